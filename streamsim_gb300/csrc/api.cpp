@@ -246,8 +246,8 @@ uint32_t run_sweeps(facetcu_context* ctx, float sky, float relax, uint32_t count
     for (uint32_t i = 0; i < count; ++i) {
         const float* in = ping == 0 ? a : b;
         float* out = ping == 0 ? b : a;
-        jacobi_plain_sweep(ctx->graph, ctx->optics.as<facetcu_surface_optics>(), sky, relax, in,
-                           out, res + first_slot + i, ctx->stream);
+        jacobi_sweep(ctx->graph, ctx->optics.as<facetcu_surface_optics>(), sky, relax, in, out,
+                     res + first_slot + i, ctx->stream);
         ping ^= 1u;
     }
     return ping;
