@@ -234,6 +234,9 @@ void upload(DeviceBuffer& buf, const void* src, size_t bytes, cudaStream_t s)
     if (bytes) FCU_CHECK(cudaMemcpyAsync(buf.ptr, src, bytes, cudaMemcpyHostToDevice, s));
 }
 
+// Sweeps from which a graph's column plan pays for being made.
+constexpr uint32_t kPlanSweeps = 8;
+
 // The plain Jacobi loop shared by solve and solveAccelerated.  Runs `count`
 // sweeps starting from buffer `ping`; each sweep's max|dB| lands in
 // residual[sweep_index].  Returns the new ping.
@@ -358,13 +361,13 @@ int facetcu_destroy(facetcu_context* ctx)
     ctx->graph.denominators.release();
     ctx->graph.sky.release();
     ctx->graph.packed.release();
-    ctx->graph.packed_valid = false;
+    ctx->graph.changed();
     for (DeviceBuffer* b : {&ctx->graph.order, &ctx->graph.rank, &ctx->graph.p_rows,
                             &ctx->graph.p_packed, &ctx->graph.p_denom, &ctx->graph.p_sky})
         b->release();
-    ctx->graph.perm_valid = false;
     ctx->graph.scene_facets.clear();
     ctx->graph.p_scene.release();
+    ctx->graph.column.release();
     ctx->graph_ready = false;
     for (DeviceBuffer* b : {&ctx->raster.counts, &ctx->raster.offsets, &ctx->raster.records,
                             &ctx->raster.big_list, &ctx->raster.deep_list, &ctx->raster.stats,
@@ -435,8 +438,7 @@ int facetcu_set_geometry(facetcu_context* ctx, const facetcu_vertex* vertices,
         }
         FCU_CHECK(cudaStreamSynchronize(ctx->stream));
         ctx->graph_ready = false;
-        ctx->graph.packed_valid = false;
-        ctx->graph.perm_valid = false;
+        ctx->graph.changed();
         ctx->graph.scene_facets.clear();
         ctx->bvh_ready = false;
         ctx->facets = uint32_t(vertex_count / 3);
@@ -798,8 +800,7 @@ int facetcu_set_graph(facetcu_context* ctx, uint32_t surface_count, const uint32
         upload(g.edges, edges, nnz * 8 + 8, s);
         upload(g.denominators, denominators, size_t(surface_count) * 4, s);
         upload(g.sky, sky_counts, size_t(surface_count) * 4, s);
-        g.packed_valid = false;
-        g.perm_valid = false;
+        g.changed();
         g.scene_facets.clear();
         float closure;
         uint32_t sampled;
@@ -831,6 +832,7 @@ int facetcu_solve(facetcu_context* ctx, const facetcu_surface_optics* optics,
         FCU_CHECK(cudaMemsetAsync(ctx->rad_a.ptr, 0, size_t(S) * 4, s));
         FCU_CHECK(cudaMemsetAsync(ctx->rad_b.ptr, 0, size_t(S) * 4, s));
         FCU_CHECK(cudaMemsetAsync(ctx->residual.ptr, 0, (size_t(iterations) + 1) * 4, s));
+        if (iterations >= kPlanSweeps) column_plan(ctx->graph, ctx->ws, s);
         const uint32_t ping = run_sweeps(ctx, sky, relaxation, iterations, 0, 0);
         const float* final_buf = ping == 0 ? ctx->rad_a.as<float>() : ctx->rad_b.as<float>();
         uint32_t bits = 0;
@@ -883,6 +885,7 @@ int facetcu_solve_accelerated(facetcu_context* ctx, const facetcu_surface_optics
             FCU_CHECK(cudaMemsetAsync(ctx->rad_a.ptr, 0, size_t(S) * 4, s));
             FCU_CHECK(cudaMemsetAsync(ctx->rad_b.ptr, 0, size_t(S) * 4, s));
         }
+        if (maximum_iterations >= kPlanSweeps) column_plan(ctx->graph, ctx->ws, s);
         uint32_t done = 0, ping = 0;
         float md = 0.0f;
         while (done < maximum_iterations) {
@@ -1574,8 +1577,7 @@ int facetcu_scene_batch(facetcu_context* ctx, facetcu_context* const* scenes,
         FCU_CHECK(cudaMemcpyAsync(g.row_offsets.as<uint32_t>() + S, &last, 4,
                                   cudaMemcpyHostToDevice, s));
         g.max_count = max_count;
-        g.packed_valid = false;
-        g.perm_valid = false;
+        g.changed();
         // the scenes' facet ranges: converged scenes leave the int8 steps
         g.scene_facets.assign(1, 0u);
         for (uint32_t i = 0, f = 0; i < scene_count; ++i) {

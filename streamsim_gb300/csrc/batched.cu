@@ -39,12 +39,12 @@
 #include <type_traits>
 
 #include "internal.h"
+#include "sweep_math.cuh"
 
 namespace facetcu {
 namespace {
 
 constexpr int kWarps = 8;  // warps per CTA
-constexpr int kMaxP = 128;
 #ifndef FCU_NARROW_U
 // loads in flight per lane for 1-4 column panels (the 32-scene batch of
 // 4.7 M facets, whose thermal band is a 1-column panel: 172.0 ms at 8, 172.6
@@ -62,18 +62,6 @@ struct PanelParams {
     const float* colmax;  // [P] max|B| of the previous sweep (floor of the per-side test)
     const float* omega;   // [P] Chebyshev weight of the int8 step being formed (or null)
 };
-
-// The per-side stop test: |dB_s| / max(|B_s|, kSideFloor * max|B|) <= tol
-// per column, the form of the accuracy bar (relative error per side, with
-// sides below 1e-6 of the column's maximum measured against that floor).
-constexpr float kSideFloor = 1e-6f;
-__device__ __forceinline__ float rel_change(float d, float b, float floor_abs)
-{
-    d = fabsf(d);
-    if (d == 0.0f) return 0.0f;
-    const float den = fmaxf(fabsf(b), floor_abs);
-    return den > 0.0f ? d / den : INFINITY;
-}
 
 struct GraphView {
     const uint32_t* rows;
@@ -2673,7 +2661,9 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
     const bool fp64 = cfg.precision == FACETCU_PRECISION_FP64;
     const bool mixed = cfg.precision == FACETCU_PRECISION_MIXED;
     const size_t elem = fp64 ? 8 : 4;
-    ensure_permuted(gr, p, ws, s);
+    // A single right-hand side runs in the caller's side order on the graph's
+    // column plan, and needs no renumbered copy.
+    if (fp64 || R != 1 || !column_plan(gr, ws, s)) ensure_permuted(gr, p, ws, s);
     const bool perm = gr.perm_valid;
     // caller facet -> solver facet, for the panel transposes
     const uint32_t* rank = perm ? gr.rank.as<uint32_t>() : nullptr;
@@ -2759,6 +2749,13 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
 
     for (uint32_t c0 = 0; c0 < R;) {
         const int P = panel_width(R - c0, cfg.panel_width, uint32_t(Pmax));
+        // One column over a large graph: FP32 sweeps through the column plan,
+        // in every precision but FP64 (on the 200,000-facet forest's 74 M
+        // edges 78 us against 203 for k_sweep<1>; the BF16 defect sweeps
+        // gather the same 32-byte sectors).
+        const bool column = !fp64 && P == 1 && column_plan(gr, ws, s);
+        const bool low = mixed && !column;
+        const uint32_t* side_rank = column ? nullptr : rank;
         const size_t cells = size_t(S) * P;
         float* prho = prm;
         float* ptau = prm + cells;
@@ -2766,7 +2763,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
         float* pdir = prm + 3 * cells;
         float* psky = prm + 4 * cells;
         PanelParams pp{prho, ptau, pemis, pdir, psky, colmax,
-                       mixed && P >= 32 ? cheb + 2 * kMaxP : nullptr};
+                       low && P >= 32 ? cheb + 2 * kMaxP : nullptr};
         __nv_bfloat16* d0 = dbuf;
         __nv_bfloat16* d1 = dbuf ? dbuf + cells : nullptr;
         // Per-cell bytes: full sweep = state in + out + rho, tau, emission,
@@ -2777,7 +2774,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
         const double full_bytes = graph_bytes + double(cells) * (double(elem) * 2.0 + 16.0);
         const double defect_bytes = graph_bytes + double(cells) * (P >= 32 ? 26.0 : 20.0);
         auto timed_sweep = [&](bool defect, auto&& launch) {
-            const bool count = timed && (defect == mixed);
+            const bool count = timed && (defect == low);
             if (count) FCU_CHECK(cudaEventRecord(t0, s));
             launch();
             ++launches;
@@ -2793,7 +2790,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
             }
         };
         launches += 4;  // prepare, sky, panel in, panel out
-        k_prepare_panel<<<blocks_for(S, kPanelTile), 256, 0, s>>>(S, p.bands, R, c0, P, rank, p.rho,
+        k_prepare_panel<<<blocks_for(S, kPanelTile), 256, 0, s>>>(S, p.bands, R, c0, P, side_rank, p.rho,
                                                                 p.tau, p.emis, p.beam, p.dgeo,
                                                                 prho, ptau, pemis, pdir);
         FCU_LAUNCH("k_prepare_panel");
@@ -2803,10 +2800,10 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
         const float* init = cfg.warm_start == FACETCU_WARM_GIVEN ? d_initial : nullptr;
         if (fp64)
             k_panel_in<double><<<blocks_for(S, kPanelTile), 256, 0, s>>>(
-                init, S, R, c0, P, rank, reinterpret_cast<double*>(x0));
+                init, S, R, c0, P, side_rank, reinterpret_cast<double*>(x0));
         else
             k_panel_in<float><<<blocks_for(S, kPanelTile), 256, 0, s>>>(
-                init, S, R, c0, P, rank, reinterpret_cast<float*>(x0));
+                init, S, R, c0, P, side_rank, reinterpret_cast<float*>(x0));
         FCU_LAUNCH("k_panel_in");
         // A solve from zero: its first sweep gathers nothing (null input).
         const bool zero_start = init == nullptr;
@@ -2814,7 +2811,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
         uint32_t it = 0;
         int cur = 0;
         uint32_t host_flag[3] = {0, 0, 0};
-        if (!mixed) {
+        if (!low) {
             while (it < max_it) {
                 const uint32_t batch = std::min(timed ? 1u : check_every, max_it - it);
                 for (uint32_t k = 0; k < batch; ++k) {
@@ -2822,7 +2819,11 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                     char* in = sweep == 0 && zero_start ? nullptr : (sweep & 1u) ? x1 : x0;
                     char* out = (sweep & 1u) ? x0 : x1;
                     timed_sweep(false, [&] {
-                        if (fp64)
+                        if (column)
+                            column_sweep(gr, prho, ptau, pemis, pdir, psky, colmax,
+                                         reinterpret_cast<const float*>(in),
+                                         reinterpret_cast<float*>(out), stats, flag, s);
+                        else if (fp64)
                             launch_sweep<double>(P, g, pp, reinterpret_cast<const double*>(in),
                                                  reinterpret_cast<double*>(out), stats, counter,
                                                  flag, s);
@@ -3046,10 +3047,10 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
         const char* final_buf = cur ? x1 : x0;
         if (fp64)
             k_panel_out<double><<<blocks_for(S, kPanelTile), 256, 0, s>>>(
-                reinterpret_cast<const double*>(final_buf), S, R, c0, P, rank, d_out);
+                reinterpret_cast<const double*>(final_buf), S, R, c0, P, side_rank, d_out);
         else
             k_panel_out<float><<<blocks_for(S, kPanelTile), 256, 0, s>>>(
-                reinterpret_cast<const float*>(final_buf), S, R, c0, P, rank, d_out);
+                reinterpret_cast<const float*>(final_buf), S, R, c0, P, side_rank, d_out);
         FCU_LAUNCH("k_panel_out");
         worst_iterations = std::max(worst_iterations, host_flag[1]);
         float change;

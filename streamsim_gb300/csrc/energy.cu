@@ -532,6 +532,10 @@ void window_incident(const DeviceGraph& g, uint32_t W, const float* B, const flo
     const facetcu_csr_edge* edges = g.edges.as<facetcu_csr_edge>();
     const uint32_t* den = g.denominators.as<uint32_t>();
     const uint32_t* skyc = g.sky.as<uint32_t>();
+    if (W == 1 && !dgeo && g.column.state == ColumnPlan::kMade) {
+        column_incident(g, B, sky, H, s);
+        return;
+    }
     if (W == 1 && !dgeo) {
         k_incident_one<<<blocks(S * 32, 256), 256, 0, s>>>(uint32_t(S), rows, edges, den, skyc, B,
                                                             sky, H);

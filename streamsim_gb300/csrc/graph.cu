@@ -178,8 +178,7 @@ void graph_from_pairs(uint64_t* d_pairs, size_t n, int side_bits, DeviceGraph& g
     k_csr_fill<<<grid(m + 1, 256), 256, 0, s>>>(dkeys, dvals, m, side_bits, S, rows, edges);
     FCU_LAUNCH("k_csr_fill");
     FCU_CHECK(cudaStreamSynchronize(s));
-    g.packed_valid = false;
-    g.perm_valid = false;
+    g.changed();
     g.scene_facets.clear();
 }
 
@@ -206,7 +205,6 @@ bool graph_pack(DeviceGraph& g, Workspace& ws, cudaStream_t s)
 {
     (void)ws;
     if (g.packed_valid) return true;
-    g.perm_valid = false;
     // neighbour in the low nb_bits (at least 22), count above: exact while the
     // largest count fits the remaining bits (1023 up to 2^22 sides, 511 up
     // to 2^23, 255 up to 2^24); otherwise the 8-byte edges are used

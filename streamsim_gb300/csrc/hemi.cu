@@ -482,8 +482,7 @@ void hemisphere_graph(const facetcu_vertex* d_vertices, uint32_t facets, const L
     k_hemi_compact<<<(S * 32 + 255) / 256, 256, 0, s>>>(tmp_edges, rows, S, top_k, edges);
     FCU_LAUNCH("k_hemi_compact");
     FCU_CHECK(cudaStreamSynchronize(s));
-    g.packed_valid = false;
-    g.perm_valid = false;
+    g.changed();
     if (dropped) *dropped = host[0];
 }
 

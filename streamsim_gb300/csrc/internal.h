@@ -130,6 +130,18 @@ void raster_resolve_sunlit(const RasterFrame& frame, uint32_t chain_cap, RasterB
                            uint32_t* d_total, uint32_t* d_visible, RasterStats& stats,
                            cudaStream_t s);
 
+// ---- one-column sweeps from shared memory (column.cu) --------------------
+// The edge words of a graph laid out by tiles of the column, and the sums of
+// (side, tile) pairs of the sweep in flight; made by column_plan at the first
+// one-column solve of the graph.
+struct ColumnPlan {
+    enum State { kUnknown, kNone, kMade };
+    State state = kUnknown;
+    uint32_t ctas = 0, tiles = 0;
+    DeviceBuffer shares, groups, meta, words, partial;
+    void release();
+};
+
 // ---- graph assembly (graph.cu) ------------------------------------------
 struct DeviceGraph {
     uint32_t surfaces = 0;
@@ -153,6 +165,14 @@ struct DeviceGraph {
     // one scene); with the Morton copy, the scene of each renumbered facet.
     std::vector<uint32_t> scene_facets;
     DeviceBuffer p_scene;       // F u16, built with the Morton copy for 2..65535 scenes
+    ColumnPlan column;
+    // Other edges or rows: what was derived from the old ones is stale.
+    void changed()
+    {
+        packed_valid = false;
+        perm_valid = false;
+        column.state = ColumnPlan::kUnknown;
+    }
 };
 // Sort undirected pair keys, count runs, emit the symmetric CSR.
 void graph_from_pairs(uint64_t* d_pairs, size_t pair_count, int side_bits, DeviceGraph& g,
@@ -168,7 +188,8 @@ void graph_closure(const DeviceGraph& g, float* closure, uint32_t* sampled, Work
 bool graph_pack(DeviceGraph& g, Workspace& ws, cudaStream_t s);
 
 // ---- solves (solve.cu) ---------------------------------------------------
-// One sweep of the reference's solver.
+// One sweep of the reference's solver; through the graph's column plan where
+// it has one.
 void jacobi_sweep(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
                   float relaxation, const float* d_in, float* d_out, uint32_t* d_max_delta_bits,
                   cudaStream_t s);
@@ -180,6 +201,22 @@ void jacobi_sweep_raw(uint32_t surfaces, uint64_t edges_hint, const uint32_t* ro
                       const float* d_in, float* d_out, uint32_t* d_max_delta_bits, cudaStream_t s);
 void incident_irradiance(const DeviceGraph& g, const facetcu_surface_optics* d_optics,
                          float sky, const float* d_radiosity, float* d_out, cudaStream_t s);
+
+// ---- one-column sweeps (column.cu) ---------------------------------------
+// Makes the graph's plan once; false where the CSR sweeps are to be used.
+bool column_plan(DeviceGraph& g, Workspace& ws, cudaStream_t s);
+// With a plan: the reference's sweep (as jacobi_sweep), the batched solver's
+// sweep of a one-column panel in the caller's side order (in == nullptr:
+// zeros), and max(0, incident diffuse radiation) with compensated sums.
+// Inputs are 16-byte aligned.
+void column_jacobi(const DeviceGraph& g, const facetcu_surface_optics* optics, float sky,
+                   float relax, const float* in, float* out, uint32_t* max_delta_bits,
+                   cudaStream_t s);
+void column_sweep(const DeviceGraph& g, const float* rho, const float* tau, const float* emis,
+                  const float* direct, const float* skyL, const float* colmax, const float* in,
+                  float* out, uint32_t* stats, const uint32_t* done, cudaStream_t s);
+void column_incident(const DeviceGraph& g, const float* B, const float* sky, float* out,
+                     cudaStream_t s);
 
 // ---- batched solver (batched.cu) ---------------------------------------
 struct BatchProblem {

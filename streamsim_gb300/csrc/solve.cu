@@ -3,7 +3,8 @@
 // k_jacobi_rows is the sweep of the reference's radiosity.comp:49-106
 // (FacetrtVulkan::solve): FP32 gather over the count-form CSR, both sides of a
 // facet updated together, mix() relaxation, max|dB| as an atomicMax over float
-// bits.
+// bits.  It serves the graphs that column.cu's plan is not made for (few
+// edges, short rows) and callers that bring their own arrays.
 #include "internal.h"
 
 namespace facetcu {
@@ -123,6 +124,10 @@ void jacobi_sweep(const DeviceGraph& g, const facetcu_surface_optics* d_optics, 
                   float relaxation, const float* d_in, float* d_out, uint32_t* d_max_delta_bits,
                   cudaStream_t s)
 {
+    if (g.column.state == ColumnPlan::kMade) {
+        column_jacobi(g, d_optics, sky, relaxation, d_in, d_out, d_max_delta_bits, s);
+        return;
+    }
     jacobi_sweep_raw(g.surfaces, g.nnz, g.row_offsets.as<uint32_t>(), g.edges.as<facetcu_csr_edge>(),
                      g.denominators.as<uint32_t>(), g.sky.as<uint32_t>(), d_optics, sky, relaxation,
                      d_in, d_out, d_max_delta_bits, s);

@@ -1,5 +1,6 @@
 """One-column sweeps on the device against a float64 Jacobi iteration in numpy:
-the CSR kernel (k_jacobi_rows) at the edges of its lane groups.
+the CSR kernel (k_jacobi_rows) at the edges of its lane groups, and the
+shared-memory plan (column.cu) at the edges of its tiles, windows and groups.
 
 Tolerance: a sweep adds at most `deg` products in FP32, so a row's relative
 error per sweep is below (deg + 8) 2^-24, and the iteration (rho + tau = c)
@@ -90,3 +91,68 @@ def test_csr_sweep_lane_groups(S, mean):
     m.close()
     want = _jacobi(graph, o[:, 3].astype(np.float64), o[:, 2].astype(np.float64), 9, 0.75)
     assert np.max(np.abs(got - want) / want) < _tolerance(graph)
+
+
+# sides: one tile less 2, exactly one tile, a second tile of 2 sides, and a
+# ragged last window; row lengths with empty rows and one far above the rest
+@pytest.fixture(scope="module", params=[49150, 49152, 49154, 102402])
+def planned(request):
+    require_gpu()
+    S = request.param
+    rng = np.random.default_rng(S)
+    deg = rng.integers(150, 330, S)
+    deg[rng.choice(S, S // 50)] = 0
+    deg[rng.choice(S, 200)] = np.arange(1, 201) % 40
+    deg[7] = 3000
+    graph = _graph(S, deg, rng, counts=[255, 256, 257, 511, 512, 4097, 65535])
+    assert int(graph[0][-1]) >= 10 << 20  # large enough for the plan
+    m = _model(S, graph)
+    yield dict(S=S, graph=graph, model=m, optics=_optics(S, rng))
+    m.close()
+
+
+def test_planned_sweep(planned):
+    o = planned["optics"]
+    got = planned["model"].solve(o, SKY, 12, 0.75)["radiosity"]
+    want = _jacobi(planned["graph"], o[:, 3].astype(np.float64), o[:, 2].astype(np.float64), 12,
+                   0.75)
+    assert np.max(np.abs(got - want) / want) < _tolerance(planned["graph"])
+    again = planned["model"].solve(o, SKY, 12, 0.75)["radiosity"]
+    assert np.array_equal(got, again)
+
+
+@pytest.mark.parametrize("precision", [facetcu.PRECISION_FP32, facetcu.PRECISION_MIXED])
+def test_planned_panel(planned, precision):
+    S, o = planned["S"], planned["optics"]
+    col = lambda k: o[:, k][None, :]  # noqa: E731
+    out, res = planned["model"].solveBatched(
+        col(0), col(1), np.float32([SKY]), np.float32([1.0]), col(3), emission=col(2),
+        precision=precision, tolerance=1e-6)
+    want = _jacobi(planned["graph"], o[:, 3].astype(np.float64), o[:, 2].astype(np.float64), 60)
+    assert res["converged"]
+    # the stop rule leaves at most tolerance / (1 - c)
+    assert np.max(np.abs(out[0] - want) / want) < _tolerance(planned["graph"]) + 1e-6 / (1 - RHO - TAU)
+
+
+def test_planned_incident_in_a_node(planned):
+    """The node's net radiation of object facets is the sum over both sides of
+    eps H - E with the longwave radiosity it returns."""
+    S, graph = planned["S"], planned["graph"]
+    F = S // 2
+    rng = np.random.default_rng(1)
+    p, keep = facetcu.energy_parameters(
+        F, [facetcu.EnergySurface([0.1], [0.0], 0.3, 0.1, vegetation=False)], np.zeros(F, np.uint32),
+        coupling_iterations=1, solver_tolerance=1e-6)
+    T0 = rng.uniform(285, 305, F).astype(np.float32).repeat(2)
+    meteo = dict(air_temperature=20.0, vapor_pressure=12.0, pressure=1000.0, wind_speed=2.0,
+                 shortwave=0.0, longwave=SKY)
+    out, _ = planned["model"].facetebNode(p, meteo, np.float32([0, 1, 0]), np.zeros(S, np.float32),
+                                          None, T0, fields=("longwave_radiosity", "net_radiation"))
+    eps = 1.0 - np.float64(np.float32(0.3)) - np.float64(np.float32(0.1))
+    H = _incident(graph, out["longwave_radiosity"].astype(np.float64))
+    # the emitted part from the final temperature the node returns
+    E = eps * 5.670374419e-8 * out["temperature"].astype(np.float64) ** 4
+    want = (eps * H - E).reshape(-1, 2).sum(1).repeat(2)
+    # H is rounded once to float and the two products and sums are floats
+    scale = 2 * (eps * H.max() + E.max())
+    assert np.max(np.abs(out["net_radiation"] - want)) < 12 * 2.0 ** -24 * scale + 1e-6 * scale
