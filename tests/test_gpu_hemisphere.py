@@ -192,3 +192,31 @@ def test_hemisphere_graph_config2_scale_bit_exact(oracle):
     assert graphs_equal(gpu_graph, g) is None
     assert dropped == dropped_o
     assert np.array_equal(lit, oracle.hemisphere_sunlit_bvh(sc.vertices, suv, 256, 32, sun))
+
+
+@pytest.mark.parametrize("rays,top_k", [(1, 1), (31, 7), (32, 32), (33, 5), (65, 64), (129, 3),
+                                        (257, 40), (511, 256), (1000, 17), (1023, 1023)])
+@pytest.mark.parametrize("leaves,grid,neighbours", [(1, 1, 0), (37, 3, 4), (300, 5, 0)])
+def test_hemisphere_sizes_bit_exact(oracle, rays, top_k, leaves, grid, neighbours):
+    """Every sort width of the row kernel, ragged ray counts, trees of 3 to 350
+    facets, and directions along the axes (zero components)."""
+    sc = scenes.config1(seed=rays, leaves=leaves, grid=grid)
+    uv, dirs = scenes.hemisphere_samples(rays, 4, seed=rays)
+    dirs[0, ::3] = [0.0, 0.0, 1.0]
+    dirs[1, ::4] = [1.0, 0.0, 0.0]
+    dirs[2, ::5] = [1e-30, 1.0, 1e-12]
+    m = facetcu.FacetrtCuda()
+    m.initialize(64, 64, 64, 0, neighbours, 10.0, 10.0)
+    m.setGeometry(sc.vertices)
+    _, dropped = m.buildHemisphereGraph(uv, dirs, rays, top_k, 4)
+    periodic = (neighbours, 10.0, 10.0)
+    g, dropped_o = oracle.hemisphere_graph(sc.vertices, uv, dirs, rays, 4, top_k, periodic=periodic)
+    assert graphs_equal(m.graph(), g) is None
+    assert dropped == dropped_o
+    for sun in ([0.0, 1.0, 0.0], [1.0, 0.0, 0.0], [0.3, -0.5, 0.8]):
+        sun = np.float32(sun)
+        n = min(rays, 100)
+        lit = m.hemisphereSunlit(sun, uv[:, :n], n, 4)
+        assert np.array_equal(lit, oracle.hemisphere_sunlit(sc.vertices, uv[:, :n], n, 4, sun,
+                                                            periodic=periodic))
+    m.close()
