@@ -2148,8 +2148,8 @@ int facetcu_render_sensor_image(facetcu_context* ctx, const facetcu_sensor* sens
         const size_t S = 2 * size_t(F);
         cudaStream_t st = ctx->stream;
         auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-        const size_t bytes = al(size_t(F) * 3 * image::kProjBytes) + al(size_t(F) * 4) +
-                             al(n * 8) + al(n * 4) * 2 + al(size_t(band_count) * S * 4) +
+        const size_t bytes = al(size_t(F) * 4) + al(n * 16) + al(n * 4) * 2 +
+                             al(size_t(band_count) * S * 4) +
                              al(size_t(band_count) * 4) + al(size_t(band_count) * n * 4) + al(8);
         char* c = static_cast<char*>(ctx->img_io.reserve(bytes));
         auto take = [&](size_t b) {
@@ -2158,9 +2158,8 @@ int facetcu_render_sensor_image(facetcu_context* ctx, const facetcu_sensor* sens
             return r;
         };
         image::Scratch w{};
-        w.proj = take(size_t(F) * 3 * image::kProjBytes);
         w.side = reinterpret_cast<int32_t*>(take(size_t(F) * 4));
-        w.zbuf = reinterpret_cast<unsigned long long*>(take(n * 8));
+        w.zbuf = reinterpret_cast<ulonglong2*>(take(n * 16));
         w.index = reinterpret_cast<int32_t*>(take(n * 4));
         int32_t* d_sides = reinterpret_cast<int32_t*>(take(n * 4));
         float* d_values = reinterpret_cast<float*>(take(size_t(band_count) * S * 4));

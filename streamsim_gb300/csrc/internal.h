@@ -411,12 +411,10 @@ struct Camera {
     int32_t perspective;
 };
 struct Scratch {
-    void* proj;               // 3F projected vertices
-    int32_t* side;            // F observed sides
-    unsigned long long* zbuf; // W*H depth keys
-    int32_t* index;           // W*H facet indices, then observed sides
+    int32_t* side;     // F observed sides
+    ulonglong2* zbuf;  // W*H nearest fragments (depth key, facet)
+    int32_t* index;    // W*H observed sides
 };
-constexpr size_t kProjBytes = 32;  // one projected vertex
 Camera camera(const facetcu_sensor& s, double* naming_zenith, double* naming_azimuth);
 void render(const Camera& c, uint32_t F, const facetcu_vertex* V, const float* values,
             uint32_t nb, size_t S, const float* wavelengths, bool as_temperature, double sky_t,

@@ -111,3 +111,37 @@ def test_rejects_bad_arguments(site):
         m.renderSensorImage(facetcu.sensor(8, 8), site["values"], WAVELENGTHS[:1])
     with pytest.raises(ValueError):
         m.renderSensorImage(facetcu.sensor(8, 8), site["values"][:1], [np.nan])
+
+
+@pytest.mark.parametrize("case", [
+    dict(width=1, height=1, perspective=False, vza=0.0, vaa=0.0, scene_x=12.0, scene_y=12.0),
+    dict(width=3, height=700, perspective=False, vza=20.0, vaa=10.0, scene_x=12.0, scene_y=12.0),
+    dict(width=333, height=77, perspective=False, vza=50.0, vaa=300.0, scene_x=9.0, scene_y=12.0),
+    dict(width=130, height=97, perspective=True, vza=85.0, vaa=30.0, fov=100.0, scene_x=12.0,
+         scene_y=12.0, position=(6.3, 6.1, 0.4)),
+])
+def test_boxes_of_every_size_and_equal_depths(case):
+    """Facets from far below a pixel to larger than the image (thread and warp
+    boxes), each also as an exact copy with a higher index: equal depths, the
+    first facet is seen."""
+    require_gpu()
+    rng = np.random.default_rng(case["width"])
+    parts = [scenes._triangles_to_vertices(*scenes.equilateral(
+        np.stack([rng.uniform(-6, 6, n), rng.uniform(0.1, 2.5, n), rng.uniform(-6, 6, n)], 1),
+        scenes.uniform_sphere(n, rng), edge, rng)) for n, edge in ((300, 0.01), (300, 0.2),
+                                                                   (60, 1.5), (3, 40.0))]
+    one = np.concatenate(parts)
+    v = np.concatenate([one, one])
+    m = model_for(v, 64, 64)
+    F = len(v) // 3
+    values = rng.uniform(0.0, 1.0, (1, 2 * F)).astype(np.float32)
+    s = facetcu.sensor(case["width"], case["height"], case["perspective"], case["vza"],
+                       case["vaa"], case.get("fov", 0.0), case["scene_x"], case["scene_y"],
+                       case.get("position", (np.nan,) * 3))
+    img, idx, _ = m.renderSensorImage(s, values, [450.0])
+    m.close()
+    cam, want = _oracle(case, v.reshape(-1, 3, 6)[:, :, :3])
+    assert np.array_equal(idx, want), f"{np.sum(idx != want)} pixels differ"
+    assert idx.max() < F  # the copies lose every tie
+    seen = want >= 0
+    assert np.array_equal(img[0][seen], values[0][want[seen]])
