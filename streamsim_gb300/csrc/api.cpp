@@ -390,7 +390,7 @@ int facetcu_destroy(facetcu_context* ctx)
                             &ctx->net.grad})
         b->release();
     for (DeviceBuffer* b : {&ctx->mlp_scratch.z1, &ctx->mlp_scratch.a1, &ctx->mlp_scratch.z2,
-                            &ctx->mlp_scratch.a2, &ctx->mlp_scratch.y, &ctx->mlp_scratch.dy,
+                            &ctx->mlp_scratch.a2, &ctx->mlp_scratch.dy,
                             &ctx->mlp_scratch.da, &ctx->mlp_scratch.dz, &ctx->mlp_scratch.part,
                             &ctx->mlp_scratch.lossp, &ctx->mlp_scratch.idx, &ctx->mlp_scratch.xb,
                             &ctx->mlp_scratch.tb, &ctx->mlp_tensor.xb, &ctx->mlp_tensor.a1,

@@ -308,7 +308,7 @@ struct Net {
     uint32_t steps_done = 0;
 };
 struct Scratch {
-    DeviceBuffer z1, a1, z2, a2, y, dy, da, dz, part, lossp, idx, xb, tb;
+    DeviceBuffer z1, a1, z2, a2, dy, da, dz, part, lossp, idx, xb, tb;
 };
 // Buffers of the tensor-core inference (mlp_tc.cu).
 struct TensorScratch {
@@ -323,8 +323,8 @@ void infer_tensor(Net& net, const float* X, size_t n, TensorScratch& ts, float* 
 uint32_t tensor_error(TensorScratch& ts, cudaStream_t s);
 void init_params(Net& net, uint32_t seed, cudaStream_t s);
 void set_params(Net& net, const float* host, cudaStream_t s);
-// Rows per forward pass: kMaxRows keeps the GEMM grid (64 rows per CTA in
-// y) under 65,535 CTAs; inference is chunked at kInferChunk rows.
+// Most rows of a gradient or training batch (its activations take 4 GB);
+// inference is chunked at kInferChunk rows.
 constexpr size_t kMaxRows = size_t(1) << 21;
 constexpr size_t kInferChunk = size_t(1) << 19;
 void forward_full(Net& net, const float* X, int n, Scratch& sc, float* Y, cudaStream_t s);

@@ -8,12 +8,15 @@
 // row-major [n][features] FP32.  The loss is the mean squared error over
 // all n x 64 outputs.
 //
-// GEMMs are one tiled kernel (64 x 64 output tile per CTA, 16-deep K
-// slices staged in shared memory, 4 x 4 outputs per thread) with optional
-// transposes, a BF16 operand, a bias + GELU epilogue, and split-K for the
-// weight gradients (K = batch): each split writes its own partial and a
-// second kernel sums the partials in a fixed order, so a training step is
-// deterministic.
+// GEMMs (FP32 FMA: activations and gradients are FP32, and so are the sums).
+//   k_layer  128 rows per CTA against a whole weight matrix in shared memory
+//            (at most 128 x 128 floats), 8 x 8 or 8 x 4 outputs per thread;
+//            the epilogue is the layer's own: bias and GELU, bias and loss,
+//            or the product with GELU'(Z)
+//   k_wgrad  a weight gradient dZ^T A over a share of the rows per CTA, with
+//            the bias gradient beside it; every CTA writes its own partial
+//            and k_sum_partials adds them in a fixed order, so a training
+//            step is deterministic.
 #include <cuda_bf16.h>
 
 #include <cmath>
@@ -26,8 +29,6 @@ namespace mlp {
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16;
-
 __device__ __forceinline__ float gelu(float z)
 {
     return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
@@ -39,140 +40,336 @@ __device__ __forceinline__ float gelu_grad(float z)
     return cdf + z * pdf;
 }
 
-template <typename T> __device__ __forceinline__ float ld(const T* p);
-template <> __device__ __forceinline__ float ld<float>(const float* p) { return *p; }
-template <> __device__ __forceinline__ float ld<__nv_bfloat16>(const __nv_bfloat16* p)
+// acc[i][j] += a[i] * b[j], two columns at a time (fma.rn.f32x2: each half is
+// an fma of its own).
+__device__ __forceinline__ void fma2(float& c0, float& c1, float a, float b0, float b1)
 {
-    return __bfloat162float(*p);
+    asm("{ .reg .b64 c, x, y;\n  mov.b64 c, {%0, %1};\n  mov.b64 x, {%2, %2};\n"
+        "  mov.b64 y, {%3, %4};\n  fma.rn.f32x2 c, x, y, c;\n  mov.b64 {%0, %1}, c; }"
+        : "+f"(c0), "+f"(c1)
+        : "f"(a), "f"(b0), "f"(b1));
 }
 
-// C[m][n] (+)= sum_k opA(m,k) * opB(k,n)   (split-K: C += z * M * N)
-// opA(m,k) = TA ? A[k*lda + m] : A[m*lda + k]
-// opB(k,n) = TB ? B[n*ldb + k] : B[k*ldb + n]
-// epilogue: EPI 0 = store; 1 = + bias[n], store Z and GELU(Z) to C2.
-template <bool TA, bool TB, typename TBT, int EPI>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float* __restrict__ A,
-                                              int lda, const TBT* __restrict__ B, int ldb,
-                                              float* __restrict__ C, int ldc,
-                                              const float* __restrict__ bias, float* __restrict__ C2,
-                                              int k_per_split)
+// ---- layers -------------------------------------------------------------------
+enum Epilogue {
+    kGelu,      // Z = acc + bias to out (where given), GELU(Z) to out2
+    kOutput,    // acc + bias to out
+    kLoss,      // Y = acc + bias; out = 2 (Y - T) scale, the CTA's sum of (Y - T)^2
+    kGeluBack,  // acc * GELU'(Z)
+};
+struct LayerArgs {
+    const float* bias;
+    const float* other;  // kLoss: the targets T; kGeluBack: Z
+    float *out, *out2;
+    double* loss_part;
+    float scale;
+};
+
+constexpr int kRows = 128;      // rows of a CTA
+constexpr int kPad = kRows + 4;
+
+// Bound: FP32 FMA issue and, in the epilogues, erf and exp.  The layers of a
+// 65,536-row gradient take 243 us and the weight gradients 95 (10.3 GFLOP: 31
+// TFLOP/s over both); with 64 x 64 tiles, 4 x 4 outputs per thread, separate
+// loss, GELU and bias kernels they took 1,440, and a one-thread sum of the loss
+// 963 more.
+// out[rows][N] = A[rows][K] B, B = W^T (kT: W is [N][K]) or W ([K][N]), in K
+// slices of KS whose A values are fetched while the slice before is summed.
+template <int K, int N, int KS, bool kT, Epilogue E>
+__global__ void __launch_bounds__(256, 2) k_layer(int rows, const float* __restrict__ A,
+                                                  const __nv_bfloat16* __restrict__ W,
+                                                  LayerArgs args)
 {
-    __shared__ float As[TK][TM + 4];
-    __shared__ float Bs[TK][TN + 4];
+    static_assert(K % KS == 0 && KS % 4 == 0 && (N == 128 || N == 64), "shape");
+    constexpr int C = N / 16;                          // columns per thread
+    constexpr int kQuads = kRows * KS / 4;             // float4 of a slice
+    constexpr int kFetch = (kQuads + 255) / 256;
+    extern __shared__ __align__(16) float smem[];
+    float(*Bs)[N] = reinterpret_cast<float(*)[N]>(smem);                 // [K][N]
+    float(*As)[KS][kPad] = reinterpret_cast<float(*)[KS][kPad]>(smem + K * N);  // [2][KS][rows]
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    const int kb = blockIdx.z * k_per_split;
-    const int ke = min(K, kb + k_per_split);
-    float acc[4][4] = {};
-    for (int k0 = kb; k0 < ke; k0 += TK) {
-        for (int i = threadIdx.x; i < TM * TK; i += 256) {
-            const int mm = TA ? i % TM : i / TK;
-            const int kk = TA ? i / TM : i % TK;
-            const int m = m0 + mm, k = k0 + kk;
-            As[kk][mm] = (m < M && k < ke) ? (TA ? A[size_t(k) * lda + m] : A[size_t(m) * lda + k])
-                                            : 0.0f;
+    if (kT) {  // lanes over n: the stores of a warp are side by side
+        constexpr int V = K % 8 == 0 ? 8 : 4;  // weights per load
+        for (int i = threadIdx.x; i < K / V * N; i += 256) {
+            const int n = i % N, k = i / N * V;
+            __nv_bfloat16 w[V];
+            if (V == 8) *reinterpret_cast<uint4*>(w) = *reinterpret_cast<const uint4*>(W + n * K + k);
+            else *reinterpret_cast<uint2*>(w) = *reinterpret_cast<const uint2*>(W + n * K + k);
+#pragma unroll
+            for (int j = 0; j < V; ++j) Bs[k + j][n] = __bfloat162float(w[j]);
         }
-        for (int i = threadIdx.x; i < TN * TK; i += 256) {
-            const int nn = TB ? i / TK : i % TN;
-            const int kk = TB ? i % TK : i / TN;
-            const int n = n0 + nn, k = k0 + kk;
-            Bs[kk][nn] = (n < N && k < ke)
-                             ? (TB ? ld(B + size_t(n) * ldb + k) : ld(B + size_t(k) * ldb + n))
-                             : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < TK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a[i] = As[kk][ty * 4 + i];
-                b[i] = Bs[kk][tx * 4 + i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * b[j];
-        }
-        __syncthreads();
+    } else {
+        for (int i = threadIdx.x; i < K * N; i += 256) Bs[i / N][i % N] = __bfloat162float(W[i]);
     }
-    float* Cz = C + size_t(blockIdx.z) * M * ldc;
+    float loss = 0.0f, loss_low = 0.0f;  // compensated: about twice the float precision
+    for (int r0 = blockIdx.x * kRows; r0 < rows; r0 += gridDim.x * kRows) {
+    float4 next[kFetch];
+    auto fetch = [&](int k0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= M) continue;
+        for (int q = 0; q < kFetch; ++q) {
+            const int i = threadIdx.x + q * 256, r = i / (KS / 4), k = i % (KS / 4) * 4;
+            next[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if ((kQuads % 256 == 0 || i < kQuads) && r0 + r < rows)
+                next[q] = *reinterpret_cast<const float4*>(A + size_t(r0 + r) * K + k0 + k);
+        }
+    };
+    auto put = [&](int buf) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n >= N) continue;
-            if (EPI == 0) {
-                Cz[size_t(m) * ldc + n] = acc[i][j];
-            } else {
-                const float z = acc[i][j] + bias[n];
-                Cz[size_t(m) * ldc + n] = z;
-                C2[size_t(m) * ldc + n] = gelu(z);
+        for (int q = 0; q < kFetch; ++q) {
+            const int i = threadIdx.x + q * 256, r = i / (KS / 4), k = i % (KS / 4) * 4;
+            if (kQuads % 256 == 0 || i < kQuads) {
+                As[buf][k][r] = next[q].x;
+                As[buf][k + 1][r] = next[q].y;
+                As[buf][k + 2][r] = next[q].z;
+                As[buf][k + 3][r] = next[q].w;
             }
         }
+    };
+    float acc[8][C] = {};
+    fetch(0);
+    put(0);
+    __syncthreads();
+#pragma unroll 1
+    for (int k0 = 0, buf = 0; k0 < K; k0 += KS, buf ^= 1) {
+        if (k0 + KS < K) fetch(k0 + KS);
+#pragma unroll
+        for (int k = 0; k < KS; ++k) {
+            float a[8], b[C];
+            // rows 4 ty .. and 64 + 4 ty .., columns 4 tx .. and 64 + 4 tx ..
+            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&As[buf][k][4 * ty]);
+            *reinterpret_cast<float4*>(a + 4) =
+                *reinterpret_cast<const float4*>(&As[buf][k][64 + 4 * ty]);
+            *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&Bs[k0 + k][4 * tx]);
+            if (C == 8)
+                *reinterpret_cast<float4*>(b + C - 4) =
+                    *reinterpret_cast<const float4*>(&Bs[k0 + k][N - 64 + 4 * tx]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < C; j += 2)
+                    fma2(acc[i][j], acc[i][j + 1], a[i], b[j], b[j + 1]);
+        }
+        if (k0 + KS < K) put(buf ^ 1);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = r0 + (i < 4 ? 0 : 64) + 4 * ty + i % 4;
+        if (r >= rows) continue;
+#pragma unroll
+        for (int h = 0; h < C / 4; ++h) {
+            const int n = h * 64 + 4 * tx;
+            const size_t at = size_t(r) * N + n;
+            float v[4], w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = acc[i][h * 4 + j];
+            if (E != kGeluBack) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] += args.bias[n + j];
+            }
+            if (E == kLoss || E == kGeluBack)
+                *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(args.other + at);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (E == kGelu) w[j] = gelu(v[j]);
+                if (E == kGeluBack) v[j] *= gelu_grad(w[j]);
+                if (E == kLoss) {
+                    const float d = v[j] - w[j];
+                    const float q = __fmul_rn(d, d), t = __fadd_rn(loss, q);
+                    const float e = fabsf(loss) >= q ? __fadd_rn(__fadd_rn(loss, -t), q)
+                                                     : __fadd_rn(__fadd_rn(q, -t), loss);
+                    loss = t;
+                    loss_low = __fadd_rn(loss_low, __fadd_rn(e, __fmaf_rn(d, d, -q)));
+                    v[j] = 2.0f * d * args.scale;
+                }
+            }
+            if (E != kGelu || args.out)
+                *reinterpret_cast<float4*>(args.out + at) = make_float4(v[0], v[1], v[2], v[3]);
+            if (E == kGelu)
+                *reinterpret_cast<float4*>(args.out2 + at) = make_float4(w[0], w[1], w[2], w[3]);
+        }
+    }
+    }
+    if (E == kLoss) {
+        double* red = reinterpret_cast<double*>(smem);  // (the operands are done with)
+        red[threadIdx.x] = double(loss) + double(loss_low);
+        __syncthreads();
+        for (int o = 128; o > 0; o >>= 1) {
+            if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) args.loss_part[blockIdx.x] = red[0];
     }
 }
 
-// out[i] = sum_z part[z * n + i], fixed order.
-__global__ void k_sum_splits(const float* part, int splits, size_t n, float* out, float scale)
+// CTAs of a layer: two per SM, each loads the weights once.
+inline int layer_ctas(int rows)
 {
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += part[size_t(z) * n + i];
-    out[i] = s * scale;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return std::min((rows + kRows - 1) / kRows, 2 * std::max(sms, 1));
 }
 
-// Column sums of X[n][cols] in fixed order: one thread per column, rows
-// split in `splits` chunks written to part[split][col].
-__global__ void k_colsum_part(const float* X, int rows, int cols, int rows_per_split, float* part)
+template <int K, int N, int KS, bool kT, Epilogue E>
+void layer(int rows, const float* A, const __nv_bfloat16* W, const LayerArgs& args, cudaStream_t s)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int z = blockIdx.y;
-    if (c >= cols) return;
-    const int r0 = z * rows_per_split, r1 = min(rows, r0 + rows_per_split);
-    float s = 0.0f;
-    for (int r = r0; r < r1; ++r) s += X[size_t(r) * cols + c];
-    part[size_t(z) * cols + c] = s;
+    constexpr int smem = (K * N + 2 * KS * kPad) * 4;
+    FCU_CHECK(cudaFuncSetAttribute(k_layer<K, N, KS, kT, E>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_layer<K, N, KS, kT, E><<<layer_ctas(rows), 256, smem, s>>>(rows, A, W, args);
+    FCU_LAUNCH("k_layer");
 }
 
-// dY = 2 (Y - T) / (n * 64); loss partials per block.
-__global__ void k_mse_grad(const float* Y, const float* T, size_t count, float scale, float* dY,
-                           double* loss_part)
+// ---- weight gradients ---------------------------------------------------------
+constexpr int kSlice = 16;  // rows in shared memory at a time
+
+// part[cta][o * I + i] = sum of D[r][o] X[r][i] over the CTA's rows, and
+// bias_part[cta][o] = sum of D[r][o]; `stride` floats from one CTA's partials to
+// the next's.  I = 128: 8 x 8 (O = 128) or 4 x 8 (O = 64) outputs per thread.
+template <int O>
+__global__ void __launch_bounds__(256, 2) k_wgrad(int rows, int rows_per_cta,
+                                                  const float* __restrict__ D,
+                                                  const float* __restrict__ X, size_t stride,
+                                                  float* __restrict__ part,
+                                                  float* __restrict__ bias_part)
+{
+    constexpr int I = 128, R = O / 16;
+    __shared__ __align__(16) float Ds[2][kSlice][O];
+    __shared__ __align__(16) float Xs[2][kSlice][I];
+    constexpr int kFd = kSlice * O / 4 / 256, kFx = kSlice * I / 4 / 256;
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const int begin = blockIdx.x * rows_per_cta, end = min(rows, begin + rows_per_cta);
+    float4 nd[kFd], nx[kFx];
+    auto fetch = [&](int r0) {
+#pragma unroll
+        for (int q = 0; q < kFd; ++q) {
+            const int i = threadIdx.x + q * 256, r = r0 + i / (O / 4);
+            nd[q] = r < end ? reinterpret_cast<const float4*>(D + size_t(r) * O)[i % (O / 4)]
+                            : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int q = 0; q < kFx; ++q) {
+            const int i = threadIdx.x + q * 256, r = r0 + i / (I / 4);
+            nx[q] = r < end ? reinterpret_cast<const float4*>(X + size_t(r) * I)[i % (I / 4)]
+                            : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    auto put = [&](int buf) {
+#pragma unroll
+        for (int q = 0; q < kFd; ++q) reinterpret_cast<float4*>(Ds[buf])[threadIdx.x + q * 256] = nd[q];
+#pragma unroll
+        for (int q = 0; q < kFx; ++q) reinterpret_cast<float4*>(Xs[buf])[threadIdx.x + q * 256] = nx[q];
+    };
+    float acc[R][8] = {}, bias = 0.0f;
+    fetch(begin);
+    put(0);
+    __syncthreads();
+#pragma unroll 1
+    for (int r0 = begin, buf = 0; r0 < end; r0 += kSlice, buf ^= 1) {
+        if (r0 + kSlice < end) fetch(r0 + kSlice);
+#pragma unroll
+        for (int k = 0; k < kSlice; ++k) {
+            float a[R], b[8];
+            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&Ds[buf][k][4 * ty]);
+            if (R == 8)
+                *reinterpret_cast<float4*>(a + R - 4) =
+                    *reinterpret_cast<const float4*>(&Ds[buf][k][O - 64 + 4 * ty]);
+            *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&Xs[buf][k][4 * tx]);
+            *reinterpret_cast<float4*>(b + 4) =
+                *reinterpret_cast<const float4*>(&Xs[buf][k][64 + 4 * tx]);
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; j += 2)
+                    fma2(acc[i][j], acc[i][j + 1], a[i], b[j], b[j + 1]);
+        }
+        if (threadIdx.x < O) {
+#pragma unroll
+            for (int k = 0; k < kSlice; ++k) bias += Ds[buf][k][threadIdx.x];
+        }
+        if (r0 + kSlice < end) put(buf ^ 1);
+        __syncthreads();
+    }
+    float* p = part + size_t(blockIdx.x) * stride;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int o = (i < 4 ? 0 : 64) + 4 * ty + i % 4;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            *reinterpret_cast<float4*>(p + o * I + h * 64 + 4 * tx) = make_float4(
+                acc[i][h * 4], acc[i][h * 4 + 1], acc[i][h * 4 + 2], acc[i][h * 4 + 3]);
+    }
+    if (threadIdx.x < O) bias_part[size_t(blockIdx.x) * stride + threadIdx.x] = bias;
+}
+
+// The first layer's gradient (I = 12 inputs): thread (o, half) sums 6 of a
+// weight row's 12 outputs.
+__global__ void __launch_bounds__(256) k_wgrad_first(int rows, int rows_per_cta,
+                                                     const float* __restrict__ D,
+                                                     const float* __restrict__ X, size_t stride,
+                                                     float* __restrict__ part,
+                                                     float* __restrict__ bias_part)
+{
+    constexpr int kTake = 64, U = 16;  // rows of X kept, rows of D in flight
+    __shared__ __align__(16) float Xs[kTake][kIn];
+    const int o = threadIdx.x % kH, half = threadIdx.x / kH;
+    const int begin = blockIdx.x * rows_per_cta, end = min(rows, begin + rows_per_cta);
+    float acc[6] = {}, bias = 0.0f;
+    for (int r0 = begin; r0 < end; r0 += kTake) {
+        const int n = min(kTake, end - r0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < n * kIn; i += 256) (&Xs[0][0])[i] = X[size_t(r0) * kIn + i];
+        __syncthreads();
+        for (int k = 0; k < n; k += U) {
+            float d[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) d[u] = k + u < n ? D[size_t(r0 + k + u) * kH + o] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (k + u >= n) break;
+                bias += d[u];
+#pragma unroll
+                for (int j = 0; j < 6; ++j) acc[j] += d[u] * Xs[k + u][half * 6 + j];
+            }
+        }
+    }
+    float* p = part + size_t(blockIdx.x) * stride;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) p[o * kIn + half * 6 + j] = acc[j];
+    if (half == 0) bias_part[size_t(blockIdx.x) * stride + o] = bias;
+}
+
+// out[i] = sum over the CTAs' partials, in order within each of 8 interleaved
+// runs and then over the runs.
+__global__ void __launch_bounds__(256) k_sum_partials(const float* __restrict__ part, int ctas,
+                                                      int n, float* __restrict__ out)
+{
+    __shared__ float red[8][32];
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31), run = threadIdx.x >> 5;
+    float s = 0.0f;
+    if (i < n)
+        for (int z = run; z < ctas; z += 8) s += part[size_t(z) * n + i];
+    red[run][threadIdx.x & 31] = s;
+    __syncthreads();
+    if (run == 0 && i < n) {
+        for (int k = 1; k < 8; ++k) s += red[k][threadIdx.x];
+        out[i] = s;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_sum_double(const double* part, int n, double* out)
 {
     __shared__ double red[256];
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    double l = 0.0;
-    if (i < count) {
-        const float d = Y[i] - T[i];
-        dY[i] = 2.0f * d * scale;
-        l = double(d) * double(d);
-    }
-    red[threadIdx.x] = l;
+    double s = 0.0;
+    for (int i = threadIdx.x; i < n; i += 256) s += part[i];
+    red[threadIdx.x] = s;
     __syncthreads();
     for (int o = 128; o > 0; o >>= 1) {
         if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) loss_part[blockIdx.x] = red[0];
-}
-
-__global__ void k_sum_double(const double* part, int n, double* out)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += part[i];
-    *out = s;
-}
-
-// dZ = dA * gelu'(Z)
-__global__ void k_gelu_back(const float* dA, const float* Z, size_t n, float* dZ)
-{
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) dZ[i] = dA[i] * gelu_grad(Z[i]);
+    if (threadIdx.x == 0) *out = red[0];
 }
 
 __global__ void k_to_bf16(const float* p, size_t n, __nv_bfloat16* q)
@@ -270,54 +467,27 @@ void set_params(Net& net, const float* host, cudaStream_t s)
     net.steps_done = 0;
 }
 
-namespace {
-
-template <bool TA, bool TB, typename TBT, int EPI>
-void gemm(int M, int N, int K, const float* A, int lda, const TBT* B, int ldb, float* C, int ldc,
-          const float* bias, float* C2, int splits, cudaStream_t s)
-{
-    const int kps = ((K + splits - 1) / splits + TK - 1) / TK * TK;
-    dim3 grid(unsigned((N + TN - 1) / TN), unsigned((M + TM - 1) / TM), unsigned(splits));
-    k_gemm<TB ? TA : TA, TB, TBT, EPI><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, bias,
-                                                           C2, kps);
-    FCU_LAUNCH("k_gemm");
-}
-
-}  // namespace
-
-// Forward pass of n rows (activations kept in sc for a backward pass).
-static void forward(Net& net, const float* X, int n, Scratch& sc, float* Y, cudaStream_t s)
+// The hidden layers of n rows: GELU(Z) to sc.a1, sc.a2 and, for a backward
+// pass, Z to sc.z1, sc.z2.
+static void hidden(Net& net, const float* X, int n, Scratch& sc, bool keep_z, cudaStream_t s)
 {
     const __nv_bfloat16* w = net.bf16.as<__nv_bfloat16>();
     const float* p = net.params.as<float>();
-    float* z1 = static_cast<float*>(sc.z1.reserve(size_t(n) * kH * 4));
+    float* z1 = keep_z ? static_cast<float*>(sc.z1.reserve(size_t(n) * kH * 4)) : nullptr;
     float* a1 = static_cast<float*>(sc.a1.reserve(size_t(n) * kH * 4));
-    float* z2 = static_cast<float*>(sc.z2.reserve(size_t(n) * kH * 4));
+    float* z2 = keep_z ? static_cast<float*>(sc.z2.reserve(size_t(n) * kH * 4)) : nullptr;
     float* a2 = static_cast<float*>(sc.a2.reserve(size_t(n) * kH * 4));
-    // Z1 = X W1^T + b1 ; A1 = gelu(Z1)
-    gemm<false, true, __nv_bfloat16, 1>(n, kH, kIn, X, kIn, w + kOffW1, kIn, z1, kH, p + kOffB1,
-                                        a1, 1, s);
-    gemm<false, true, __nv_bfloat16, 1>(n, kH, kH, a1, kH, w + kOffW2, kH, z2, kH, p + kOffB2, a2,
-                                        1, s);
-    // Y = A2 W3^T + b3 (no activation): use EPI 1 into a scratch then copy?
-    // The output layer has no GELU: EPI 0, then add the bias in the loss or
-    // here with a tiny kernel.
-    gemm<false, true, __nv_bfloat16, 0>(n, kOut, kH, a2, kH, w + kOffW3, kH, Y, kOut, nullptr,
-                                        nullptr, 1, s);
-}
-
-static __global__ void k_add_bias(float* Y, const float* b, size_t rows, int cols)
-{
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < rows * cols) Y[i] += b[i % cols];
+    layer<kIn, kH, kIn, true, kGelu>(n, X, w + kOffW1, {p + kOffB1, nullptr, z1, a1, nullptr, 0.0f}, s);
+    layer<kH, kH, 16, true, kGelu>(n, a1, w + kOffW2, {p + kOffB2, nullptr, z2, a2, nullptr, 0.0f}, s);
 }
 
 void forward_full(Net& net, const float* X, int n, Scratch& sc, float* Y, cudaStream_t s)
 {
-    forward(net, X, n, sc, Y, s);
-    k_add_bias<<<blocks(size_t(n) * kOut, 256), 256, 0, s>>>(Y, net.params.as<float>() + kOffB3,
-                                                             size_t(n), kOut);
-    FCU_LAUNCH("k_add_bias");
+    hidden(net, X, n, sc, false, s);
+    layer<kH, kOut, 16, true, kOutput>(n, sc.a2.as<float>(), net.bf16.as<__nv_bfloat16>() + kOffW3,
+                                       {net.params.as<float>() + kOffB3, nullptr, Y, nullptr,
+                                        nullptr, 0.0f},
+                                       s);
 }
 
 // Inference over any number of rows: chunks of kInferChunk rows keep the
@@ -334,52 +504,38 @@ void infer(Net& net, const float* X, size_t n, Scratch& sc, float* Y, cudaStream
 double loss_and_grad(Net& net, const float* X, const float* T, int n, Scratch& sc, cudaStream_t s,
                      bool want_loss)
 {
-    float* Y = static_cast<float*>(sc.y.reserve(size_t(n) * kOut * 4));
-    forward_full(net, X, n, sc, Y, s);
-    float* dY = static_cast<float*>(sc.dy.reserve(size_t(n) * kOut * 4));
-    const size_t cnt = size_t(n) * kOut;
-    const unsigned lb = blocks(cnt, 256);
-    double* lossp = static_cast<double*>(sc.lossp.reserve((lb + 1) * 8));
-    k_mse_grad<<<lb, 256, 0, s>>>(Y, T, cnt, 1.0f / float(cnt), dY, lossp);
-    FCU_LAUNCH("k_mse_grad");
     const __nv_bfloat16* w = net.bf16.as<__nv_bfloat16>();
-    float* g = net.grad.as<float>();
-    const int splits = std::max(1, std::min(64, n / 512));
-    float* part = static_cast<float*>(sc.part.reserve(size_t(splits) * kH * kH * 4 + 64));
-    float* da = static_cast<float*>(sc.da.reserve(size_t(n) * kH * 4));
-    float* dz = static_cast<float*>(sc.dz.reserve(size_t(n) * kH * 4));
-    const int rps = (n + splits - 1) / splits;
-    // layer 3: dW3[o][h] = sum_r dY[r][o] A2[r][h]; db3 = colsum dY
-    gemm<true, false, float, 0>(kOut, kH, n, dY, kOut, sc.a2.as<float>(), kH, part, kH, nullptr,
-                                nullptr, splits, s);
-    k_sum_splits<<<blocks(kW3, 256), 256, 0, s>>>(part, splits, kW3, g + kOffW3, 1.0f);
-    k_colsum_part<<<dim3(blocks(kOut, 128), splits), 128, 0, s>>>(dY, n, kOut, rps, part);
-    k_sum_splits<<<1, 128, 0, s>>>(part, splits, kB3, g + kOffB3, 1.0f);
-    // dA2 = dY W3 ; dZ2 = dA2 gelu'(Z2)
-    gemm<false, false, __nv_bfloat16, 0>(n, kH, kOut, dY, kOut, w + kOffW3, kH, da, kH, nullptr,
-                                         nullptr, 1, s);
-    k_gelu_back<<<blocks(size_t(n) * kH, 256), 256, 0, s>>>(da, sc.z2.as<float>(), size_t(n) * kH,
-                                                            dz);
-    // layer 2: dW2 = dZ2^T A1 ; db2 = colsum dZ2
-    gemm<true, false, float, 0>(kH, kH, n, dz, kH, sc.a1.as<float>(), kH, part, kH, nullptr,
-                                nullptr, splits, s);
-    k_sum_splits<<<blocks(kW2, 256), 256, 0, s>>>(part, splits, kW2, g + kOffW2, 1.0f);
-    k_colsum_part<<<dim3(blocks(kH, 128), splits), 128, 0, s>>>(dz, n, kH, rps, part);
-    k_sum_splits<<<1, 128, 0, s>>>(part, splits, kB2, g + kOffB2, 1.0f);
-    // dA1 = dZ2 W2 ; dZ1 = dA1 gelu'(Z1)
-    gemm<false, false, __nv_bfloat16, 0>(n, kH, kH, dz, kH, w + kOffW2, kH, da, kH, nullptr,
-                                         nullptr, 1, s);
-    k_gelu_back<<<blocks(size_t(n) * kH, 256), 256, 0, s>>>(da, sc.z1.as<float>(), size_t(n) * kH,
-                                                            dz);
-    // layer 1: dW1 = dZ1^T X ; db1 = colsum dZ1
-    gemm<true, false, float, 0>(kH, kIn, n, dz, kH, X, kIn, part, kIn, nullptr, nullptr, splits, s);
-    k_sum_splits<<<blocks(kW1, 256), 256, 0, s>>>(part, splits, kW1, g + kOffW1, 1.0f);
-    k_colsum_part<<<dim3(blocks(kH, 128), splits), 128, 0, s>>>(dz, n, kH, rps, part);
-    k_sum_splits<<<1, 128, 0, s>>>(part, splits, kB1, g + kOffB1, 1.0f);
+    const float* p = net.params.as<float>();
+    hidden(net, X, n, sc, true, s);
+    const float *z1 = sc.z1.as<float>(), *a1 = sc.a1.as<float>(), *z2 = sc.z2.as<float>(),
+                *a2 = sc.a2.as<float>();
+    float* dy = static_cast<float*>(sc.dy.reserve(size_t(n) * kOut * 4));
+    float* dz2 = static_cast<float*>(sc.da.reserve(size_t(n) * kH * 4));
+    float* dz1 = static_cast<float*>(sc.dz.reserve(size_t(n) * kH * 4));
+    const size_t cnt = size_t(n) * kOut;
+    const int tiles = layer_ctas(n);
+    double* lossp = static_cast<double*>(sc.lossp.reserve((size_t(tiles) + 1) * 8));
+    layer<kH, kOut, 16, true, kLoss>(n, a2, w + kOffW3,
+                                     {p + kOffB3, T, dy, nullptr, lossp, 1.0f / float(cnt)}, s);
+    // dZ2 = dY W3 gelu'(Z2) ; dZ1 = dZ2 W2 gelu'(Z1)
+    layer<kOut, kH, 16, false, kGeluBack>(n, dy, w + kOffW3, {nullptr, z2, dz2, nullptr, nullptr, 0.0f}, s);
+    layer<kH, kH, 16, false, kGeluBack>(n, dz2, w + kOffW2, {nullptr, z1, dz1, nullptr, nullptr, 0.0f}, s);
+    // weight and bias gradients: two CTAs per SM, at least 64 rows each
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int want = std::max(1, std::min(2 * std::max(sms, 1), n / 64));
+    const int per = (n + want - 1) / want;
+    const int ctas = (n + per - 1) / per;
+    float* part = static_cast<float*>(sc.part.reserve(size_t(ctas) * kParams * 4));
+    k_wgrad<kOut><<<ctas, 256, 0, s>>>(n, per, dy, a2, kParams, part + kOffW3, part + kOffB3);
+    k_wgrad<kH><<<ctas, 256, 0, s>>>(n, per, dz2, a1, kParams, part + kOffW2, part + kOffB2);
+    k_wgrad_first<<<ctas, 256, 0, s>>>(n, per, dz1, X, kParams, part + kOffW1, part + kOffB1);
+    k_sum_partials<<<blocks(kParams, 32), 256, 0, s>>>(part, ctas, kParams, net.grad.as<float>());
     FCU_LAUNCH("mlp backward");
     if (!want_loss) return 0.0;
-    double* total = lossp + lb;
-    k_sum_double<<<1, 1, 0, s>>>(lossp, int(lb), total);
+    double* total = lossp + tiles;
+    k_sum_double<<<1, 256, 0, s>>>(lossp, tiles, total);
     double host = 0.0;
     FCU_CHECK(cudaMemcpyAsync(&host, total, 8, cudaMemcpyDeviceToHost, s));
     FCU_CHECK(cudaStreamSynchronize(s));

@@ -229,3 +229,36 @@ def test_tensor_core_wait_times_out_and_context_survives(model, monkeypatch):
     monkeypatch.delenv("FACETCU_TEST_STALL_TENSOR_WAIT")
     y = model.mlpForwardTensor(x)
     assert np.max(np.abs(y - M.forward_bf16_activations(params, x))) <= 5e-3 * max(1.0, np.abs(y).max())
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 127, 128, 129, 1000, 38912, 38913, 39041])
+def test_forward_and_gradient_at_tile_edges(model, n):
+    """Row counts around the layers' 128-row tiles, the weight gradients' 64
+    rows per CTA and 2 x 152 tiles (where a CTA starts to take a second tile).
+    Tolerance: FP32 products and sums over K = 128 and over n rows in shares,
+    whose rounding stays below sqrt(K + n) 2^-24 of a tensor's norm, through
+    three layers and back: 6 sqrt(128 + n) 2^-24."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    params = rng.normal(scale=0.15, size=M.COUNT).astype(np.float32)
+    model.mlpSetParameters(params)
+    x = rng.normal(size=(n, 12)).astype(np.float32)
+    t = rng.normal(size=(n, 64)).astype(np.float32)
+    parts = {k: torch.from_numpy(v).requires_grad_() for k, v in M.effective(params).items()}
+    h = torch.from_numpy(x).double()
+    for k in ("1", "2"):
+        h = torch.nn.functional.gelu(h @ parts["W" + k].T + parts["b" + k])
+    y = h @ parts["W3"].T + parts["b3"]
+    loss = ((y - torch.from_numpy(t).double()) ** 2).mean()
+    loss.backward()
+    tol = 6 * np.sqrt(128 + n) * 2.0 ** -24
+    got = model.mlpForward(x)
+    assert np.linalg.norm(got - y.detach().numpy()) <= tol * np.linalg.norm(y.detach().numpy())
+    got_loss, g = model.mlpLossAndGradient(x, t)
+    assert abs(got_loss - loss.item()) <= tol * loss.item()
+    off = 0
+    for name, shape in M.SIZES:
+        k = int(np.prod(shape))
+        want = parts[name].grad.numpy().ravel()
+        assert np.linalg.norm(g[off:off + k] - want) <= tol * np.linalg.norm(want), name
+        off += k
