@@ -414,7 +414,8 @@ __device__ __forceinline__ void gather_split(const uint32_t* __restrict__ rows,
         for (int k = 0; k < CPL; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
 }
 
-// The same product for 8 or 16 FP32 columns: L = P / 4 lanes per row, so one
+// The same product for 8 or 16 FP32 columns, for graphs without packed words
+// (k_sweep_mid has those): L = P / 4 lanes per row, so one
 // load instruction covers G = 32 / L = 16 or 8 edges, and a round of
 // 32 * G / 4 edges (128 or 64, G / 4 packed words per lane) gives every lane
 // eight 16-byte loads in flight (a 32-edge chunk would fill only two or four
@@ -652,6 +653,151 @@ __global__ void __launch_bounds__(kWarps * 32, SweepBlocks<P>::value) k_sweep_wi
         }
     });
     publish_cols<CPL>(md, mb, mr, col0, owner, P, stats);
+}
+
+// The FP32 sweep of 8 or 16 columns over packed edges.  A row of P floats is L =
+// P / 4 vectors of 16 bytes, so a load instruction covers G = 32 / L edges and a
+// round of 4 G edges x 2 (128 or 64) gives a lane eight loads in flight.  What
+// bounds it is latency (32- or 64-byte rows from L2, 5 TB/s where 64-byte
+// rows can reach 15.8), so the chain of dependent loads is taken apart: chunk
+// numbers are drawn two chunks ahead, row offsets read one chunk ahead, a
+// round's edge words while the round before is gathered, and the facet's own
+// values before its rows.  The lanes' partial sums of both sides are folded
+// together by a reduce-scatter (8 shuffles per facet; 64 when every lane
+// kept all sums), after which a lane owns one (side, column).
+// On the forest's 74.4 M edges 8 columns take 287 us and 16 columns 326
+// (k_sweep_wide: 448 and 537), about one row per clock and SM, what the L1's
+// tags take.  CTAs per SM measured: 8 columns 296, 287 and 304 us at 2, 3 and
+// 4, 16 columns 412, 336 and 326.
+template <int P>
+__global__ void __launch_bounds__(kWarps * 32, P == 8 ? 3 : 4) k_sweep_mid(GraphView g, PanelParams pp,
+                                                               const float* __restrict__ Bin,
+                                                               float* __restrict__ Bout,
+                                                               uint32_t* stats, uint32_t* counter,
+                                                               const uint32_t* done)
+{
+    if (*done) return;
+    static_assert(P == 8 || P == 16, "8 or 16 columns");
+    constexpr int L = P / 4, G = 32 / L, U = 8, E = G * U, W = E / 32;
+    constexpr uint32_t C = 2;  // facets per chunk
+    __shared__ uint32_t s_stat[3][P];
+    const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
+    for (int i = threadIdx.x; i < 3 * P; i += blockDim.x) (&s_stat[0][0])[i] = 0u;
+    __syncthreads();
+    // after the fold: lane -> (side, column); 8 columns have two lanes each
+    const int side = lane >> 4;
+    const int col = sub * 4 + (lane >> 3 & 1) * 2 + (lane >> 2 & 1);
+    const bool owner = P == 16 || (lane & 2) == 0;
+    const float Lsky = pp.skyL[col], floor_abs = kSideFloor * pp.colmax[col];
+    float md = 0.0f, mb = 0.0f, mr = 0.0f;
+    const uint32_t S = 2u * g.facets, chunks = (g.facets + C - 1) / C;
+    const uint32_t mask = (1u << g.nb_bits) - 1u;
+    const float4* __restrict__ X4 = reinterpret_cast<const float4*>(Bin);
+    auto draw = [&] { return lane == 0 ? atomicAdd(counter, 1u) : 0u; };
+    auto offsets = [&](uint32_t ch) {
+        const uint32_t s = min(S, ch * 2u * C + uint32_t(min(lane, int(2 * C))));
+        return ch < chunks ? __ldg(g.rows + s) : 0u;
+    };
+    auto words = [&](uint32_t base, uint32_t end, uint32_t (&x)[W]) {
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+            const uint32_t e = base + uint32_t(q * 32 + lane);
+            x[q] = e < end ? __ldcs(g.packed + e) : 0u;
+        }
+    };
+    uint32_t ch = __shfl_sync(0xffffffffu, draw(), 0);
+    uint32_t row = offsets(ch);
+    uint32_t drawn = draw();
+    uint32_t w[W], held = 0xffffffffu, held_end = 0u;  // words of [held, held_end)
+    while (ch < chunks) {
+        const uint32_t chn = __shfl_sync(0xffffffffu, drawn, 0);
+        const uint32_t rown = offsets(chn);
+        drawn = draw();
+        const uint32_t fe = min(g.facets, (ch + 1) * C);
+        for (uint32_t f = ch * C; f < fe; ++f) {
+            // the facet's own values, in the lanes that will use them
+            const uint32_t s_own = 2u * f + uint32_t(side);
+            const size_t i = size_t(s_own) * P + col;
+            const uint32_t d = __ldg(g.denom + s_own), sk = __ldg(g.skyc + s_own);
+            const float dir = __ldcs(pp.direct + i), em = __ldcs(pp.emis + i),
+                        rh = __ldcs(pp.rho + i), ta = __ldcs(pp.tau + i), old = Bin[i];
+            float acc[2][4] = {};
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int r = int(2u * (f - ch * C)) + k;
+                const uint32_t start = __shfl_sync(0xffffffffu, row, r);
+                const uint32_t end = __shfl_sync(0xffffffffu, row, r + 1);
+                // where the round after the side's last one begins and ends
+                const bool last = r + 1 == int(2u * C) || (k == 1 && f + 1 == fe);
+                const uint32_t after = __shfl_sync(0xffffffffu, last ? rown : row, last ? 0 : r + 1);
+                const uint32_t after_end =
+                    __shfl_sync(0xffffffffu, last ? rown : row, last ? 1 : min(r + 2, 31));
+                for (uint32_t base = start; base < end; base += E) {
+                    // (after an empty row nothing was read ahead)
+                    if (held != base || held_end != end) words(base, end, w);
+                    float4 q[U];
+                    float c[U];
+                    uint32_t x[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int idx = u * G + grp;
+                        x[u] = __shfl_sync(0xffffffffu, w[(u * G) / 32], idx & 31);
+                    }
+                    const bool more = base + E < end;
+                    held = more ? base + E : after;
+                    held_end = more ? end : after_end;
+                    words(held, held_end, w);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const bool on = base + uint32_t(u * G + grp) < end;
+                        c[u] = float(x[u] >> g.nb_bits);
+                        q[u] = on ? __ldg(X4 + size_t(x[u] & mask) * L + sub)
+                                  : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        acc[k][0] += c[u] * q[u].x;
+                        acc[k][1] += c[u] * q[u].y;
+                        acc[k][2] += c[u] * q[u].z;
+                        acc[k][3] += c[u] * q[u].w;
+                    }
+                }
+            }
+            // reduce-scatter: lane bit 4 keeps a side, bit 3 two columns, bit 2 one
+            float v4[4], v2[2], v;
+            const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float give = b4 ? acc[0][j] : acc[1][j];
+                v4[j] = (b4 ? acc[1][j] : acc[0][j]) + __shfl_xor_sync(0xffffffffu, give, 16);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float give = b3 ? v4[j] : v4[2 + j];
+                v2[j] = (b3 ? v4[2 + j] : v4[j]) + __shfl_xor_sync(0xffffffffu, give, 8);
+            }
+            {
+                const float give = b2 ? v2[0] : v2[1];
+                v = (b2 ? v2[1] : v2[0]) + __shfl_xor_sync(0xffffffffu, give, 4);
+            }
+            if (P == 8) v += __shfl_xor_sync(0xffffffffu, v, 2);
+            const float h = (d != 0u ? (float(sk) * Lsky + v) / float(d) : Lsky) + dir;
+            const float ho = __shfl_xor_sync(0xffffffffu, h, 16);  // the facet's other side
+            const float b = em + rh * h + ta * ho;
+            if (owner) Bout[i] = b;
+            md = fmaxf(md, fabsf(b - old));
+            mb = fmaxf(mb, fabsf(b));
+            mr = fmaxf(mr, rel_change(b - old, b, floor_abs));
+        }
+        ch = chn;
+        row = rown;
+    }
+    atomicMax(&s_stat[0][col], __float_as_uint(md));
+    atomicMax(&s_stat[1][col], __float_as_uint(mb));
+    atomicMax(&s_stat[2][col], __float_as_uint(mr));
+    __syncthreads();
+    for (int k = threadIdx.x; k < 3 * P; k += blockDim.x)
+        atomicMax(stats + (k / P) * kMaxP + k % P, s_stat[k / P][k % P]);
 }
 
 // The first sweep of a solve from zero, B = T(0): no gather, so one thread
@@ -2218,6 +2364,17 @@ void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in,
             default: k_sweep_zero<128><<<grid, 256, 0, s>>>(g, pp, out, stats, done); break;
             }
             FCU_LAUNCH("k_sweep_zero");
+            return;
+        }
+        if ((P == 8 || P == 16) && g.packed) {
+            if (P == 8) {
+                static const int grid = grid_for(k_sweep_mid<8>);
+                k_sweep_mid<8><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+            } else {
+                static const int grid = grid_for(k_sweep_mid<16>);
+                k_sweep_mid<16><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+            }
+            FCU_LAUNCH("k_sweep_mid");
             return;
         }
         if (P == 8 || P == 16) {

@@ -1,6 +1,7 @@
-"""One-column sweeps on the device against a float64 Jacobi iteration in numpy:
+"""Sweeps of one and of a few columns on the device against a float64 Jacobi iteration in numpy:
 the CSR kernel (k_jacobi_rows) at the edges of its lane groups, and the
-shared-memory plan (column.cu) at the edges of its tiles, windows and groups.
+shared-memory plan (column.cu) at the edges of its tiles, windows and groups,
+and the 8- and 16-column panels (k_sweep_mid) at the edges of their rounds.
 
 Tolerance: a sweep adds at most `deg` products in FP32, so a row's relative
 error per sweep is below (deg + 8) 2^-24, and the iteration (rho + tau = c)
@@ -156,3 +157,26 @@ def test_planned_incident_in_a_node(planned):
     # H is rounded once to float and the two products and sums are floats
     scale = 2 * (eps * H.max() + E.max())
     assert np.max(np.abs(out["net_radiation"] - want)) < 12 * 2.0 ** -24 * scale + 1e-6 * scale
+
+
+@pytest.mark.parametrize("bands", [5, 8, 11, 16])  # panels of 8 and 16 columns
+@pytest.mark.parametrize("S", [2, 6, 1030])
+def test_few_columns(S, bands):
+    """Rows around 64 and 128 edges (one round of 16 and 8 columns), empty rows
+    before, between and after others, an odd number of facets."""
+    require_gpu()
+    rng = np.random.default_rng(S + bands)
+    edge = np.array([0, 1, 63, 64, 65, 0, 0, 127, 128, 129, 255, 256, 257, 3, 0, 500])
+    graph = _graph(S, np.resize(edge, S), rng, counts=[255, 256, 257, 1000])
+    m = _model(S, graph)
+    scale = np.linspace(0.5, 2.0, bands, dtype=np.float32)
+    o = _optics(S, rng)
+    rep = lambda v: np.repeat(v[None, :], bands, 0)  # noqa: E731
+    out, res = m.solveBatched(rep(o[:, 0]), rep(o[:, 1]), np.full(bands, SKY, np.float32), scale,
+                              o[:, 3][None, :], emission=rep(o[:, 2]), tolerance=1e-7)
+    m.close()
+    tol = _tolerance(graph) + 1e-7 / (1 - RHO - TAU)
+    for b in range(bands):
+        direct = (o[:, 3] * scale[b]).astype(np.float64)
+        want = _jacobi(graph, direct, o[:, 2].astype(np.float64), 60)
+        assert np.max(np.abs(out[b] - want) / want) < tol
