@@ -32,8 +32,7 @@ struct facetcu_context {
     cudaStream_t stream = nullptr;
 
     uint32_t facets = 0;
-    std::vector<facetcu_vertex> vertices_host;
-    DeviceBuffer vertices;
+    DeviceBuffer vertices, vertices_next;
     float bmin[3] = {0, 0, 0}, bmax[3] = {0, 0, 0};
     bool bounds_override = false;
     float omin[3] = {0, 0, 0}, omax[3] = {0, 0, 0};
@@ -356,6 +355,8 @@ int facetcu_destroy(facetcu_context* ctx)
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     ctx->vertices.release();
+    ctx->vertices_next.release();
+    ctx->ws.release();
     ctx->graph.row_offsets.release();
     ctx->graph.edges.release();
     ctx->graph.denominators.release();
@@ -371,8 +372,7 @@ int facetcu_destroy(facetcu_context* ctx)
     ctx->graph_ready = false;
     for (DeviceBuffer* b : {&ctx->raster.counts, &ctx->raster.offsets, &ctx->raster.records,
                             &ctx->raster.big_list, &ctx->raster.deep_list, &ctx->raster.stats,
-                            &ctx->pairs, &ctx->pair_count, &ctx->denom_tmp, &ctx->ws.a, &ctx->ws.b,
-                            &ctx->ws.c, &ctx->ws.d, &ctx->ws.e, &ctx->optics, &ctx->rad_a,
+                            &ctx->pairs, &ctx->pair_count, &ctx->denom_tmp, &ctx->optics, &ctx->rad_a,
                             &ctx->rad_b, &ctx->residual, &ctx->host_io, &ctx->scratch,
                             &ctx->sun_total, &ctx->sun_visible, &ctx->batch.x0, &ctx->batch.x1,
                             &ctx->batch.half, &ctx->batch.colstats, &ctx->batch.q,
@@ -398,7 +398,6 @@ int facetcu_destroy(facetcu_context* ctx)
         b->release();
     ctx->net.ready = false;
     ctx->bvh_ready = false;
-    ctx->vertices_host.clear();
     ctx->bounds_override = false;
     ctx->initialized = false;
     return FACETCU_OK;
@@ -426,34 +425,26 @@ int facetcu_set_geometry(facetcu_context* ctx, const facetcu_vertex* vertices,
             throw Error(FACETCU_INVALID_ARGUMENT, "Geometry must be a non-empty triangle list");
         if (vertex_count / 3 > (1ull << 30))
             throw Error(FACETCU_OVERFLOW_ERROR, "Geometry exceeds 2^30 facets");
-        for (uint64_t i = 0; i < vertex_count; ++i) {
-            const facetcu_vertex& v = vertices[i];
-            for (float c : v.position)
-                if (!std::isfinite(c))
-                    throw Error(FACETCU_INVALID_ARGUMENT, "Geometry contains a non-finite position");
-            const float len = std::sqrt(v.normal[0] * v.normal[0] + v.normal[1] * v.normal[1] +
-                                        v.normal[2] * v.normal[2]);
-            if (!(len > 0.99f && len < 1.01f))
-                throw Error(FACETCU_INVALID_ARGUMENT, "Facet normals must be normalized");
-        }
-        FCU_CHECK(cudaStreamSynchronize(ctx->stream));
+        // checked on the device before anything of the old geometry changes
+        DeviceBuffer& next = ctx->vertices_next;
+        upload(next, vertices, vertex_count * sizeof(facetcu_vertex), ctx->stream);
+        const GeometryCheck check =
+            check_geometry(next.as<facetcu_vertex>(), vertex_count, ctx->ws, ctx->stream);
+        if (check.bad_position != 0xffffffffu && check.bad_position <= check.bad_normal)
+            throw Error(FACETCU_INVALID_ARGUMENT, "Geometry contains a non-finite position");
+        if (check.bad_normal != 0xffffffffu)
+            throw Error(FACETCU_INVALID_ARGUMENT, "Facet normals must be normalized");
         ctx->graph_ready = false;
         ctx->graph.changed();
         ctx->graph.scene_facets.clear();
         ctx->bvh_ready = false;
         ctx->facets = uint32_t(vertex_count / 3);
-        ctx->vertices_host.assign(vertices, vertices + vertex_count);
+        std::swap(ctx->vertices.ptr, next.ptr);
+        std::swap(ctx->vertices.bytes, next.bytes);
         for (int a = 0; a < 3; ++a) {
-            ctx->bmin[a] = std::numeric_limits<float>::max();
-            ctx->bmax[a] = std::numeric_limits<float>::lowest();
+            ctx->bmin[a] = check.lo[a];
+            ctx->bmax[a] = check.hi[a];
         }
-        for (uint64_t i = 0; i < vertex_count; ++i)
-            for (int a = 0; a < 3; ++a) {
-                ctx->bmin[a] = std::min(ctx->bmin[a], vertices[i].position[a]);
-                ctx->bmax[a] = std::max(ctx->bmax[a], vertices[i].position[a]);
-            }
-        upload(ctx->vertices, vertices, vertex_count * sizeof(facetcu_vertex), ctx->stream);
-        FCU_CHECK(cudaStreamSynchronize(ctx->stream));
         return FACETCU_OK;
     });
 }
@@ -588,16 +579,13 @@ int facetcu_compute_sunlit_fraction(facetcu_context* ctx, const facetcu_directio
         uint32_t* visible = static_cast<uint32_t*>(ctx->sun_visible.reserve(size_t(S) * 4));
         FCU_CHECK(cudaMemsetAsync(total, 0, size_t(S) * 4, s));
         FCU_CHECK(cudaMemsetAsync(visible, 0, size_t(S) * 4, s));
-        raster_resolve_sunlit(frame, chain_cap(ctx), ctx->raster, total, visible, st, s);
+        float* d_fraction = static_cast<float*>(ctx->fraction.reserve(size_t(S) * 4));
+        raster_resolve_sunlit(frame, chain_cap(ctx), ctx->raster, total, visible, d_fraction, st, s);
         if (st.overflow)
             throw Error(FACETCU_RUNTIME_ERROR,
                         "Direct-light A-buffer overflow; increase Config::maxFragmentsPerPixel");
-        std::vector<uint32_t> t(S), v(S);
-        FCU_CHECK(cudaMemcpyAsync(t.data(), total, size_t(S) * 4, cudaMemcpyDeviceToHost, s));
-        FCU_CHECK(cudaMemcpyAsync(v.data(), visible, size_t(S) * 4, cudaMemcpyDeviceToHost, s));
+        FCU_CHECK(cudaMemcpyAsync(fraction, d_fraction, size_t(S) * 4, cudaMemcpyDeviceToHost, s));
         FCU_CHECK(cudaStreamSynchronize(s));
-        for (uint32_t i = 0; i < S; ++i)
-            fraction[i] = t[i] ? float(v[i]) / float(t[i]) : 0.0f;
         return FACETCU_OK;
     });
 }
@@ -732,7 +720,7 @@ int facetcu_hemisphere_sunlit(facetcu_context* ctx, const facetcu_direction* sun
         float* d = static_cast<float*>(ctx->fraction.reserve(size_t(S) * 4));
         hemisphere_sunlit(ctx->vertices.as<facetcu_vertex>(), ctx->facets, ctx->bvh,
                           ctx->samples_uv.as<float>(), samples, sample_sets,
-                          make_float3(sun->x, sun->y, sun->z), make_tiles(ctx), d, s);
+                          make_float3(sun->x, sun->y, sun->z), make_tiles(ctx), d, ctx->ws, s);
         FCU_CHECK(cudaMemcpyAsync(fraction, d, size_t(S) * 4, cudaMemcpyDeviceToHost, s));
         FCU_CHECK(cudaStreamSynchronize(s));
         return FACETCU_OK;
@@ -1540,14 +1528,17 @@ int facetcu_scene_batch(facetcu_context* ctx, facetcu_context* const* scenes,
         uint32_t n = 1;
         while (uint64_t(n) * n * n < scene_count) ++n;
         const float cell = 1.25f * std::max(extent, 1.0f);
-        std::vector<facetcu_vertex> all;
+        std::vector<facetcu_vertex> all, part;
         all.reserve(size_t(facets) * 3);
         for (uint32_t i = 0; i < scene_count; ++i) {
             const facetcu_context* sc = scenes[i];
             const float off[3] = {float(i % n) * cell - sc->bmin[0],
                                   float((i / n) % n) * cell - sc->bmin[1],
                                   float(i / (n * n)) * cell - sc->bmin[2]};
-            for (facetcu_vertex v : sc->vertices_host) {
+            part.resize(size_t(sc->facets) * 3);
+            FCU_CHECK(cudaMemcpy(part.data(), sc->vertices.ptr, part.size() * sizeof(facetcu_vertex),
+                                 cudaMemcpyDeviceToHost));
+            for (facetcu_vertex v : part) {
                 for (int a = 0; a < 3; ++a) v.position[a] += off[a];
                 all.push_back(v);
             }

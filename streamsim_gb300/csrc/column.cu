@@ -564,7 +564,7 @@ bool make_plan(DeviceGraph& g, Workspace& ws, cudaStream_t s)
     const uint32_t* packed = g.packed_valid ? g.packed.as<uint32_t>() : nullptr;
     const facetcu_csr_edge* edges = g.edges.as<facetcu_csr_edge>();
 
-    DeviceBuffer seg_buf, slot_buf, ng_buf, first_buf, group_buf;
+    ScratchBuffer seg_buf(ws), slot_buf(ws), ng_buf(ws), first_buf(ws), group_buf(ws);
     uint16_t* seg = static_cast<uint16_t*>(seg_buf.reserve(size_t(tiles) * S * 2));
     uint16_t* slot = static_cast<uint16_t*>(slot_buf.reserve(size_t(tiles) * S * 2));
     uint32_t* ng = static_cast<uint32_t*>(ng_buf.reserve(size_t(cells) * 4));

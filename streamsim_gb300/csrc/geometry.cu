@@ -1,0 +1,98 @@
+// geometry.cu — the checks of setGeometry on the device.
+//
+// FacetrtVulkan::validateGeometry (facetrt_vulkan.cpp:425-453) refuses the
+// first vertex whose position is not finite or whose normal is not of unit
+// length, and the bounds of the positions frame the raster.  On the host the
+// pass over the vertices took 3 ms for 200,000 facets, more than the raster
+// build that follows; here it is one read of the uploaded vertices (compiled
+// with -fmad=false: the normal's length rounds as the host's did).
+#include <cfloat>
+
+#include "internal.h"
+
+namespace facetcu {
+namespace {
+
+struct Result {
+    uint32_t bad_position, bad_normal;
+    uint32_t lo[3], hi[3];  // ordered keys
+};
+
+// Order-preserving key of a finite float.
+__device__ __host__ inline uint32_t key_of(uint32_t bits)
+{
+    return bits & 0x80000000u ? ~bits : bits | 0x80000000u;
+}
+inline float value_of(uint32_t key)
+{
+    const uint32_t bits = key & 0x80000000u ? key & 0x7fffffffu : ~key;
+    float f;
+    std::memcpy(&f, &bits, 4);
+    return f;
+}
+
+__global__ void __launch_bounds__(256) k_check_geometry(const float* __restrict__ v, uint64_t count,
+                                                        Result* r)
+{
+    uint32_t bad_position = 0xffffffffu, bad_normal = 0xffffffffu;
+    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) {
+        const float2* q = reinterpret_cast<const float2*>(v + 6 * i);
+        const float2 a = q[0], b = q[1], c = q[2];
+        const float p[3] = {a.x, a.y, b.x}, n[3] = {b.y, c.x, c.y};
+        bool finite = true;
+        for (int k = 0; k < 3; ++k) {
+            finite &= isfinite(p[k]);
+            lo[k] = fminf(lo[k], p[k]);
+            hi[k] = fmaxf(hi[k], p[k]);
+        }
+        if (!finite) bad_position = min(bad_position, uint32_t(i));
+        const float len = sqrtf(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+        if (!(len > 0.99f && len < 1.01f)) bad_normal = min(bad_normal, uint32_t(i));
+    }
+    const bool first = (threadIdx.x & 31) == 0;
+    bad_position = __reduce_min_sync(0xffffffffu, bad_position);
+    bad_normal = __reduce_min_sync(0xffffffffu, bad_normal);
+    if (first && bad_position != 0xffffffffu) atomicMin(&r->bad_position, bad_position);
+    if (first && bad_normal != 0xffffffffu) atomicMin(&r->bad_normal, bad_normal);
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t l = __reduce_min_sync(0xffffffffu, key_of(__float_as_uint(lo[k])));
+        const uint32_t h = __reduce_max_sync(0xffffffffu, key_of(__float_as_uint(hi[k])));
+        if (first) {
+            atomicMin(&r->lo[k], l);
+            atomicMax(&r->hi[k], h);
+        }
+    }
+}
+
+}  // namespace
+
+GeometryCheck check_geometry(const facetcu_vertex* d_vertices, uint64_t count, Workspace& ws,
+                             cudaStream_t s)
+{
+    ScratchBuffer buf(ws);
+    Result* d = static_cast<Result*>(buf.reserve(sizeof(Result)));
+    Result r;
+    std::memset(&r, 0xff, sizeof(r));
+    for (uint32_t& h : r.hi) h = 0;
+    FCU_CHECK(cudaMemcpyAsync(d, &r, sizeof(r), cudaMemcpyHostToDevice, s));
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const unsigned grid = unsigned(std::min<uint64_t>((count + 255) / 256, uint64_t(std::max(sms, 1)) * 8));
+    k_check_geometry<<<grid, 256, 0, s>>>(reinterpret_cast<const float*>(d_vertices), count, d);
+    FCU_LAUNCH("k_check_geometry");
+    FCU_CHECK(cudaMemcpyAsync(&r, d, sizeof(r), cudaMemcpyDeviceToHost, s));
+    FCU_CHECK(cudaStreamSynchronize(s));
+    GeometryCheck c;
+    c.bad_position = r.bad_position;
+    c.bad_normal = r.bad_normal;
+    for (int k = 0; k < 3; ++k) {
+        c.lo[k] = value_of(r.lo[k]);
+        c.hi[k] = value_of(r.hi[k]);
+    }
+    return c;
+}
+
+}  // namespace facetcu

@@ -154,7 +154,7 @@ void graph_from_pairs(uint64_t* d_pairs, size_t n, int side_bits, DeviceGraph& g
         u = size_t(total);
     }
     // unique keys go to `other`, their run starts reuse `heads` storage after compaction
-    DeviceBuffer upos_buf;
+    ScratchBuffer upos_buf(ws);
     uint32_t* upos = static_cast<uint32_t*>(upos_buf.reserve((u + 1) * 4));
     if (n) {
         k_compact_heads<<<grid(n, 256), 256, 0, s>>>(keys, n, heads, index, other, upos);
@@ -162,7 +162,7 @@ void graph_from_pairs(uint64_t* d_pairs, size_t n, int side_bits, DeviceGraph& g
     }
     const size_t m = 2 * u;
     if (m >= (1ull << 32)) throw Error(FACETCU_OVERFLOW_ERROR, "visibility graph exceeds 2^32 edges");
-    DeviceBuffer dk, dk2, dv, dv2;
+    ScratchBuffer dk(ws), dk2(ws), dv(ws), dv2(ws);
     uint64_t* dkeys = static_cast<uint64_t*>(dk.reserve((m + 1) * 8));
     uint64_t* dkeys2 = static_cast<uint64_t*>(dk2.reserve((m + 1) * 8));
     uint32_t* dvals = static_cast<uint32_t*>(dv.reserve((m + 1) * 4));

@@ -682,7 +682,7 @@ void hemisphere_graph(const facetcu_vertex* d_vertices, uint32_t facets, const L
     const uint32_t S = 2u * facets;
     top_k = std::min(top_k, rays);
     g.surfaces = S;
-    DeviceBuffer tmp, counters;
+    ScratchBuffer tmp(ws), counters(ws);
     uint2* tmp_edges = static_cast<uint2*>(tmp.reserve(size_t(S) * top_k * 8 + 8));
     uint32_t* rows = static_cast<uint32_t*>(g.row_offsets.reserve((size_t(S) + 1) * 4));
     uint32_t* den = static_cast<uint32_t*>(g.denominators.reserve(size_t(S) * 4));
@@ -701,7 +701,7 @@ void hemisphere_graph(const facetcu_vertex* d_vertices, uint32_t facets, const L
                                                       facets / (kBlocksPerSm * uint32_t(std::max(sms, 1)))}));
     // hit ids of a run of facets at a time
     const uint32_t run = std::min(facets, std::max(per_block, uint32_t((size_t(1) << 30) / (size_t(8) * rays)) / per_block * per_block));
-    DeviceBuffer traced_buf;
+    ScratchBuffer traced_buf(ws);
     uint32_t* traced = static_cast<uint32_t*>(traced_buf.reserve(size_t(run) * 2 * rays * 4));
     const size_t smem_trace = size_t(2) * (size_t(2) * per_block << shift);
     FCU_CHECK(cudaFuncSetAttribute(k_hemi_trace, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -746,10 +746,11 @@ void hemisphere_graph(const facetcu_vertex* d_vertices, uint32_t facets, const L
 
 void hemisphere_sunlit(const facetcu_vertex* d_vertices, uint32_t facets, const Lbvh& bvh,
                        const float* d_uv, uint32_t samples, uint32_t sets, float3 sun,
-                       const PeriodicTiles& periodic, float* d_fraction, cudaStream_t s)
+                       const PeriodicTiles& periodic, float* d_fraction, Workspace& ws,
+                       cudaStream_t s)
 {
     const uint32_t S = 2u * facets;
-    DeviceBuffer err;
+    ScratchBuffer err(ws);
     uint32_t* d_error = static_cast<uint32_t*>(err.reserve(16));
     FCU_CHECK(cudaMemsetAsync(d_error, 0, 16, s));
     k_hemi_sunlit<<<(facets * 32 + 255) / 256, 256, 0, s>>>(d_vertices, bvh.nodes.as<float4>(),

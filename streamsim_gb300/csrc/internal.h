@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <initializer_list>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -75,9 +76,93 @@ struct RasterFrame {
     float tile_dz[21];
 };
 
-// Scratch used by the device sort and scan.
+// Scratch used by the device sort and scan, and the blocks that builds borrow
+// (ScratchBuffer): kept for the next build up to kKeep bytes in all, given
+// back by release().  A context's work is on one stream, so a block may be
+// lent again as soon as it is handed back.
 struct Workspace {
     DeviceBuffer a, b, c, d, e;
+
+    static constexpr size_t kKeep = size_t(256) << 20;
+    struct Block {
+        void* ptr;
+        size_t bytes;
+    };
+    std::vector<Block> free_blocks;
+    size_t kept = 0;
+
+    Workspace() = default;
+    Workspace(const Workspace&) = delete;
+    Workspace& operator=(const Workspace&) = delete;
+    ~Workspace() { release(); }
+    Block borrow(size_t n)
+    {
+        // the smallest kept block that holds n bytes and is not far larger
+        size_t best = free_blocks.size();
+        for (size_t i = 0; i < free_blocks.size(); ++i)
+            if (free_blocks[i].bytes >= n && free_blocks[i].bytes <= 8 * n + 65536 &&
+                (best == free_blocks.size() || free_blocks[i].bytes < free_blocks[best].bytes))
+                best = i;
+        if (best < free_blocks.size()) {
+            const Block b = free_blocks[best];
+            free_blocks.erase(free_blocks.begin() + long(best));
+            kept -= b.bytes;
+            return b;
+        }
+        Block b{nullptr, n ? n : 16};
+        if (cudaMalloc(&b.ptr, b.bytes) == cudaErrorMemoryAllocation && kept) {
+            cudaGetLastError();
+            drop_blocks();  // make room
+            cuda_check(cudaMalloc(&b.ptr, b.bytes), "cudaMalloc");
+        } else if (!b.ptr) {
+            cudaGetLastError();
+            cuda_check(cudaMalloc(&b.ptr, b.bytes), "cudaMalloc");
+        }
+        return b;
+    }
+    void hand_back(const Block& b) noexcept
+    {
+        if (b.bytes <= kKeep / 4 && kept + b.bytes <= kKeep) {
+            try {
+                free_blocks.push_back(b);
+                kept += b.bytes;
+                return;
+            } catch (...) {
+            }
+        }
+        cudaFree(b.ptr);
+    }
+    void drop_blocks()
+    {
+        for (const Block& b : free_blocks) cudaFree(b.ptr);
+        free_blocks.clear();
+        kept = 0;
+    }
+    void release()
+    {
+        for (DeviceBuffer* x : {&a, &b, &c, &d, &e}) x->release();
+        drop_blocks();
+    }
+};
+
+// A device block borrowed from a workspace for one call.
+struct ScratchBuffer {
+    Workspace& ws;
+    Workspace::Block block{nullptr, 0};
+    explicit ScratchBuffer(Workspace& w) : ws(w) {}
+    ScratchBuffer(const ScratchBuffer&) = delete;
+    ScratchBuffer& operator=(const ScratchBuffer&) = delete;
+    ~ScratchBuffer()
+    {
+        if (block.ptr) ws.hand_back(block);
+    }
+    void* reserve(size_t n)
+    {
+        if (block.ptr) ws.hand_back(block);
+        block = {nullptr, 0};
+        block = ws.borrow(n);
+        return block.ptr;
+    }
 };
 
 // ---- device utilities (sort.cu) ----------------------------------------
@@ -125,10 +210,11 @@ void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t
                           RasterBuffers& rb, uint32_t* d_denominators, uint32_t* d_sky,
                           uint64_t* d_pairs, unsigned long long* d_pair_count, int side_bits,
                           RasterStats& stats, cudaStream_t s);
-// Resolve one direction's lists into sunlit total/visible counts.
+// Resolve one direction's lists into sunlit total/visible counts and their
+// ratio (0 where nothing was seen).
 void raster_resolve_sunlit(const RasterFrame& frame, uint32_t chain_cap, RasterBuffers& rb,
-                           uint32_t* d_total, uint32_t* d_visible, RasterStats& stats,
-                           cudaStream_t s);
+                           uint32_t* d_total, uint32_t* d_visible, float* d_fraction,
+                           RasterStats& stats, cudaStream_t s);
 
 // ---- one-column sweeps from shared memory (column.cu) --------------------
 // The edge words of a graph laid out by tiles of the column, and the sums of
@@ -288,7 +374,16 @@ void hemisphere_graph(const facetcu_vertex* d_vertices, uint32_t facets, const L
                       unsigned long long* dropped, Workspace& ws, cudaStream_t s);
 void hemisphere_sunlit(const facetcu_vertex* d_vertices, uint32_t facets, const Lbvh& bvh,
                        const float* d_uv, uint32_t samples, uint32_t sets, float3 sun,
-                       const PeriodicTiles& periodic, float* d_fraction, cudaStream_t s);
+                       const PeriodicTiles& periodic, float* d_fraction, Workspace& ws,
+                       cudaStream_t s);
+// First vertices with a non-finite position and with a normal that is not
+// normalized (~0: none), and the bounds of the positions (geometry.cu).
+struct GeometryCheck {
+    uint32_t bad_position, bad_normal;
+    float lo[3], hi[3];
+};
+GeometryCheck check_geometry(const facetcu_vertex* d_vertices, uint64_t count, Workspace& ws,
+                             cudaStream_t s);
 
 // ---- warm-start MLP (mlp.cu) -----------------------------------------------
 namespace mlp {

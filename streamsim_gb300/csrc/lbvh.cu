@@ -274,7 +274,7 @@ void lbvh_build(const facetcu_vertex* d_vertices, uint32_t n, Lbvh& bvh, Workspa
         sb.hi[a] = bvh.scene_max[a];
     }
     const float margin = 2.0f * bvh.hit_margin;
-    DeviceBuffer keys_a, keys_b, ids_a, ids_b, leaf_box, int_box, child, parent_int, parent_leaf;
+    ScratchBuffer keys_a(ws), keys_b(ws), ids_a(ws), ids_b(ws), leaf_box(ws), int_box(ws), child(ws), parent_int(ws), parent_leaf(ws);
     uint64_t* ka = static_cast<uint64_t*>(keys_a.reserve(size_t(n) * 8));
     uint64_t* kb = static_cast<uint64_t*>(keys_b.reserve(size_t(n) * 8));
     uint32_t* ia = static_cast<uint32_t*>(ids_a.reserve(size_t(n) * 4));
@@ -315,7 +315,7 @@ void morton_order(const facetcu_vertex* d_vertices, uint32_t n, const float lo[3
         sb.lo[a] = lo[a];
         sb.hi[a] = hi[a];
     }
-    DeviceBuffer keys_a, keys_b, ids_b, boxes;
+    ScratchBuffer keys_a(ws), keys_b(ws), ids_b(ws), boxes(ws);
     uint64_t* ka = static_cast<uint64_t*>(keys_a.reserve(size_t(n) * 8));
     uint64_t* kb = static_cast<uint64_t*>(keys_b.reserve(size_t(n) * 8));
     uint32_t* ia = d_order;

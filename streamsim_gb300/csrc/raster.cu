@@ -531,6 +531,12 @@ __global__ void __launch_bounds__(256) k_resolve_sunlit(const uint32_t* offsets,
     atomicAdd(&visible[frag_side(best.key, c_frame.facets)], 1u);
 }
 
+__global__ void k_fraction(uint32_t S, const uint32_t* total, const uint32_t* visible, float* out)
+{
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < S) out[s] = total[s] ? float(visible[s]) / float(total[s]) : 0.0f;
+}
+
 __global__ void k_set_last_offset(uint32_t* offsets, uint64_t n, const unsigned long long* total)
 {
     offsets[n] = uint32_t(*total);
@@ -621,8 +627,8 @@ void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t
 }
 
 void raster_resolve_sunlit(const RasterFrame& frame, uint32_t chain_cap, RasterBuffers& rb,
-                           uint32_t* d_total, uint32_t* d_visible, RasterStats& stats,
-                           cudaStream_t s)
+                           uint32_t* d_total, uint32_t* d_visible, float* d_fraction,
+                           RasterStats& stats, cudaStream_t s)
 {
     const uint64_t npix = uint64_t(frame.width) * frame.height;
     RasterStats* dstats = rb.stats.as<RasterStats>();
@@ -630,6 +636,9 @@ void raster_resolve_sunlit(const RasterFrame& frame, uint32_t chain_cap, RasterB
         rb.offsets.as<uint32_t>(), rb.records.as<uint64_t>(), npix, chain_cap,
         d_total, d_visible, dstats);
     FCU_LAUNCH("k_resolve_sunlit");
+    k_fraction<<<(2 * frame.facets + 255) / 256, 256, 0, s>>>(2 * frame.facets, d_total, d_visible,
+                                                              d_fraction);
+    FCU_LAUNCH("k_fraction");
     RasterStats host{};
     FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
     FCU_CHECK(cudaStreamSynchronize(s));
