@@ -370,8 +370,8 @@ int facetcu_destroy(facetcu_context* ctx)
     ctx->graph.p_scene.release();
     ctx->graph.column.release();
     ctx->graph_ready = false;
-    for (DeviceBuffer* b : {&ctx->raster.counts, &ctx->raster.offsets, &ctx->raster.records,
-                            &ctx->raster.big_list, &ctx->raster.deep_list, &ctx->raster.stats,
+    for (DeviceBuffer* b : {&ctx->raster.heads, &ctx->raster.nodes, &ctx->raster.planes,
+                            &ctx->raster.jobs, &ctx->raster.list, &ctx->raster.stats,
                             &ctx->pairs, &ctx->pair_count, &ctx->denom_tmp, &ctx->optics, &ctx->rad_a,
                             &ctx->rad_b, &ctx->residual, &ctx->host_io, &ctx->scratch,
                             &ctx->sun_total, &ctx->sun_visible, &ctx->batch.x0, &ctx->batch.x1,
@@ -492,14 +492,16 @@ int facetcu_build_visibility_graph(facetcu_context* ctx, const facetcu_direction
         g.surfaces = S;
         uint32_t* denom = static_cast<uint32_t*>(g.denominators.reserve(size_t(S) * 4));
         uint32_t* sky = static_cast<uint32_t*>(g.sky.reserve(size_t(S) * 4));
-        FCU_CHECK(cudaMemsetAsync(denom, 0, size_t(S) * 4, s));
+        uint32_t* frags = static_cast<uint32_t*>(ctx->denom_tmp.reserve(size_t(S) * 4));
+        FCU_CHECK(cudaMemsetAsync(frags, 0, size_t(S) * 4, s));
         FCU_CHECK(cudaMemsetAsync(sky, 0, size_t(S) * 4, s));
         unsigned long long* pair_count =
             static_cast<unsigned long long*>(ctx->pair_count.reserve(16));
         FCU_CHECK(cudaMemsetAsync(pair_count, 0, 8, s));
-        // directions per chunk: keep the per-pixel count/offset arrays near 1 GiB
+        // directions per chunk: keep the per-pixel arrays (4 bytes a pixel and
+        // the pool's first 8) near 1 GiB
         const uint64_t pixels = uint64_t(frame.width) * frame.height;
-        uint32_t chunk = uint32_t(std::max<uint64_t>(1, (1ull << 30) / (8 * pixels)));
+        uint32_t chunk = uint32_t(std::max<uint64_t>(1, (1ull << 30) / (12 * pixels)));
         chunk = std::min<uint32_t>(std::min<uint32_t>(chunk, 64u), direction_count);
         uint64_t overflow = 0, pairs_used = 0, pairs_cap = ctx->pairs.bytes / 8;
         uint32_t capacity_error = 0, max_chain = 0;
@@ -507,7 +509,7 @@ int facetcu_build_visibility_graph(facetcu_context* ctx, const facetcu_direction
             const uint32_t n = std::min(chunk, direction_count - d0);
             RasterStats st{};
             raster_fragments(ctx->vertices.as<facetcu_vertex>(), frame, views.data() + d0, n,
-                             ctx->raster, ctx->ws, st, s);
+                             ctx->raster, frags, st, s);
             // pairs of this chunk are at most the fragments of it
             const uint64_t need = pairs_used + st.fragments + 1;
             if (need > pairs_cap) {
@@ -521,7 +523,7 @@ int facetcu_build_visibility_graph(facetcu_context* ctx, const facetcu_direction
                 std::swap(ctx->pairs.bytes, grown.bytes);
                 pairs_cap = ctx->pairs.bytes / 8;
             }
-            raster_resolve_graph(frame, n, chain_cap(ctx), ctx->raster, denom, sky,
+            raster_resolve_graph(frame, n, chain_cap(ctx), ctx->raster, sky,
                                  ctx->pairs.as<uint64_t>(), pair_count, side_bits, st, s);
             unsigned long long used = 0;
             FCU_CHECK(cudaMemcpyAsync(&used, pair_count, 8, cudaMemcpyDeviceToHost, s));
@@ -531,6 +533,7 @@ int facetcu_build_visibility_graph(facetcu_context* ctx, const facetcu_direction
             capacity_error += st.capacity_error;
             max_chain = std::max(max_chain, st.max_chain);
         }
+        raster_denominators(ctx->facets, frags, denom, s);
         facetcu_graph_diagnostics diag{};
         diag.facet_count = ctx->facets;
         diag.surface_count = S;
@@ -573,12 +576,12 @@ int facetcu_compute_sunlit_fraction(facetcu_context* ctx, const facetcu_directio
         const RasterFrame frame = make_frame(ctx);
         cudaStream_t s = ctx->stream;
         RasterStats st{};
-        raster_fragments(ctx->vertices.as<facetcu_vertex>(), frame, &view, 1, ctx->raster, ctx->ws,
-                         st, s);
         uint32_t* total = static_cast<uint32_t*>(ctx->sun_total.reserve(size_t(S) * 4));
         uint32_t* visible = static_cast<uint32_t*>(ctx->sun_visible.reserve(size_t(S) * 4));
         FCU_CHECK(cudaMemsetAsync(total, 0, size_t(S) * 4, s));
         FCU_CHECK(cudaMemsetAsync(visible, 0, size_t(S) * 4, s));
+        raster_fragments(ctx->vertices.as<facetcu_vertex>(), frame, &view, 1, ctx->raster, total, st,
+                         s);
         float* d_fraction = static_cast<float*>(ctx->fraction.reserve(size_t(S) * 4));
         raster_resolve_sunlit(frame, chain_cap(ctx), ctx->raster, total, visible, d_fraction, st, s);
         if (st.overflow)

@@ -179,41 +179,45 @@ void radix_sort_u64(uint64_t*& keys, uint64_t*& keys_alt, uint32_t*& values,
 
 // ---- raster visibility (raster.cu) --------------------------------------
 struct RasterBuffers {
-    DeviceBuffer counts;    // dirs * pixels
-    DeviceBuffer offsets;   // dirs * pixels + 1
-    DeviceBuffer records;   // fragments (u64: depth bits << 32 | key)
-    DeviceBuffer big_list;  // large-triangle work items
-    DeviceBuffer deep_list; // pixels with more than the fast-path chain
-    DeviceBuffer stats;     // small counters
+    DeviceBuffer heads;   // dirs * pixels: 1 + the newest node of the pixel's list, or 0
+    DeviceBuffer nodes;   // fragments (depth bits, key, the older node)
+    DeviceBuffer planes;  // facets as three planes of float4
+    DeviceBuffer jobs;    // triangles for warps (from the front) and blocks (from the back)
+    DeviceBuffer list;    // pixels with more than the register path's chain
+    DeviceBuffer stats;   // RasterStats
 };
 
 struct RasterStats {
     unsigned long long fragments;
     unsigned long long overflow;   // sum over pixels of max(0, count - cap)
-    unsigned long long pairs;
-    unsigned int big;
-    unsigned int deep;
+    unsigned int mid, big;         // triangles listed for warps and for blocks
+    unsigned int listed;           // pixels in RasterBuffers::list
     unsigned int capacity_error;
     unsigned int max_chain;
 };
 
-// Rasterise `dir_count` directions (views[0..dir_count)) into exact-size
-// per-pixel fragment lists.  Leaves counts/offsets/records filled.
+// Rasterise `dir_count` directions (views[0..dir_count)) into per-pixel lists
+// of fragments (heads, nodes), and add the fragments of every facet to
+// d_frags[2 facet + (camera-side flip)].
 void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame,
                       const RasterView* views, uint32_t dir_count, RasterBuffers& rb,
-                      Workspace& ws, RasterStats& stats, cudaStream_t s);
-// Resolve the lists of a chunk into denominators, sky counts and pair keys
+                      uint32_t* d_frags, RasterStats& stats, cudaStream_t s);
+// Denominators of both sides of every facet from d_frags.
+void raster_denominators(uint32_t facets, const uint32_t* d_frags, uint32_t* d_denominators,
+                         cudaStream_t s);
+// Resolve the lists of a chunk (stats as raster_fragments left it) into sky
+// counts and pair keys
 // (lo << side_bits | hi), appended at pairs[pair_count..].
 // chain_cap = the reference's maxFragmentsPerPixel: longer chains count as
 // fragment overflow (UINT32_MAX = no limit).
 void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t chain_cap,
-                          RasterBuffers& rb, uint32_t* d_denominators, uint32_t* d_sky,
-                          uint64_t* d_pairs, unsigned long long* d_pair_count, int side_bits,
-                          RasterStats& stats, cudaStream_t s);
-// Resolve one direction's lists into sunlit total/visible counts and their
-// ratio (0 where nothing was seen).
+                          RasterBuffers& rb, uint32_t* d_sky, uint64_t* d_pairs,
+                          unsigned long long* d_pair_count, int side_bits, RasterStats& stats,
+                          cudaStream_t s);
+// Resolve one direction's lists into visible counts per side, and their ratio
+// to the totals (the raster's d_frags; 0 where there are none).
 void raster_resolve_sunlit(const RasterFrame& frame, uint32_t chain_cap, RasterBuffers& rb,
-                           uint32_t* d_total, uint32_t* d_visible, float* d_fraction,
+                           const uint32_t* d_total, uint32_t* d_visible, float* d_fraction,
                            RasterStats& stats, cudaStream_t s);
 
 // ---- one-column sweeps from shared memory (column.cu) --------------------

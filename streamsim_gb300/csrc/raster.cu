@@ -14,17 +14,33 @@
 //     chains replay the introsort step for step.
 //
 // GB300 layout: instead of a fixed W x H x L A-buffer (512 MB per direction
-// at 1024^2 x 64) the raster runs twice — count, exclusive scan, fill — into
-// exact-size per-pixel lists for a whole chunk of directions at once, so a
-// single launch covers all 40 directions and HBM holds only real fragments.
+// at 1024^2 x 64) every pixel heads a list of its fragments, in one pool for a
+// whole chunk of directions, so a single launch covers all 40 directions, each
+// triangle is rasterised once, and HBM holds only real fragments.  A block
+// takes its room in the pool with one atomic.  A pool that turns out too small
+// is grown to the exact number and the chunk rasterised again.  A facet's
+// fragments are counted by the threads that rasterise it, not fragment by
+// fragment when the lists are resolved.
 #include "internal.h"
 
 namespace facetcu {
 namespace {
 
-constexpr uint32_t kBigPixels = 1024;  // bbox area above which a CTA takes the triangle
-constexpr uint32_t kFastChain = 64;    // per-thread chain capacity of the main resolve
+// Who takes a triangle, by the area of its bounding box.  Build of the graph,
+// us, 4,096 facets of terrain (boxes of some 500 pixels) / 200,000 facets of
+// forest (most below 10, the ground's about 100), 40 directions of 1024^2:
+//   a thread up to 8, 16, 32 pixels:  925 / 5288,  929 / 2095,  876 / 2005
+//   above, 4, 8, 16, 32 lanes:        839 / 1709,  848 / 1777,  870 / 1904,
+//                                     894 / 2194
+// and the one direction of the sun pass with 4, 8, 32 lanes: 144 / 157,
+// 121 / 155, 110 / 169.
+constexpr uint32_t kSmallPixels = 32;  // (a thread's covered pixels are bits of a word)
+constexpr uint32_t kMidLanes = 8;
+constexpr uint32_t kBigPixels = 1024;  // above: blocks
+constexpr int kFast = 8;               // chains ordered in registers
+constexpr uint32_t kMidChain = 64;     // per-thread chain capacity of the middle resolve
 constexpr uint32_t kDeepChain = 1024;  // capacity of the deep-chain resolve
+constexpr uint32_t kResolvePixels = 2048;  // pixels of a resolving block
 constexpr uint32_t kKeyMask = 0x7fffffffu;
 
 __constant__ RasterView c_views[64];
@@ -40,24 +56,70 @@ __device__ __forceinline__ float dot3(const float a[3], float b0, float b1, floa
 }
 
 // facetrtcore.cpp:1259-1275
-__device__ __forceinline__ void project(const facetcu_vertex* V, uint32_t f, uint32_t tile,
-                                        const RasterView& v, Projected& p, uint32_t& flip)
+__device__ __forceinline__ void project_vertex(float px, float py, float pz, uint32_t tile,
+                                               const RasterView& v, float& x, float& y, float& d)
 {
-    const float ox = c_frame.tile_dx[tile], oz = c_frame.tile_dz[tile];
     const float r = c_frame.radius;
-    const float w = float(c_frame.width), h = float(c_frame.height);
+    const float rx = (px + c_frame.tile_dx[tile]) - c_frame.center[0];
+    const float ry = py - c_frame.center[1];
+    const float rz = (pz + c_frame.tile_dz[tile]) - c_frame.center[2];
+    x = (0.5f + 0.5f * dot3(v.right, rx, ry, rz) / r) * float(c_frame.width);
+    y = (0.5f + 0.5f * dot3(v.up, rx, ry, rz) / r) * float(c_frame.height);
+    d = 0.5f - dot3(v.view, rx, ry, rz) / (2.0f * r);
+}
+
+// The triangles as three planes of 16 bytes a facet (corners, then the first
+// corner's normal): a warp of facets reads them in 12 wavefronts, where the
+// vertices' 24-byte records take some 200 and bounded the raster of 200,000
+// facets.
+__global__ void k_planes(const facetcu_vertex* __restrict__ V, uint32_t facets,
+                         float4* __restrict__ planes)
+{
+    const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= facets) return;
+    const facetcu_vertex &a = V[3 * f], &b = V[3 * f + 1], &c = V[3 * f + 2];
+    planes[f] = make_float4(a.position[0], a.position[1], a.position[2], b.position[0]);
+    planes[facets + f] = make_float4(b.position[1], b.position[2], c.position[0], c.position[1]);
+    planes[2 * size_t(facets) + f] =
+        make_float4(c.position[2], a.normal[0], a.normal[1], a.normal[2]);
+}
+
+struct Facet {
+    float4 q0, q1, q2;
+};
+__device__ __forceinline__ Facet load_facet(const float4* planes, uint32_t f)
+{
+    const size_t F = c_frame.facets;
+    return {__ldg(planes + f), __ldg(planes + F + f), __ldg(planes + 2 * F + f)};
+}
+__device__ __forceinline__ uint32_t facing(const Facet& t, const RasterView& v)
+{
+    return dot3(v.view, t.q2.y, t.q2.z, t.q2.w) >= 0.0f ? 0u : 1u;
+}
+__device__ __forceinline__ void project(const Facet& t, uint32_t tile, const RasterView& v,
+                                        Projected& p)
+{
+    project_vertex(t.q0.x, t.q0.y, t.q0.z, tile, v, p.x[0], p.y[0], p.d[0]);
+    project_vertex(t.q0.w, t.q1.x, t.q1.y, tile, v, p.x[1], p.y[1], p.d[1]);
+    project_vertex(t.q1.z, t.q1.w, t.q2.x, tile, v, p.x[2], p.y[2], p.d[2]);
+}
+// The same by kLanes lanes: they take a corner each and exchange.
+template <uint32_t kLanes>
+__device__ __forceinline__ void project_lanes(const Facet& t, uint32_t tile, const RasterView& v,
+                                             Projected& p)
+{
+    const uint32_t c = (threadIdx.x % kLanes) % 3u;
+    const float px = c == 0u ? t.q0.x : c == 1u ? t.q0.w : t.q1.z;
+    const float py = c == 0u ? t.q0.y : c == 1u ? t.q1.x : t.q1.w;
+    const float pz = c == 0u ? t.q0.z : c == 1u ? t.q1.y : t.q2.x;
+    float x, y, d;
+    project_vertex(px, py, pz, tile, v, x, y, d);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const facetcu_vertex& vx = V[3 * f + c];
-        const float rx = (vx.position[0] + ox) - c_frame.center[0];
-        const float ry = vx.position[1] - c_frame.center[1];
-        const float rz = (vx.position[2] + oz) - c_frame.center[2];
-        p.x[c] = (0.5f + 0.5f * dot3(v.right, rx, ry, rz) / r) * w;
-        p.y[c] = (0.5f + 0.5f * dot3(v.up, rx, ry, rz) / r) * h;
-        p.d[c] = 0.5f - dot3(v.view, rx, ry, rz) / (2.0f * r);
+    for (int k = 0; k < 3; ++k) {
+        p.x[k] = __shfl_sync(0xffffffffu, x, k, kLanes);
+        p.y[k] = __shfl_sync(0xffffffffu, y, k, kLanes);
+        p.d[k] = __shfl_sync(0xffffffffu, d, k, kLanes);
     }
-    const facetcu_vertex& v0 = V[3 * f];
-    flip = dot3(v.view, v0.normal[0], v0.normal[1], v0.normal[2]) >= 0.0f ? 0u : 1u;
 }
 
 // edge() of facetrtcore.cpp:1287-1290, argument order kept.
@@ -117,85 +179,278 @@ __device__ __forceinline__ bool cover(const Projected& p, float area, int x, int
     return true;
 }
 
-struct ItemRef {
-    uint32_t dir, tile, facet;
-};
-
-__device__ __forceinline__ ItemRef decode_item(uint64_t w)
+__device__ __forceinline__ bool inside(const Projected& p, float area, int x, int y)
 {
-    const uint64_t per_dir = uint64_t(c_frame.tiles) * c_frame.facets;
-    ItemRef r;
-    r.dir = uint32_t(w / per_dir);
-    const uint64_t rem = w - uint64_t(r.dir) * per_dir;
-    r.tile = uint32_t(rem / c_frame.facets);
-    r.facet = uint32_t(rem - uint64_t(r.tile) * c_frame.facets);
-    return r;
+    float unused;
+    return cover(p, area, x, y, unused);
 }
 
-// Count (kFill = false) or fill (kFill = true) the fragments of one
-// triangle; big triangles are queued for the CTA kernel in the count pass.
-template <bool kFill>
-__global__ void __launch_bounds__(256) k_raster_small(const facetcu_vertex* V, uint64_t items,
-                                                      uint32_t* counts, const uint32_t* offsets,
-                                                      uint64_t* records, uint32_t* big_list,
-                                                      uint32_t* big_count)
+struct Pool {
+    uint32_t* heads;                 // per pixel: 1 + its newest node, or 0
+    uint4* nodes;                    // depth bits, key, the older node (1 + index, or 0)
+    uint64_t capacity;
+    unsigned long long* used;        // also counts what found no room
+};
+
+__device__ __forceinline__ void put(const Pool& pool, size_t pix, uint64_t slot, float depth,
+                                    uint32_t key)
 {
-    const uint64_t w = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (w >= items) return;
-    const ItemRef it = decode_item(w);
-    Projected p;
-    uint32_t flip;
-    project(V, it.facet, it.tile, c_views[it.dir], p, flip);
-    const Bbox b = triangle_bbox(p);
-    if (!b.valid) return;
-    const uint32_t area_px = uint32_t(b.x1 - b.x0 + 1) * uint32_t(b.y1 - b.y0 + 1);
-    if (area_px > kBigPixels) {
-        if (!kFill) big_list[atomicAdd(big_count, 1u)] = uint32_t(w);
-        return;
+    if (slot >= pool.capacity) return;
+    const uint32_t older = atomicExch(&pool.heads[pix], uint32_t(slot) + 1u);
+    pool.nodes[slot] = make_uint4(__float_as_uint(depth), key, older, 0u);
+}
+
+// Room in the pool for `mine` fragments of each warp of the block, one atomic
+// per block (a single counter takes about one atomic a clock).  All threads
+// call; `mine` is the warp's.
+struct Room {
+    uint32_t warp[8];
+    unsigned long long base;
+};
+__device__ __forceinline__ uint64_t take_room(Room& r, uint32_t mine, unsigned long long* counter)
+{
+    const uint32_t warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31u) == 0u) r.warp[warp] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t all = 0;
+        for (int w = 0; w < 8; ++w) all += r.warp[w];
+        r.base = all ? atomicAdd(counter, (unsigned long long)all) : 0ull;
     }
-    const size_t plane = size_t(it.dir) * c_frame.width * c_frame.height;
-    const uint32_t key = (it.tile * c_frame.facets + it.facet) | (flip << 31);
-    for (int y = b.y0; y <= b.y1; ++y) {
-        for (int x = b.x0; x <= b.x1; ++x) {
-            float depth;
-            if (!cover(p, b.area, x, y, depth)) continue;
-            const size_t pix = plane + size_t(y) * c_frame.width + size_t(x);
-            if (!kFill) {
-                atomicAdd(&counts[pix], 1u);
-            } else {
-                const uint32_t slot = offsets[pix] + atomicAdd(&counts[pix], 1u);
-                records[slot] = (uint64_t(__float_as_uint(depth)) << 32) | key;
+    __syncthreads();
+    uint64_t base = r.base;
+    for (uint32_t w = 0; w < warp; ++w) base += r.warp[w];
+    return base;
+}
+
+__device__ __forceinline__ uint32_t scan_inclusive(uint32_t v)
+{
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31u) >= uint32_t(o)) v += y;
+    }
+    return v;
+}
+
+// A triangle, tile and direction (blockIdx.y) per thread.  Boxes of up to
+// kSmallPixels pixels are done here: one thread walking a box of hundreds waits
+// for as many atomics in turn.  Larger ones are listed, for some lanes each
+// from the front of `jobs` and for whole blocks from its back.
+// Bound by instructions (69 % of the issue slots; nine IEEE divides to project
+// a triangle): 351 us for the 8 M triangles of the forest, where counting and
+// filling in two passes took 268 + 448.
+__global__ void __launch_bounds__(256) k_raster(const float4* __restrict__ planes, uint32_t per_dir,
+                                                Pool pool, uint32_t* jobs, uint32_t items,
+                                                RasterStats* stats, uint32_t* frags)
+{
+    __shared__ Room room;
+    __shared__ uint32_t warp_mid[8], warp_big[8], base_mid, base_big;
+    const uint32_t w = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31u,
+                   warp = threadIdx.x >> 5;
+    const uint32_t item = blockIdx.y * per_dir + w;
+    Projected p;
+    Bbox b;
+    b.valid = false;
+    uint32_t box = 0, side = 0, key = 0, mask = 0;
+    if (w < per_dir) {
+        const uint32_t tile = c_frame.tiles == 1u ? 0u : w / c_frame.facets;
+        const uint32_t facet = w - tile * c_frame.facets;
+        const Facet t = load_facet(planes, facet);
+        const uint32_t flip = facing(t, c_views[blockIdx.y]);
+        project(t, tile, c_views[blockIdx.y], p);
+        b = triangle_bbox(p);
+        key = w | (flip << 31);
+        side = 2u * facet + flip;
+        if (b.valid) box = uint32_t(b.x1 - b.x0 + 1) * uint32_t(b.y1 - b.y0 + 1);
+        if (box <= kSmallPixels && b.valid) {
+            uint32_t bit = 1u;
+            for (int y = b.y0; y <= b.y1; ++y)
+                for (int x = b.x0; x <= b.x1; ++x, bit <<= 1)
+                    if (inside(p, b.area, x, y)) mask |= bit;
+        }
+    }
+    const uint32_t n = __popc(mask);
+    if (n && frags) atomicAdd(&frags[side], n);
+    const uint32_t incl = scan_inclusive(n);
+    const uint32_t mid = __ballot_sync(0xffffffffu, box > kSmallPixels && box <= kBigPixels);
+    const uint32_t big = __ballot_sync(0xffffffffu, box > kBigPixels);
+    if (lane == 0) {
+        warp_mid[warp] = __popc(mid);
+        warp_big[warp] = __popc(big);
+    }
+    uint64_t slot = take_room(room, __shfl_sync(0xffffffffu, incl, 31), pool.used) + (incl - n);
+    if (threadIdx.x < 2) {
+        const uint32_t* from = threadIdx.x ? warp_big : warp_mid;
+        uint32_t all = 0;
+        for (int k = 0; k < 8; ++k) all += from[k];
+        if (all) all = atomicAdd(threadIdx.x ? &stats->big : &stats->mid, all);
+        (threadIdx.x ? base_big : base_mid) = all;
+    }
+    if (mask) {
+        const size_t plane = size_t(blockIdx.y) * c_frame.width * c_frame.height;
+        for (int y = b.y0; y <= b.y1; ++y) {
+            for (int x = b.x0; x <= b.x1; ++x, mask >>= 1) {
+                if (!(mask & 1u)) continue;
+                float depth;
+                cover(p, b.area, x, y, depth);
+                put(pool, plane + size_t(y) * c_frame.width + size_t(x), slot++, depth, key);
             }
         }
     }
+    __syncthreads();
+    if (box <= kSmallPixels) return;
+    const bool whole = box > kBigPixels;
+    const uint32_t before = (whole ? big : mid) & ((1u << lane) - 1u);
+    uint32_t at = (whole ? base_big : base_mid) + uint32_t(__popc(before));
+    for (uint32_t k = 0; k < warp; ++k) at += whole ? warp_big[k] : warp_mid[k];
+    jobs[whole ? items - 1u - at : at] = item;
 }
 
-template <bool kFill>
-__global__ void __launch_bounds__(256) k_raster_big(const facetcu_vertex* V,
-                                                    const uint32_t* big_list, uint32_t* counts,
-                                                    const uint32_t* offsets, uint64_t* records)
+// kLanes lanes' share of a listed triangle: pixels [first, first + count) of
+// its box, at most 32 kLanes, so that a lane's covered ones are the bits of a
+// word.  Called by all threads of the block (count 0 where there is none).
+// The atomics of four steps are in flight together.
+template <uint32_t kLanes>
+__device__ __forceinline__ void raster_span(const Projected& p, const Bbox& b, size_t plane,
+                                            uint32_t key, uint32_t first, uint32_t count,
+                                            const Pool& pool, Room& room, uint32_t* count_at)
 {
-    const uint64_t w = big_list[blockIdx.x];
-    const ItemRef it = decode_item(w);
-    Projected p;
-    uint32_t flip;
-    project(V, it.facet, it.tile, c_views[it.dir], p, flip);
-    const Bbox b = triangle_bbox(p);
-    const uint32_t bw = uint32_t(b.x1 - b.x0 + 1), bh = uint32_t(b.y1 - b.y0 + 1);
-    const size_t plane = size_t(it.dir) * c_frame.width * c_frame.height;
-    const uint32_t key = (it.tile * c_frame.facets + it.facet) | (flip << 31);
-    for (uint32_t i = threadIdx.x; i < bw * bh; i += blockDim.x) {
-        const int x = b.x0 + int(i % bw), y = b.y0 + int(i / bw);
-        float depth;
-        if (!cover(p, b.area, x, y, depth)) continue;
-        const size_t pix = plane + size_t(y) * c_frame.width + size_t(x);
-        if (!kFill) {
-            atomicAdd(&counts[pix], 1u);
-        } else {
-            const uint32_t slot = offsets[pix] + atomicAdd(&counts[pix], 1u);
-            records[slot] = (uint64_t(__float_as_uint(depth)) << 32) | key;
+    const uint32_t lane = threadIdx.x & 31u, sub = lane % kLanes;
+    const uint32_t bw = count ? uint32_t(b.x1 - b.x0 + 1) : 1u;
+    const uint32_t steps = (count + kLanes - 1u) / kLanes;
+    const uint32_t col0 = (first + sub) % bw, row0 = (first + sub) / bw;
+    const uint32_t step_x = kLanes % bw, step_y = kLanes / bw;
+    uint32_t mask = 0;
+    uint32_t cx = col0, cy = row0;
+    for (uint32_t r = 0; r < steps; ++r) {
+        if (r * kLanes + sub < count && inside(p, b.area, b.x0 + int(cx), b.y0 + int(cy)))
+            mask |= 1u << r;
+        cx += step_x;
+        cy += step_y;
+        if (cx >= bw) {
+            cx -= bw;
+            ++cy;
         }
     }
+    __syncwarp();
+    uint32_t n = __popc(mask);
+#pragma unroll
+    for (uint32_t o = 1; o < kLanes; o <<= 1) n += __shfl_xor_sync(0xffffffffu, n, int(o));
+    if (sub == 0 && n && count_at) atomicAdd(count_at, n);
+#pragma unroll
+    for (uint32_t o = kLanes; o < 32u; o <<= 1) n += __shfl_xor_sync(0xffffffffu, n, int(o));
+    uint64_t slot = take_room(room, n, pool.used);
+    const uint32_t most = __reduce_max_sync(0xffffffffu, steps);
+    cx = col0;
+    cy = row0;
+    for (uint32_t r = 0; r < most; r += 4) {
+        uint32_t older[4];
+        float depth[4];
+        uint64_t at[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            const bool on = r + k < steps && (mask >> (r + k)) & 1u;
+            const uint32_t lanes = __ballot_sync(0xffffffffu, on);
+            at[k] = on ? slot + uint32_t(__popc(lanes & ((1u << lane) - 1u))) : ~0ull;
+            slot += uint32_t(__popc(lanes));
+            if (at[k] < pool.capacity) {
+                const int x = b.x0 + int(cx), y = b.y0 + int(cy);
+                cover(p, b.area, x, y, depth[k]);
+                older[k] = atomicExch(&pool.heads[plane + size_t(y) * c_frame.width + size_t(x)],
+                                      uint32_t(at[k]) + 1u);
+            }
+            cx += step_x;
+            cy += step_y;
+            if (cx >= bw) {
+                cx -= bw;
+                ++cy;
+            }
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+            if (at[k] < pool.capacity)
+                pool.nodes[at[k]] = make_uint4(__float_as_uint(depth[k]), key, older[k], 0u);
+    }
+    __syncthreads();  // room is free again
+}
+
+struct Job {
+    Projected p;
+    Bbox b;
+    size_t plane;
+    uint32_t key, side;
+};
+template <uint32_t kLanes>
+__device__ __forceinline__ void load_job(const float4* planes, uint32_t per_dir, uint32_t item,
+                                         Job& j)
+{
+    const uint32_t dir = item / per_dir, w = item - dir * per_dir;
+    const uint32_t tile = w / c_frame.facets, facet = w - tile * c_frame.facets;
+    const Facet t = load_facet(planes, facet);
+    const uint32_t flip = facing(t, c_views[dir]);
+    project_lanes<kLanes>(t, tile, c_views[dir], j.p);
+    j.b = triangle_bbox(j.p);
+    j.plane = size_t(dir) * c_frame.width * c_frame.height;
+    j.key = w | (flip << 31);
+    j.side = 2u * facet + flip;
+}
+
+// Bound by instructions and the latency of its rounds (issue 57 %): 323 us for
+// the forest's 0.8 M ground triangles, 190 us for the terrain's 164,000, which
+// took 160 + 495 in two passes of a thread each.
+template <uint32_t kLanes>
+__global__ void __launch_bounds__(256) k_raster_mid(const float4* __restrict__ planes,
+                                                    uint32_t per_dir, Pool pool,
+                                                    const uint32_t* __restrict__ jobs,
+                                                    const uint32_t* __restrict__ job_count,
+                                                    uint32_t* frags)
+{
+    __shared__ Room room;
+    const uint32_t count = *job_count;
+    constexpr uint32_t kJobs = 256 / kLanes, kSpan = 32 * kLanes;
+    for (uint32_t k = blockIdx.x * kJobs; k < count; k += gridDim.x * kJobs) {
+        const uint32_t mine = k + threadIdx.x / kLanes;
+        Job j;
+        load_job<kLanes>(planes, per_dir, jobs[mine < count ? mine : k], j);
+        const uint32_t box = mine < count ? uint32_t(j.b.x1 - j.b.x0 + 1) *
+                                                uint32_t(j.b.y1 - j.b.y0 + 1) : 0u;
+        for (uint32_t first = 0; __syncthreads_or(int(first < box)); first += kSpan)
+            raster_span<kLanes>(j.p, j.b, j.plane, j.key, first,
+                                first < box ? min(box - first, kSpan) : 0u, pool, room,
+                                frags ? frags + j.side : nullptr);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_raster_big(const float4* __restrict__ planes,
+                                                    uint32_t per_dir, Pool pool,
+                                                    const uint32_t* __restrict__ jobs_end,
+                                                    const uint32_t* __restrict__ job_count,
+                                                    uint32_t* frags)
+{
+    __shared__ Room room;
+    const uint32_t count = *job_count, warp = threadIdx.x >> 5;
+    for (uint32_t k = blockIdx.x; k < count; k += gridDim.x) {
+        Job j;
+        load_job<32>(planes, per_dir, *(jobs_end - 1 - k), j);
+        const uint32_t box = uint32_t(j.b.x1 - j.b.x0 + 1) * uint32_t(j.b.y1 - j.b.y0 + 1);
+        for (uint32_t f = blockIdx.y * 8 * kBigPixels; f < box; f += gridDim.y * 8 * kBigPixels) {
+            const uint32_t first = f + warp * kBigPixels;
+            raster_span<32>(j.p, j.b, j.plane, j.key, first < box ? first : 0u,
+                        first < box ? min(box - first, kBigPixels) : 0u, pool, room,
+                        frags ? frags + j.side : nullptr);
+        }
+    }
+}
+
+// Both sides of a facet have the denominator of all its fragments.
+__global__ void k_denominators(uint32_t facets, const uint2* __restrict__ frags,
+                               uint2* __restrict__ denom)
+{
+    const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= facets) return;
+    const uint32_t n = frags[f].x + frags[f].y;
+    denom[f] = make_uint2(n, n);
 }
 
 // ---- per-pixel ordering ------------------------------------------------------
@@ -402,17 +657,11 @@ __device__ __forceinline__ uint32_t frag_side(uint32_t key, uint32_t facets)
     return 2u * (order % facets) + (key >> 31);
 }
 
-// Emit denominators, sky counts and adjacent pairs of an ordered chain
+// Emit sky counts and adjacent pairs of an ordered chain
 // (facetrtcore.cpp:1374-1392; visibility_resolve.comp:102-116).
-__device__ void emit_chain(const Frag* f, int n, uint32_t facets, uint32_t* denom, uint32_t* sky,
-                           uint64_t* pairs, unsigned long long* pair_count, int side_bits,
-                           bool warp_aggregate)
+__device__ void emit_chain(const Frag* f, int n, uint32_t facets, uint32_t* sky, uint64_t* pairs,
+                           unsigned long long* pair_count, int side_bits)
 {
-    for (int i = 0; i < n; ++i) {
-        const uint32_t s = frag_side(f[i].key, facets);
-        atomicAdd(&denom[s], 1u);
-        atomicAdd(&denom[s ^ 1u], 1u);
-    }
     if (n > 0) {
         atomicAdd(&sky[frag_side(f[0].key, facets)], 1u);
         atomicAdd(&sky[frag_side(f[n - 1].key, facets) ^ 1u], 1u);
@@ -424,24 +673,7 @@ __device__ void emit_chain(const Frag* f, int n, uint32_t facets, uint32_t* deno
         if ((a >> 1) != (b >> 1)) ++np;
     }
     unsigned long long base = 0;
-    if (warp_aggregate) {
-        // called by all 32 lanes of the warp (threads without a chain pass n = 0)
-        __syncwarp();
-        const unsigned lane = threadIdx.x & 31u;
-        unsigned incl = np;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= unsigned(o)) incl += y;
-        }
-        const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
-        unsigned long long b0 = 0;
-        if (lane == 31u && total) b0 = atomicAdd(pair_count, (unsigned long long)total);
-        b0 = __shfl_sync(0xffffffffu, b0, 31);
-        base = b0 + (incl - np);
-    } else if (np) {
-        base = atomicAdd(pair_count, (unsigned long long)np);
-    }
+    if (np) base = atomicAdd(pair_count, (unsigned long long)np);
     uint32_t k = 0;
     for (int i = 0; i + 1 < n; ++i) {
         const uint32_t a = frag_side(f[i].key, facets) ^ 1u;
@@ -453,82 +685,274 @@ __device__ void emit_chain(const Frag* f, int n, uint32_t facets, uint32_t* deno
     }
 }
 
-__device__ __forceinline__ Frag unpack(uint64_t r)
+// A fragment as a number whose order is the chain's: depth, then append order
+// (frag_less_stable); the flip bit lies below both.
+__device__ __forceinline__ uint64_t chain_key(const uint4& node)
 {
-    Frag f;
-    f.depth = __uint_as_float(uint32_t(r >> 32));
-    f.key = uint32_t(r);
-    return f;
+    const uint32_t bits = __float_as_uint(__uint_as_float(node.x) + 0.0f);  // -0 is 0
+    const uint32_t depth = bits & 0x80000000u ? ~bits : bits | 0x80000000u;
+    return (uint64_t(depth) << 32) | uint64_t((node.y << 1) | (node.y >> 31));
+}
+__device__ __forceinline__ uint32_t key_side(uint64_t k, uint32_t facets)
+{
+    const uint32_t low = uint32_t(k);  // the side itself where there is one tile
+    return c_frame.tiles == 1u ? low : 2u * ((low >> 1) % facets) + (low & 1u);
 }
 
-__global__ void __launch_bounds__(128) k_resolve_graph(
-    const uint32_t* offsets, const uint64_t* records, uint64_t npix, uint32_t cap,
-    uint32_t* denom, uint32_t* sky, uint64_t* pairs, unsigned long long* pair_count,
-    int side_bits, uint32_t* deep_list, uint32_t* deep_count, RasterStats* stats)
+__device__ __forceinline__ void order2(uint64_t& a, uint64_t& b)
 {
-    const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const bool valid = i < npix;
-    uint32_t n = 0, start = 0;
-    if (valid) {
-        start = offsets[i];
-        n = offsets[i + 1] - start;
-    }
-    if (valid && n > cap) atomicAdd(&stats->overflow, (unsigned long long)(n - cap));
-    if (valid && n > 0) atomicMax(&stats->max_chain, n);
-    if (valid && n > kFastChain) {
-        deep_list[atomicAdd(deep_count, 1u)] = uint32_t(i);
-        n = 0;
-    }
-    Frag f[kFastChain];
-    for (uint32_t k = 0; k < n; ++k) f[k] = unpack(records[start + k]);
-    order_chain(f, int(n));
-    // every thread of the warp reaches the aggregated allocation
-    emit_chain(f, int(n), c_frame.facets, denom, sky, pairs, pair_count, side_bits, true);
+    const uint64_t lo = a < b ? a : b, hi = a < b ? b : a;
+    a = lo;
+    b = hi;
 }
 
-__global__ void __launch_bounds__(32) k_resolve_graph_deep(
-    const uint32_t* offsets, const uint64_t* records, const uint32_t* deep_list,
-    const uint32_t* deep_count, uint32_t* denom, uint32_t* sky, uint64_t* pairs,
-    unsigned long long* pair_count, int side_bits, RasterStats* stats)
+// The run of lanes with the same side that this lane begins: its length, or 0
+// where it begins none.  Neighbouring pixels mostly show one side, so that a
+// count takes one atomic per run.
+__device__ __forceinline__ uint32_t side_run(uint32_t side, bool on)
 {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= *deep_count) return;
-    const uint32_t i = deep_list[j];
-    const uint32_t start = offsets[i];
-    const uint32_t n = offsets[i + 1] - start;
-    if (n > kDeepChain) {
-        atomicAdd(&stats->capacity_error, 1u);
-        return;
-    }
-    Frag f[kDeepChain];
-    for (uint32_t k = 0; k < n; ++k) f[k] = unpack(records[start + k]);
-    order_chain(f, int(n));
-    emit_chain(f, int(n), c_frame.facets, denom, sky, pairs, pair_count, side_bits, false);
+    const uint32_t lane = threadIdx.x & 31u, key = on ? side : 0xffffffffu;
+    const uint32_t left = __shfl_up_sync(0xffffffffu, key, 1);
+    const bool head = lane == 0u || left != key;
+    const uint32_t later = __ballot_sync(0xffffffffu, head) & (0xfffffffeu << lane);
+    return head && on ? (later ? uint32_t(__ffs(int(later)) - 1) : 32u) - lane : 0u;
+}
+__device__ __forceinline__ void add_sides(uint32_t* count, uint32_t side, bool on)
+{
+    const uint32_t run = side_run(side, on);
+    if (run) atomicAdd(&count[side], run);
 }
 
-// computeCpuSunlit per pixel (facetrtcore.cpp:1448-1466): every fragment
-// counts towards its side's total; the nearest (first in append order among
-// equal depths) is visible.
-__global__ void __launch_bounds__(256) k_resolve_sunlit(const uint32_t* offsets,
-                                                        const uint64_t* records, uint64_t npix,
-                                                        uint32_t cap, uint32_t* total,
-                                                        uint32_t* visible, RasterStats* stats)
+// The longest chain that a thread has met.
+__device__ __forceinline__ void note_longest(RasterStats* stats, uint32_t n)
 {
-    const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= npix) return;
-    const uint32_t start = offsets[i];
-    const uint32_t n = offsets[i + 1] - start;
-    if (n == 0) return;
-    if (n > cap) atomicAdd(&stats->overflow, (unsigned long long)(n - cap));
-    atomicMax(&stats->max_chain, n);
-    Frag best = unpack(records[start]);
-    atomicAdd(&total[frag_side(best.key, c_frame.facets)], 1u);
-    for (uint32_t k = 1; k < n; ++k) {
-        const Frag f = unpack(records[start + k]);
-        atomicAdd(&total[frag_side(f.key, c_frame.facets)], 1u);
-        if (frag_less_stable(f, best)) best = f;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31u) == 0u && most > *const_cast<volatile uint32_t*>(&stats->max_chain))
+        atomicMax(&stats->max_chain, most);
+}
+
+// The block's 2,048 pixels, those that hold fragments packed into `queue`
+// (three quarters of the pixels are empty, and whole threads with them).
+struct Covered {
+    uint32_t queue[2048];
+    uint32_t warp[8];
+};
+__device__ __forceinline__ uint32_t gather_covered(const uint32_t* heads, Covered& c)
+{
+    const uint4* h = reinterpret_cast<const uint4*>(heads) + size_t(blockIdx.x) * 512 + threadIdx.x;
+    const uint4 a = __ldcs(h), b = __ldcs(h + 256);
+    const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t n = 0;  // both halves' counts, 16 bits each
+#pragma unroll
+    for (int k = 0; k < 8; ++k) n += v[k] ? (k < 4 ? 1u : 0x10000u) : 0u;
+    const uint32_t incl = scan_inclusive(n), warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31u) == 31u) c.warp[warp] = incl;
+    __syncthreads();
+    uint32_t before = incl - n, all = 0;
+    for (uint32_t w = 0; w < 8; ++w) {
+        if (w < warp) before += c.warp[w];
+        all += c.warp[w];
     }
-    atomicAdd(&visible[frag_side(best.key, c_frame.facets)], 1u);
+    uint32_t at = before & 0xffffu;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (k == 4) at = (all & 0xffffu) + (before >> 16);
+        if (v[k]) c.queue[at++] = v[k];
+    }
+    __syncthreads();
+    return (all & 0xffffu) + (all >> 16);
+}
+
+// A thread per covered pixel, chains of at most kFast fragments ordered in
+// registers (most have one); longer ones are listed for k_resolve_list.  The
+// block's pairs wait in shared memory and leave together: with one atomic and a
+// barrier per 256 pixels this took 208 us for the terrain's 42 M pixels and 252
+// for the forest's, now 171 and 181; 64 fragments of local memory for every
+// pixel and two denominator atomics per fragment took 871 and 460.  Bound by
+// instructions and the two loads in a row, pixel and fragment.
+constexpr uint32_t kHeldPairs = 1024;
+__global__ void __launch_bounds__(256) k_resolve_graph(
+    const uint32_t* __restrict__ heads, const uint4* __restrict__ nodes, uint32_t cap,
+    uint32_t* sky, uint64_t* pairs, unsigned long long* pair_count, int side_bits, uint2* list,
+    RasterStats* stats)
+{
+    __shared__ Covered c;
+    __shared__ uint64_t held[kHeldPairs];
+    __shared__ uint32_t held_count, held_end;
+    __shared__ unsigned long long out;
+    if (threadIdx.x == 0) held_count = 0;
+    const uint32_t covered = gather_covered(heads, c);
+    if (!covered) return;
+    const uint32_t facets = c_frame.facets, lane = threadIdx.x & 31u;
+    uint32_t longest = 0;
+    for (uint32_t first = threadIdx.x & ~31u; first < covered; first += 256) {
+        const uint32_t head = first + lane < covered ? c.queue[first + lane] : 0u;
+        uint64_t k[kFast];
+        uint32_t n = 0, next = 0;
+        k[0] = ~0ull;
+        if (head) {
+            const uint4 node = __ldcs(nodes + (head - 1u));
+            k[0] = chain_key(node);
+            next = node.z;
+            n = 1;
+        }
+        if (!__any_sync(0xffffffffu, next != 0u)) {
+            const uint32_t side = key_side(k[0], facets), run = side_run(side, n != 0u);
+            if (run) {
+                atomicAdd(&sky[side], run);
+                atomicAdd(&sky[side ^ 1u], run);
+            }
+            if (n > cap) atomicAdd(&stats->overflow, (unsigned long long)(n - cap));
+            longest = max(longest, n);
+            continue;
+        }
+#pragma unroll
+        for (int q = 1; q < kFast; ++q) {
+            k[q] = ~0ull;
+            if (next) {
+                const uint4 node = __ldcs(nodes + (next - 1u));
+                k[q] = chain_key(node);
+                next = node.z;
+                ++n;
+            }
+        }
+        if (next) {
+            while (next) {
+                next = nodes[next - 1u].z;
+                ++n;
+            }
+            list[atomicAdd(&stats->listed, 1u)] = make_uint2(head, n);
+        }
+        if (n > cap) atomicAdd(&stats->overflow, (unsigned long long)(n - cap));
+        longest = max(longest, n);
+        if (n > uint32_t(kFast)) n = 0;
+        const uint32_t most = __reduce_max_sync(0xffffffffu, n);
+        // Batcher's networks for 2, 4 and 8 keys
+        order2(k[0], k[1]);
+        if (most > 2u) {
+            order2(k[2], k[3]);
+            order2(k[0], k[2]);
+            order2(k[1], k[3]);
+            order2(k[1], k[2]);
+        }
+        if (most > 4u) {
+            order2(k[4], k[5]);
+            order2(k[6], k[7]);
+            order2(k[4], k[6]);
+            order2(k[5], k[7]);
+            order2(k[5], k[6]);
+            order2(k[0], k[4]);
+            order2(k[1], k[5]);
+            order2(k[2], k[6]);
+            order2(k[3], k[7]);
+            order2(k[2], k[4]);
+            order2(k[3], k[5]);
+            order2(k[1], k[2]);
+            order2(k[3], k[4]);
+            order2(k[5], k[6]);
+        }
+        uint32_t side[kFast], mine = 0;
+        side[0] = key_side(k[0], facets);
+        uint32_t last = side[0];
+#pragma unroll
+        for (int q = 1; q < kFast; ++q) {
+            if (uint32_t(q) >= most) break;
+            side[q] = key_side(k[q], facets);
+            if (uint32_t(q) < n) {
+                last = side[q];
+                if ((side[q - 1] >> 1) != (side[q] >> 1)) ++mine;
+            }
+        }
+        add_sides(sky, side[0], n != 0u);
+        add_sides(sky, last ^ 1u, n != 0u);
+        if (!__any_sync(0xffffffffu, mine != 0u)) continue;
+        const uint32_t incl = scan_inclusive(mine);
+        const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(&held_count, all);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        uint64_t* to = held + (base + incl - mine);
+        if (base + all > kHeldPairs) {
+            // No room: straight out.  All later requests end here too, and the
+            // first of them marks the end of what is held.
+            if (lane == 0 && base <= kHeldPairs) held_end = base;
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(pair_count, (unsigned long long)all);
+            to = pairs + __shfl_sync(0xffffffffu, at, 0) + (incl - mine);
+        }
+#pragma unroll
+        for (int q = 1; q < kFast; ++q) {
+            if (uint32_t(q) >= most) break;
+            if (uint32_t(q) >= n || (side[q - 1] >> 1) == (side[q] >> 1)) continue;
+            const uint32_t a = side[q - 1] ^ 1u, b = side[q];
+            const uint64_t lo = a < b ? a : b, hi = a < b ? b : a;
+            *to++ = (lo << side_bits) | hi;
+        }
+    }
+    note_longest(stats, longest);
+    __syncthreads();
+    const uint32_t keep = held_count > kHeldPairs ? held_end : held_count;
+    if (threadIdx.x == 0 && keep) out = atomicAdd(pair_count, (unsigned long long)keep);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < keep; i += 256) pairs[out + i] = held[i];
+}
+
+// The listed pixels with more than `above` and at most kCap fragments, a thread
+// each, in local memory; chains above kDeepChain are an error.
+template <uint32_t kCap>
+__global__ void __launch_bounds__(64) k_resolve_list(
+    const uint4* __restrict__ nodes, const uint2* __restrict__ list, uint32_t above, uint32_t* sky,
+    uint64_t* pairs, unsigned long long* pair_count, int side_bits, RasterStats* stats)
+{
+    const uint32_t listed = stats->listed;
+    for (uint32_t j = blockIdx.x * 64 + threadIdx.x; j < listed; j += gridDim.x * 64) {
+        const uint32_t n = list[j].y;
+        if (n > kCap) {
+            // (kMidChain: the next launch's)
+            if (kCap == kDeepChain) atomicAdd(&stats->capacity_error, 1u);
+            continue;
+        }
+        if (n <= above) continue;
+        Frag f[kCap];
+        uint32_t next = list[j].x;
+        for (uint32_t k = 0; k < n; ++k) {
+            const uint4 node = nodes[next - 1u];
+            f[k].depth = __uint_as_float(node.x);
+            f[k].key = node.y;
+            next = node.z;
+        }
+        order_chain(f, int(n));
+        emit_chain(f, int(n), c_frame.facets, sky, pairs, pair_count, side_bits);
+    }
+}
+
+// computeCpuSunlit per pixel (facetrtcore.cpp:1448-1466): the nearest fragment
+// (first in append order among equal depths) is visible.  (Every fragment
+// counts towards its side's total: counted by the raster.)
+__global__ void __launch_bounds__(256) k_resolve_sunlit(const uint32_t* __restrict__ heads,
+                                                        const uint4* __restrict__ nodes,
+                                                        uint32_t cap, uint32_t* visible,
+                                                        RasterStats* stats)
+{
+    __shared__ Covered c;
+    const uint32_t covered = gather_covered(heads, c), lane = threadIdx.x & 31u;
+    uint32_t longest = 0;
+    for (uint32_t first = threadIdx.x & ~31u; first < covered; first += 256) {
+        uint32_t next = first + lane < covered ? c.queue[first + lane] : 0u, n = 0;
+        uint64_t best = ~0ull;
+        while (next) {
+            const uint4 node = __ldcs(nodes + (next - 1u));
+            const uint64_t key = chain_key(node);
+            best = key < best ? key : best;
+            next = node.z;
+            ++n;
+        }
+        __syncwarp();
+        if (n > cap) atomicAdd(&stats->overflow, (unsigned long long)(n - cap));
+        longest = max(longest, n);
+        add_sides(visible, key_side(best, c_frame.facets), n != 0u);
+    }
+    note_longest(stats, longest);
 }
 
 __global__ void k_fraction(uint32_t S, const uint32_t* total, const uint32_t* visible, float* out)
@@ -537,16 +961,11 @@ __global__ void k_fraction(uint32_t S, const uint32_t* total, const uint32_t* vi
     if (s < S) out[s] = total[s] ? float(visible[s]) / float(total[s]) : 0.0f;
 }
 
-__global__ void k_set_last_offset(uint32_t* offsets, uint64_t n, const unsigned long long* total)
-{
-    offsets[n] = uint32_t(*total);
-}
-
 }  // namespace
 
 void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame,
                       const RasterView* views, uint32_t dir_count, RasterBuffers& rb,
-                      Workspace& ws, RasterStats& stats, cudaStream_t s)
+                      uint32_t* d_frags, RasterStats& stats, cudaStream_t s)
 {
     if (dir_count > 64) throw Error(FACETCU_INVALID_ARGUMENT, "raster chunk exceeds 64 directions");
     FCU_CHECK(cudaMemcpyToSymbolAsync(c_views, views, sizeof(RasterView) * dir_count, 0,
@@ -554,87 +973,98 @@ void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame
     FCU_CHECK(cudaMemcpyToSymbolAsync(c_frame, &frame, sizeof(RasterFrame), 0,
                                       cudaMemcpyHostToDevice, s));
     const uint64_t npix = uint64_t(dir_count) * frame.width * frame.height;
-    const uint64_t items = uint64_t(dir_count) * frame.tiles * frame.facets;
+    const uint64_t per_dir = uint64_t(frame.tiles) * frame.facets, items = dir_count * per_dir;
     if (items >= (1ull << 32)) throw Error(FACETCU_OVERFLOW_ERROR, "raster work exceeds 2^32 triangles");
-    uint32_t* counts = static_cast<uint32_t*>(rb.counts.reserve(npix * 4));
-    uint32_t* offsets = static_cast<uint32_t*>(rb.offsets.reserve((npix + 1) * 4));
-    uint32_t* big = static_cast<uint32_t*>(rb.big_list.reserve(items * 4));
-    RasterStats* dstats = static_cast<RasterStats*>(rb.stats.reserve(sizeof(RasterStats) + 64));
-    unsigned long long* dtotal = reinterpret_cast<unsigned long long*>(
-        static_cast<char*>(rb.stats.ptr) + sizeof(RasterStats));
-    FCU_CHECK(cudaMemsetAsync(counts, 0, npix * 4, s));
-    FCU_CHECK(cudaMemsetAsync(dstats, 0, sizeof(RasterStats), s));
-    const unsigned blocks = unsigned((items + 255) / 256);
-    k_raster_small<false><<<blocks, 256, 0, s>>>(d_vertices, items, counts, nullptr, nullptr,
-                                                 big, &dstats->big);
-    FCU_LAUNCH("k_raster_small<count>");
+    // whole blocks of the resolve
+    const uint64_t padded = (npix + kResolvePixels - 1) / kResolvePixels * kResolvePixels;
+    uint32_t* heads = static_cast<uint32_t*>(rb.heads.reserve(padded * 4));
+    uint32_t* jobs = static_cast<uint32_t*>(rb.jobs.reserve(items * 4));
+    float4* planes = static_cast<float4*>(rb.planes.reserve(size_t(frame.facets) * 48));
+    RasterStats* dstats = static_cast<RasterStats*>(rb.stats.reserve(sizeof(RasterStats)));
+    k_planes<<<(frame.facets + 255) / 256, 256, 0, s>>>(d_vertices, frame.facets, planes);
+    FCU_LAUNCH("k_planes");
+    // A pool of one fragment for two pixels to begin with: the forest of
+    // 200,000 facets has 0.29 a pixel over the 40 directions, 4,096 facets of
+    // terrain 0.25.
     RasterStats host{};
-    FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
-    FCU_CHECK(cudaStreamSynchronize(s));
-    if (host.big) {
-        k_raster_big<false><<<host.big, 256, 0, s>>>(d_vertices, big, counts, nullptr, nullptr);
-        FCU_LAUNCH("k_raster_big<count>");
+    uint64_t capacity = std::max<uint64_t>(rb.nodes.bytes / 16, npix / 2 + 1);
+    for (uint32_t* counted = d_frags;; counted = nullptr) {
+        capacity = std::min<uint64_t>(capacity, 0xffffffffull);
+        const Pool pool{heads, static_cast<uint4*>(rb.nodes.reserve(capacity * 16)), capacity,
+                        &dstats->fragments};
+        FCU_CHECK(cudaMemsetAsync(heads, 0, padded * 4, s));
+        FCU_CHECK(cudaMemsetAsync(dstats, 0, sizeof(RasterStats), s));
+        k_raster<<<dim3(unsigned((per_dir + 255) / 256), dir_count), 256, 0, s>>>(
+            planes, uint32_t(per_dir), pool, jobs, uint32_t(items), dstats, counted);
+        FCU_LAUNCH("k_raster");
+        k_raster_mid<kMidLanes><<<unsigned(std::min<uint64_t>((items + 31) / 32, 8 * 152)), 256, 0, s>>>(
+            planes, uint32_t(per_dir), pool, jobs, &dstats->mid, counted);
+        FCU_LAUNCH("k_raster_mid");
+        k_raster_big<<<dim3(unsigned(std::min<uint64_t>(items, 152)), 16), 256, 0, s>>>(
+            planes, uint32_t(per_dir), pool, jobs + items, &dstats->big, counted);
+        FCU_LAUNCH("k_raster_big");
+        FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
+        FCU_CHECK(cudaStreamSynchronize(s));
+        if (host.fragments >= (1ull << 32))
+            throw Error(FACETCU_OVERFLOW_ERROR, "more than 2^32 fragments in one raster chunk");
+        if (host.fragments <= capacity) break;
+        capacity = host.fragments;
     }
-    exclusive_scan_u32(counts, offsets, npix, dtotal, ws, s);
-    unsigned long long total = 0;
-    FCU_CHECK(cudaMemcpyAsync(&total, dtotal, 8, cudaMemcpyDeviceToHost, s));
-    FCU_CHECK(cudaStreamSynchronize(s));
-    if (total >= (1ull << 32))
-        throw Error(FACETCU_OVERFLOW_ERROR, "more than 2^32 fragments in one raster chunk");
-    k_set_last_offset<<<1, 1, 0, s>>>(offsets, npix, dtotal);
-    FCU_LAUNCH("k_set_last_offset");
-    uint64_t* records = static_cast<uint64_t*>(rb.records.reserve((total + 1) * 8));
-    FCU_CHECK(cudaMemsetAsync(counts, 0, npix * 4, s));
-    k_raster_small<true><<<blocks, 256, 0, s>>>(d_vertices, items, counts, offsets, records,
-                                                nullptr, nullptr);
-    FCU_LAUNCH("k_raster_small<fill>");
-    if (host.big) {
-        k_raster_big<true><<<host.big, 256, 0, s>>>(d_vertices, big, counts, offsets, records);
-        FCU_LAUNCH("k_raster_big<fill>");
-    }
-    stats.fragments = total;
+    stats.fragments = host.fragments;
     stats.big = host.big;
 }
 
+void raster_denominators(uint32_t facets, const uint32_t* d_frags, uint32_t* d_denominators,
+                         cudaStream_t s)
+{
+    k_denominators<<<(facets + 255) / 256, 256, 0, s>>>(
+        facets, reinterpret_cast<const uint2*>(d_frags), reinterpret_cast<uint2*>(d_denominators));
+    FCU_LAUNCH("k_denominators");
+}
+
 void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t chain_cap,
-                          RasterBuffers& rb, uint32_t* d_denominators, uint32_t* d_sky,
-                          uint64_t* d_pairs, unsigned long long* d_pair_count, int side_bits,
-                          RasterStats& stats, cudaStream_t s)
+                          RasterBuffers& rb, uint32_t* d_sky, uint64_t* d_pairs,
+                          unsigned long long* d_pair_count, int side_bits, RasterStats& stats,
+                          cudaStream_t s)
 {
     const uint64_t npix = uint64_t(dir_count) * frame.width * frame.height;
     RasterStats* dstats = rb.stats.as<RasterStats>();
-    uint32_t* deep = static_cast<uint32_t*>(rb.deep_list.reserve(npix * 4));
-    FCU_CHECK(cudaMemsetAsync(&dstats->deep, 0, 4, s));
-    k_resolve_graph<<<unsigned((npix + 127) / 128), 128, 0, s>>>(
-        rb.offsets.as<uint32_t>(), rb.records.as<uint64_t>(), npix, chain_cap,
-        d_denominators, d_sky, d_pairs, d_pair_count, side_bits, deep, &dstats->deep, dstats);
+    uint2* list = static_cast<uint2*>(rb.list.reserve((stats.fragments / (kFast + 1) + 1) * 8));
+    const uint4* nodes = rb.nodes.as<uint4>();
+    k_resolve_graph<<<unsigned((npix + kResolvePixels - 1) / kResolvePixels), 256, 0, s>>>(
+        rb.heads.as<uint32_t>(), nodes, chain_cap, d_sky, d_pairs, d_pair_count, side_bits, list,
+        dstats);
     FCU_LAUNCH("k_resolve_graph");
+    const unsigned list_blocks = 16 * 152;
+    k_resolve_list<kMidChain><<<list_blocks, 64, 0, s>>>(nodes, list, 0u, d_sky, d_pairs,
+                                                         d_pair_count, side_bits, dstats);
+    FCU_LAUNCH("k_resolve_list");
     RasterStats host{};
-    FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
-    FCU_CHECK(cudaStreamSynchronize(s));
-    if (host.deep) {
-        k_resolve_graph_deep<<<(host.deep + 31) / 32, 32, 0, s>>>(
-            rb.offsets.as<uint32_t>(), rb.records.as<uint64_t>(), deep, &dstats->deep,
-            d_denominators, d_sky, d_pairs, d_pair_count, side_bits, dstats);
-        FCU_LAUNCH("k_resolve_graph_deep");
+    auto read = [&] {
         FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
         FCU_CHECK(cudaStreamSynchronize(s));
+    };
+    read();
+    if (host.max_chain > kMidChain) {
+        // (launched only then: its local memory is a few GB)
+        k_resolve_list<kDeepChain><<<list_blocks, 64, 0, s>>>(
+            nodes, list, kMidChain, d_sky, d_pairs, d_pair_count, side_bits, dstats);
+        FCU_LAUNCH("k_resolve_list");
+        read();
     }
     stats.overflow = host.overflow;
-    stats.deep = host.deep;
     stats.max_chain = host.max_chain;
     stats.capacity_error = host.capacity_error;
 }
 
 void raster_resolve_sunlit(const RasterFrame& frame, uint32_t chain_cap, RasterBuffers& rb,
-                           uint32_t* d_total, uint32_t* d_visible, float* d_fraction,
+                           const uint32_t* d_total, uint32_t* d_visible, float* d_fraction,
                            RasterStats& stats, cudaStream_t s)
 {
     const uint64_t npix = uint64_t(frame.width) * frame.height;
     RasterStats* dstats = rb.stats.as<RasterStats>();
-    k_resolve_sunlit<<<unsigned((npix + 255) / 256), 256, 0, s>>>(
-        rb.offsets.as<uint32_t>(), rb.records.as<uint64_t>(), npix, chain_cap,
-        d_total, d_visible, dstats);
+    k_resolve_sunlit<<<unsigned((npix + kResolvePixels - 1) / kResolvePixels), 256, 0, s>>>(
+        rb.heads.as<uint32_t>(), rb.nodes.as<uint4>(), chain_cap, d_visible, dstats);
     FCU_LAUNCH("k_resolve_sunlit");
     k_fraction<<<(2 * frame.facets + 255) / 256, 256, 0, s>>>(2 * frame.facets, d_total, d_visible,
                                                               d_fraction);
