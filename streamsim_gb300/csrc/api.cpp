@@ -245,6 +245,10 @@ uint32_t run_sweeps(facetcu_context* ctx, float sky, float relax, uint32_t count
     float* a = ctx->rad_a.as<float>();
     float* b = ctx->rad_b.as<float>();
     uint32_t* res = ctx->residual.as<uint32_t>();
+    if (jacobi_sweeps_cluster(ctx->graph, ctx->optics.as<facetcu_surface_optics>(), sky, relax,
+                              ping == 0 ? a : b, ping == 0 ? b : a, count, res + first_slot,
+                              ctx->stream))
+        return ping ^ (count & 1u);
     for (uint32_t i = 0; i < count; ++i) {
         const float* in = ping == 0 ? a : b;
         float* out = ping == 0 ? b : a;

@@ -283,6 +283,11 @@ bool graph_pack(DeviceGraph& g, Workspace& ws, cudaStream_t s);
 void jacobi_sweep(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
                   float relaxation, const float* d_in, float* d_out, uint32_t* d_max_delta_bits,
                   cudaStream_t s);
+// All `sweeps` sweeps of a small graph in one launch, from d_in, alternating
+// with d_other as single sweeps would; false where the graph is not for it.
+bool jacobi_sweeps_cluster(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
+                           float relaxation, float* d_in, float* d_other, uint32_t sweeps,
+                           uint32_t* d_max_delta_bits, cudaStream_t s);
 // The same sweep on raw device pointers (used by facetcu_solve_noalloc);
 // edges_hint: about how many edges there are.
 void jacobi_sweep_raw(uint32_t surfaces, uint64_t edges_hint, const uint32_t* rows,

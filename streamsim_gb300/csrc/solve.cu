@@ -7,6 +7,8 @@
 // edges, short rows) and callers that bring their own arrays.
 #include "internal.h"
 
+#include <cooperative_groups.h>
+
 namespace facetcu {
 namespace {
 
@@ -76,6 +78,176 @@ __global__ void __launch_bounds__(256) k_jacobi_rows(
     }
 }
 
+// ---- all sweeps of a small graph in one launch ----------------------------
+// A sweep of 98,000 edges takes 2.6 us on the device and its launch 5 us of the
+// host, so 64 of them took 333 us.  Here a cluster of 16 blocks runs all of
+// them in 175 (249 with the copies): every block holds the whole radiosity
+// twice (this sweep's and the next), its share of the sides and their edges in
+// shared memory, and writes its new values into the others'.  Bound by the
+// exchange and the cluster's barrier (1 us a sweep for 1,152 sides, 2.5 for
+// 8,192); blocks that wait on a count of received bytes instead (asynchronous
+// stores, bulk copies) gave 291 and 232.
+// The cluster's 16 SMs are the limit for larger graphs; a solve of 64 sweeps in
+// single launches and here, us:
+//     edges    6,708   40,442   98,058   138,606   325,582   610,067
+//     launches   306      332      333       408       486       465
+//     cluster    126      212      249       264       435       511
+// (two lanes a side; four: 125, 235, 279, 278, 468, 499; eight blocks: 304 at
+// 98,058 edges.)  Setting up costs as much as some launches: 6,708 edges break
+// even at 3 sweeps (48, 50), 98,058 at 6 (90, 89), 325,582 at 12 (160, 161).
+constexpr uint32_t kCtas = 16, kClusterThreads = 1024, kGroup = 16, kDeltas = 64;
+constexpr int kClusterLanes = 2;
+constexpr uint64_t kClusterEdges = 400000;
+constexpr size_t kClusterShared = 227 * 1024 - 1024;  // (static arrays besides)
+
+struct ClusterShape {
+    uint32_t padded;  // sides, the same whole number of groups for every block
+    uint32_t owned;   // a block's, whole groups
+    uint32_t words;   // edges that fit; the rest is read from memory
+};
+
+// Sides go to the blocks in groups of 16 in turn, so that rows of different
+// lengths even out.
+__device__ __forceinline__ uint32_t owned_side(uint32_t j, uint32_t rank)
+{
+    return (rank + kCtas * (j / kGroup)) * kGroup + j % kGroup;
+}
+
+template <int L>
+__global__ void __launch_bounds__(kClusterThreads, 1) k_jacobi_cluster(
+    ClusterShape shape, uint32_t surfaces, const uint32_t* __restrict__ rows,
+    const facetcu_csr_edge* __restrict__ edges, const uint32_t* __restrict__ denom,
+    const uint32_t* __restrict__ skyc, const facetcu_surface_optics* __restrict__ optics, float sky,
+    float relax, const float* first, float* out_even, float* out_odd, uint32_t sweeps,
+    uint32_t* max_delta_bits)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank(), tid = threadIdx.x, lane = tid & 31u;
+    extern __shared__ float4 shared4[];
+    float* x = reinterpret_cast<float*>(shared4);                       // [2][padded]
+    float4* opt = shared4 + 2 * shape.padded / 4;                       // [owned]
+    float2* norm = reinterpret_cast<float2*>(opt + shape.owned);        // [owned]
+    uint32_t* start = reinterpret_cast<uint32_t*>(norm + shape.owned);  // [owned + 4]
+    uint32_t* words = start + shape.owned + 4;
+    __shared__ uint32_t warp_sum[kClusterThreads / 32];
+    __shared__ uint32_t block_delta[kDeltas];  // of kDeltas sweeps, sent off together
+    if (tid < kDeltas) block_delta[tid] = 0;
+    for (uint32_t i = tid; i < shape.padded; i += kClusterThreads) x[i] = i < surfaces ? first[i] : 0.0f;
+    uint32_t base = 0;
+    for (uint32_t j0 = 0; j0 < shape.owned; j0 += kClusterThreads) {
+        const uint32_t j = j0 + tid, s = owned_side(j, rank);
+        const bool on = j < shape.owned && s < surfaces;
+        const uint32_t n = on ? rows[s + 1] - rows[s] : 0u;
+        uint32_t incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= uint32_t(o)) incl += y;
+        }
+        if (lane == 31u) warp_sum[tid >> 5] = incl;
+        __syncthreads();
+        uint32_t before = base, all = 0;
+        for (uint32_t w = 0; w < kClusterThreads / 32; ++w) {
+            if (w < tid >> 5) before += warp_sum[w];
+            all += warp_sum[w];
+        }
+        if (j < shape.owned) {
+            start[j] = before + incl - n;
+            if (j + 1 == shape.owned) start[j + 1] = before + incl;
+            opt[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            norm[j] = make_float2(0.0f, 0.0f);
+            if (on) {
+                const facetcu_surface_optics o = optics[s];
+                opt[j] = make_float4(o.reflectance, o.transmittance, o.emission, o.direct_irradiance);
+                norm[j] = make_float2(float(skyc[s]), float(denom[s]));
+            }
+        }
+        base += all;
+        __syncthreads();
+    }
+    for (uint32_t j = tid / 8; j < shape.owned; j += kClusterThreads / 8) {
+        const uint32_t s = owned_side(j, rank);
+        if (s >= surfaces) continue;
+        const uint32_t from = rows[s], n = rows[s + 1] - from, at = start[j];
+        for (uint32_t e = tid % 8; e < n && at + e < shape.words; e += 8) {
+            const facetcu_csr_edge ed = edges[from + e];
+            words[at + e] = ed.neighbor << 16 | ed.count;
+        }
+    }
+    cluster.sync();
+    constexpr int U = 2;
+    for (uint32_t it = 0; it < sweeps; ++it) {
+        const float* now = x + (it & 1u ? shape.padded : 0u);
+        float* next = x + (it & 1u ? 0u : shape.padded);
+        float delta = 0.0f;
+        for (uint32_t j = tid / L; j < shape.owned; j += kClusterThreads / L) {
+            const uint32_t at = start[j], n = start[j + 1] - at, s = owned_side(j, rank);
+            const uint32_t held = at >= shape.words ? 0u : min(n, shape.words - at);
+            float acc = 0.0f;
+            uint32_t e = tid % L;
+            for (; e < held; e += L * U) {
+                uint32_t w[U];
+                float v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) w[u] = e + u * L < held ? words[at + e + u * L] : 0u;
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = now[w[u] >> 16];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (e + u * L < held) acc += float(w[u] & 0xffffu) * v[u];
+            }
+            e = held + (tid % L + L - held % L) % L;
+            if (e < n) {
+                const uint32_t from = rows[s];
+                for (; e < n; e += L) {
+                    const facetcu_csr_edge ed = edges[from + e];
+                    acc += float(ed.count) * now[ed.neighbor];
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 1; k < L; k <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
+            const float4 o = opt[j];
+            const float2 d = norm[j];
+            const float h = (d.y == 0.0f ? sky : (d.x * sky + acc) / d.y) + o.w;
+            const float other = __shfl_xor_sync(0xffffffffu, h, L);  // the facet's other side
+            if (tid % L == 0) {
+                const float old = now[s], t = o.z + o.x * h + o.y * other;
+                const float b = s < surfaces ? old * (1.0f - relax) + t * relax : 0.0f;
+                next[s] = b;
+                delta = fmaxf(delta, fabsf(b - old));
+            }
+        }
+        const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(delta));
+        if (lane == 0) atomicMax(&block_delta[it % kDeltas], most);
+        __syncthreads();
+        // this block's values to the others, two warps to each, 16 bytes a lane
+        for (uint32_t w = tid >> 5; w < 2 * (kCtas - 1); w += kClusterThreads / 32) {
+            float* there = cluster.map_shared_rank(next, (rank + 1 + w / 2) % kCtas);
+            for (uint32_t p = (w & 1u) * 32 + lane; p < shape.owned / 4; p += 64) {
+                const uint32_t s = owned_side(4 * p, rank);
+                *reinterpret_cast<float4*>(there + s) = *reinterpret_cast<const float4*>(next + s);
+            }
+        }
+        if (it % kDeltas == kDeltas - 1 || it + 1 == sweeps) {
+            // (a global atomic in every sweep would have to be waited for at the barrier)
+            const uint32_t k = it - it % kDeltas + tid;
+            if (k <= it && tid < kDeltas) {
+                atomicMax(max_delta_bits + k, block_delta[tid]);
+                block_delta[tid] = 0;
+            }
+        }
+        cluster.sync();
+    }
+    for (uint32_t j = tid; j < shape.owned; j += kClusterThreads) {
+        const uint32_t s = owned_side(j, rank);
+        if (s >= surfaces) continue;
+        out_even[s] = x[s];
+        out_odd[s] = x[shape.padded + s];
+    }
+}
+
 // FacetrtVulkan::incidentIrradiance / incidentIrradianceCpu
 // (facetrt_vulkan.cpp:1360-1399, facetrtcore.cpp:1531-1559): FP64 gather.
 __global__ void __launch_bounds__(128) k_incident(
@@ -131,6 +303,52 @@ void jacobi_sweep(const DeviceGraph& g, const facetcu_surface_optics* d_optics, 
     jacobi_sweep_raw(g.surfaces, g.nnz, g.row_offsets.as<uint32_t>(), g.edges.as<facetcu_csr_edge>(),
                      g.denominators.as<uint32_t>(), g.sky.as<uint32_t>(), d_optics, sky, relaxation,
                      d_in, d_out, d_max_delta_bits, s);
+}
+
+bool jacobi_sweeps_cluster(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
+                           float relaxation, float* d_in, float* d_other, uint32_t sweeps,
+                           uint32_t* d_max_delta_bits, cudaStream_t s)
+{
+    const uint32_t S = g.surfaces;
+    if (sweeps < 5 + g.nnz / 50000 || S < 2 || S > 0xffffu || g.max_count > 0xffffu || g.nnz > kClusterEdges)
+        return false;
+    ClusterShape shape;
+    const uint32_t groups = (S + kGroup - 1) / kGroup;
+    shape.owned = (groups + kCtas - 1) / kCtas * kGroup;
+    shape.padded = shape.owned * kCtas;
+    const size_t fixed = size_t(shape.padded) * 8 + size_t(shape.owned) * 28 + 16;
+    if (fixed >= kClusterShared) return false;
+    // an even share of the edges fits; a block whose share is larger than what
+    // it has room for reads the rest from memory
+    const size_t room = (kClusterShared - fixed) / 4;
+    if (g.nnz / kCtas > room) return false;
+    shape.words = uint32_t(std::min<size_t>(room, g.nnz / kCtas * 2 + 1024));
+    auto kernel = k_jacobi_cluster<kClusterLanes>;
+    const size_t shared = fixed + size_t(shape.words) * 4;
+    FCU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shared)));
+    FCU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t config{};
+    config.gridDim = kCtas;
+    config.blockDim = kClusterThreads;
+    config.dynamicSmemBytes = shared;
+    config.stream = s;
+    cudaLaunchAttribute cluster{};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim = {kCtas, 1, 1};
+    config.attrs = &cluster;
+    config.numAttrs = 1;
+    int fits = 0;
+    if (cudaOccupancyMaxActiveClusters(&fits, kernel, &config) != cudaSuccess || fits < 1) {
+        cudaGetLastError();
+        return false;
+    }
+    // after `sweeps` sweeps the values lie where single sweeps would leave them
+    FCU_CHECK(cudaLaunchKernelEx(&config, kernel, shape, S, (const uint32_t*)g.row_offsets.ptr,
+                                 (const facetcu_csr_edge*)g.edges.ptr,
+                                 (const uint32_t*)g.denominators.ptr, (const uint32_t*)g.sky.ptr,
+                                 d_optics, sky, relaxation, (const float*)d_in, d_in, d_other, sweeps,
+                                 d_max_delta_bits));
+    return true;
 }
 
 void incident_irradiance(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
