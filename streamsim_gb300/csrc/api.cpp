@@ -529,10 +529,7 @@ int facetcu_build_visibility_graph(facetcu_context* ctx, const facetcu_direction
             }
             raster_resolve_graph(frame, n, chain_cap(ctx), ctx->raster, sky,
                                  ctx->pairs.as<uint64_t>(), pair_count, side_bits, st, s);
-            unsigned long long used = 0;
-            FCU_CHECK(cudaMemcpyAsync(&used, pair_count, 8, cudaMemcpyDeviceToHost, s));
-            FCU_CHECK(cudaStreamSynchronize(s));
-            pairs_used = used;
+            pairs_used = st.pairs;
             overflow += st.overflow;
             capacity_error += st.capacity_error;
             max_chain = std::max(max_chain, st.max_chain);

@@ -3,9 +3,12 @@
 // The reference counts pairs in a std::unordered_map (buildCpuGraph,
 // facetrtcore.cpp:1390) or a GPU open-addressing hash compacted on the host
 // (visibility_resolve.comp:52-72, facetrt_vulkan.cpp:1006-1037).  Here the
-// pair keys are radix-sorted on the device, run-length counted, mirrored to
-// directed entries and sorted again, so each CSR row comes out ordered by
-// neighbour and the build is deterministic and needs no capacity guess.
+// pair keys (lo, hi) are radix-sorted on the device and run-length counted; a
+// second sort by hi alone, which is stable, gives the mirrored entries.  A row
+// is its mirrored entries (neighbours below it), then its forward ones (above),
+// so each CSR row comes out ordered by neighbour and the build is deterministic
+// and needs no capacity guess.  (Sorting all directed entries by both sides
+// moved twice the entries over twice the digits.)
 #include "internal.h"
 
 namespace facetcu {
@@ -29,36 +32,50 @@ __global__ void k_compact_heads(const uint64_t* keys, size_t n, const uint32_t* 
     }
 }
 
-// Directed entries 2u, 2u+1 of undirected edge u: (lo -> hi) and (hi -> lo)
-// with the run length as value.
+// The mirrored entry (hi -> lo) of every undirected edge, with its run length.
 __global__ void k_mirror(const uint64_t* ukeys, const uint32_t* upos, size_t u, size_t n,
-                         int side_bits, uint64_t* dkeys, uint32_t* dvals)
+                         int side_bits, uint64_t* mkeys, uint32_t* mvals)
 {
     const size_t j = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (j >= u) return;
     const uint64_t mask = (1ull << side_bits) - 1ull;
-    const uint64_t lo = ukeys[j] >> side_bits, hi = ukeys[j] & mask;
-    const uint32_t count = (j + 1 < u ? upos[j + 1] : uint32_t(n)) - upos[j];
-    dkeys[2 * j] = (lo << side_bits) | hi;
-    dkeys[2 * j + 1] = (hi << side_bits) | lo;
-    dvals[2 * j] = count;
-    dvals[2 * j + 1] = count;
+    mkeys[j] = (ukeys[j] & mask) << side_bits | ukeys[j] >> side_bits;
+    mvals[j] = (j + 1 < u ? upos[j + 1] : uint32_t(n)) - upos[j];
 }
 
-__global__ void k_csr_fill(const uint64_t* dkeys, const uint32_t* dvals, size_t n, int side_bits,
-                           uint32_t surfaces, uint32_t* row_offsets, facetcu_csr_edge* edges)
+// starts[r] = the first of the n sorted entries whose side is r or above:
+// of the forward entries (blockIdx.y 0) and of the mirrored ones.  A search per
+// row: an entry per thread that fills the gap before it took 157 us for 400,000
+// sides, of which one thread walked the tens of thousands that have no entry.
+__global__ void k_row_starts(const uint64_t* forward, const uint64_t* mirrored, uint32_t n,
+                             int side_bits, uint32_t surfaces, uint32_t* starts)
+{
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r > surfaces) return;
+    const uint64_t* keys = blockIdx.y ? mirrored : forward;
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2u;
+        if (uint32_t(keys[mid] >> side_bits) < r) lo = mid + 1u;
+        else hi = mid;
+    }
+    starts[(blockIdx.y ? surfaces + 1u : 0u) + r] = lo;
+}
+
+__global__ void k_csr_fill(const uint64_t* ukeys, const uint32_t* upos, size_t pairs,
+                           const uint64_t* mkeys, const uint32_t* mvals, size_t u, int side_bits,
+                           uint32_t surfaces, const uint32_t* starts, uint32_t* row_offsets,
+                           facetcu_csr_edge* edges)
 {
     const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i > n) return;
-    const uint64_t mask = (1ull << side_bits) - 1ull;
-    // row boundaries: rows (prev, cur] start at i
-    const int64_t prev = i == 0 ? -1 : int64_t(dkeys[i - 1] >> side_bits);
-    const int64_t cur = i == n ? int64_t(surfaces) : int64_t(dkeys[i] >> side_bits);
-    for (int64_t r = prev + 1; r <= cur; ++r) row_offsets[r] = uint32_t(i);
-    if (i < n) {
-        edges[i].neighbor = uint32_t(dkeys[i] & mask);
-        edges[i].count = dvals[i];
-    }
+    const uint32_t* mstarts = starts + surfaces + 1u;
+    const uint32_t mask = uint32_t((1ull << side_bits) - 1ull);
+    if (i <= surfaces) row_offsets[i] = starts[i] + mstarts[i];
+    if (i >= u) return;
+    const uint32_t s = uint32_t(ukeys[i] >> side_bits), m = uint32_t(mkeys[i] >> side_bits);
+    edges[i + mstarts[s + 1u]] = {uint32_t(ukeys[i]) & mask,
+                                  (i + 1 < u ? upos[i + 1] : uint32_t(pairs)) - upos[i]};
+    edges[i + starts[m]] = {uint32_t(mkeys[i]) & mask, mvals[i]};
 }
 
 // Closure diagnostic of buildCpuGraph / buildVisibilityGraph
@@ -136,7 +153,7 @@ void graph_from_pairs(uint64_t* d_pairs, size_t n, int side_bits, DeviceGraph& g
     uint64_t* alt = static_cast<uint64_t*>(ws.a.reserve((n + 1) * 8));
     uint32_t* nov = nullptr;
     uint32_t* nov2 = nullptr;
-    radix_sort_u64(keys, alt, nov, nov2, n, 2 * side_bits, ws, s);
+    radix_sort_u64(keys, alt, nov, nov2, n, 0, 2 * side_bits, ws, s);
     // keys now holds the sorted pairs (either d_pairs or ws.a); use the other
     // buffer for the unique keys.
     uint64_t* other = keys == d_pairs ? alt : d_pairs;
@@ -162,22 +179,26 @@ void graph_from_pairs(uint64_t* d_pairs, size_t n, int side_bits, DeviceGraph& g
     }
     const size_t m = 2 * u;
     if (m >= (1ull << 32)) throw Error(FACETCU_OVERFLOW_ERROR, "visibility graph exceeds 2^32 edges");
-    ScratchBuffer dk(ws), dk2(ws), dv(ws), dv2(ws);
-    uint64_t* dkeys = static_cast<uint64_t*>(dk.reserve((m + 1) * 8));
-    uint64_t* dkeys2 = static_cast<uint64_t*>(dk2.reserve((m + 1) * 8));
-    uint32_t* dvals = static_cast<uint32_t*>(dv.reserve((m + 1) * 4));
-    uint32_t* dvals2 = static_cast<uint32_t*>(dv2.reserve((m + 1) * 4));
+    ScratchBuffer mk(ws), mk2(ws), mv(ws), mv2(ws), st(ws);
+    uint64_t* mkeys = static_cast<uint64_t*>(mk.reserve((u + 1) * 8));
+    uint64_t* mkeys2 = static_cast<uint64_t*>(mk2.reserve((u + 1) * 8));
+    uint32_t* mvals = static_cast<uint32_t*>(mv.reserve((u + 1) * 4));
+    uint32_t* mvals2 = static_cast<uint32_t*>(mv2.reserve((u + 1) * 4));
     if (u) {
-        k_mirror<<<grid(u, 256), 256, 0, s>>>(other, upos, u, n, side_bits, dkeys, dvals);
+        k_mirror<<<grid(u, 256), 256, 0, s>>>(other, upos, u, n, side_bits, mkeys, mvals);
         FCU_LAUNCH("k_mirror");
-        radix_sort_u64(dkeys, dkeys2, dvals, dvals2, m, 2 * side_bits, ws, s);
+        radix_sort_u64(mkeys, mkeys2, mvals, mvals2, u, side_bits, 2 * side_bits, ws, s);
     }
     g.nnz = m;
+    uint32_t* starts = static_cast<uint32_t*>(st.reserve((size_t(S) + 1) * 2 * 4));
     uint32_t* rows = static_cast<uint32_t*>(g.row_offsets.reserve((size_t(S) + 1) * 4));
     facetcu_csr_edge* edges = static_cast<facetcu_csr_edge*>(g.edges.reserve((m + 1) * 8));
-    k_csr_fill<<<grid(m + 1, 256), 256, 0, s>>>(dkeys, dvals, m, side_bits, S, rows, edges);
+    k_row_starts<<<dim3(grid(size_t(S) + 1, 256), 2), 256, 0, s>>>(other, mkeys, uint32_t(u),
+                                                                  side_bits, S, starts);
+    FCU_LAUNCH("k_row_starts");
+    k_csr_fill<<<grid(std::max<size_t>(u, size_t(S) + 1), 256), 256, 0, s>>>(
+        other, upos, n, mkeys, mvals, u, side_bits, S, starts, rows, edges);
     FCU_LAUNCH("k_csr_fill");
-    FCU_CHECK(cudaStreamSynchronize(s));
     g.changed();
     g.scene_facets.clear();
 }

@@ -170,11 +170,11 @@ struct ScratchBuffer {
 // *total_dev (optional) receives the 64-bit sum on the device.
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n,
                         unsigned long long* total_dev, Workspace& ws, cudaStream_t s);
-// LSD radix sort of 64-bit keys on bits [0, key_bits), with optional 32-bit
+// LSD radix sort of 64-bit keys on bits [first_bit, end_bit), with optional 32-bit
 // values; stable.  Result ends in keys/values (the buffers are swapped with
 // the alternates as needed).
 void radix_sort_u64(uint64_t*& keys, uint64_t*& keys_alt, uint32_t*& values,
-                    uint32_t*& values_alt, size_t n, int key_bits, Workspace& ws,
+                    uint32_t*& values_alt, size_t n, int first_bit, int end_bit, Workspace& ws,
                     cudaStream_t s);
 
 // ---- raster visibility (raster.cu) --------------------------------------
@@ -194,6 +194,7 @@ struct RasterStats {
     unsigned int listed;           // pixels in RasterBuffers::list
     unsigned int capacity_error;
     unsigned int max_chain;
+    unsigned long long pairs;      // (host copy only) pairs so far
 };
 
 // Rasterise `dir_count` directions (views[0..dir_count)) into per-pixel lists

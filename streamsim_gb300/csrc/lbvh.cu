@@ -282,7 +282,7 @@ void lbvh_build(const facetcu_vertex* d_vertices, uint32_t n, Lbvh& bvh, Workspa
     float* lb = static_cast<float*>(leaf_box.reserve(size_t(n) * 24));
     k_morton<<<grid(n, 256), 256, 0, s>>>(d_vertices, n, sb, ka, ia, lb, margin, true);
     FCU_LAUNCH("k_morton");
-    radix_sort_u64(ka, kb, ia, ib, n, 30, ws, s);
+    radix_sort_u64(ka, kb, ia, ib, n, 0, 30, ws, s);
     float* lbs = static_cast<float*>(bvh.parent.reserve(size_t(n) * 24));  // sorted leaf boxes
     float4* tri = static_cast<float4*>(bvh.tri.reserve(size_t(n) * 48));
     k_leaves<<<grid(n, 256), 256, 0, s>>>(d_vertices, ia, n, lb, lbs, tri);
@@ -323,7 +323,7 @@ void morton_order(const facetcu_vertex* d_vertices, uint32_t n, const float lo[3
     float* lb = static_cast<float*>(boxes.reserve(size_t(n) * 24));
     k_morton<<<grid(n, 256), 256, 0, s>>>(d_vertices, n, sb, ka, ia, lb, 0.0f, false);
     FCU_LAUNCH("k_morton");
-    radix_sort_u64(ka, kb, ia, ib, n, 30, ws, s);
+    radix_sort_u64(ka, kb, ia, ib, n, 0, 30, ws, s);
     if (ia != d_order)
         FCU_CHECK(cudaMemcpyAsync(d_order, ia, size_t(n) * 4, cudaMemcpyDeviceToDevice, s));
     FCU_CHECK(cudaStreamSynchronize(s));

@@ -1042,6 +1042,7 @@ void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t
     RasterStats host{};
     auto read = [&] {
         FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
+        FCU_CHECK(cudaMemcpyAsync(&stats.pairs, d_pair_count, 8, cudaMemcpyDeviceToHost, s));
         FCU_CHECK(cudaStreamSynchronize(s));
     };
     read();

@@ -62,3 +62,18 @@ def test_triangle_sizes(oracle, size):
     v = _triangles(rng, n, s, rng.uniform(-0.9, 0.9, n), rng.choice([-1.0, 1.0], n))
     dirs = scenes.hemisphere_directions()[::9]
     _check(oracle, v, 128, 512, dirs, scenes.sun_direction(30, 135))
+
+
+@pytest.mark.parametrize("raster,sheets", [(32, 3), (1024, 3), (1024, 6)])
+def test_pair_sort_tiles(oracle, raster, sheets):
+    """2,048 pairs (one tile of the sort), 2 M, and 5.2 M: more tiles than a
+    digit's scan takes at once.  No facet lies below or above all others, so that
+    sides have mirrored entries, forward entries, both or none."""
+    require_gpu()
+    rng = np.random.default_rng(sheets)
+    v = np.zeros((sheets, 3, 6), np.float32)
+    v[:, :, [0, 2]] = np.float32([[-3, -3], [3.5, -3], [-3, 3.5]])
+    v[:, :, 1] = (rng.permutation(sheets)[:, None] - sheets / 2) / sheets
+    v[:, :, 4] = rng.choice([-1.0, 1.0], sheets)[:, None]
+    g = _check(oracle, v.reshape(-1, 6), raster, 64, UP, UP[0])
+    assert int(g.counts.astype(np.int64).sum()) == 2 * raster * raster * (sheets - 1)
