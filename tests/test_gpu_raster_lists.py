@@ -72,7 +72,7 @@ def test_pair_sort_tiles(oracle, raster, sheets):
     require_gpu()
     rng = np.random.default_rng(sheets)
     v = np.zeros((sheets, 3, 6), np.float32)
-    v[:, :, [0, 2]] = np.float32([[-3, -3], [3.5, -3], [-3, 3.5]])
+    v[:, :, [0, 2]] = np.float32([[-20, -20], [30, -20], [-20, 30]])  # the whole frame
     v[:, :, 1] = (rng.permutation(sheets)[:, None] - sheets / 2) / sheets
     v[:, :, 4] = rng.choice([-1.0, 1.0], sheets)[:, None]
     g = _check(oracle, v.reshape(-1, 6), raster, 64, UP, UP[0])
