@@ -56,7 +56,7 @@ struct PanelParams {
     // per side and column, [S][P]
     const float* rho;
     const float* tau;
-    const float* emis;
+    const float* emis;    // null (32 and more FP32 columns only): none
     const float* direct;
     const float* skyL;    // [P]
     const float* colmax;  // [P] max|B| of the previous sweep (floor of the per-side test)
@@ -625,8 +625,13 @@ __global__ void __launch_bounds__(kWarps * 32, SweepBlocks<P>::value) k_sweep_wi
                 const size_t i0 = size_t(2u * f) * P + col0, i1 = i0 + P;
                 float e0[CPL], e1[CPL], r0[CPL], r1[CPL], t0[CPL], t1[CPL], o0[CPL], o1[CPL];
                 float b0[CPL], b1[CPL];
-                load4(pp.emis + i0, e0);
-                load4(pp.emis + i1, e1);
+                if (pp.emis) {
+                    load4(pp.emis + i0, e0);
+                    load4(pp.emis + i1, e1);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < CPL; ++k) e0[k] = e1[k] = 0.0f;
+                }
                 load4(pp.rho + i0, r0);
                 load4(pp.rho + i1, r1);
                 load4(pp.tau + i0, t0);
@@ -824,8 +829,9 @@ __global__ void __launch_bounds__(256) k_sweep_zero(GraphView g, PanelParams pp,
         const size_t i0 = size_t(s0) * P + c, i1 = i0 + P;
         const float h0 = (d0 != 0u ? (k0 * L) / float(d0) : L) + __ldcs(pp.direct + i0);
         const float h1 = (d1 != 0u ? (k1 * L) / float(d1) : L) + __ldcs(pp.direct + i1);
-        const float b0 = __ldcs(pp.emis + i0) + __ldcs(pp.rho + i0) * h0 + __ldcs(pp.tau + i0) * h1;
-        const float b1 = __ldcs(pp.emis + i1) + __ldcs(pp.rho + i1) * h1 + __ldcs(pp.tau + i1) * h0;
+        const float e0 = pp.emis ? __ldcs(pp.emis + i0) : 0.0f, e1 = pp.emis ? __ldcs(pp.emis + i1) : 0.0f;
+        const float b0 = e0 + __ldcs(pp.rho + i0) * h0 + __ldcs(pp.tau + i0) * h1;
+        const float b1 = e1 + __ldcs(pp.rho + i1) * h1 + __ldcs(pp.tau + i1) * h0;
         Bout[i0] = b0;
         Bout[i1] = b1;
         md = fmaxf(md, fmaxf(fabsf(b0), fabsf(b1)));
@@ -1806,7 +1812,7 @@ __global__ void k_scene_init_md(const float* __restrict__ X, const float* __rest
             m = 0.0f;
         }
         const size_t i = size_t(sd) * P + c;
-        m = fmaxf(m, fabsf(Y[i] - X[i]));
+        m = fmaxf(m, fabsf(X ? Y[i] - X[i] : Y[i]));
     }
     if (cur != 0xffffffffu) atomicMax(mdr + size_t(cur) * kMaxP + c, __float_as_uint(m));
 }
@@ -1826,20 +1832,32 @@ __global__ void k_scene_init_sigma(uint32_t* mdr, float* sig, float* cheb, uint3
 }
 
 // R = Y - X and Q = round(R / sigma) for the first int8 step (X unchanged).
-__global__ void k_init_i8(const float* __restrict__ X, const float* __restrict__ Y,
-                          float* __restrict__ R, int8_t* __restrict__ Q,
-                          const float* __restrict__ sig, size_t n, int P, uint32_t* it_dev,
-                          uint32_t it, const uint16_t* __restrict__ scene = nullptr,
-                          const float* __restrict__ scene_sig = nullptr)
+// X null: X is 0 and Y itself becomes R (the caller takes the two buffers for
+// one another).  Four columns a thread; n4 = cells / 4.  Bound by the planes:
+// on 400,000 sides of 64 columns 108 us with a column a thread, two planes in
+// and R and Q out; 35 from zero.
+__global__ void __launch_bounds__(256) k_init_i8(
+    const float4* __restrict__ X, const float4* __restrict__ Y, float4* __restrict__ R,
+    char4* __restrict__ Q, const float* __restrict__ sig, uint32_t n4, uint32_t P, uint32_t* it_dev,
+    uint32_t it, const uint16_t* __restrict__ scene = nullptr,
+    const float* __restrict__ scene_sig = nullptr)
 {
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
     if (i == 0) *it_dev = it;  // sweep index of the first step's check
-    if (i >= n) return;
-    const float r = Y[i] - X[i];
-    const size_t c = i % size_t(P);
-    const float sg = scene ? scene_sig[size_t(scene[(i / size_t(P)) >> 1]) * kMaxP + c] : sig[c];
-    R[i] = r;
-    Q[i] = int8_t(sg > 0.0f ? max(-127, min(127, __float2int_rn(r / sg))) : 0);
+    if (i >= n4) return;
+    const uint32_t side = i / (P / 4), c = (i - side * (P / 4)) * 4;
+    float4 r = Y[i];
+    if (X) {
+        const float4 x = X[i];
+        r = make_float4(r.x - x.x, r.y - x.y, r.z - x.z, r.w - x.w);
+        R[i] = r;
+    }
+    const float4 sg = *reinterpret_cast<const float4*>(
+        (scene ? scene_sig + size_t(scene[side >> 1]) * kMaxP : sig) + c);
+    auto q = [](float v, float s) {
+        return (signed char)(s > 0.0f ? max(-127, min(127, __float2int_rn(v / s))) : 0);
+    };
+    Q[i] = make_char4(q(r.x, sg.x), q(r.y, sg.y), q(r.z, sg.z), q(r.w, sg.w));
 }
 
 // Narrow-panel sweep (FP32 or FP64 state; also used for the FP64 truth);
@@ -2171,7 +2189,7 @@ __global__ void __launch_bounds__(256) k_prepare_panel(
             const size_t o = size_t(dest[ls]) * P + j0 + j;
             prho[o] = tile[0][ls][j];
             ptau[o] = tile[1][ls][j];
-            pemis[o] = tile[2][ls][j];
+            if (pemis) pemis[o] = tile[2][ls][j];
             pdir[o] = tile[3][ls][j];
         }
     }
@@ -2767,12 +2785,28 @@ __global__ void k_validate_inputs(const float* __restrict__ rho, const float* __
     uint32_t f = 0;
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     const size_t first = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    for (size_t i = first; i < n; i += stride) {
-        const float r = rho[i], t = tau[i], e = emis ? emis[i] : 0.0f;
+    auto check = [&](float r, float t, float e) {
         if (!isfinite(r) || !isfinite(t) || !isfinite(e) || r < 0.0f || t < 0.0f || e < 0.0f ||
             r + t > 1.0001f)
             f |= 1u;
+    };
+    // four values a load where the arrays allow it (57 us for 25.6 M cells with
+    // one, 44 with four)
+    const bool wide = ((reinterpret_cast<uintptr_t>(rho) | reinterpret_cast<uintptr_t>(tau) |
+                        reinterpret_cast<uintptr_t>(emis)) & 15u) == 0u;
+    const size_t n4 = wide ? n / 4 : 0;
+    for (size_t i = first; i < n4; i += stride) {
+        const float4 r = reinterpret_cast<const float4*>(rho)[i],
+                     t = reinterpret_cast<const float4*>(tau)[i];
+        const float4 e = emis ? reinterpret_cast<const float4*>(emis)[i]
+                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        check(r.x, t.x, e.x);
+        check(r.y, t.y, e.y);
+        check(r.z, t.z, e.z);
+        check(r.w, t.w, e.w);
     }
+    for (size_t i = 4 * n4 + first; i < n; i += stride)
+        check(rho[i], tau[i], emis ? emis[i] : 0.0f);
     if (first < bands) {
         const float k = sky[first], b = beam[first];
         if (!isfinite(k) || k < 0.0f) f |= 2u;
@@ -2916,7 +2950,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
         const size_t cells = size_t(S) * P;
         float* prho = prm;
         float* ptau = prm + cells;
-        float* pemis = prm + 2 * cells;
+        float* pemis = !p.emis && !fp64 && P >= 32 ? nullptr : prm + 2 * cells;
         float* pdir = prm + 3 * cells;
         float* psky = prm + 4 * cells;
         PanelParams pp{prho, ptau, pemis, pdir, psky, colmax,
@@ -2946,7 +2980,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                 ++timed_sweeps;
             }
         };
-        launches += 4;  // prepare, sky, panel in, panel out
+        launches += d_initial && cfg.warm_start == FACETCU_WARM_GIVEN ? 4 : 3;  // prepare, sky, panel in, panel out
         k_prepare_panel<<<blocks_for(S, kPanelTile), 256, 0, s>>>(S, p.bands, R, c0, P, side_rank, p.rho,
                                                                 p.tau, p.emis, p.beam, p.dgeo,
                                                                 prho, ptau, pemis, pdir);
@@ -2955,18 +2989,25 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
         FCU_LAUNCH("k_panel_sky");
         FCU_CHECK(cudaMemsetAsync(stats, 0, (4 * kMaxP + 16) * 4, s));  // stats, flags, colmax
         const float* init = cfg.warm_start == FACETCU_WARM_GIVEN ? d_initial : nullptr;
-        if (fp64)
-            k_panel_in<double><<<blocks_for(S, kPanelTile), 256, 0, s>>>(
-                init, S, R, c0, P, side_rank, reinterpret_cast<double*>(x0));
-        else
-            k_panel_in<float><<<blocks_for(S, kPanelTile), 256, 0, s>>>(
-                init, S, R, c0, P, side_rank, reinterpret_cast<float*>(x0));
-        FCU_LAUNCH("k_panel_in");
+        if (!init) {
+            // The first sweep takes no input; what follows it in MIXED steps
+            // from the zeros (a memset at 5.9 TB/s, where the transposing
+            // kernel wrote them at 1.4).
+            if (low) FCU_CHECK(cudaMemsetAsync(x0, 0, cells * elem, s));
+        } else {
+            if (fp64)
+                k_panel_in<double><<<blocks_for(S, kPanelTile), 256, 0, s>>>(
+                    init, S, R, c0, P, side_rank, reinterpret_cast<double*>(x0));
+            else
+                k_panel_in<float><<<blocks_for(S, kPanelTile), 256, 0, s>>>(
+                    init, S, R, c0, P, side_rank, reinterpret_cast<float*>(x0));
+            FCU_LAUNCH("k_panel_in");
+        }
         // A solve from zero: its first sweep gathers nothing (null input).
         const bool zero_start = init == nullptr;
 
         uint32_t it = 0;
-        int cur = 0;
+        const char* final_buf = x0;
         uint32_t host_flag[3] = {0, 0, 0};
         if (!low) {
             while (it < max_it) {
@@ -3002,7 +3043,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                     break;
                 }
             }
-            cur = int(host_flag[1] & 1u);
+            final_buf = host_flag[1] & 1u ? x1 : x0;
         } else if (P >= 32) {
             // FP32 sweep; then residual-tracked int8 steps until the
             // per-side test holds on their exact residual R (R_s is the
@@ -3017,6 +3058,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
             const float step_tol = tol;
             float* X = reinterpret_cast<float*>(x0);
             float* Y = reinterpret_cast<float*>(x1);
+            float* res = rbuf;
             int8_t* qb[2] = {qbuf, qbuf + cells};
             float* slot[2] = {sig, sig + kMaxP};
             while (it < max_it) {
@@ -3045,22 +3087,27 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                     std::swap(X, Y);
                     continue;
                 }
+                const bool from_zero = it == 1 && zero_start;  // X is 0: R is Y
                 if (g.scene) {
                     // every scene takes part in a new int8 phase, with its
                     // own first scales max|Y - X| / 127
                     FCU_CHECK(cudaMemsetAsync(g.scene_stats, 0,
                                               size_t(g.scenes) * (8 * kMaxP + 1) * 4, s));
-                    k_scene_init_md<<<(S + 255) / 256, P, 0, s>>>(X, Y, g.scene, S, P, g.scene_md);
+                    k_scene_init_md<<<(S + 255) / 256, P, 0, s>>>(from_zero ? nullptr : X, Y, g.scene,
+                                                                  S, P, g.scene_md);
                     FCU_LAUNCH("k_scene_init_md");
                     k_scene_init_sigma<<<g.scenes, kMaxP, 0, s>>>(g.scene_md, g.scene_sig,
                                                                   g.scene_cheb, g.scenes, P);
                     FCU_LAUNCH("k_scene_init_sigma");
                     launches += 2;
                 }
-                k_init_i8<<<blocks_for(cells, 256), 256, 0, s>>>(X, Y, rbuf, qb[0], slot[0], cells,
-                                                                 P, flag + 12, it, g.scene,
-                                                                 g.scene_sig);
+                k_init_i8<<<blocks_for(cells / 4, 256), 256, 0, s>>>(
+                    reinterpret_cast<const float4*>(from_zero ? nullptr : X),
+                    reinterpret_cast<const float4*>(Y), reinterpret_cast<float4*>(res),
+                    reinterpret_cast<char4*>(qb[0]), slot[0], uint32_t(cells / 4), uint32_t(P),
+                    flag + 12, it, g.scene, g.scene_sig);
                 FCU_LAUNCH("k_init_i8");
+                if (from_zero) std::swap(res, Y);
                 ++launches;
                 uint32_t j = 0;
                 bool steps_done = false;
@@ -3074,10 +3121,12 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                         key.P = P;
                         key.g = g;
                         key.pp = pp;
+                        key.pp.emis = nullptr;  // (the steps read neither)
+                        key.pp.direct = nullptr;
                         key.q0 = qb[0];
                         key.q1 = qb[1];
                         key.X = X;
-                        key.R = rbuf;
+                        key.R = res;
                         key.slot0 = slot[0];
                         key.slot1 = slot[1];
                         key.stats = stats;
@@ -3109,7 +3158,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                         const float* sin = slot[j & 1u];
                         const float* sout = slot[(j + 1) & 1u];
                         timed_sweep(true, [&] {
-                            launch_step_i8(P, g, pp, qb[j & 1u], qb[(j + 1) & 1u], X, rbuf, sin,
+                            launch_step_i8(P, g, pp, qb[j & 1u], qb[(j + 1) & 1u], X, res, sin,
                                            sout, stats, counter, flag + 3, j & 1u, s);
                         });
                         // slot j & 1 (sigma of the panel just consumed) takes
@@ -3133,7 +3182,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                     }
                 }
             }
-            cur = X == reinterpret_cast<float*>(x0) ? 0 : 1;
+            final_buf = reinterpret_cast<const char*>(X);
             host_flag[1] = it;
         } else {
             // FP32 sweep, then BF16 defect sweeps until the defect has shrunk
@@ -3198,10 +3247,9 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                     }
                 }
             }
-            cur = X == reinterpret_cast<float*>(x0) ? 0 : 1;
+            final_buf = reinterpret_cast<const char*>(X);
             host_flag[1] = it;
         }
-        const char* final_buf = cur ? x1 : x0;
         if (fp64)
             k_panel_out<double><<<blocks_for(S, kPanelTile), 256, 0, s>>>(
                 reinterpret_cast<const double*>(final_buf), S, R, c0, P, side_rank, d_out);
