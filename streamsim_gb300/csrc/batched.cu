@@ -2146,7 +2146,43 @@ __device__ __forceinline__ uint32_t new_side(const uint32_t* rank, uint32_t so)
 // shared tile.  Reading in solver order instead (one 4-byte element of a
 // different band row per thread) moved 8x the bytes once the inputs
 // outgrew L2.
-constexpr int kPanelTile = 32;
+//
+// One array at a time goes over all columns of the panel, kPanelLoads loads of
+// a thread in flight: out, 400,000 sides of 64 columns, in 84 us with 32
+// columns between two barriers, 44 so (54 with 8 loads, 76 with 16).  The four
+// arrays of k_prepare_panel go 32 columns at a time, all in one pass: 115 us
+// (130 array by array; on a batch of six scenes 108 and 145).
+constexpr int kPanelTile = 32, kPanelLoads = 4;
+template <typename T>
+using PanelTile = T[kPanelTile][kMaxP + 1];
+
+// tile[side][column] <- load(side, column), band-major: a warp reads 32 sides
+// of a column.
+template <typename T, typename Load>
+__device__ __forceinline__ void tile_from_bands(PanelTile<T>& tile, int P, Load load)
+{
+    for (int k0 = threadIdx.x; k0 < kPanelTile * P; k0 += 256 * kPanelLoads) {
+        T v[kPanelLoads];
+#pragma unroll
+        for (int u = 0; u < kPanelLoads; ++u) {
+            const int k = k0 + u * 256;
+            v[u] = k < kPanelTile * P ? load(k % kPanelTile, k / kPanelTile) : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < kPanelLoads; ++u) {
+            const int k = k0 + u * 256;
+            if (k < kPanelTile * P) tile[k % kPanelTile][k / kPanelTile] = v[u];
+        }
+    }
+}
+// row(side, column) for every element, a side's columns side by side (P is a
+// power of two).
+template <typename Row>
+__device__ __forceinline__ void for_panel_rows(int P, Row row)
+{
+    const int shift = 31 - __clz(P);
+    for (int k = threadIdx.x; k < kPanelTile * P; k += 256) row(k >> shift, k & (P - 1));
+}
 
 // Panel parameters for columns [c0, c0 + P) (column c = sun * bands + band).
 __global__ void __launch_bounds__(256) k_prepare_panel(
@@ -2156,12 +2192,17 @@ __global__ void __launch_bounds__(256) k_prepare_panel(
     float* __restrict__ ptau, float* __restrict__ pemis, float* __restrict__ pdir)
 {
     __shared__ float tile[4][kPanelTile][kPanelTile + 1];
-    __shared__ uint32_t dest[kPanelTile];
+    __shared__ uint32_t dest[kPanelTile], band[kMaxP], sun[kMaxP];
     const uint32_t so0 = blockIdx.x * kPanelTile;
     if (threadIdx.x < kPanelTile) {
         const uint32_t so = so0 + threadIdx.x;
         dest[threadIdx.x] = so < S ? new_side(rank, so) : 0u;
     }
+    for (int j = threadIdx.x; j < P; j += 256) {
+        band[j] = (c0 + j) % bands;
+        sun[j] = (c0 + j) / bands;
+    }
+    const int shift = 31 - __clz(min(P, kPanelTile));  // (P is a power of two)
     for (int j0 = 0; j0 < P; j0 += kPanelTile) {
         const int w = min(P - j0, kPanelTile);
         __syncthreads();
@@ -2170,7 +2211,7 @@ __global__ void __launch_bounds__(256) k_prepare_panel(
             const uint32_t so = so0 + ls, c = c0 + j0 + j;
             float r = 0.0f, t = 0.0f, e = 0.0f, d = 0.0f;
             if (so < S && c < R) {
-                const uint32_t b = c % bands, kk = c / bands;
+                const uint32_t b = band[j0 + j], kk = sun[j0 + j];
                 const size_t bi = size_t(b) * S + so;
                 r = rho[bi];
                 t = tau[bi];
@@ -2184,7 +2225,7 @@ __global__ void __launch_bounds__(256) k_prepare_panel(
         }
         __syncthreads();
         for (int k = threadIdx.x; k < kPanelTile * w; k += blockDim.x) {
-            const int ls = k / w, j = k % w;
+            const int ls = k >> shift, j = k & (w - 1);
             if (so0 + ls >= S) continue;
             const size_t o = size_t(dest[ls]) * P + j0 + j;
             prho[o] = tile[0][ls][j];
@@ -2204,33 +2245,27 @@ __global__ void k_panel_sky(uint32_t bands, uint32_t R, uint32_t c0, int P, cons
     }
 }
 
-// [R][S] (caller order) -> [S][P] (solver order); src null: zeros
+// [R][S] (caller order) -> [S][P] (solver order)
 template <typename T>
 __global__ void __launch_bounds__(256) k_panel_in(const float* __restrict__ src, uint32_t S,
                                                   uint32_t R, uint32_t c0, int P,
                                                   const uint32_t* rank, T* __restrict__ dst)
 {
-    __shared__ float tile[kPanelTile][kPanelTile + 1];
+    __shared__ PanelTile<float> tile;
     __shared__ uint32_t dest[kPanelTile];
     const uint32_t so0 = blockIdx.x * kPanelTile;
     if (threadIdx.x < kPanelTile) {
         const uint32_t so = so0 + threadIdx.x;
         dest[threadIdx.x] = so < S ? new_side(rank, so) : 0u;
     }
-    for (int j0 = 0; j0 < P; j0 += kPanelTile) {
-        const int w = min(P - j0, kPanelTile);
-        __syncthreads();
-        for (int k = threadIdx.x; k < kPanelTile * w; k += blockDim.x) {
-            const int j = k / kPanelTile, ls = k % kPanelTile;
-            const uint32_t so = so0 + ls, c = c0 + j0 + j;
-            tile[ls][j] = (src && so < S && c < R) ? src[size_t(c) * S + so] : 0.0f;
-        }
-        __syncthreads();
-        for (int k = threadIdx.x; k < kPanelTile * w; k += blockDim.x) {
-            const int ls = k / w, j = k % w;
-            if (so0 + ls < S) dst[size_t(dest[ls]) * P + j0 + j] = T(tile[ls][j]);
-        }
-    }
+    tile_from_bands<float>(tile, P, [&](int ls, int j) {
+        const uint32_t so = so0 + ls, c = c0 + j;
+        return so < S && c < R ? src[size_t(c) * S + so] : 0.0f;
+    });
+    __syncthreads();
+    for_panel_rows(P, [&](int ls, int j) {
+        if (so0 + ls < S) dst[size_t(dest[ls]) * P + j] = T(tile[ls][j]);
+    });
 }
 
 // [S][P] (solver order) -> [R][S] (caller order)
@@ -2239,26 +2274,33 @@ __global__ void __launch_bounds__(256) k_panel_out(const T* __restrict__ src, ui
                                                    uint32_t R, uint32_t c0, int P,
                                                    const uint32_t* rank, float* __restrict__ dst)
 {
-    __shared__ float tile[kPanelTile][kPanelTile + 1];
+    __shared__ PanelTile<float> tile;
     __shared__ uint32_t from[kPanelTile];
     const uint32_t so0 = blockIdx.x * kPanelTile;
     if (threadIdx.x < kPanelTile) {
         const uint32_t so = so0 + threadIdx.x;
         from[threadIdx.x] = so < S ? new_side(rank, so) : 0u;
     }
-    for (int j0 = 0; j0 < P; j0 += kPanelTile) {
-        const int w = min(P - j0, kPanelTile);
-        __syncthreads();
-        for (int k = threadIdx.x; k < kPanelTile * w; k += blockDim.x) {
-            const int ls = k / w, j = k % w;
-            tile[ls][j] = so0 + ls < S ? float(src[size_t(from[ls]) * P + j0 + j]) : 0.0f;
+    __syncthreads();
+    const int shift = 31 - __clz(P);
+    for (int k0 = threadIdx.x; k0 < kPanelTile * P; k0 += 256 * kPanelLoads) {
+        float v[kPanelLoads];
+#pragma unroll
+        for (int u = 0; u < kPanelLoads; ++u) {
+            const int k = k0 + u * 256, ls = k >> shift, j = k & (P - 1);
+            v[u] = k < kPanelTile * P && so0 + ls < S ? float(src[size_t(from[ls]) * P + j]) : 0.0f;
         }
-        __syncthreads();
-        for (int k = threadIdx.x; k < kPanelTile * w; k += blockDim.x) {
-            const int j = k / kPanelTile, ls = k % kPanelTile;
-            const uint32_t so = so0 + ls, c = c0 + j0 + j;
-            if (so < S && c < R) dst[size_t(c) * S + so] = tile[ls][j];
+#pragma unroll
+        for (int u = 0; u < kPanelLoads; ++u) {
+            const int k = k0 + u * 256;
+            if (k < kPanelTile * P) tile[k >> shift][k & (P - 1)] = v[u];
         }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < kPanelTile * P; k += 256) {
+        const int ls = k % kPanelTile, j = k / kPanelTile;
+        const uint32_t so = so0 + ls, c = c0 + j;
+        if (so < S && c < R) dst[size_t(c) * S + so] = tile[ls][j];
     }
 }
 
