@@ -1926,7 +1926,8 @@ int facetcu_faceteb_node(facetcu_context* ctx, const facetcu_energy_parameters* 
         const float* d_zero = d_lwsky + 1;
 
         const size_t per_side = 26;  // single-column fields (below)
-        const size_t io_bytes = al(S * 4) * per_side + al(size_t(W) * S * 4) * 6 +
+        const size_t io_bytes = al(S * 4) * per_side + al(size_t(W) * S * 4) * 5 +
+                                al(size_t(energy::window_stride(W)) * S * 4) +
                                 al(size_t(nb) * S * 4) * 4;
         char* c = static_cast<char*>(ctx->eb_io.reserve(io_bytes));
         auto take = [&](size_t n) {
@@ -1960,7 +1961,7 @@ int facetcu_faceteb_node(facetcu_context* ctx, const facetcu_energy_parameters* 
         float* d_swtau = take(size_t(W) * S);
         float* d_swB = take(2 * size_t(W) * S);
         float* d_swH = take(size_t(W) * S);
-        float* d_swBT = take(size_t(W) * S);
+        float* d_swBT = take(size_t(energy::window_stride(W)) * S);
         float* d_brho = take(size_t(nb) * S);
         float* d_btau = take(size_t(nb) * S);
         float* d_bemis = take(size_t(nb) * S);

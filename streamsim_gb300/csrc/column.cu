@@ -26,6 +26,7 @@
 #include <cmath>
 #include <vector>
 
+#include "compensated.cuh"
 #include "internal.h"
 #include "sweep_math.cuh"
 
@@ -518,16 +519,15 @@ __global__ void __launch_bounds__(256) k_finish_incident(
     if (s >= S) return;
     const float L = sky[0];
     const uint32_t d = denom[s];
-    double diffuse = L;
+    float h = L;
     if (d) {
-        double sum = 0.0;
+        Csum sum{0.0f, 0.0f};
         for (uint32_t t = 0; t < tiles; ++t) {
             const float2 q = partial[size_t(t) * S + s];
-            sum += double(q.x) + double(q.y);
+            csum_add(sum, q.x, q.y);
         }
-        diffuse = (double(skyc[s]) * double(L) + sum) / double(d);
+        h = diffuse_mean(sum, skyc[s], L, d);
     }
-    const float h = float(diffuse);
     out[s] = (0.0f < h) ? h : 0.0f;
 }
 

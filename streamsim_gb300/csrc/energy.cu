@@ -32,6 +32,7 @@
 // library's are).
 #include <cmath>
 
+#include "compensated.cuh"
 #include "internal.h"
 #include "optics_math.cuh"
 
@@ -156,82 +157,128 @@ __global__ void k_direct_geometry(uint32_t F, const facetcu_vertex* __restrict__
 }
 
 // Side-major copy of the first W columns of a column-major [R][S] block.
-__global__ void k_transpose(uint32_t S, uint32_t W, const float* __restrict__ B,
-                            float* __restrict__ BT)
+__global__ void __launch_bounds__(256) k_transpose(uint32_t S, uint32_t W, uint32_t stride,
+                                                   const float* __restrict__ B,
+                                                   float* __restrict__ BT)
 {
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= size_t(S) * W) return;
-    const uint32_t s = uint32_t(i / W), w = uint32_t(i % W);
-    BT[i] = B[size_t(w) * S + s];
+    __shared__ float tile[32][33];
+    const uint32_t s0 = blockIdx.x * 32u, w0 = blockIdx.y * 32u;
+    const uint32_t x = threadIdx.x & 31u, y = threadIdx.x >> 5;
+    for (uint32_t k = y; k < 32u; k += 8u)
+        tile[k][x] = w0 + k < W && s0 + x < S ? B[size_t(w0 + k) * S + s0 + x] : 0.0f;
+    __syncthreads();
+    for (uint32_t k = y; k < 32u; k += 8u)
+        if (s0 + k < S && w0 + x < stride) BT[size_t(s0 + k) * stride + w0 + x] = tile[x][k];
 }
 
-// Compensated FP32 sum of count x B terms: each product split exactly into
-// p + e (TwoProduct with an explicit fmaf) and each addition into s + err
-// (Neumaier's TwoSum); the errors accumulate in c.  sum + c then carries
-// about twice the float precision, as close to the reference's FP64 sum as
-// its conversion back to float can tell, at FP32 throughput (GB300's FP64
-// rate is a small fraction of it).
-struct Csum {
-    float s, c;
+// Compensated sums of two windows at once in packed registers.  (Knuth's TwoSum: the
+// same exact error as Neumaier's, without the comparison.)
+typedef unsigned long long Pair;  // two floats
+__device__ __forceinline__ Pair pair_of(float lo, float hi)
+{
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ Pair add2(Pair a, Pair b)
+{
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b)
+{
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c)
+{
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+struct Csum2 {
+    Pair s, c;
 };
-__device__ __forceinline__ void csum_add(Csum& a, float t, float e)
+__device__ __forceinline__ void csum_term(Csum2& a, uint32_t count, Pair v)
 {
-    const float s = a.s + t;
-    const float err = fabsf(a.s) >= fabsf(t) ? (a.s - s) + t : (t - s) + a.s;
-    a.s = s;
-    a.c += err + e;
-}
-__device__ __forceinline__ void csum_term(Csum& a, uint32_t count, float v)
-{
+    const Pair minus = pair_of(-1.0f, -1.0f);
     const float n = float(count);  // exact below 2^24
-    const float p = n * v;
-    csum_add(a, p, fmaf(n, v, -p));
+    const Pair n2 = pair_of(n, n), p = mul2(n2, v), e = fma2(n2, v, mul2(p, minus));
+    const Pair s = add2(a.s, p), grown = fma2(a.s, minus, s);
+    const Pair err = add2(fma2(fma2(grown, minus, s), minus, a.s), fma2(grown, minus, p));
+    a.s = s;
+    a.c = add2(a.c, add2(err, e));
 }
-__device__ __forceinline__ double csum_value(const Csum& a) { return double(a.s) + double(a.c); }
-
-// H[w][s] = max(0, diffuse + D): one warp per side, lane w of each 32-wide
-// window group sums its window's gather in the reference's edge order (each
-// edge is one broadcast load, its W values one contiguous row of BT).
-__global__ void k_window_incident(uint32_t S, uint32_t W, const uint32_t* __restrict__ rows,
-                                  const facetcu_csr_edge* __restrict__ edges,
-                                  const uint32_t* __restrict__ denom,
-                                  const uint32_t* __restrict__ skyc, const float* __restrict__ BT,
-                                  const float* __restrict__ sky, const float* __restrict__ dni,
-                                  const float* __restrict__ dgeo, float* __restrict__ H)
+__device__ __forceinline__ Csum half_of(const Csum2& a, int half)
 {
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t lane = threadIdx.x & 31u;
-    if (warp >= S) return;
-    const uint32_t s = warp;
-    const uint32_t d = denom[s], start = rows[s], end = rows[s + 1];
+    return {__uint_as_float(uint32_t(a.s >> (32 * half))),
+            __uint_as_float(uint32_t(a.c >> (32 * half)))};
+}
+
+// H[w][s] = max(0, diffuse + D): one warp per side, a pair of windows per lane
+// and as many edges at a time as there are groups of lanes for the pairs (three
+// for 20 windows).  A row of BT holds a side's windows in 128-byte lines of
+// their own where there are 17 to 32.  Bound by instructions and the gather's
+// rows: 2.18 ms for the 74 M edges of the 200,000-facet forest and 20 windows
+// with a window per lane, 1.08 here (issue 67 %).
+__global__ void __launch_bounds__(256) k_window_incident(
+    uint32_t S, uint32_t W, uint32_t stride, const uint32_t* __restrict__ rows,
+    const facetcu_csr_edge* __restrict__ edges, const uint32_t* __restrict__ denom,
+    const uint32_t* __restrict__ skyc, const float* __restrict__ BT, const float* __restrict__ sky,
+    const float* __restrict__ dni, const float* __restrict__ dgeo, float* __restrict__ H)
+{
+    constexpr int U = 4;
+    const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (s >= S) return;
+    const uint32_t d = denom[s], start = rows[s], end = d != 0u ? rows[s + 1] : start;
     const float g = dgeo ? dgeo[s] : 0.0f;
-    for (uint32_t w0 = 0; w0 < W; w0 += 32) {
-        const uint32_t w = w0 + lane;
-        const bool on = w < W;
-        const float L = on ? sky[w] : 0.0f;
-        double diffuse = L;
-        if (d != 0u) {
-            Csum acc{0.0f, 0.0f};
-            uint32_t e = start;
-            for (; e + 4 <= end; e += 4) {
-                facetcu_csr_edge ed[4];
-                float v[4];
+    for (uint32_t w0 = 0; w0 < W; w0 += 64) {
+        const uint32_t pairs = min(32u, (W - w0 + 1u) / 2u), groups = 32u / pairs;
+        const uint32_t group = lane / pairs, q = lane - group * pairs, w = w0 + 2u * q;
+        const float* base = BT + w;
+        Csum2 acc{0ull, 0ull};
+        if (group < groups) {
+            uint32_t e = start + group;
+            for (; e + (U - 1) * groups < end; e += groups * U) {
+                facetcu_csr_edge ed[U];
+                Pair v[U];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) ed[k] = edges[e + k];
+                for (int k = 0; k < U; ++k) ed[k] = edges[e + k * groups];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) v[k] = on ? BT[size_t(ed[k].neighbor) * W + w] : 0.0f;
+                for (int k = 0; k < U; ++k)
+                    v[k] = *reinterpret_cast<const Pair*>(base + size_t(ed[k].neighbor) * stride);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) csum_term(acc, ed[k].count, v[k]);
+                for (int k = 0; k < U; ++k) csum_term(acc, ed[k].count, v[k]);
             }
-            for (; e < end; ++e) {
+            for (; e < end; e += groups) {
                 const facetcu_csr_edge ed = edges[e];
-                csum_term(acc, ed.count, on ? BT[size_t(ed.neighbor) * W + w] : 0.0f);
+                csum_term(acc, ed.count,
+                          *reinterpret_cast<const Pair*>(base + size_t(ed.neighbor) * stride));
             }
-            diffuse = (double(skyc[s]) * double(L) + csum_value(acc)) / double(d);
         }
-        if (on) {
-            const float D = dgeo ? g * dni[w] : 0.0f;
-            H[size_t(w) * S + s] = smax(0.0f, float(diffuse) + D);
+        __syncwarp();
+        const Csum2 mine = acc;
+        Csum sum[2] = {half_of(acc, 0), half_of(acc, 1)};
+        for (uint32_t k = 1; k < groups; ++k) {
+            const int from = int(q + k * pairs);
+            const Csum2 other{__shfl_sync(0xffffffffu, mine.s, from),
+                              __shfl_sync(0xffffffffu, mine.c, from)};
+            for (int half = 0; half < 2; ++half) {
+                const Csum o = half_of(other, half);
+                csum_add(sum[half], o.s, o.c);
+            }
+        }
+        if (group) continue;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const uint32_t at = w + uint32_t(half);
+            if (at >= W) break;
+            const float L = sky[at];
+            const float diffuse = d != 0u ? diffuse_mean(sum[half], skyc[s], L, d) : L;
+            const float D = dgeo ? g * dni[at] : 0.0f;
+            H[size_t(at) * S + s] = smax(0.0f, diffuse + D);
         }
     }
 }
@@ -265,9 +312,7 @@ __global__ void k_incident_one(uint32_t S, const uint32_t* __restrict__ rows,
         csum_add(acc, os, oc);
     }
     if (lane == 0) {
-        double diffuse = L;
-        if (d != 0u) diffuse = (double(skyc[s]) * double(L) + csum_value(acc)) / double(d);
-        H[s] = smax(0.0f, float(diffuse));
+        H[s] = smax(0.0f, d != 0u ? diffuse_mean(acc, skyc[s], L, d) : L);
     }
 }
 
@@ -523,6 +568,11 @@ void direct_geometry(uint32_t F, const facetcu_vertex* V, facetcu_direction sun,
     FCU_LAUNCH("k_direct_geometry");
 }
 
+uint32_t window_stride(uint32_t W)
+{
+    return W <= 8 ? 8 : W <= 16 ? 16 : (W + 31) / 32 * 32;
+}
+
 void window_incident(const DeviceGraph& g, uint32_t W, const float* B, const float* sky,
                      const float* dni, const float* dgeo, float* BT, float* H, cudaStream_t s)
 {
@@ -542,10 +592,11 @@ void window_incident(const DeviceGraph& g, uint32_t W, const float* B, const flo
         FCU_LAUNCH("k_incident_one");
         return;
     }
-    k_transpose<<<blocks(S * W, 256), 256, 0, s>>>(uint32_t(S), W, B, BT);
+    const uint32_t stride = window_stride(W);
+    k_transpose<<<dim3(blocks(S, 32), (stride + 31) / 32), 256, 0, s>>>(uint32_t(S), W, stride, B, BT);
     FCU_LAUNCH("k_transpose");
-    k_window_incident<<<blocks(S * 32, 256), 256, 0, s>>>(uint32_t(S), W, rows, edges, den, skyc,
-                                                          BT, sky, dni, dgeo, H);
+    k_window_incident<<<blocks(S * 32, 256), 256, 0, s>>>(uint32_t(S), W, stride, rows, edges, den,
+                                                          skyc, BT, sky, dni, dgeo, H);
     FCU_LAUNCH("k_window_incident");
 }
 
