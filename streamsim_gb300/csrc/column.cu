@@ -315,23 +315,19 @@ __device__ __forceinline__ void comp_term(float& s, float& c, float n, float v)
 // queue of groups shared by the CTAs of a tile, longest first or in order, 100-125.
 // kComp: compensated sums, two floats per partial.
 template <bool kComp>
-__global__ void __launch_bounds__(kThreads, 1) k_gather(View v, const float* __restrict__ B,
+__global__ void __launch_bounds__(kThreads, 1) k_gather(View v, const float* B,
                                                         float* __restrict__ partial,
                                                         const uint32_t* done)
 {
-    if (done && *done) return;
     extern __shared__ __align__(16) float tile[];
+    start_next();
     const uint32_t lane = threadIdx.x & 31;
+    // The plan's own arrays first: no kernel that may still run writes them.
     const Share p = v.shares[blockIdx.x];
     const uint32_t at = p.tile * kTile, m = min(kTile, v.surfaces - at);
     __shared__ uint32_t queue;
     if (threadIdx.x == 0) queue = kThreads / 32;
     uint32_t g = p.begin + threadIdx.x / 32;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < m / 4; i += kThreads) cp_async16(tile + 4 * i, B + at + 4 * i);
-    if (threadIdx.x < (m & 3)) tile[(m & ~3u) + threadIdx.x] = B[at + (m & ~3u) + threadIdx.x];
-    cp_commit();
-    if (threadIdx.x == 0) tile[kPad] = 0.0f;
     const size_t out = size_t(p.tile) * v.surfaces;
     constexpr int U = 8;
     uint32_t meta = 0, meta1 = 0;          // heads of this group and the next
@@ -351,6 +347,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_gather(View v, const float* __r
 #pragma unroll
     for (int u = 0; u < U; ++u)
         if (uint32_t(u) < n) x[u] = __ldcs(w + u * 32);
+    wait_for_previous();
+    if (done && *done) return;
+    for (uint32_t i = threadIdx.x; i < m / 4; i += kThreads) cp_async16(tile + 4 * i, B + at + 4 * i);
+    if (threadIdx.x < (m & 3)) tile[(m & ~3u) + threadIdx.x] = B[at + (m & ~3u) + threadIdx.x];
+    cp_commit();
+    if (threadIdx.x == 0) tile[kPad] = 0.0f;
+    __syncthreads();  // the queue's start
     uint32_t g1 = take();
     if (g1 < p.end) {
         meta1 = __ldcs(v.meta + size_t(g1) * 32 + lane);
@@ -434,11 +437,12 @@ __device__ __forceinline__ float2 sum_pair(const float* partial, uint32_t tiles,
 
 // A thread per facet: the reference's update (as k_jacobi_rows in solve.cu).
 __global__ void __launch_bounds__(256) k_finish_jacobi(
-    uint32_t facets, uint32_t tiles, const float* __restrict__ partial,
-    const uint2* __restrict__ denom, const uint2* __restrict__ skyc,
-    const float4* __restrict__ optics, float sky, float relax, const float2* __restrict__ in,
-    float2* __restrict__ out, uint32_t* max_delta_bits)
+    uint32_t facets, uint32_t tiles, const float* partial, const uint2* __restrict__ denom,
+    const uint2* __restrict__ skyc, const float4* __restrict__ optics, float sky, float relax,
+    const float2* in, float2* out, uint32_t* max_delta_bits)
 {
+    start_next();
+    wait_for_previous();
     __shared__ float block_delta[8];
     const uint32_t f = blockIdx.x * 256 + threadIdx.x;
     float delta = 0.0f;
@@ -469,13 +473,13 @@ __global__ void __launch_bounds__(256) k_finish_jacobi(
 // A thread per facet: the batched solver's update and statistics (as
 // k_sweep<1> in batched.cu); in == nullptr stands for zeros.
 __global__ void __launch_bounds__(256) k_finish_panel(
-    uint32_t facets, uint32_t tiles, const float* __restrict__ partial,
-    const uint2* __restrict__ denom, const uint2* __restrict__ skyc, const float2* __restrict__ rho,
-    const float2* __restrict__ tau, const float2* __restrict__ emis,
-    const float2* __restrict__ direct, const float* __restrict__ skyL,
-    const float* __restrict__ colmax, const float2* __restrict__ in, float2* __restrict__ out,
+    uint32_t facets, uint32_t tiles, const float* partial, const uint2* __restrict__ denom,
+    const uint2* __restrict__ skyc, const float2* rho, const float2* tau, const float2* emis,
+    const float2* direct, const float* skyL, const float* colmax, const float2* in, float2* out,
     uint32_t* stats, const uint32_t* done)
 {
+    start_next();
+    wait_for_previous();
     if (*done) return;
     __shared__ float red[3][8];
     const uint32_t f = blockIdx.x * 256 + threadIdx.x;
@@ -511,10 +515,11 @@ __global__ void __launch_bounds__(256) k_finish_panel(
 // A thread per side: max(0, incident diffuse radiation) from compensated
 // partials (the FacetEB node).
 __global__ void __launch_bounds__(256) k_finish_incident(
-    uint32_t S, uint32_t tiles, const float2* __restrict__ partial,
-    const uint32_t* __restrict__ denom, const uint32_t* __restrict__ skyc,
-    const float* __restrict__ sky, float* __restrict__ out)
+    uint32_t S, uint32_t tiles, const float2* partial, const uint32_t* __restrict__ denom,
+    const uint32_t* __restrict__ skyc, const float* sky, float* out)
 {
+    start_next();
+    wait_for_previous();
     const uint32_t s = blockIdx.x * 256 + threadIdx.x;
     if (s >= S) return;
     const float L = sky[0];
@@ -537,6 +542,11 @@ float2* compensated(const DeviceGraph& g)
                                      size_t(g.column.tiles) * g.surfaces);
 }
 
+// The gathers and what finishes them follow one another without the 2 us
+// between two launches: each starts while the one before it ends and waits
+// inside, the gather with its plan's first words in registers (64 sweeps of the
+// 200,000-facet forest 6.91 -> 6.63 ms).  The arrays that a kernel before writes
+// are not __restrict__, so that no load of them moves above the wait.
 template <bool kComp>
 void gather(const DeviceGraph& g, const float* B, const uint32_t* done, cudaStream_t s)
 {
@@ -547,8 +557,7 @@ void gather(const DeviceGraph& g, const float* B, const uint32_t* done, cudaStre
     FCU_CHECK(cudaFuncSetAttribute(k_gather<kComp>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    smem));
     float* partial = kComp ? reinterpret_cast<float*>(compensated(g)) : c.partial.as<float>();
-    k_gather<kComp><<<c.ctas, kThreads, smem, s>>>(v, B, partial, done);
-    FCU_LAUNCH("k_gather");
+    launch_early(k_gather<kComp>, c.ctas, kThreads, smem, s, v, B, partial, done);
 }
 
 bool make_plan(DeviceGraph& g, Workspace& ws, cudaStream_t s)
@@ -693,11 +702,11 @@ void column_jacobi(const DeviceGraph& g, const facetcu_surface_optics* optics, f
 {
     const uint32_t facets = g.surfaces / 2;
     gather<false>(g, in, nullptr, s);
-    k_finish_jacobi<<<blocks(facets, 256), 256, 0, s>>>(
-        facets, g.column.tiles, g.column.partial.as<float>(), g.denominators.as<uint2>(),
-        g.sky.as<uint2>(), reinterpret_cast<const float4*>(optics), sky, relax,
-        reinterpret_cast<const float2*>(in), reinterpret_cast<float2*>(out), max_delta_bits);
-    FCU_LAUNCH("k_finish_jacobi");
+    launch_early(k_finish_jacobi, blocks(facets, 256), 256, 0, s, facets, g.column.tiles,
+                 g.column.partial.as<float>(), g.denominators.as<uint2>(), g.sky.as<uint2>(),
+                 reinterpret_cast<const float4*>(optics), sky, relax,
+                 reinterpret_cast<const float2*>(in), reinterpret_cast<float2*>(out),
+                 max_delta_bits);
 }
 
 void column_sweep(const DeviceGraph& g, const float* rho, const float* tau, const float* emis,
@@ -707,21 +716,18 @@ void column_sweep(const DeviceGraph& g, const float* rho, const float* tau, cons
     const uint32_t facets = g.surfaces / 2;
     if (in) gather<false>(g, in, done, s);
     auto pair = [](const float* p) { return reinterpret_cast<const float2*>(p); };
-    k_finish_panel<<<blocks(facets, 256), 256, 0, s>>>(
-        facets, g.column.tiles, g.column.partial.as<float>(), g.denominators.as<uint2>(),
-        g.sky.as<uint2>(), pair(rho), pair(tau), pair(emis), pair(direct), skyL, colmax, pair(in),
-        reinterpret_cast<float2*>(out), stats, done);
-    FCU_LAUNCH("k_finish_panel");
+    launch_early(k_finish_panel, blocks(facets, 256), 256, 0, s, facets, g.column.tiles,
+                 g.column.partial.as<float>(), g.denominators.as<uint2>(), g.sky.as<uint2>(),
+                 pair(rho), pair(tau), pair(emis), pair(direct), skyL, colmax, pair(in),
+                 reinterpret_cast<float2*>(out), stats, done);
 }
 
 void column_incident(const DeviceGraph& g, const float* B, const float* sky, float* out,
                      cudaStream_t s)
 {
     gather<true>(g, B, nullptr, s);
-    k_finish_incident<<<blocks(g.surfaces, 256), 256, 0, s>>>(
-        g.surfaces, g.column.tiles, compensated(g), g.denominators.as<uint32_t>(),
-        g.sky.as<uint32_t>(), sky, out);
-    FCU_LAUNCH("k_finish_incident");
+    launch_early(k_finish_incident, blocks(g.surfaces, 256), 256, 0, s, g.surfaces, g.column.tiles,
+                 compensated(g), g.denominators.as<uint32_t>(), g.sky.as<uint32_t>(), sky, out);
 }
 
 }  // namespace facetcu

@@ -32,6 +32,35 @@ inline void cuda_check(cudaError_t e, const char* what)
 #define FCU_CHECK(x) ::facetcu::cuda_check((x), #x)
 #define FCU_LAUNCH(what) ::facetcu::cuda_check(cudaGetLastError(), what)
 
+// A launch that may begin before the kernel in front of it has ended.  The
+// kernel calls wait_for_previous() before it touches anything that a kernel
+// before it writes or reads; the one in front says start_next() as early as it
+// likes.
+template <typename... P, typename... A>
+void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t shared, cudaStream_t s,
+                  A&&... args)
+{
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = shared;
+    config.stream = s;
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &early;
+    config.numAttrs = 1;
+    FCU_CHECK(cudaLaunchKernelEx(&config, kernel, P(args)...));
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void start_next()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
+
 // Owning device buffer that only grows.
 struct DeviceBuffer {
     void* ptr = nullptr;
