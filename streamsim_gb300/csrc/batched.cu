@@ -582,6 +582,8 @@ __global__ void __launch_bounds__(kWarps * 32, SweepBlocks<P>::value) k_sweep_wi
                                                             uint32_t* stats, uint32_t* counter,
                                                             const uint32_t* done)
 {
+    start_next();
+    wait_for_previous();
     if (*done) return;
     constexpr int CPL = 4;
     constexpr int L = P / CPL;
@@ -681,6 +683,8 @@ __global__ void __launch_bounds__(kWarps * 32, P == 8 ? 3 : 4) k_sweep_mid(Graph
                                                                uint32_t* stats, uint32_t* counter,
                                                                const uint32_t* done)
 {
+    start_next();
+    wait_for_previous();
     if (*done) return;
     static_assert(P == 8 || P == 16, "8 or 16 columns");
     constexpr int L = P / 4, G = 32 / L, U = 8, E = G * U, W = E / 32;
@@ -2089,6 +2093,8 @@ __global__ void k_check(uint32_t* stats, uint32_t* flag, int P, float tol, uint3
                         bool per_side, float* colmax, float* cheb = nullptr, int cheb_mode = 0,
                         const float* scale_prev = nullptr)
 {
+    start_next();
+    wait_for_previous();
     __shared__ int all_ok, abs_ok;
     __shared__ float worst;
     if (it_dev) it = *it_dev;  // the sweep index kept on the device (graph replays)
@@ -2403,6 +2409,8 @@ int grid_for(K kernel)
     return std::max(1, sms) * std::max(1, per_sm);
 }
 
+// (The FP32 sweeps of a panel and k_check follow one another: each is launched
+// while the one before it ends and waits inside.)
 template <typename T>
 void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in, T* out,
                   uint32_t* stats, uint32_t* counter, const uint32_t* done, cudaStream_t s)
@@ -2429,10 +2437,10 @@ void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in,
         if ((P == 8 || P == 16) && g.packed) {
             if (P == 8) {
                 static const int grid = grid_for(k_sweep_mid<8>);
-                k_sweep_mid<8><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                launch_early(k_sweep_mid<8>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
             } else {
                 static const int grid = grid_for(k_sweep_mid<16>);
-                k_sweep_mid<16><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                launch_early(k_sweep_mid<16>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
             }
             FCU_LAUNCH("k_sweep_mid");
             return;
@@ -2441,10 +2449,10 @@ void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in,
             // 16-byte row vectors in rounds of 8 loads per lane
             if (P == 8) {
                 static const int grid = grid_for(k_sweep_wide<8>);
-                k_sweep_wide<8><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                launch_early(k_sweep_wide<8>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
             } else {
                 static const int grid = grid_for(k_sweep_wide<16>);
-                k_sweep_wide<16><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                launch_early(k_sweep_wide<16>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
             }
             FCU_LAUNCH("k_sweep_wide");
             return;
@@ -2453,17 +2461,17 @@ void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in,
             switch (P) {
             case 32: {
                 static const int grid = grid_for(k_sweep_wide<32>);
-                k_sweep_wide<32><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                launch_early(k_sweep_wide<32>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
                 break;
             }
             case 64: {
                 static const int grid = grid_for(k_sweep_wide<64>);
-                k_sweep_wide<64><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                launch_early(k_sweep_wide<64>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
                 break;
             }
             default: {
                 static const int grid = grid_for(k_sweep_wide<128>);
-                k_sweep_wide<128><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                launch_early(k_sweep_wide<128>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
                 break;
             }
             }
@@ -3072,9 +3080,8 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                                                 reinterpret_cast<float*>(out), stats, counter,
                                                 flag, s);
                     });
-                    k_check<<<1, kMaxP, 0, s>>>(stats, flag, P, tol, sweep, counter, nullptr,
-                                                nullptr, nullptr, true, colmax);
-                    FCU_LAUNCH("k_check");
+                    launch_early(k_check, 1, kMaxP, 0, s, stats, flag, P, tol, sweep, counter, nullptr,
+                                 nullptr, nullptr, true, colmax, nullptr, 0, nullptr);
                     ++launches;
                 }
                 it += batch;
