@@ -16,14 +16,18 @@ namespace {
 // each lane has U edges in flight and the chain of dependent loads of a row
 // (offsets, edge words, neighbour values) is paid once for all of them.
 // (One thread per facet walked ~30 such chains: 7.2 us per sweep on the
-// 4,096-facet scene of 98,000 edges, 4.1 here.)  L follows the mean row length.
-template <int L>
+// 4,096-facet scene of 98,000 edges, 4.1 here, 2.9 where a sweep begins while
+// the one before it ends: 64 sweeps 333 -> 243 us, of 1.3 M edges 669 -> 521.)
+// L follows the mean row length.
+// kEarly: launched while the sweep before it ends; only Bin is waited for.
+template <int L, bool kEarly>
 __global__ void __launch_bounds__(256) k_jacobi_rows(
     uint32_t facets, const uint32_t* __restrict__ rows, const facetcu_csr_edge* __restrict__ edges,
     const uint32_t* __restrict__ denom, const uint32_t* __restrict__ skyc,
     const facetcu_surface_optics* __restrict__ optics, float sky, float relax,
-    const float* __restrict__ Bin, float* __restrict__ Bout, uint32_t* max_delta_bits)
+    const float* Bin, float* Bout, uint32_t* max_delta_bits)
 {
+    if (kEarly) start_next();
     constexpr int U = 4;
     __shared__ float block_delta[8];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -35,14 +39,19 @@ __global__ void __launch_bounds__(256) k_jacobi_rows(
     float acc = 0.0f, old = 0.0f;
     uint32_t d = 0, sc = 0;
     facetcu_surface_optics o{};
+    uint32_t start = 0, end = 0;
     if (valid) {
-        const uint32_t start = rows[s], end = rows[s + 1];
+        start = rows[s];
+        end = rows[s + 1];
         d = denom[s];
         if (eg == 0) {
             sc = skyc[s];
             o = optics[s];
-            old = Bin[s];
         }
+    }
+    if (kEarly) wait_for_previous();
+    if (valid) {
+        if (eg == 0) old = Bin[s];
         for (uint32_t e = start + eg; e < end; e += L * U) {
             facetcu_csr_edge ed[U];
             float v[U];
@@ -79,25 +88,25 @@ __global__ void __launch_bounds__(256) k_jacobi_rows(
 }
 
 // ---- all sweeps of a small graph in one launch ----------------------------
-// A sweep of 98,000 edges takes 2.6 us on the device and its launch 5 us of the
-// host, so 64 of them took 333 us.  Here a cluster of 16 blocks runs all of
-// them in 175 (249 with the copies): every block holds the whole radiosity
-// twice (this sweep's and the next), its share of the sides and their edges in
-// shared memory, and writes its new values into the others'.  Bound by the
-// exchange and the cluster's barrier (1 us a sweep for 1,152 sides, 2.5 for
-// 8,192); blocks that wait on a count of received bytes instead (asynchronous
-// stores, bulk copies) gave 291 and 232.
-// The cluster's 16 SMs are the limit for larger graphs; a solve of 64 sweeps in
-// single launches and here, us:
-//     edges    6,708   40,442   98,058   138,606   325,582   610,067
-//     launches   306      332      333       408       486       465
-//     cluster    126      212      249       264       435       511
-// (two lanes a side; four: 125, 235, 279, 278, 468, 499; eight blocks: 304 at
-// 98,058 edges.)  Setting up costs as much as some launches: 6,708 edges break
-// even at 3 sweeps (48, 50), 98,058 at 6 (90, 89), 325,582 at 12 (160, 161).
+// A sweep of the smallest graphs is shorter than a launch, even one that begins
+// early.  Here a cluster of 16 blocks runs all of them: every block holds the
+// whole radiosity twice (this sweep's and the next), its share of the sides and
+// their edges in shared memory, and writes its new values into the others'.
+// Bound by that exchange and the cluster's barrier: 1 us a sweep for 1,152
+// sides, 2.5 for 8,192 (with blocks that wait on a count of received bytes
+// instead, 2.2 by bulk copies and 3.2 by asynchronous stores).  64 sweeps in
+// early launches and here, us:
+//     sides      1,152   2,048   3,200   4,608   6,272   8,192
+//     edges      6,708  18,923  33,350  50,392  72,020  98,058
+//     launches     160     173     187     202     211     243
+//     cluster      126     142     160     195     225     249
+// (two lanes a side; four: 125 and 279 for the first and the last; eight blocks:
+// 304 for the last.)  Setting up costs some launches: 8 sweeps of 6,708 edges
+// take 58 and 59, 12 take 64 and 60.
 constexpr uint32_t kCtas = 16, kClusterThreads = 1024, kGroup = 16, kDeltas = 64;
 constexpr int kClusterLanes = 2;
-constexpr uint64_t kClusterEdges = 400000;
+constexpr uint32_t kClusterSides = 4096, kClusterSweeps = 12;
+constexpr uint64_t kClusterEdges = 100000;
 constexpr size_t kClusterShared = 227 * 1024 - 1024;  // (static arrays besides)
 
 struct ClusterShape {
@@ -272,24 +281,43 @@ __global__ void __launch_bounds__(128) k_incident(
 
 }  // namespace
 
+namespace {
+
+template <bool kEarly>
+void sweep_rows(uint32_t surfaces, uint64_t edges_hint, const uint32_t* rows,
+                const facetcu_csr_edge* edges, const uint32_t* denom, const uint32_t* skyc,
+                const facetcu_surface_optics* d_optics, float sky, float relaxation,
+                const float* d_in, float* d_out, uint32_t* d_max_delta_bits, cudaStream_t s)
+{
+    const uint32_t facets = surfaces / 2u;
+    if (!facets) return;
+    auto launch = [&](auto kernel, uint32_t lanes) {
+        const unsigned grid = unsigned((uint64_t(surfaces) * lanes + 255) / 256);
+        if (kEarly)
+            launch_early(kernel, grid, 256, 0, s, facets, rows, edges, denom, skyc, d_optics, sky,
+                         relaxation, d_in, d_out, d_max_delta_bits);
+        else
+            kernel<<<grid, 256, 0, s>>>(facets, rows, edges, denom, skyc, d_optics, sky, relaxation,
+                                        d_in, d_out, d_max_delta_bits);
+    };
+    const uint64_t mean = edges_hint / surfaces;
+    if (mean < 8) launch(k_jacobi_rows<4, kEarly>, 4);
+    else if (mean < 48) launch(k_jacobi_rows<8, kEarly>, 8);
+    else launch(k_jacobi_rows<16, kEarly>, 16);
+    FCU_LAUNCH("k_jacobi_rows");
+}
+
+}  // namespace
+
+// (The caller's arrays may have been written by the kernel just before: no
+// early start here.)
 void jacobi_sweep_raw(uint32_t surfaces, uint64_t edges_hint, const uint32_t* rows,
                       const facetcu_csr_edge* edges, const uint32_t* denom, const uint32_t* skyc,
                       const facetcu_surface_optics* d_optics, float sky, float relaxation,
                       const float* d_in, float* d_out, uint32_t* d_max_delta_bits, cudaStream_t s)
 {
-    const uint32_t facets = surfaces / 2u;
-    if (!facets) return;
-    auto launch = [&](auto kernel, uint32_t lanes) {
-        const uint64_t threads = uint64_t(surfaces) * lanes;
-        kernel<<<unsigned((threads + 255) / 256), 256, 0, s>>>(facets, rows, edges, denom, skyc,
-                                                              d_optics, sky, relaxation, d_in,
-                                                              d_out, d_max_delta_bits);
-    };
-    const uint64_t mean = edges_hint / surfaces;
-    if (mean < 8) launch(k_jacobi_rows<4>, 4);
-    else if (mean < 48) launch(k_jacobi_rows<8>, 8);
-    else launch(k_jacobi_rows<16>, 16);
-    FCU_LAUNCH("k_jacobi_rows");
+    sweep_rows<false>(surfaces, edges_hint, rows, edges, denom, skyc, d_optics, sky, relaxation, d_in,
+                      d_out, d_max_delta_bits, s);
 }
 
 void jacobi_sweep(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
@@ -300,7 +328,7 @@ void jacobi_sweep(const DeviceGraph& g, const facetcu_surface_optics* d_optics, 
         column_jacobi(g, d_optics, sky, relaxation, d_in, d_out, d_max_delta_bits, s);
         return;
     }
-    jacobi_sweep_raw(g.surfaces, g.nnz, g.row_offsets.as<uint32_t>(), g.edges.as<facetcu_csr_edge>(),
+    sweep_rows<true>(g.surfaces, g.nnz, g.row_offsets.as<uint32_t>(), g.edges.as<facetcu_csr_edge>(),
                      g.denominators.as<uint32_t>(), g.sky.as<uint32_t>(), d_optics, sky, relaxation,
                      d_in, d_out, d_max_delta_bits, s);
 }
@@ -310,18 +338,17 @@ bool jacobi_sweeps_cluster(const DeviceGraph& g, const facetcu_surface_optics* d
                            uint32_t* d_max_delta_bits, cudaStream_t s)
 {
     const uint32_t S = g.surfaces;
-    if (sweeps < 5 + g.nnz / 50000 || S < 2 || S > 0xffffu || g.max_count > 0xffffu || g.nnz > kClusterEdges)
+    if (sweeps < kClusterSweeps || S < 2 || S > kClusterSides || g.nnz > kClusterEdges ||
+        g.max_count > 0xffffu)
         return false;
     ClusterShape shape;
     const uint32_t groups = (S + kGroup - 1) / kGroup;
     shape.owned = (groups + kCtas - 1) / kCtas * kGroup;
     shape.padded = shape.owned * kCtas;
     const size_t fixed = size_t(shape.padded) * 8 + size_t(shape.owned) * 28 + 16;
-    if (fixed >= kClusterShared) return false;
-    // an even share of the edges fits; a block whose share is larger than what
-    // it has room for reads the rest from memory
+    // a block whose share of the edges is larger than what it has room for
+    // reads the rest from memory
     const size_t room = (kClusterShared - fixed) / 4;
-    if (g.nnz / kCtas > room) return false;
     shape.words = uint32_t(std::min<size_t>(room, g.nnz / kCtas * 2 + 1024));
     auto kernel = k_jacobi_cluster<kClusterLanes>;
     const size_t shared = fixed + size_t(shape.words) * 4;
