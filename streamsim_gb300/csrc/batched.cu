@@ -13,7 +13,9 @@
 // vector load per lane per edge (float / float2 / float4 in FP32, 1/2/4
 // packed BF16 in the defect sweep), one warp shuffle per packed 4-byte edge
 // (22-bit neighbour, 10-bit count), full 32-edge chunks without predication.
-// Narrow panels (P < 32, few RHS) split the warp into 32/P edge groups.
+// 8 and 16 columns on the packed graph have a sweep of their own
+// (k_sweep_mid), one column of a large graph the column plan (column.cu); other
+// narrow panels split the warp into 32/P edge groups.
 // The graph is renumbered once along a Morton curve of facet centroids and
 // every warp sweeps a contiguous run of facets, so the neighbour rows a CTA
 // touches stay hot in L1/L2.  The grid is persistent (a multiple of the SM
@@ -1836,13 +1838,11 @@ __global__ void k_scene_init_sigma(uint32_t* mdr, float* sig, float* cheb, uint3
 }
 
 // R = Y - X and Q = round(R / sigma) for the first int8 step (X unchanged).
-// X null: X is 0 and Y itself becomes R (the caller takes the two buffers for
-// one another).  Four columns a thread; n4 = cells / 4.  Bound by the planes:
+// R may be Y's own buffer; with X null, X is 0 and Y is R already.  Four columns a thread; n4 = cells / 4.  Bound by the planes:
 // on 400,000 sides of 64 columns 108 us with a column a thread, two planes in
 // and R and Q out; 35 from zero.
 __global__ void __launch_bounds__(256) k_init_i8(
-    const float4* __restrict__ X, const float4* __restrict__ Y, float4* __restrict__ R,
-    char4* __restrict__ Q, const float* __restrict__ sig, uint32_t n4, uint32_t P, uint32_t* it_dev,
+    const float4* __restrict__ X, const float4* Y, float4* R, char4* __restrict__ Q, const float* __restrict__ sig, uint32_t n4, uint32_t P, uint32_t* it_dev,
     uint32_t it, const uint16_t* __restrict__ scene = nullptr,
     const float* __restrict__ scene_sig = nullptr)
 {
@@ -3137,6 +3137,9 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                     continue;
                 }
                 const bool from_zero = it == 1 && zero_start;  // X is 0: R is Y
+                // The first residual takes Y's place, later ones are written
+                // where it was (the captured steps know one R).
+                const bool in_place = res == rbuf;
                 if (g.scene) {
                     // every scene takes part in a new int8 phase, with its
                     // own first scales max|Y - X| / 127
@@ -3152,11 +3155,11 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                 }
                 k_init_i8<<<blocks_for(cells / 4, 256), 256, 0, s>>>(
                     reinterpret_cast<const float4*>(from_zero ? nullptr : X),
-                    reinterpret_cast<const float4*>(Y), reinterpret_cast<float4*>(res),
+                    reinterpret_cast<const float4*>(Y), reinterpret_cast<float4*>(in_place ? Y : res),
                     reinterpret_cast<char4*>(qb[0]), slot[0], uint32_t(cells / 4), uint32_t(P),
                     flag + 12, it, g.scene, g.scene_sig);
                 FCU_LAUNCH("k_init_i8");
-                if (from_zero) std::swap(res, Y);
+                if (in_place) std::swap(res, Y);
                 ++launches;
                 uint32_t j = 0;
                 bool steps_done = false;

@@ -382,7 +382,7 @@ int batched_solve(const DeviceGraph& g, const BatchProblem& p, const facetcu_bat
 // ---- hemisphere ray casting (lbvh.cu, hemi.cu) ----------------------------
 struct Lbvh {
     uint32_t leaves = 0;
-    DeviceBuffer nodes;      // internal nodes: 2 children (u32, leaf bit 31) + aabb
+    DeviceBuffer nodes;      // 64-byte nodes of four children, boxes in 7 bits
     DeviceBuffer tri;        // per sorted leaf: a, e1, e2 (9 floats) + facet id
     DeviceBuffer parent;     // build scratch
     DeviceBuffer flags;      // build scratch

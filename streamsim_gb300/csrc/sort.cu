@@ -1,8 +1,8 @@
 // sort.cu — device exclusive scan and stable LSD radix sort.
 //
-// Both are written for the graph build: the scan turns per-pixel fragment
-// counts into list offsets, the sort groups (side, side) pair keys so that
-// the symmetric CSR comes out row-sorted and deterministic (the reference
+// Both are written for the graph build: the scan turns row lengths and marks
+// into offsets, the sort groups (side, side) pair keys so that the symmetric
+// CSR comes out row-sorted and deterministic (the reference
 // uses a hash map on the CPU, facetrtcore.cpp:1358-1412, and a 64-bit-key
 // GPU hash compacted on the host, facetrt_vulkan.cpp:979-1037).
 #include "internal.h"
