@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(256) k_raster(const float4* __restrict__ plane
                                                 Pool pool, uint32_t* jobs, uint32_t items,
                                                 RasterStats* stats, uint32_t* frags)
 {
+    start_next();
     __shared__ Room room;
     __shared__ uint32_t warp_mid[8], warp_big[8], base_mid, base_big;
     const uint32_t w = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31u,
@@ -402,10 +403,12 @@ __device__ __forceinline__ void load_job(const float4* planes, uint32_t per_dir,
 template <uint32_t kLanes>
 __global__ void __launch_bounds__(256) k_raster_mid(const float4* __restrict__ planes,
                                                     uint32_t per_dir, Pool pool,
-                                                    const uint32_t* __restrict__ jobs,
-                                                    const uint32_t* __restrict__ job_count,
+                                                    const uint32_t* jobs,
+                                                    const uint32_t* job_count,
                                                     uint32_t* frags)
 {
+    start_next();
+    wait_for_previous();
     __shared__ Room room;
     const uint32_t count = *job_count;
     constexpr uint32_t kJobs = 256 / kLanes, kSpan = 32 * kLanes;
@@ -424,10 +427,12 @@ __global__ void __launch_bounds__(256) k_raster_mid(const float4* __restrict__ p
 
 __global__ void __launch_bounds__(256) k_raster_big(const float4* __restrict__ planes,
                                                     uint32_t per_dir, Pool pool,
-                                                    const uint32_t* __restrict__ jobs_end,
-                                                    const uint32_t* __restrict__ job_count,
+                                                    const uint32_t* jobs_end,
+                                                    const uint32_t* job_count,
                                                     uint32_t* frags)
 {
+    start_next();
+    wait_for_previous();
     __shared__ Room room;
     const uint32_t count = *job_count, warp = threadIdx.x >> 5;
     for (uint32_t k = blockIdx.x; k < count; k += gridDim.x) {
@@ -997,12 +1002,10 @@ void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame
         k_raster<<<dim3(unsigned((per_dir + 255) / 256), dir_count), 256, 0, s>>>(
             planes, uint32_t(per_dir), pool, jobs, uint32_t(items), dstats, counted);
         FCU_LAUNCH("k_raster");
-        k_raster_mid<kMidLanes><<<unsigned(std::min<uint64_t>((items + 31) / 32, 8 * 152)), 256, 0, s>>>(
-            planes, uint32_t(per_dir), pool, jobs, &dstats->mid, counted);
-        FCU_LAUNCH("k_raster_mid");
-        k_raster_big<<<dim3(unsigned(std::min<uint64_t>(items, 152)), 16), 256, 0, s>>>(
-            planes, uint32_t(per_dir), pool, jobs + items, &dstats->big, counted);
-        FCU_LAUNCH("k_raster_big");
+        launch_early(k_raster_mid<kMidLanes>, unsigned(std::min<uint64_t>((items + 31) / 32, 8 * 152)),
+                     256, 0, s, planes, uint32_t(per_dir), pool, jobs, &dstats->mid, counted);
+        launch_early(k_raster_big, dim3(unsigned(std::min<uint64_t>(items, 152)), 16), 256, 0, s, planes,
+                     uint32_t(per_dir), pool, jobs + items, &dstats->big, counted);
         FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
         FCU_CHECK(cudaStreamSynchronize(s));
         if (host.fragments >= (1ull << 32))

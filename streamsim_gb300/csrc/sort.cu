@@ -117,6 +117,8 @@ __global__ void __launch_bounds__(kThreads) k_digit_histogram(const uint64_t* ke
                                                               int shift, uint32_t* hist,
                                                               uint32_t blocks)
 {
+    start_next();
+    wait_for_previous();
     __shared__ uint32_t h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -134,6 +136,8 @@ __global__ void __launch_bounds__(kThreads) k_digit_histogram(const uint64_t* ke
 __global__ void __launch_bounds__(kThreads) k_digit_scan(uint32_t* hist, uint32_t blocks,
                                                          uint32_t* totals)
 {
+    start_next();
+    wait_for_previous();
     __shared__ uint32_t ws[kThreads / 32];
     uint32_t* row = hist + size_t(blockIdx.x) * blocks;
     uint32_t carry = 0;
@@ -162,6 +166,8 @@ __global__ void __launch_bounds__(kThreads) k_digit_scatter(
     const uint64_t* keys, const uint32_t* values, uint64_t* keys_out, uint32_t* values_out,
     size_t n, int shift, const uint32_t* offsets, const uint32_t* totals, uint32_t blocks)
 {
+    start_next();
+    wait_for_previous();
     __shared__ uint32_t s_base[256];
     __shared__ uint32_t s_scan[kThreads / 32];
     __shared__ uint32_t s_warp[kThreads / 32][256];
@@ -247,7 +253,8 @@ void exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n,
 
 // Three launches a digit: the digits' own bases are scanned by every scattering
 // block, which costs less than the launches of a scan over all counts (the
-// graph of 164,000 pairs took 64 launches in its two sorts; 18 now).
+// graph of 164,000 pairs took 64 launches in its two sorts; 18 now).  Each is
+// launched while the one before it ends and waits inside.
 void radix_sort_u64(uint64_t*& keys, uint64_t*& keys_alt, uint32_t*& values,
                     uint32_t*& values_alt, size_t n, int first_bit, int end_bit, Workspace& ws,
                     cudaStream_t s)
@@ -257,13 +264,10 @@ void radix_sort_u64(uint64_t*& keys, uint64_t*& keys_alt, uint32_t*& values,
     uint32_t* hist = static_cast<uint32_t*>(ws.c.reserve((size_t(blocks) + 1) * 256 * 4));
     uint32_t* totals = hist + size_t(blocks) * 256;
     for (int shift = first_bit; shift < end_bit; shift += 8) {
-        k_digit_histogram<<<blocks, kThreads, 0, s>>>(keys, n, shift, hist, blocks);
-        FCU_LAUNCH("k_digit_histogram");
-        k_digit_scan<<<256, kThreads, 0, s>>>(hist, blocks, totals);
-        FCU_LAUNCH("k_digit_scan");
-        k_digit_scatter<<<blocks, kThreads, 0, s>>>(keys, values, keys_alt, values_alt, n, shift,
-                                                    hist, totals, blocks);
-        FCU_LAUNCH("k_digit_scatter");
+        launch_early(k_digit_histogram, blocks, kThreads, 0, s, keys, n, shift, hist, blocks);
+        launch_early(k_digit_scan, 256, kThreads, 0, s, hist, blocks, totals);
+        launch_early(k_digit_scatter, blocks, kThreads, 0, s, keys, values, keys_alt, values_alt, n,
+                     shift, hist, totals, blocks);
         std::swap(keys, keys_alt);
         if (values) std::swap(values, values_alt);
     }
