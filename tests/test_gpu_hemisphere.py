@@ -220,3 +220,20 @@ def test_hemisphere_sizes_bit_exact(oracle, rays, top_k, leaves, grid, neighbour
         assert np.array_equal(lit, oracle.hemisphere_sunlit(sc.vertices, uv[:, :n], n, 4, sun,
                                                             periodic=periodic))
     m.close()
+
+
+@pytest.mark.parametrize("samples", [33, 64, 128, 129, 255, 300])
+@pytest.mark.parametrize("leaves,grid", [(1, 1), (37, 3), (300, 5)])
+def test_sun_samples_shared_by_warps(oracle, samples, leaves, grid):
+    """Two, four and eight warps to a facet, with facets that leave the last
+    block in part empty and samples that leave some of the warps without any."""
+    sc = scenes.config1(seed=samples, leaves=leaves, grid=grid)
+    uv, _ = scenes.hemisphere_samples(samples, 4, seed=samples)
+    m = facetcu.FacetrtCuda()
+    m.initialize(64, 64, 64)
+    m.setGeometry(sc.vertices)
+    for sun in ([0.0, 1.0, 0.0], [0.6, 0.5, -0.3]):
+        sun = np.float32(sun) / np.float32(np.linalg.norm(sun))
+        lit = m.hemisphereSunlit(sun, uv, samples, 4)
+        assert np.array_equal(lit, oracle.hemisphere_sunlit(sc.vertices, uv, samples, 4, sun))
+    m.close()
