@@ -21,6 +21,8 @@
 // is grown to the exact number and the chunk rasterised again.  A facet's
 // fragments are counted by the threads that rasterise it, not fragment by
 // fragment when the lists are resolved.
+#include <algorithm>
+
 #include "internal.h"
 
 namespace facetcu {
@@ -43,8 +45,14 @@ constexpr uint32_t kDeepChain = 1024;  // capacity of the deep-chain resolve
 constexpr uint32_t kResolvePixels = 2048;  // pixels of a resolving block
 constexpr uint32_t kKeyMask = 0x7fffffffu;
 
-__constant__ RasterView c_views[64];
-__constant__ RasterFrame c_frame;
+// What a raster kernel looks at, by value in its parameters: __constant__
+// copies would be one per device, and another context's build on its own stream
+// would change them between this one's kernels.
+constexpr uint32_t kMaxViews = 64;
+struct Scene {
+    RasterFrame frame;
+    RasterView views[kMaxViews];
+};
 
 struct Projected {
     float x[3], y[3], d[3];
@@ -56,15 +64,16 @@ __device__ __forceinline__ float dot3(const float a[3], float b0, float b1, floa
 }
 
 // facetrtcore.cpp:1259-1275
-__device__ __forceinline__ void project_vertex(float px, float py, float pz, uint32_t tile,
-                                               const RasterView& v, float& x, float& y, float& d)
+__device__ __forceinline__ void project_vertex(const RasterFrame& frame, float px, float py,
+                                               float pz, uint32_t tile, const RasterView& v,
+                                               float& x, float& y, float& d)
 {
-    const float r = c_frame.radius;
-    const float rx = (px + c_frame.tile_dx[tile]) - c_frame.center[0];
-    const float ry = py - c_frame.center[1];
-    const float rz = (pz + c_frame.tile_dz[tile]) - c_frame.center[2];
-    x = (0.5f + 0.5f * dot3(v.right, rx, ry, rz) / r) * float(c_frame.width);
-    y = (0.5f + 0.5f * dot3(v.up, rx, ry, rz) / r) * float(c_frame.height);
+    const float r = frame.radius;
+    const float rx = (px + frame.tile_dx[tile]) - frame.center[0];
+    const float ry = py - frame.center[1];
+    const float rz = (pz + frame.tile_dz[tile]) - frame.center[2];
+    x = (0.5f + 0.5f * dot3(v.right, rx, ry, rz) / r) * float(frame.width);
+    y = (0.5f + 0.5f * dot3(v.up, rx, ry, rz) / r) * float(frame.height);
     d = 0.5f - dot3(v.view, rx, ry, rz) / (2.0f * r);
 }
 
@@ -87,33 +96,33 @@ __global__ void k_planes(const facetcu_vertex* __restrict__ V, uint32_t facets,
 struct Facet {
     float4 q0, q1, q2;
 };
-__device__ __forceinline__ Facet load_facet(const float4* planes, uint32_t f)
+__device__ __forceinline__ Facet load_facet(const RasterFrame& frame, const float4* planes, uint32_t f)
 {
-    const size_t F = c_frame.facets;
+    const size_t F = frame.facets;
     return {__ldg(planes + f), __ldg(planes + F + f), __ldg(planes + 2 * F + f)};
 }
 __device__ __forceinline__ uint32_t facing(const Facet& t, const RasterView& v)
 {
     return dot3(v.view, t.q2.y, t.q2.z, t.q2.w) >= 0.0f ? 0u : 1u;
 }
-__device__ __forceinline__ void project(const Facet& t, uint32_t tile, const RasterView& v,
-                                        Projected& p)
+__device__ __forceinline__ void project(const RasterFrame& frame, const Facet& t, uint32_t tile,
+                                        const RasterView& v, Projected& p)
 {
-    project_vertex(t.q0.x, t.q0.y, t.q0.z, tile, v, p.x[0], p.y[0], p.d[0]);
-    project_vertex(t.q0.w, t.q1.x, t.q1.y, tile, v, p.x[1], p.y[1], p.d[1]);
-    project_vertex(t.q1.z, t.q1.w, t.q2.x, tile, v, p.x[2], p.y[2], p.d[2]);
+    project_vertex(frame, t.q0.x, t.q0.y, t.q0.z, tile, v, p.x[0], p.y[0], p.d[0]);
+    project_vertex(frame, t.q0.w, t.q1.x, t.q1.y, tile, v, p.x[1], p.y[1], p.d[1]);
+    project_vertex(frame, t.q1.z, t.q1.w, t.q2.x, tile, v, p.x[2], p.y[2], p.d[2]);
 }
 // The same by kLanes lanes: they take a corner each and exchange.
 template <uint32_t kLanes>
-__device__ __forceinline__ void project_lanes(const Facet& t, uint32_t tile, const RasterView& v,
-                                             Projected& p)
+__device__ __forceinline__ void project_lanes(const RasterFrame& frame, const Facet& t, uint32_t tile,
+                                              const RasterView& v, Projected& p)
 {
     const uint32_t c = (threadIdx.x % kLanes) % 3u;
     const float px = c == 0u ? t.q0.x : c == 1u ? t.q0.w : t.q1.z;
     const float py = c == 0u ? t.q0.y : c == 1u ? t.q1.x : t.q1.w;
     const float pz = c == 0u ? t.q0.z : c == 1u ? t.q1.y : t.q2.x;
     float x, y, d;
-    project_vertex(px, py, pz, tile, v, x, y, d);
+    project_vertex(frame, px, py, pz, tile, v, x, y, d);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         p.x[k] = __shfl_sync(0xffffffffu, x, k, kLanes);
@@ -150,15 +159,15 @@ struct Bbox {
 };
 
 // facetrtcore.cpp:1292-1308
-__device__ __forceinline__ Bbox triangle_bbox(const Projected& p)
+__device__ __forceinline__ Bbox triangle_bbox(const RasterFrame& frame, const Projected& p)
 {
     Bbox b;
     b.area = edgef(p.x[0], p.y[0], p.x[1], p.y[1], p.x[2], p.y[2]);
     b.valid = !(fabsf(b.area) < 1.0e-8f);
     b.x0 = max(0, int(floorf(min3(p.x[0], p.x[1], p.x[2]))));
-    b.x1 = min(int(c_frame.width) - 1, int(ceilf(max3(p.x[0], p.x[1], p.x[2]))));
+    b.x1 = min(int(frame.width) - 1, int(ceilf(max3(p.x[0], p.x[1], p.x[2]))));
     b.y0 = max(0, int(floorf(min3(p.y[0], p.y[1], p.y[2]))));
-    b.y1 = min(int(c_frame.height) - 1, int(ceilf(max3(p.y[0], p.y[1], p.y[2]))));
+    b.y1 = min(int(frame.height) - 1, int(ceilf(max3(p.y[0], p.y[1], p.y[2]))));
     if (b.x1 < b.x0 || b.y1 < b.y0) b.valid = false;
     return b;
 }
@@ -240,7 +249,8 @@ __device__ __forceinline__ uint32_t scan_inclusive(uint32_t v)
 // Bound by instructions (69 % of the issue slots; nine IEEE divides to project
 // a triangle): 351 us for the 8 M triangles of the forest, where counting and
 // filling in two passes took 268 + 448.
-__global__ void __launch_bounds__(256) k_raster(const float4* __restrict__ planes, uint32_t per_dir,
+__global__ void __launch_bounds__(256) k_raster(const __grid_constant__ Scene scene,
+                                                const float4* __restrict__ planes, uint32_t per_dir,
                                                 Pool pool, uint32_t* jobs, uint32_t items,
                                                 RasterStats* stats, uint32_t* frags)
 {
@@ -255,12 +265,13 @@ __global__ void __launch_bounds__(256) k_raster(const float4* __restrict__ plane
     b.valid = false;
     uint32_t box = 0, side = 0, key = 0, mask = 0;
     if (w < per_dir) {
-        const uint32_t tile = c_frame.tiles == 1u ? 0u : w / c_frame.facets;
-        const uint32_t facet = w - tile * c_frame.facets;
-        const Facet t = load_facet(planes, facet);
-        const uint32_t flip = facing(t, c_views[blockIdx.y]);
-        project(t, tile, c_views[blockIdx.y], p);
-        b = triangle_bbox(p);
+        const RasterFrame& frame = scene.frame;
+        const uint32_t tile = frame.tiles == 1u ? 0u : w / frame.facets;
+        const uint32_t facet = w - tile * frame.facets;
+        const Facet t = load_facet(frame, planes, facet);
+        const uint32_t flip = facing(t, scene.views[blockIdx.y]);
+        project(frame, t, tile, scene.views[blockIdx.y], p);
+        b = triangle_bbox(frame, p);
         key = w | (flip << 31);
         side = 2u * facet + flip;
         if (b.valid) box = uint32_t(b.x1 - b.x0 + 1) * uint32_t(b.y1 - b.y0 + 1);
@@ -289,13 +300,14 @@ __global__ void __launch_bounds__(256) k_raster(const float4* __restrict__ plane
         (threadIdx.x ? base_big : base_mid) = all;
     }
     if (mask) {
-        const size_t plane = size_t(blockIdx.y) * c_frame.width * c_frame.height;
+        const uint32_t width = scene.frame.width;
+        const size_t plane = size_t(blockIdx.y) * width * scene.frame.height;
         for (int y = b.y0; y <= b.y1; ++y) {
             for (int x = b.x0; x <= b.x1; ++x, mask >>= 1) {
                 if (!(mask & 1u)) continue;
                 float depth;
                 cover(p, b.area, x, y, depth);
-                put(pool, plane + size_t(y) * c_frame.width + size_t(x), slot++, depth, key);
+                put(pool, plane + size_t(y) * width + size_t(x), slot++, depth, key);
             }
         }
     }
@@ -314,7 +326,7 @@ __global__ void __launch_bounds__(256) k_raster(const float4* __restrict__ plane
 // The atomics of four steps are in flight together.
 template <uint32_t kLanes>
 __device__ __forceinline__ void raster_span(const Projected& p, const Bbox& b, size_t plane,
-                                            uint32_t key, uint32_t first, uint32_t count,
+                                            uint32_t width, uint32_t key, uint32_t first, uint32_t count,
                                             const Pool& pool, Room& room, uint32_t* count_at)
 {
     const uint32_t lane = threadIdx.x & 31u, sub = lane % kLanes;
@@ -358,7 +370,7 @@ __device__ __forceinline__ void raster_span(const Projected& p, const Bbox& b, s
             if (at[k] < pool.capacity) {
                 const int x = b.x0 + int(cx), y = b.y0 + int(cy);
                 cover(p, b.area, x, y, depth[k]);
-                older[k] = atomicExch(&pool.heads[plane + size_t(y) * c_frame.width + size_t(x)],
+                older[k] = atomicExch(&pool.heads[plane + size_t(y) * width + size_t(x)],
                                       uint32_t(at[k]) + 1u);
             }
             cx += step_x;
@@ -383,16 +395,17 @@ struct Job {
     uint32_t key, side;
 };
 template <uint32_t kLanes>
-__device__ __forceinline__ void load_job(const float4* planes, uint32_t per_dir, uint32_t item,
-                                         Job& j)
+__device__ __forceinline__ void load_job(const Scene& scene, const float4* planes, uint32_t per_dir,
+                                         uint32_t item, Job& j)
 {
     const uint32_t dir = item / per_dir, w = item - dir * per_dir;
-    const uint32_t tile = w / c_frame.facets, facet = w - tile * c_frame.facets;
-    const Facet t = load_facet(planes, facet);
-    const uint32_t flip = facing(t, c_views[dir]);
-    project_lanes<kLanes>(t, tile, c_views[dir], j.p);
-    j.b = triangle_bbox(j.p);
-    j.plane = size_t(dir) * c_frame.width * c_frame.height;
+    const RasterFrame& frame = scene.frame;
+    const uint32_t tile = w / frame.facets, facet = w - tile * frame.facets;
+    const Facet t = load_facet(frame, planes, facet);
+    const uint32_t flip = facing(t, scene.views[dir]);
+    project_lanes<kLanes>(frame, t, tile, scene.views[dir], j.p);
+    j.b = triangle_bbox(frame, j.p);
+    j.plane = size_t(dir) * frame.width * frame.height;
     j.key = w | (flip << 31);
     j.side = 2u * facet + flip;
 }
@@ -401,7 +414,8 @@ __device__ __forceinline__ void load_job(const float4* planes, uint32_t per_dir,
 // the forest's 0.8 M ground triangles, 190 us for the terrain's 164,000, which
 // took 160 + 495 in two passes of a thread each.
 template <uint32_t kLanes>
-__global__ void __launch_bounds__(256) k_raster_mid(const float4* __restrict__ planes,
+__global__ void __launch_bounds__(256) k_raster_mid(const __grid_constant__ Scene scene,
+                                                    const float4* __restrict__ planes,
                                                     uint32_t per_dir, Pool pool,
                                                     const uint32_t* jobs,
                                                     const uint32_t* job_count,
@@ -415,17 +429,18 @@ __global__ void __launch_bounds__(256) k_raster_mid(const float4* __restrict__ p
     for (uint32_t k = blockIdx.x * kJobs; k < count; k += gridDim.x * kJobs) {
         const uint32_t mine = k + threadIdx.x / kLanes;
         Job j;
-        load_job<kLanes>(planes, per_dir, jobs[mine < count ? mine : k], j);
+        load_job<kLanes>(scene, planes, per_dir, jobs[mine < count ? mine : k], j);
         const uint32_t box = mine < count ? uint32_t(j.b.x1 - j.b.x0 + 1) *
                                                 uint32_t(j.b.y1 - j.b.y0 + 1) : 0u;
         for (uint32_t first = 0; __syncthreads_or(int(first < box)); first += kSpan)
-            raster_span<kLanes>(j.p, j.b, j.plane, j.key, first,
+            raster_span<kLanes>(j.p, j.b, j.plane, scene.frame.width, j.key, first,
                                 first < box ? min(box - first, kSpan) : 0u, pool, room,
                                 frags ? frags + j.side : nullptr);
     }
 }
 
-__global__ void __launch_bounds__(256) k_raster_big(const float4* __restrict__ planes,
+__global__ void __launch_bounds__(256) k_raster_big(const __grid_constant__ Scene scene,
+                                                    const float4* __restrict__ planes,
                                                     uint32_t per_dir, Pool pool,
                                                     const uint32_t* jobs_end,
                                                     const uint32_t* job_count,
@@ -437,11 +452,11 @@ __global__ void __launch_bounds__(256) k_raster_big(const float4* __restrict__ p
     const uint32_t count = *job_count, warp = threadIdx.x >> 5;
     for (uint32_t k = blockIdx.x; k < count; k += gridDim.x) {
         Job j;
-        load_job<32>(planes, per_dir, *(jobs_end - 1 - k), j);
+        load_job<32>(scene, planes, per_dir, *(jobs_end - 1 - k), j);
         const uint32_t box = uint32_t(j.b.x1 - j.b.x0 + 1) * uint32_t(j.b.y1 - j.b.y0 + 1);
         for (uint32_t f = blockIdx.y * 8 * kBigPixels; f < box; f += gridDim.y * 8 * kBigPixels) {
             const uint32_t first = f + warp * kBigPixels;
-            raster_span<32>(j.p, j.b, j.plane, j.key, first < box ? first : 0u,
+            raster_span<32>(j.p, j.b, j.plane, scene.frame.width, j.key, first < box ? first : 0u,
                         first < box ? min(box - first, kBigPixels) : 0u, pool, room,
                         frags ? frags + j.side : nullptr);
         }
@@ -698,10 +713,10 @@ __device__ __forceinline__ uint64_t chain_key(const uint4& node)
     const uint32_t depth = bits & 0x80000000u ? ~bits : bits | 0x80000000u;
     return (uint64_t(depth) << 32) | uint64_t((node.y << 1) | (node.y >> 31));
 }
-__device__ __forceinline__ uint32_t key_side(uint64_t k, uint32_t facets)
+__device__ __forceinline__ uint32_t key_side(uint64_t k, uint32_t facets, uint32_t tiles)
 {
     const uint32_t low = uint32_t(k);  // the side itself where there is one tile
-    return c_frame.tiles == 1u ? low : 2u * ((low >> 1) % facets) + (low & 1u);
+    return tiles == 1u ? low : 2u * ((low >> 1) % facets) + (low & 1u);
 }
 
 __device__ __forceinline__ void order2(uint64_t& a, uint64_t& b)
@@ -777,7 +792,7 @@ __device__ __forceinline__ uint32_t gather_covered(const uint32_t* heads, Covere
 // instructions and the two loads in a row, pixel and fragment.
 constexpr uint32_t kHeldPairs = 1024;
 __global__ void __launch_bounds__(256) k_resolve_graph(
-    const uint32_t* __restrict__ heads, const uint4* __restrict__ nodes, uint32_t cap,
+    uint32_t facets, uint32_t tiles, const uint32_t* __restrict__ heads, const uint4* __restrict__ nodes, uint32_t cap,
     uint32_t* sky, uint64_t* pairs, unsigned long long* pair_count, int side_bits, uint2* list,
     RasterStats* stats)
 {
@@ -788,7 +803,7 @@ __global__ void __launch_bounds__(256) k_resolve_graph(
     if (threadIdx.x == 0) held_count = 0;
     const uint32_t covered = gather_covered(heads, c);
     if (!covered) return;
-    const uint32_t facets = c_frame.facets, lane = threadIdx.x & 31u;
+    const uint32_t lane = threadIdx.x & 31u;
     uint32_t longest = 0;
     for (uint32_t first = threadIdx.x & ~31u; first < covered; first += 256) {
         const uint32_t head = first + lane < covered ? c.queue[first + lane] : 0u;
@@ -802,7 +817,7 @@ __global__ void __launch_bounds__(256) k_resolve_graph(
             n = 1;
         }
         if (!__any_sync(0xffffffffu, next != 0u)) {
-            const uint32_t side = key_side(k[0], facets), run = side_run(side, n != 0u);
+            const uint32_t side = key_side(k[0], facets, tiles), run = side_run(side, n != 0u);
             if (run) {
                 atomicAdd(&sky[side], run);
                 atomicAdd(&sky[side ^ 1u], run);
@@ -857,12 +872,12 @@ __global__ void __launch_bounds__(256) k_resolve_graph(
             order2(k[5], k[6]);
         }
         uint32_t side[kFast], mine = 0;
-        side[0] = key_side(k[0], facets);
+        side[0] = key_side(k[0], facets, tiles);
         uint32_t last = side[0];
 #pragma unroll
         for (int q = 1; q < kFast; ++q) {
             if (uint32_t(q) >= most) break;
-            side[q] = key_side(k[q], facets);
+            side[q] = key_side(k[q], facets, tiles);
             if (uint32_t(q) < n) {
                 last = side[q];
                 if ((side[q - 1] >> 1) != (side[q] >> 1)) ++mine;
@@ -906,7 +921,7 @@ __global__ void __launch_bounds__(256) k_resolve_graph(
 // each, in local memory; chains above kDeepChain are an error.
 template <uint32_t kCap>
 __global__ void __launch_bounds__(64) k_resolve_list(
-    const uint4* __restrict__ nodes, const uint2* __restrict__ list, uint32_t above, uint32_t* sky,
+    uint32_t facets, const uint4* __restrict__ nodes, const uint2* __restrict__ list, uint32_t above, uint32_t* sky,
     uint64_t* pairs, unsigned long long* pair_count, int side_bits, RasterStats* stats)
 {
     const uint32_t listed = stats->listed;
@@ -927,14 +942,15 @@ __global__ void __launch_bounds__(64) k_resolve_list(
             next = node.z;
         }
         order_chain(f, int(n));
-        emit_chain(f, int(n), c_frame.facets, sky, pairs, pair_count, side_bits);
+        emit_chain(f, int(n), facets, sky, pairs, pair_count, side_bits);
     }
 }
 
 // computeCpuSunlit per pixel (facetrtcore.cpp:1448-1466): the nearest fragment
 // (first in append order among equal depths) is visible.  (Every fragment
 // counts towards its side's total: counted by the raster.)
-__global__ void __launch_bounds__(256) k_resolve_sunlit(const uint32_t* __restrict__ heads,
+__global__ void __launch_bounds__(256) k_resolve_sunlit(uint32_t facets, uint32_t tiles,
+                                                        const uint32_t* __restrict__ heads,
                                                         const uint4* __restrict__ nodes,
                                                         uint32_t cap, uint32_t* visible,
                                                         RasterStats* stats)
@@ -955,7 +971,7 @@ __global__ void __launch_bounds__(256) k_resolve_sunlit(const uint32_t* __restri
         __syncwarp();
         if (n > cap) atomicAdd(&stats->overflow, (unsigned long long)(n - cap));
         longest = max(longest, n);
-        add_sides(visible, key_side(best, c_frame.facets), n != 0u);
+        add_sides(visible, key_side(best, facets, tiles), n != 0u);
     }
     note_longest(stats, longest);
 }
@@ -972,11 +988,11 @@ void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame
                       const RasterView* views, uint32_t dir_count, RasterBuffers& rb,
                       uint32_t* d_frags, RasterStats& stats, cudaStream_t s)
 {
-    if (dir_count > 64) throw Error(FACETCU_INVALID_ARGUMENT, "raster chunk exceeds 64 directions");
-    FCU_CHECK(cudaMemcpyToSymbolAsync(c_views, views, sizeof(RasterView) * dir_count, 0,
-                                      cudaMemcpyHostToDevice, s));
-    FCU_CHECK(cudaMemcpyToSymbolAsync(c_frame, &frame, sizeof(RasterFrame), 0,
-                                      cudaMemcpyHostToDevice, s));
+    if (dir_count > kMaxViews)
+        throw Error(FACETCU_INVALID_ARGUMENT, "raster chunk exceeds 64 directions");
+    Scene scene{};
+    scene.frame = frame;
+    std::copy(views, views + dir_count, scene.views);
     const uint64_t npix = uint64_t(dir_count) * frame.width * frame.height;
     const uint64_t per_dir = uint64_t(frame.tiles) * frame.facets, items = dir_count * per_dir;
     if (items >= (1ull << 32)) throw Error(FACETCU_OVERFLOW_ERROR, "raster work exceeds 2^32 triangles");
@@ -1000,12 +1016,12 @@ void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame
         FCU_CHECK(cudaMemsetAsync(heads, 0, padded * 4, s));
         FCU_CHECK(cudaMemsetAsync(dstats, 0, sizeof(RasterStats), s));
         k_raster<<<dim3(unsigned((per_dir + 255) / 256), dir_count), 256, 0, s>>>(
-            planes, uint32_t(per_dir), pool, jobs, uint32_t(items), dstats, counted);
+            scene, planes, uint32_t(per_dir), pool, jobs, uint32_t(items), dstats, counted);
         FCU_LAUNCH("k_raster");
         launch_early(k_raster_mid<kMidLanes>, unsigned(std::min<uint64_t>((items + 31) / 32, 8 * 152)),
-                     256, 0, s, planes, uint32_t(per_dir), pool, jobs, &dstats->mid, counted);
-        launch_early(k_raster_big, dim3(unsigned(std::min<uint64_t>(items, 152)), 16), 256, 0, s, planes,
-                     uint32_t(per_dir), pool, jobs + items, &dstats->big, counted);
+                     256, 0, s, scene, planes, uint32_t(per_dir), pool, jobs, &dstats->mid, counted);
+        launch_early(k_raster_big, dim3(unsigned(std::min<uint64_t>(items, 152)), 16), 256, 0, s, scene,
+                     planes, uint32_t(per_dir), pool, jobs + items, &dstats->big, counted);
         FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
         FCU_CHECK(cudaStreamSynchronize(s));
         if (host.fragments >= (1ull << 32))
@@ -1035,12 +1051,12 @@ void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t
     uint2* list = static_cast<uint2*>(rb.list.reserve((stats.fragments / (kFast + 1) + 1) * 8));
     const uint4* nodes = rb.nodes.as<uint4>();
     k_resolve_graph<<<unsigned((npix + kResolvePixels - 1) / kResolvePixels), 256, 0, s>>>(
-        rb.heads.as<uint32_t>(), nodes, chain_cap, d_sky, d_pairs, d_pair_count, side_bits, list,
+        frame.facets, frame.tiles, rb.heads.as<uint32_t>(), nodes, chain_cap, d_sky, d_pairs, d_pair_count, side_bits, list,
         dstats);
     FCU_LAUNCH("k_resolve_graph");
     const unsigned list_blocks = 16 * 152;
-    k_resolve_list<kMidChain><<<list_blocks, 64, 0, s>>>(nodes, list, 0u, d_sky, d_pairs,
-                                                         d_pair_count, side_bits, dstats);
+    k_resolve_list<kMidChain><<<list_blocks, 64, 0, s>>>(frame.facets, nodes, list, 0u, d_sky,
+                                                         d_pairs, d_pair_count, side_bits, dstats);
     FCU_LAUNCH("k_resolve_list");
     RasterStats host{};
     auto read = [&] {
@@ -1052,7 +1068,7 @@ void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t
     if (host.max_chain > kMidChain) {
         // (launched only then: its local memory is a few GB)
         k_resolve_list<kDeepChain><<<list_blocks, 64, 0, s>>>(
-            nodes, list, kMidChain, d_sky, d_pairs, d_pair_count, side_bits, dstats);
+            frame.facets, nodes, list, kMidChain, d_sky, d_pairs, d_pair_count, side_bits, dstats);
         FCU_LAUNCH("k_resolve_list");
         read();
     }
@@ -1068,7 +1084,8 @@ void raster_resolve_sunlit(const RasterFrame& frame, uint32_t chain_cap, RasterB
     const uint64_t npix = uint64_t(frame.width) * frame.height;
     RasterStats* dstats = rb.stats.as<RasterStats>();
     k_resolve_sunlit<<<unsigned((npix + kResolvePixels - 1) / kResolvePixels), 256, 0, s>>>(
-        rb.heads.as<uint32_t>(), rb.nodes.as<uint4>(), chain_cap, d_visible, dstats);
+        frame.facets, frame.tiles, rb.heads.as<uint32_t>(), rb.nodes.as<uint4>(), chain_cap,
+        d_visible, dstats);
     FCU_LAUNCH("k_resolve_sunlit");
     k_fraction<<<(2 * frame.facets + 255) / 256, 256, 0, s>>>(2 * frame.facets, d_total, d_visible,
                                                               d_fraction);
