@@ -623,7 +623,6 @@ __global__ void __launch_bounds__(kWarps * 32, SweepBlocks<P>::value) k_sweep_wi
                                                             const uint32_t* done)
 {
     start_next();
-    wait_for_previous();
     if (*done) return;
     constexpr int CPL = 4;
     constexpr int L = P / CPL;
@@ -718,7 +717,7 @@ __global__ void __launch_bounds__(kWarps * 32, SweepBlocks<P>::value) k_sweep_wi
 // 4, 16 columns 412, 336 and 326.
 template <int P>
 __global__ void __launch_bounds__(kWarps * 32, P == 8 ? 3 : 4) k_sweep_mid(GraphView g, PanelParams pp,
-                                                               const float* __restrict__ Bin,
+                                                               const float* Bin,
                                                                float* __restrict__ Bout,
                                                                uint32_t* stats, uint32_t* counter,
                                                                const uint32_t* done)
@@ -741,7 +740,7 @@ __global__ void __launch_bounds__(kWarps * 32, P == 8 ? 3 : 4) k_sweep_mid(Graph
     float md = 0.0f, mb = 0.0f, mr = 0.0f;
     const uint32_t S = 2u * g.facets, chunks = (g.facets + C - 1) / C;
     const uint32_t mask = (1u << g.nb_bits) - 1u;
-    const float4* __restrict__ X4 = reinterpret_cast<const float4*>(Bin);
+    const float4* X4 = reinterpret_cast<const float4*>(Bin);
     auto draw = [&] { return lane == 0 ? atomicAdd(counter, 1u) : 0u; };
     auto offsets = [&](uint32_t ch) {
         const uint32_t s = min(S, ch * 2u * C + uint32_t(min(lane, int(2 * C))));
@@ -800,7 +799,7 @@ __global__ void __launch_bounds__(kWarps * 32, P == 8 ? 3 : 4) k_sweep_mid(Graph
                     for (int u = 0; u < U; ++u) {
                         const bool on = base + uint32_t(u * G + grp) < end;
                         c[u] = float(x[u] >> g.nb_bits);
-                        q[u] = on ? __ldg(X4 + size_t(x[u] & mask) * L + sub)
+                        q[u] = on ? X4[size_t(x[u] & mask) * L + sub]
                                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
 #pragma unroll
@@ -2447,8 +2446,11 @@ int grid_for(K kernel)
     return std::max(1, sms) * std::max(1, per_sm);
 }
 
-// (The FP32 sweeps of a panel and k_check follow one another: each is launched
-// while the one before it ends and waits inside.)
+// (The 8- and 16-column sweeps and k_check are launched while the kernel in front
+// of them ends and wait inside.  k_sweep_wide is not: it gathers its panel through
+// the read-only path, which an early kernel may not do, and with plain loads the
+// 32-column sweeps cost more than the 2 us of a launch: the energy node 28.7 ms
+// instead of 27.8.)
 template <typename T>
 void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in, T* out,
                   uint32_t* stats, uint32_t* counter, const uint32_t* done, cudaStream_t s)
@@ -2487,10 +2489,10 @@ void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in,
             // 16-byte row vectors in rounds of 8 loads per lane
             if (P == 8) {
                 static const int grid = grid_for(k_sweep_wide<8>);
-                launch_early(k_sweep_wide<8>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
+                k_sweep_wide<8><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
             } else {
                 static const int grid = grid_for(k_sweep_wide<16>);
-                launch_early(k_sweep_wide<16>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
+                k_sweep_wide<16><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
             }
             FCU_LAUNCH("k_sweep_wide");
             return;
@@ -2499,17 +2501,17 @@ void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in,
             switch (P) {
             case 32: {
                 static const int grid = grid_for(k_sweep_wide<32>);
-                launch_early(k_sweep_wide<32>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
+                k_sweep_wide<32><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
                 break;
             }
             case 64: {
                 static const int grid = grid_for(k_sweep_wide<64>);
-                launch_early(k_sweep_wide<64>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
+                k_sweep_wide<64><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
                 break;
             }
             default: {
                 static const int grid = grid_for(k_sweep_wide<128>);
-                launch_early(k_sweep_wide<128>, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
+                k_sweep_wide<128><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
                 break;
             }
             }

@@ -35,7 +35,10 @@ inline void cuda_check(cudaError_t e, const char* what)
 // A launch that may begin before the kernel in front of it has ended.  The
 // kernel calls wait_for_previous() before it touches anything that a kernel
 // before it writes or reads; the one in front says start_next() as early as it
-// likes.
+// likes.  What a kernel before it writes is read with plain loads: the
+// parameter is not const __restrict__ and no __ldg takes it, because the
+// read-only path wants data that nobody writes while the kernel is resident,
+// and this one is resident while the writer runs.
 template <typename... P, typename... A>
 void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t shared, cudaStream_t s,
                   A&&... args)

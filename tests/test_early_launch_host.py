@@ -1,0 +1,60 @@
+"""Kernels that are launched before the kernel in front of them ends (launch_early)
+are resident while it still writes.  Read from the sources: such a kernel waits
+for it, and the arrays that a predecessor writes don't come through the read-only
+path (const __restrict__ parameters, __ldg)."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                    "streamsim_gb300", "csrc")
+# parameters that the kernel in front may write: panels and columns, what is
+# summed from them, and the lists and counts of a sort or raster
+WRITTEN = ("Bin", "in", "B", "partial", "stats", "done", "keys", "values", "hist", "offsets",
+           "totals", "jobs", "jobs_end", "job_count")
+
+
+def _sources():
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith(".cu"):
+            with open(os.path.join(CSRC, name)) as f:
+                yield name, f.read()
+
+
+def _kernel(text, name):
+    """Parameter list and body of a __global__ function."""
+    at = re.search(r"__global__[^;{]*?\b%s\(" % name, text, re.S)
+    assert at, name
+    depth, i = 1, at.end()
+    while depth:
+        depth += {"(": 1, ")": -1}.get(text[i], 0)
+        i += 1
+    params, start = text[at.end():i - 1], text.index("{", i)
+    depth, j = 1, start + 1
+    while depth:
+        depth += {"{": 1, "}": -1}.get(text[j], 0)
+        j += 1
+    return params, text[start:j]
+
+
+def _early_kernels():
+    for name, text in _sources():
+        found = set(re.findall(r"launch_early\(\s*(k_\w+)", text))
+        if name == "solve.cu":  # launched through a generic lambda
+            found.add("k_jacobi_rows")
+        for kernel in sorted(found):
+            yield name, kernel
+
+
+@pytest.mark.parametrize("source,kernel", list(_early_kernels()))
+def test_early_kernel(source, kernel):
+    text = dict(_sources())[source]
+    params, body = _kernel(text, kernel)
+    assert "wait_for_previous()" in body
+    for p in params.split(","):
+        words = p.replace("*", " ").split()
+        if words and words[-1].split("=")[0] in WRITTEN and "*" in p:
+            assert not ("const" in words and "__restrict__" in p), p
+    for arg in re.findall(r"__ldg\(\s*(?:reinterpret_cast<[^>]*>\()?(\w+)", body):
+        assert arg not in WRITTEN + ("X4",)
