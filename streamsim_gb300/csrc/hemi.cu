@@ -719,8 +719,9 @@ void hemisphere_graph(const facetcu_vertex* d_vertices, uint32_t facets, const L
     ScratchBuffer traced_buf(ws);
     uint32_t* traced = static_cast<uint32_t*>(traced_buf.reserve(size_t(run) * 2 * rays * 4));
     const size_t smem_trace = size_t(2) * (size_t(2) * per_block << shift);
+    // (the limit belongs to the function, not to this context: always the most)
     FCU_CHECK(cudaFuncSetAttribute(k_hemi_trace, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   int(smem_trace)));
+                                   int(2 * kBlockRays)));
     for (uint32_t f0 = 0; f0 < facets; f0 += run) {
         const uint32_t f1 = std::min(facets, f0 + run);
         k_hemi_trace<<<(f1 - f0 + per_block - 1) / per_block, kTraceThreads, smem_trace, s>>>(

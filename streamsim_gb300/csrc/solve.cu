@@ -352,7 +352,9 @@ bool jacobi_sweeps_cluster(const DeviceGraph& g, const facetcu_surface_optics* d
     shape.words = uint32_t(std::min<size_t>(room, g.nnz / kCtas * 2 + 1024));
     auto kernel = k_jacobi_cluster<kClusterLanes>;
     const size_t shared = fixed + size_t(shape.words) * 4;
-    FCU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shared)));
+    // (the limits belong to the function, not to this context: always the most)
+    FCU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(kClusterShared)));
     FCU_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t config{};
     config.gridDim = kCtas;
