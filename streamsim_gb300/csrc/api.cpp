@@ -253,7 +253,7 @@ uint32_t run_sweeps(facetcu_context* ctx, float sky, float relax, uint32_t count
         const float* in = ping == 0 ? a : b;
         float* out = ping == 0 ? b : a;
         jacobi_sweep(ctx->graph, ctx->optics.as<facetcu_surface_optics>(), sky, relax, in, out,
-                     res + first_slot + i, ctx->stream);
+                     res + first_slot + i, i > 0, ctx->stream);
         ping ^= 1u;
     }
     return ping;

@@ -438,7 +438,7 @@ __device__ __forceinline__ float2 sum_pair(const float* partial, uint32_t tiles,
 // A thread per facet: the reference's update (as k_jacobi_rows in solve.cu).
 __global__ void __launch_bounds__(256) k_finish_jacobi(
     uint32_t facets, uint32_t tiles, const float* partial, const uint2* __restrict__ denom,
-    const uint2* __restrict__ skyc, const float4* __restrict__ optics, float sky, float relax,
+    const uint2* __restrict__ skyc, const float4* optics, float sky, float relax,
     const float2* in, float2* out, uint32_t* max_delta_bits)
 {
     start_next();

@@ -19,7 +19,9 @@ namespace {
 // 4,096-facet scene of 98,000 edges, 4.1 here, 2.9 where a sweep begins while
 // the one before it ends: 64 sweeps 333 -> 243 us, of 1.3 M edges 669 -> 521.)
 // L follows the mean row length.
-// kEarly: launched while the sweep before it ends; only Bin is waited for.
+// kEarly: launched while the sweep before it ends; only what that one writes is
+// waited for.  (With optics read after the wait, so that any kernel might write
+// them, 64 sweeps of the 4,096-facet scene took 1.3 % longer.)
 template <int L, bool kEarly>
 __global__ void __launch_bounds__(256) k_jacobi_rows(
     uint32_t facets, const uint32_t* __restrict__ rows, const facetcu_csr_edge* __restrict__ edges,
@@ -322,15 +324,16 @@ void jacobi_sweep_raw(uint32_t surfaces, uint64_t edges_hint, const uint32_t* ro
 
 void jacobi_sweep(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
                   float relaxation, const float* d_in, float* d_out, uint32_t* d_max_delta_bits,
-                  cudaStream_t s)
+                  bool follows, cudaStream_t s)
 {
     if (g.column.state == ColumnPlan::kMade) {
         column_jacobi(g, d_optics, sky, relaxation, d_in, d_out, d_max_delta_bits, s);
         return;
     }
-    sweep_rows<true>(g.surfaces, g.nnz, g.row_offsets.as<uint32_t>(), g.edges.as<facetcu_csr_edge>(),
-                     g.denominators.as<uint32_t>(), g.sky.as<uint32_t>(), d_optics, sky, relaxation,
-                     d_in, d_out, d_max_delta_bits, s);
+    (follows ? sweep_rows<true> : sweep_rows<false>)(
+        g.surfaces, g.nnz, g.row_offsets.as<uint32_t>(), g.edges.as<facetcu_csr_edge>(),
+        g.denominators.as<uint32_t>(), g.sky.as<uint32_t>(), d_optics, sky, relaxation, d_in, d_out,
+        d_max_delta_bits, s);
 }
 
 bool jacobi_sweeps_cluster(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,

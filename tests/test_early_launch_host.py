@@ -9,9 +9,9 @@ import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
                     "streamsim_gb300", "csrc")
-# parameters that the kernel in front may write: panels and columns, what is
-# summed from them, and the lists and counts of a sort or raster
-WRITTEN = ("Bin", "in", "B", "partial", "stats", "done", "keys", "values", "hist", "offsets",
+# parameters that the kernel in front may write: optics, panels and columns, what
+# is summed from them, and the lists and counts of a sort or raster
+WRITTEN = ("optics", "Bin", "in", "B", "partial", "stats", "done", "keys", "values", "hist", "offsets",
            "totals", "jobs", "jobs_end", "job_count")
 
 
@@ -52,9 +52,27 @@ def test_early_kernel(source, kernel):
     text = dict(_sources())[source]
     params, body = _kernel(text, kernel)
     assert "wait_for_previous()" in body
+    written = WRITTEN
+    if kernel == "k_jacobi_rows":  # see test_first_sweep
+        written = tuple(w for w in WRITTEN if w != "optics")
     for p in params.split(","):
         words = p.replace("*", " ").split()
-        if words and words[-1].split("=")[0] in WRITTEN and "*" in p:
+        if words and words[-1].split("=")[0] in written and "*" in p:
             assert not ("const" in words and "__restrict__" in p), p
+    # before the wait only the graph's and the plan's arrays are read
+    before = body[:body.index("wait_for_previous()")]
+    assert not re.search(r"\b(%s)\s*\[" % "|".join(written), before)
     for arg in re.findall(r"__ldg\(\s*(?:reinterpret_cast<[^>]*>\()?(\w+)", body):
         assert arg not in WRITTEN + ("X4",)
+
+
+def test_first_sweep():
+    """k_jacobi_rows reads optics before it waits, so only a sweep behind another
+    sweep of the same call may start early."""
+    with open(os.path.join(CSRC, "api.cpp")) as f:
+        api = f.read()
+    call = re.search(r"jacobi_sweep\(ctx->graph[^;]*;", api).group(0)
+    assert re.search(r",\s*i > 0,\s*ctx->stream\)", call)
+    solve = dict(_sources())["solve.cu"]
+    assert re.search(r"follows \? sweep_rows<true> : sweep_rows<false>", solve)
+    assert len(re.findall(r"sweep_rows<true>", solve)) == 1
