@@ -236,11 +236,20 @@ void upload(DeviceBuffer& buf, const void* src, size_t bytes, cudaStream_t s)
 // Sweeps from which a graph's column plan pays for being made.
 constexpr uint32_t kPlanSweeps = 8;
 
+// Whether a solve of up to `sweeps` sweeps runs through the graph's column plan.
+// The call's own arguments decide, not whether a plan is there already: the two
+// ways add in different orders, and a call returns the same bits whatever was
+// solved before it.
+bool sweeps_planned(facetcu_context* ctx, uint32_t sweeps)
+{
+    return sweeps >= kPlanSweeps && column_plan(ctx->graph, ctx->ws, ctx->stream);
+}
+
 // The plain Jacobi loop shared by solve and solveAccelerated.  Runs `count`
 // sweeps starting from buffer `ping`; each sweep's max|dB| lands in
 // residual[sweep_index].  Returns the new ping.
-uint32_t run_sweeps(facetcu_context* ctx, float sky, float relax, uint32_t count, uint32_t ping,
-                    uint32_t first_slot)
+uint32_t run_sweeps(facetcu_context* ctx, bool planned, float sky, float relax, uint32_t count,
+                    uint32_t ping, uint32_t first_slot)
 {
     float* a = ctx->rad_a.as<float>();
     float* b = ctx->rad_b.as<float>();
@@ -252,7 +261,7 @@ uint32_t run_sweeps(facetcu_context* ctx, float sky, float relax, uint32_t count
     for (uint32_t i = 0; i < count; ++i) {
         const float* in = ping == 0 ? a : b;
         float* out = ping == 0 ? b : a;
-        jacobi_sweep(ctx->graph, ctx->optics.as<facetcu_surface_optics>(), sky, relax, in, out,
+        jacobi_sweep(ctx->graph, planned, ctx->optics.as<facetcu_surface_optics>(), sky, relax, in, out,
                      res + first_slot + i, i > 0, ctx->stream);
         ping ^= 1u;
     }
@@ -824,8 +833,8 @@ int facetcu_solve(facetcu_context* ctx, const facetcu_surface_optics* optics,
         FCU_CHECK(cudaMemsetAsync(ctx->rad_a.ptr, 0, size_t(S) * 4, s));
         FCU_CHECK(cudaMemsetAsync(ctx->rad_b.ptr, 0, size_t(S) * 4, s));
         FCU_CHECK(cudaMemsetAsync(ctx->residual.ptr, 0, (size_t(iterations) + 1) * 4, s));
-        if (iterations >= kPlanSweeps) column_plan(ctx->graph, ctx->ws, s);
-        const uint32_t ping = run_sweeps(ctx, sky, relaxation, iterations, 0, 0);
+        const bool planned = sweeps_planned(ctx, iterations);
+        const uint32_t ping = run_sweeps(ctx, planned, sky, relaxation, iterations, 0, 0);
         const float* final_buf = ping == 0 ? ctx->rad_a.as<float>() : ctx->rad_b.as<float>();
         uint32_t bits = 0;
         if (radiosity)
@@ -877,12 +886,12 @@ int facetcu_solve_accelerated(facetcu_context* ctx, const facetcu_surface_optics
             FCU_CHECK(cudaMemsetAsync(ctx->rad_a.ptr, 0, size_t(S) * 4, s));
             FCU_CHECK(cudaMemsetAsync(ctx->rad_b.ptr, 0, size_t(S) * 4, s));
         }
-        if (maximum_iterations >= kPlanSweeps) column_plan(ctx->graph, ctx->ws, s);
+        const bool planned = sweeps_planned(ctx, maximum_iterations);
         uint32_t done = 0, ping = 0;
         float md = 0.0f;
         while (done < maximum_iterations) {
             const uint32_t count = std::min(batch_iterations, maximum_iterations - done);
-            ping = run_sweeps(ctx, sky, relaxation, count, ping, done);
+            ping = run_sweeps(ctx, planned, sky, relaxation, count, ping, done);
             done += count;
             uint32_t bits = 0;
             FCU_CHECK(cudaMemcpyAsync(&bits, ctx->residual.as<uint32_t>() + done - 1, 4,

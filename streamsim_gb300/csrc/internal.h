@@ -311,12 +311,12 @@ void graph_closure(const DeviceGraph& g, float* closure, uint32_t* sampled, Work
 bool graph_pack(DeviceGraph& g, Workspace& ws, cudaStream_t s);
 
 // ---- solves (solve.cu) ---------------------------------------------------
-// One sweep of the reference's solver; through the graph's column plan where
-// it has one.  follows: the work in front of it on the stream is another sweep of
+// One sweep of the reference's solver; planned: through the graph's column plan,
+// which column_plan has made.  follows: the work in front of it on the stream is another sweep of
 // the same solve, so that it may start early and read graph and optics before it
 // waits; the first sweep of a call does not.
-void jacobi_sweep(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
-                  float relaxation, const float* d_in, float* d_out, uint32_t* d_max_delta_bits,
+void jacobi_sweep(const DeviceGraph& g, bool planned, const facetcu_surface_optics* d_optics,
+                  float sky, float relaxation, const float* d_in, float* d_out, uint32_t* d_max_delta_bits,
                   bool follows, cudaStream_t s);
 // All `sweeps` sweeps of a small graph in one launch, from d_in, alternating
 // with d_other as single sweeps would; false where the graph is not for it.

@@ -322,11 +322,11 @@ void jacobi_sweep_raw(uint32_t surfaces, uint64_t edges_hint, const uint32_t* ro
                       d_out, d_max_delta_bits, s);
 }
 
-void jacobi_sweep(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
-                  float relaxation, const float* d_in, float* d_out, uint32_t* d_max_delta_bits,
+void jacobi_sweep(const DeviceGraph& g, bool planned, const facetcu_surface_optics* d_optics,
+                  float sky, float relaxation, const float* d_in, float* d_out, uint32_t* d_max_delta_bits,
                   bool follows, cudaStream_t s)
 {
-    if (g.column.state == ColumnPlan::kMade) {
+    if (planned) {
         column_jacobi(g, d_optics, sky, relaxation, d_in, d_out, d_max_delta_bits, s);
         return;
     }
