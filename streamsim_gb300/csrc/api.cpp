@@ -233,16 +233,14 @@ void upload(DeviceBuffer& buf, const void* src, size_t bytes, cudaStream_t s)
     if (bytes) FCU_CHECK(cudaMemcpyAsync(buf.ptr, src, bytes, cudaMemcpyHostToDevice, s));
 }
 
-// Sweeps from which a graph's column plan pays for being made.
-constexpr uint32_t kPlanSweeps = 8;
-
 // Whether a solve of up to `sweeps` sweeps runs through the graph's column plan.
 // The call's own arguments decide, not whether a plan is there already: the two
 // ways add in different orders, and a call returns the same bits whatever was
 // solved before it.
 bool sweeps_planned(facetcu_context* ctx, uint32_t sweeps)
 {
-    return sweeps >= kPlanSweeps && column_plan(ctx->graph, ctx->ws, ctx->stream);
+    return column_plan_pays(ctx->graph, sweeps) &&
+           column_plan(ctx->graph, ctx->ws, ctx->stream);
 }
 
 // The plain Jacobi loop shared by solve and solveAccelerated.  Runs `count`

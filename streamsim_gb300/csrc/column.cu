@@ -46,11 +46,11 @@ constexpr uint32_t kPad = kTile;
 constexpr uint32_t kMaxCount = 0xffffu;
 constexpr uint32_t kGroupCost = 4;   // of a group beside its words, in words, when work is split
 constexpr int kThreads = 1024;
-// From here on a first solve of 64 sweeps, the making of the plan included,
-// is not slower than over the CSR (k_jacobi_rows): 6.9 M edges 2.9 ms against
-// 2.5 and 20 us a sweep against 25, 13.1 M edges 3.4 against 3.8 and 26
-// against 45; below 4 M edges the fixed cost of a sweep (tiles, two launches:
-// 14 us) is more than the CSR sweep's.
+// Fewer edges: the fixed cost of a sweep (tiles, two launches: 14 us) takes what
+// the gather saves.  From here on one column of the batched solver, the making of
+// the plan included, is faster than over the CSR, whose renumbered copy it does
+// not need (first call, 9 sweeps: 15.9 M edges 1.37 ms against 1.82, 83.8 M 3.6
+// against 6.6).
 constexpr uint64_t kMinEdges = 10u << 20;
 // Mean edges of a (row, tile) pair: with 3.5 (13 M edges, 400,000 sides) 33 us
 // a sweep against 49; fewer leave more group heads and partials than edges.
@@ -678,6 +678,22 @@ void ColumnPlan::release()
 {
     for (DeviceBuffer* b : {&shares, &groups, &meta, &words, &partial}) b->release();
     state = kUnknown;
+}
+
+// Sweeps from which a first solve, the making of the plan included, is not slower
+// than over the CSR.  Making it takes some 0.35 ms and 14 us a million edges; a
+// sweep saves 9.5 us of 40 at 15.9 M edges and 77 of 160 at 83.8 M.  A first call
+// in ms, with the plan and without:
+//     sweeps          8           16          24          32          48          64
+//     15.9 M edges    1.15  0.70  1.37  1.00  1.61  1.32  1.85  1.62  2.28  2.25  2.75  2.87
+//     22.0 M          1.46  0.94  1.69  1.32  1.95  1.75  2.20  2.14  2.72  2.95  3.24  3.79
+//     37.4 M          1.96  1.35  2.33  2.01  2.68  2.62  3.00  3.28  3.72  4.53  4.38  5.81
+//     83.8 M          3.49  2.62  4.14  3.90  4.83  5.17  5.47  6.46  6.80  9.01  8.15  11.6
+// so the two meet at about 50, 36, 26 and 20 sweeps; the line says 46, 37, 27 and 19,
+// and 64 from the fewest edges that get a plan.
+bool column_plan_pays(const DeviceGraph& g, uint32_t sweeps)
+{
+    return sweeps >= 12u && g.nnz * (sweeps - 12u) >= 540000000ull;
 }
 
 bool column_plan(DeviceGraph& g, Workspace& ws, cudaStream_t s)

@@ -333,6 +333,8 @@ void incident_irradiance(const DeviceGraph& g, const facetcu_surface_optics* d_o
                          float sky, const float* d_radiosity, float* d_out, cudaStream_t s);
 
 // ---- one-column sweeps (column.cu) ---------------------------------------
+// Whether a plan is worth making for a solve of so many sweeps.
+bool column_plan_pays(const DeviceGraph& g, uint32_t sweeps);
 // Makes the graph's plan once; false where the CSR sweeps are to be used.
 bool column_plan(DeviceGraph& g, Workspace& ws, cudaStream_t s);
 // With a plan: the reference's sweep (as jacobi_sweep), the batched solver's
