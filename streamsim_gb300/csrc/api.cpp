@@ -2151,9 +2151,9 @@ int facetcu_render_sensor_image(facetcu_context* ctx, const facetcu_sensor* sens
         const size_t S = 2 * size_t(F);
         cudaStream_t st = ctx->stream;
         auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-        const size_t bytes = al(size_t(F) * 4) + al(n * 16) + al(n * 4) * 2 +
+        const size_t bytes = al(size_t(F) * 4) + al(size_t(F) * 4) + al(n * 16) + al(n * 4) * 2 +
                              al(size_t(band_count) * S * 4) +
-                             al(size_t(band_count) * 4) + al(size_t(band_count) * n * 4) + al(8);
+                             al(size_t(band_count) * 4) + al(size_t(band_count) * n * 4) + al(12);
         char* c = static_cast<char*>(ctx->img_io.reserve(bytes));
         auto take = [&](size_t b) {
             char* r = c;
@@ -2162,13 +2162,14 @@ int facetcu_render_sensor_image(facetcu_context* ctx, const facetcu_sensor* sens
         };
         image::Scratch w{};
         w.side = reinterpret_cast<int32_t*>(take(size_t(F) * 4));
+        w.large = reinterpret_cast<uint32_t*>(take(size_t(F) * 4));
         w.zbuf = reinterpret_cast<ulonglong2*>(take(n * 16));
         w.index = reinterpret_cast<int32_t*>(take(n * 4));
         int32_t* d_sides = reinterpret_cast<int32_t*>(take(n * 4));
         float* d_values = reinterpret_cast<float*>(take(size_t(band_count) * S * 4));
         float* d_wl = reinterpret_cast<float*>(take(size_t(band_count) * 4));
         float* d_image = reinterpret_cast<float*>(take(size_t(band_count) * n * 4));
-        uint32_t* d_counts = reinterpret_cast<uint32_t*>(take(8));
+        uint32_t* d_counts = reinterpret_cast<uint32_t*>(take(12));  // observed, output, large boxes
         if (band_count) {
             FCU_CHECK(cudaMemcpyAsync(d_values, values, size_t(band_count) * S * 4,
                                       cudaMemcpyHostToDevice, st));

@@ -10,6 +10,7 @@
 //               depths the smallest facet index, i.e. the facet the
 //               reference's sequential loop keeps (it replaces a pixel only
 //               for a strictly nearer depth)
+//   k_raster_large  the same for the facets with large boxes
 //   k_observed  facet -> observed side index image
 //   k_nadir     a parallel sensor's output grid mapped back into the
 //               observed image (:1363-1387)
@@ -163,27 +164,52 @@ __device__ __forceinline__ void test_pixel(const Camera& c, const Tri& t, uint32
     keep_nearest(zbuf + size_t(t.y0 + int(j)) * c.width + size_t(t.x0 + int(i)), depth, f);
 }
 
-// A thread per facet projects it and, for a box of at most kSmallBox pixels,
+__device__ __forceinline__ void load_facet(const facetcu_vertex* __restrict__ V, uint32_t f,
+                                           double (&p)[3][3])
+{
+    for (int k = 0; k < 3; ++k)
+        for (int a = 0; a < 3; ++a) p[k][a] = double(V[3 * size_t(f) + k].position[a]);
+}
+__device__ __forceinline__ void project_facet(const Camera& c, const double (&p)[3][3], Tri& t)
+{
+    t.a = project(c, p[0]);
+    t.b = project(c, p[1]);
+    t.c = project(c, p[2]);
+    make_box(c, t);
+}
+
+// A lane per facet projects it and, for a box of at most kSmallBox pixels,
 // tests them; the warp then takes its larger facets one by one, a lane per
 // pixel.  (A warp per facet did the projection's and the box's doubles in all
 // lanes, and two passes over the pixels, depth and index, did the test twice:
-// 2.29 ms for 200,000 facets on 1,024 x 1,024 pixels, 0.49 here.)
-constexpr uint32_t kSmallBox = 16;
+// 2.29 ms for 200,000 facets on 1,024 x 1,024 pixels, 0.49 here.)  What a warp
+// does in turn is bounded twice: it takes `per_warp` facets, fewer than 32 where
+// there would be too few warps (render), and boxes above kLargeBox are listed for
+// k_raster_large.  A side image of 1,024 x 1,024, copy included, in ms with a warp
+// per facet and box / 32 facets a warp / so:
+//     2 ground triangles        107    80.5   0.31
+//     64 facets of some metres  10.1   33.5   0.33
+//     288 soil triangles        1.77   14.3   0.39
+//     4,096 facets              0.76   2.0    0.43
+//     20,000 panels of 0.6 m    10.4   8.3    4.7
+//     200,000 facets            2.69   0.98   0.81
+// (Six blocks an SM, a few spilled words: without them the list cost the last row
+// 1.5 %.)
+constexpr uint32_t kSmallBox = 16, kLargeBox = 1024;
 constexpr int kRasterThreads = 128;
-__global__ void __launch_bounds__(kRasterThreads) k_raster(uint32_t F,
-                                                           const facetcu_vertex* __restrict__ V,
-                                                           Camera c, ulonglong2* __restrict__ zbuf,
-                                                           int32_t* __restrict__ side)
+__global__ void __launch_bounds__(kRasterThreads, 6) k_raster(
+    uint32_t F, uint32_t per_warp, const facetcu_vertex* __restrict__ V, Camera c,
+    ulonglong2* __restrict__ zbuf, int32_t* __restrict__ side, uint32_t* __restrict__ large_list,
+    uint32_t* large_count)
 {
     __shared__ Tri large[kRasterThreads / 32];
-    const uint32_t f = blockIdx.x * kRasterThreads + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t f = (blockIdx.x * (kRasterThreads / 32) + warp) * per_warp + lane;
     Tri t;
     t.w = t.h = 0;
-    if (f < F) {
+    if (lane < per_warp && f < F) {
         double p[3][3];
-        for (int k = 0; k < 3; ++k)
-            for (int a = 0; a < 3; ++a) p[k][a] = double(V[3 * size_t(f) + k].position[a]);
+        load_facet(V, f, p);
         const double e1[3] = {p[1][0] - p[0][0], p[1][1] - p[0][1], p[1][2] - p[0][2]};
         const double e2[3] = {p[2][0] - p[0][0], p[2][1] - p[0][1], p[2][2] - p[0][2]};
         const double n[3] = {e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2],
@@ -195,17 +221,18 @@ __global__ void __launch_bounds__(kRasterThreads) k_raster(uint32_t F,
             for (int a = 0; a < 3; ++a) d[a] = c.out[a];
         }
         side[f] = int32_t(2 * f + (ddot(n, d) >= 0.0 ? 0 : 1));
-        t.a = project(c, p[0]);
-        t.b = project(c, p[1]);
-        t.c = project(c, p[2]);
-        make_box(c, t);
+        project_facet(c, p, t);
     }
     const unsigned long long pixels = (unsigned long long)t.w * t.h;
     if (pixels <= kSmallBox) {
         for (uint32_t j = 0; j < t.h; ++j)
             for (uint32_t i = 0; i < t.w; ++i) test_pixel(c, t, i, j, f, zbuf);
     }
-    uint32_t todo = __ballot_sync(0xffffffffu, pixels > kSmallBox);
+    if (pixels > kLargeBox) {
+        large_list[atomicAdd(large_count, 1u)] = f;
+        t.w = t.h = 0;
+    }
+    uint32_t todo = __ballot_sync(0xffffffffu, t.w * t.h > kSmallBox);
     while (todo) {
         const int from = __ffs(int(todo)) - 1;
         todo &= todo - 1u;
@@ -225,6 +252,49 @@ __global__ void __launch_bounds__(kRasterThreads) k_raster(uint32_t F,
             }
         }
         __syncwarp();
+    }
+}
+
+// Bound by FP64, as k_raster.  The listed facets: with few of them the blocks share a facet, taking parts of
+// kPartPixels pixels of its box in turn; with more than blocks each takes whole
+// ones (the projection is done once a block and facet).
+constexpr uint32_t kPartPixels = 2048;
+__global__ void __launch_bounds__(256) k_raster_large(const facetcu_vertex* __restrict__ V, Camera c,
+                                                      ulonglong2* __restrict__ zbuf,
+                                                      const uint32_t* large_list,
+                                                      const uint32_t* large_count)
+{
+    __shared__ Tri t;
+    const uint32_t count = *large_count;
+    if (!count) return;
+    const uint32_t share = max(1u, gridDim.x / count);  // blocks of a facet
+    const uint32_t part = blockIdx.x % share;
+    for (uint32_t k = blockIdx.x / share; k < count; k += (gridDim.x + share - 1u) / share) {
+        const uint32_t f = large_list[k];
+        if (threadIdx.x == 0) {
+            double p[3][3];
+            Tri mine;
+            load_facet(V, f, p);
+            project_facet(c, p, mine);
+            t = mine;
+        }
+        __syncthreads();
+        // (at most 2^28 pixels an image)
+        const uint32_t pixels = t.w * t.h, w = t.w, dx = 256u % w, dy = 256u / w;
+        for (uint32_t first = part * kPartPixels; first < pixels; first += share * kPartPixels) {
+            const uint32_t end = min(pixels, first + kPartPixels);
+            uint32_t i = (first + threadIdx.x) % w, j = (first + threadIdx.x) / w;
+            for (uint32_t q = first + threadIdx.x; q < end; q += 256) {
+                test_pixel(c, t, i, j, f, zbuf);
+                i += dx;
+                j += dy;
+                if (i >= w) {
+                    i -= w;
+                    ++j;
+                }
+            }
+        }
+        __syncthreads();  // t is free again
     }
 }
 
@@ -490,11 +560,21 @@ void render(const Camera& c, uint32_t F, const facetcu_vertex* V, const float* v
             Scratch& w, float* image, int32_t* sides, uint32_t* counts, cudaStream_t s)
 {
     const size_t n = size_t(c.width) * c.height;
-    FCU_CHECK(cudaMemsetAsync(counts, 0, 2 * sizeof(uint32_t), s));
+    FCU_CHECK(cudaMemsetAsync(counts, 0, 3 * sizeof(uint32_t), s));
     FCU_CHECK(cudaMemsetAsync(w.zbuf, 0, n * sizeof(ulonglong2), s));
     if (F) {
-        k_raster<<<blocks(F, kRasterThreads), kRasterThreads, 0, s>>>(F, V, c, w.zbuf, w.side);
+        // 16 warps an SM before a warp takes more than one facet: enough to hide
+        // the divisions; more would do the projection's doubles in idle lanes
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const uint32_t per_warp = std::clamp(F / (16u * uint32_t(std::max(sms, 1))), 1u, 32u);
+        k_raster<<<blocks(F, per_warp * kRasterThreads / 32), kRasterThreads, 0, s>>>(
+            F, per_warp, V, c, w.zbuf, w.side, w.large, counts + 2);
         FCU_LAUNCH("k_raster");
+        k_raster_large<<<8u * uint32_t(std::max(sms, 1)), 256, 0, s>>>(V, c, w.zbuf, w.large,
+                                                                      counts + 2);
+        FCU_LAUNCH("k_raster_large");
     }
     k_observed<<<blocks(n, 256), 256, 0, s>>>(n, w.zbuf, w.side, w.index, counts);
     FCU_LAUNCH("k_observed");

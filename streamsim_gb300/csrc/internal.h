@@ -556,6 +556,7 @@ struct Camera {
 };
 struct Scratch {
     int32_t* side;     // F observed sides
+    uint32_t* large;   // F facets with large boxes
     ulonglong2* zbuf;  // W*H nearest fragments (depth key, facet)
     int32_t* index;    // W*H observed sides
 };
