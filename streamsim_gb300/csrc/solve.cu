@@ -12,6 +12,15 @@
 namespace facetcu {
 namespace {
 
+// The side of a thread where L of a block's 256 threads take one.  (As (256 block +
+// thread) / L it wrapped at 2^30 sides of four lanes.)
+constexpr __host__ __device__ uint32_t side_of(uint32_t block, uint32_t thread, uint32_t L)
+{
+    return block * (256u / L) + thread / L;
+}
+// the last side of 2^30 facets, the most that setGeometry takes
+static_assert(side_of((1u << 31) / 64u - 1u, 255u, 4u) == (1u << 31) - 1u, "4 lanes");
+
 // L lanes per side, so a facet's two rows are read at once by 2 L lanes:
 // each lane has U edges in flight and the chain of dependent loads of a row
 // (offsets, edge words, neighbour values) is paid once for all of them.
@@ -34,7 +43,7 @@ __global__ void __launch_bounds__(256) k_jacobi_rows(
     __shared__ float block_delta[8];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t eg = lane % L;
-    const uint32_t s = (blockIdx.x * 256 + threadIdx.x) / L;  // side
+    const uint32_t s = side_of(blockIdx.x, threadIdx.x, L);
     float delta = 0.0f;
     // whole warps stay for the shuffles
     const bool valid = (s >> 1) < facets;
