@@ -323,10 +323,9 @@ void jacobi_sweep(const DeviceGraph& g, bool planned, const facetcu_surface_opti
 bool jacobi_sweeps_cluster(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
                            float relaxation, float* d_in, float* d_other, uint32_t sweeps,
                            uint32_t* d_max_delta_bits, cudaStream_t s);
-// The same sweep on raw device pointers (used by facetcu_solve_noalloc);
-// edges_hint: about how many edges there are.
-void jacobi_sweep_raw(uint32_t surfaces, uint64_t edges_hint, const uint32_t* rows,
-                      const facetcu_csr_edge* edges, const uint32_t* denom, const uint32_t* skyc,
+// The same sweep on raw device pointers (used by facetcu_solve_noalloc).
+void jacobi_sweep_raw(uint32_t surfaces, const uint32_t* rows, const facetcu_csr_edge* edges,
+                      const uint32_t* denom, const uint32_t* skyc,
                       const facetcu_surface_optics* d_optics, float sky, float relaxation,
                       const float* d_in, float* d_out, uint32_t* d_max_delta_bits, cudaStream_t s);
 void incident_irradiance(const DeviceGraph& g, const facetcu_surface_optics* d_optics,

@@ -81,10 +81,9 @@ extern "C" int facetcu_solve_noalloc(const uint32_t* row_offsets, const facetcu_
         FCU_CHECK(cudaMemsetAsync(buf[0], 0, size_t(surface_count) * sizeof(float), s));
         FCU_CHECK(cudaMemsetAsync(residual, 0, size_t(iterations) * sizeof(uint32_t), s));
         for (uint32_t i = 0; i < iterations; ++i) {
-            // the number of edges is on the device: the widest rows' form
-            facetcu::jacobi_sweep_raw(surface_count, uint64_t(surface_count) * 64u, row_offsets,
-                                      edges, denominators, sky_counts, optics, sky_radiosity,
-                                      relaxation, buf[i & 1u], buf[(i + 1u) & 1u], residual + i, s);
+            facetcu::jacobi_sweep_raw(surface_count, row_offsets, edges, denominators, sky_counts,
+                                      optics, sky_radiosity, relaxation, buf[i & 1u],
+                                      buf[(i + 1u) & 1u], residual + i, s);
         }
         if (max_delta) {
             uint32_t bits = 0;

@@ -4,10 +4,14 @@
 // (FacetrtVulkan::solve): FP32 gather over the count-form CSR, both sides of a
 // facet updated together, mix() relaxation, max|dB| as an atomicMax over float
 // bits.  It serves the graphs that column.cu's plan is not made for (few
-// edges, short rows) and callers that bring their own arrays.
-#include "internal.h"
-
+// edges, short rows); k_jacobi_any is the same for callers that bring their own
+// arrays.
 #include <cooperative_groups.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "internal.h"
 
 namespace facetcu {
 namespace {
@@ -27,10 +31,84 @@ static_assert(side_of((1u << 31) / 64u - 1u, 255u, 4u) == (1u << 31) - 1u, "4 la
 // (One thread per facet walked ~30 such chains: 7.2 us per sweep on the
 // 4,096-facet scene of 98,000 edges, 4.1 here, 2.9 where a sweep begins while
 // the one before it ends: 64 sweeps 333 -> 243 us, of 1.3 M edges 669 -> 521.)
-// L follows the mean row length.
+// L follows the mean row length (lanes_for).
 // kEarly: launched while the sweep before it ends; only what that one writes is
 // waited for.  (With optics read after the wait, so that any kernel might write
 // them, 64 sweeps of the 4,096-facet scene took 1.3 % longer.)
+struct SideRow {
+    uint32_t start, end, denom, skyc;  // skyc and optics in the row's first lane
+    facetcu_surface_optics optics;
+};
+template <int L>
+__device__ __forceinline__ SideRow load_row(
+    bool valid, uint32_t s, const uint32_t* __restrict__ rows, const uint32_t* __restrict__ denom,
+    const uint32_t* __restrict__ skyc, const facetcu_surface_optics* __restrict__ optics)
+{
+    SideRow r{};
+    if (valid) {
+        r.start = rows[s];
+        r.end = rows[s + 1];
+        r.denom = denom[s];
+        if (threadIdx.x % L == 0) {
+            r.skyc = skyc[s];
+            r.optics = optics[s];
+        }
+    }
+    return r;
+}
+// The new value of side s by its L lanes (whole warps, for the shuffles); returns
+// |dB| in the first of them.
+template <int L>
+__device__ __forceinline__ float sweep_row(bool valid, uint32_t s, const SideRow& r,
+                                           const facetcu_csr_edge* __restrict__ edges, float sky,
+                                           float relax, const float* Bin, float* Bout)
+{
+    constexpr int U = 4;
+    const uint32_t eg = threadIdx.x % L;
+    float acc = 0.0f, old = 0.0f;
+    if (valid) {
+        if (eg == 0) old = Bin[s];
+        for (uint32_t e = r.start + eg; e < r.end; e += L * U) {
+            facetcu_csr_edge ed[U];
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                ed[u] = {0u, 0u};
+                if (e + u * L < r.end) ed[u] = edges[e + u * L];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = e + u * L < r.end ? Bin[ed[u].neighbor] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) acc += float(ed[u].count) * v[u];
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 1; k < L; k <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
+    const facetcu_surface_optics& o = r.optics;
+    const float h = (r.denom == 0u ? sky : (float(r.skyc) * sky + acc) / float(r.denom)) +
+                    o.direct_irradiance;
+    const float other = __shfl_xor_sync(0xffffffffu, h, L);  // the facet's other side
+    if (!valid || eg != 0) return 0.0f;
+    const float t = o.emission + o.reflectance * h + o.transmittance * other;
+    // GLSL mix(x, y, a) = x * (1 - a) + y * a
+    const float b = old * (1.0f - relax) + t * relax;
+    Bout[s] = b;
+    return fabsf(b - old);
+}
+__device__ __forceinline__ void publish_delta(float delta, uint32_t* max_delta_bits)
+{
+    __shared__ float block_delta[8];
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) delta = fmaxf(delta, __shfl_xor_sync(0xffffffffu, delta, k));
+    if ((threadIdx.x & 31) == 0) block_delta[threadIdx.x >> 5] = delta;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) delta = fmaxf(delta, block_delta[w]);
+        atomicMax(max_delta_bits, __float_as_uint(delta));
+    }
+}
+
 template <int L, bool kEarly>
 __global__ void __launch_bounds__(256) k_jacobi_rows(
     uint32_t facets, const uint32_t* __restrict__ rows, const facetcu_csr_edge* __restrict__ edges,
@@ -39,63 +117,73 @@ __global__ void __launch_bounds__(256) k_jacobi_rows(
     const float* Bin, float* Bout, uint32_t* max_delta_bits)
 {
     if (kEarly) start_next();
-    constexpr int U = 4;
-    __shared__ float block_delta[8];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t eg = lane % L;
     const uint32_t s = side_of(blockIdx.x, threadIdx.x, L);
-    float delta = 0.0f;
-    // whole warps stay for the shuffles
     const bool valid = (s >> 1) < facets;
-    float acc = 0.0f, old = 0.0f;
-    uint32_t d = 0, sc = 0;
-    facetcu_surface_optics o{};
-    uint32_t start = 0, end = 0;
-    if (valid) {
-        start = rows[s];
-        end = rows[s + 1];
-        d = denom[s];
-        if (eg == 0) {
-            sc = skyc[s];
-            o = optics[s];
-        }
-    }
+    const SideRow r = load_row<L>(valid, s, rows, denom, skyc, optics);
     if (kEarly) wait_for_previous();
-    if (valid) {
-        if (eg == 0) old = Bin[s];
-        for (uint32_t e = start + eg; e < end; e += L * U) {
-            facetcu_csr_edge ed[U];
-            float v[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                ed[u] = {0u, 0u};
-                if (e + u * L < end) ed[u] = edges[e + u * L];
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) v[u] = e + u * L < end ? Bin[ed[u].neighbor] : 0.0f;
-#pragma unroll
-            for (int u = 0; u < U; ++u) acc += float(ed[u].count) * v[u];
-        }
+    publish_delta(sweep_row<L>(valid, s, r, edges, sky, relax, Bin, Bout), max_delta_bits);
+}
+
+// Lanes of a side for rows of `mean` edges.  A sweep in us (k_jacobi_any; rows of
+// half to one and a half times the mean) with 1, 4, 8 and 16 lanes, and with one
+// thread per facet:
+//     mean              2     4     8    12    20    32    48    64
+//     40,000 sides 1  4.4   5.3   6.4   8.4  10.5  14.6  18.7  24.7
+//                  4  4.3   6.3   6.4   6.4   8.4   8.5  10.5  12.5
+//                  8  6.3   6.3   6.4   6.4   8.4   8.5  10.5  12.5
+//                 16  8.4   8.4   8.4   8.4   8.4   9.0  10.4  11.7
+//             thread  6.4   7.4   8.4  10.5  10.9  14.5  18.5  20.9
+//     1,000,000    1   12    19    35    58   107   180   271
+//                  4   27    27    37    53    76   121   182
+//                  8   49    50    52    59    77   108   155
+//                 16   95    96    97    99   103   115   157
+//             thread   23    31    46    68   101   162   230
+// (Short rows of large graphs leave most of many lanes idle; below 2,048 sides all
+// but 1 take the 4.3 us of a launch up to 20 edges.)
+constexpr __host__ __device__ int lanes_for(uint64_t mean)
+{
+    return mean < 4 ? 1 : mean < 10 ? 4 : mean < 48 ? 8 : 16;
+}
+
+// The sweep where only the device knows the number of edges, rows[surfaces]: a
+// grid of resident blocks walks the sides, with lanes by the same rule.  (With the
+// lanes of the longest rows whatever the graph, a million sides of 1 to 8 edges
+// took 92 to 107 us a sweep; one thread per facet 19 to 46, this 10 to 37.)
+template <int L>
+__device__ __forceinline__ float sweep_rows_of(uint32_t surfaces, const uint32_t* __restrict__ rows,
+                                               const facetcu_csr_edge* __restrict__ edges,
+                                               const uint32_t* __restrict__ denom,
+                                               const uint32_t* __restrict__ skyc,
+                                               const facetcu_surface_optics* __restrict__ optics,
+                                               float sky, float relax, const float* Bin, float* Bout)
+{
+    float delta = 0.0f;
+    const uint32_t blocks = (surfaces + 256u / L - 1u) / (256u / L);
+    for (uint32_t b = blockIdx.x; b < blocks; b += gridDim.x) {
+        const uint32_t s = side_of(b, threadIdx.x, L);
+        const bool valid = s < surfaces;
+        const SideRow r = load_row<L>(valid, s, rows, denom, skyc, optics);
+        delta = fmaxf(delta, sweep_row<L>(valid, s, r, edges, sky, relax, Bin, Bout));
     }
-#pragma unroll
-    for (int k = 1; k < L; k <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
-    const float h = (d == 0u ? sky : (float(sc) * sky + acc) / float(d)) + o.direct_irradiance;
-    const float other = __shfl_xor_sync(0xffffffffu, h, L);  // the facet's other side
-    if (valid && eg == 0) {
-        const float t = o.emission + o.reflectance * h + o.transmittance * other;
-        // GLSL mix(x, y, a) = x * (1 - a) + y * a
-        const float b = old * (1.0f - relax) + t * relax;
-        Bout[s] = b;
-        delta = fabsf(b - old);
-    }
-#pragma unroll
-    for (int k = 16; k > 0; k >>= 1) delta = fmaxf(delta, __shfl_xor_sync(0xffffffffu, delta, k));
-    if (lane == 0) block_delta[warp] = delta;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) delta = fmaxf(delta, block_delta[w]);
-        atomicMax(max_delta_bits, __float_as_uint(delta));
-    }
+    return delta;
+}
+__global__ void __launch_bounds__(256) k_jacobi_any(
+    uint32_t surfaces, const uint32_t* __restrict__ rows, const facetcu_csr_edge* __restrict__ edges,
+    const uint32_t* __restrict__ denom, const uint32_t* __restrict__ skyc,
+    const facetcu_surface_optics* __restrict__ optics, float sky, float relax, const float* Bin,
+    float* Bout, uint32_t* max_delta_bits)
+{
+    const int lanes = lanes_for(rows[surfaces] / surfaces);
+    auto sweep = [&](auto L) {
+        return sweep_rows_of<decltype(L)::value>(surfaces, rows, edges, denom, skyc, optics, sky, relax,
+                                                 Bin, Bout);
+    };
+    float delta;
+    if (lanes == 1) delta = sweep(std::integral_constant<int, 1>{});
+    else if (lanes == 4) delta = sweep(std::integral_constant<int, 4>{});
+    else if (lanes == 8) delta = sweep(std::integral_constant<int, 8>{});
+    else delta = sweep(std::integral_constant<int, 16>{});
+    publish_delta(delta, max_delta_bits);
 }
 
 // ---- all sweeps of a small graph in one launch ----------------------------
@@ -295,26 +383,32 @@ __global__ void __launch_bounds__(128) k_incident(
 namespace {
 
 template <bool kEarly>
-void sweep_rows(uint32_t surfaces, uint64_t edges_hint, const uint32_t* rows,
-                const facetcu_csr_edge* edges, const uint32_t* denom, const uint32_t* skyc,
-                const facetcu_surface_optics* d_optics, float sky, float relaxation,
-                const float* d_in, float* d_out, uint32_t* d_max_delta_bits, cudaStream_t s)
+void sweep_rows(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
+                float relaxation, const float* d_in, float* d_out, uint32_t* d_max_delta_bits,
+                cudaStream_t s)
 {
-    const uint32_t facets = surfaces / 2u;
+    const uint32_t facets = g.surfaces / 2u;
     if (!facets) return;
-    auto launch = [&](auto kernel, uint32_t lanes) {
-        const unsigned grid = unsigned((uint64_t(surfaces) * lanes + 255) / 256);
+    auto launch = [&](auto lanes) {
+        constexpr int L = decltype(lanes)::value;
+        const unsigned grid = unsigned((uint64_t(g.surfaces) * L + 255) / 256);
+        const uint32_t *rows = g.row_offsets.as<uint32_t>(), *denom = g.denominators.as<uint32_t>(),
+                       *skyc = g.sky.as<uint32_t>();
+        const facetcu_csr_edge* edges = g.edges.as<facetcu_csr_edge>();
         if (kEarly)
-            launch_early(kernel, grid, 256, 0, s, facets, rows, edges, denom, skyc, d_optics, sky,
-                         relaxation, d_in, d_out, d_max_delta_bits);
+            launch_early(k_jacobi_rows<L, true>, grid, 256, 0, s, facets, rows, edges, denom, skyc,
+                         d_optics, sky, relaxation, d_in, d_out, d_max_delta_bits);
         else
-            kernel<<<grid, 256, 0, s>>>(facets, rows, edges, denom, skyc, d_optics, sky, relaxation,
-                                        d_in, d_out, d_max_delta_bits);
+            k_jacobi_rows<L, false><<<grid, 256, 0, s>>>(facets, rows, edges, denom, skyc, d_optics,
+                                                         sky, relaxation, d_in, d_out,
+                                                         d_max_delta_bits);
     };
-    const uint64_t mean = edges_hint / surfaces;
-    if (mean < 8) launch(k_jacobi_rows<4, kEarly>, 4);
-    else if (mean < 48) launch(k_jacobi_rows<8, kEarly>, 8);
-    else launch(k_jacobi_rows<16, kEarly>, 16);
+    switch (lanes_for(g.nnz / g.surfaces)) {
+    case 1: launch(std::integral_constant<int, 1>{}); break;
+    case 4: launch(std::integral_constant<int, 4>{}); break;
+    case 8: launch(std::integral_constant<int, 8>{}); break;
+    default: launch(std::integral_constant<int, 16>{}); break;
+    }
     FCU_LAUNCH("k_jacobi_rows");
 }
 
@@ -322,13 +416,18 @@ void sweep_rows(uint32_t surfaces, uint64_t edges_hint, const uint32_t* rows,
 
 // (The caller's arrays may have been written by the kernel just before: no
 // early start here.)
-void jacobi_sweep_raw(uint32_t surfaces, uint64_t edges_hint, const uint32_t* rows,
-                      const facetcu_csr_edge* edges, const uint32_t* denom, const uint32_t* skyc,
+void jacobi_sweep_raw(uint32_t surfaces, const uint32_t* rows, const facetcu_csr_edge* edges,
+                      const uint32_t* denom, const uint32_t* skyc,
                       const facetcu_surface_optics* d_optics, float sky, float relaxation,
                       const float* d_in, float* d_out, uint32_t* d_max_delta_bits, cudaStream_t s)
 {
-    sweep_rows<false>(surfaces, edges_hint, rows, edges, denom, skyc, d_optics, sky, relaxation, d_in,
-                      d_out, d_max_delta_bits, s);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const unsigned most = unsigned((uint64_t(surfaces) * 16 + 255) / 256);
+    k_jacobi_any<<<std::min(most, 8u * unsigned(std::max(sms, 1))), 256, 0, s>>>(
+        surfaces, rows, edges, denom, skyc, d_optics, sky, relaxation, d_in, d_out, d_max_delta_bits);
+    FCU_LAUNCH("k_jacobi_any");
 }
 
 void jacobi_sweep(const DeviceGraph& g, bool planned, const facetcu_surface_optics* d_optics,
@@ -339,10 +438,8 @@ void jacobi_sweep(const DeviceGraph& g, bool planned, const facetcu_surface_opti
         column_jacobi(g, d_optics, sky, relaxation, d_in, d_out, d_max_delta_bits, s);
         return;
     }
-    (follows ? sweep_rows<true> : sweep_rows<false>)(
-        g.surfaces, g.nnz, g.row_offsets.as<uint32_t>(), g.edges.as<facetcu_csr_edge>(),
-        g.denominators.as<uint32_t>(), g.sky.as<uint32_t>(), d_optics, sky, relaxation, d_in, d_out,
-        d_max_delta_bits, s);
+    (follows ? sweep_rows<true> : sweep_rows<false>)(g, d_optics, sky, relaxation, d_in, d_out,
+                                                     d_max_delta_bits, s);
 }
 
 bool jacobi_sweeps_cluster(const DeviceGraph& g, const facetcu_surface_optics* d_optics, float sky,
