@@ -24,7 +24,7 @@
 
 using namespace facetcu;
 
-struct facetcu_context {
+struct facetcu_context final : facetcu::Spare {
     std::string last_error;
     bool initialized = false;
     facetcu_config config{};
@@ -67,6 +67,18 @@ struct facetcu_context {
     };
     std::map<std::string, Tuned> tuned;
     std::string gpu_name;                   // for the autotuner's key
+
+    // Kept from earlier calls for speed alone.
+    bool give_back() override
+    {
+        bool any = ws.kept != 0;
+        ws.drop_blocks();
+        any |= vertices_next.ptr != nullptr;
+        vertices_next.release();
+        any |= graph.column.give_back();
+        any |= raster.give_back();
+        return any;
+    }
 };
 
 namespace {
@@ -81,6 +93,7 @@ template <typename F>
 int guarded(facetcu_context* ctx, F&& body)
 {
     if (!ctx) return FACETCU_INVALID_ARGUMENT;
+    const SpareScope scope(ctx);
     try {
         ctx->last_error.clear();
         return body();
@@ -437,7 +450,10 @@ int facetcu_set_geometry(facetcu_context* ctx, const facetcu_vertex* vertices,
         if (vertex_count / 3 > (1ull << 30))
             throw Error(FACETCU_OVERFLOW_ERROR, "Geometry exceeds 2^30 facets");
         // checked on the device before anything of the old geometry changes
-        DeviceBuffer& next = ctx->vertices_next;
+        // (in a buffer of this call, so that nothing gives it back meanwhile)
+        DeviceBuffer next;
+        std::swap(next.ptr, ctx->vertices_next.ptr);
+        std::swap(next.bytes, ctx->vertices_next.bytes);
         upload(next, vertices, vertex_count * sizeof(facetcu_vertex), ctx->stream);
         const GeometryCheck check =
             check_geometry(next.as<facetcu_vertex>(), vertex_count, ctx->ws, ctx->stream);
@@ -452,6 +468,8 @@ int facetcu_set_geometry(facetcu_context* ctx, const facetcu_vertex* vertices,
         ctx->facets = uint32_t(vertex_count / 3);
         std::swap(ctx->vertices.ptr, next.ptr);
         std::swap(ctx->vertices.bytes, next.bytes);
+        std::swap(next.ptr, ctx->vertices_next.ptr);  // the old one, for the next call
+        std::swap(next.bytes, ctx->vertices_next.bytes);
         for (int a = 0; a < 3; ++a) {
             ctx->bmin[a] = check.lo[a];
             ctx->bmax[a] = check.hi[a];
@@ -491,6 +509,7 @@ int facetcu_build_visibility_graph(facetcu_context* ctx, const facetcu_direction
         if (!directions || direction_count == 0)
             throw Error(FACETCU_INVALID_ARGUMENT, "At least one visibility direction is required");
         ctx->graph_ready = false;
+        const RasterUse use(ctx->raster);
         const uint32_t S = ctx->facets * 2u;
         const int side_bits = side_bits_for(S);
         std::vector<RasterView> views(direction_count);
@@ -579,6 +598,7 @@ int facetcu_compute_sunlit_fraction(facetcu_context* ctx, const facetcu_directio
         if (ctx->facets == 0)
             throw Error(FACETCU_LOGIC_ERROR, "setGeometry() must be called before computeSunlitFraction()");
         if (!sun || !fraction) throw Error(FACETCU_INVALID_ARGUMENT, "sun direction and output are required");
+        const RasterUse use(ctx->raster);
         const uint32_t S = ctx->facets * 2u;
         const RasterView view = make_view(*sun);
         const RasterFrame frame = make_frame(ctx);

@@ -64,6 +64,39 @@ __device__ __forceinline__ void start_next()
 #endif
 
 
+// What the context of the running call keeps and can do without while one of
+// the call's allocations fails.  give_back() returns whether it freed anything;
+// SpareScope names the context for the calling thread.
+struct Spare {
+    virtual bool give_back() = 0;
+
+protected:
+    ~Spare() = default;
+};
+inline Spare*& spare()
+{
+    static thread_local Spare* of_this_thread = nullptr;
+    return of_this_thread;
+}
+struct SpareScope {
+    Spare* before;
+    explicit SpareScope(Spare* s) : before(spare()) { spare() = s; }
+    SpareScope(const SpareScope&) = delete;
+    SpareScope& operator=(const SpareScope&) = delete;
+    ~SpareScope() { spare() = before; }
+};
+inline void* device_alloc(size_t n)
+{
+    void* p = nullptr;
+    cudaError_t e = cudaMalloc(&p, n);
+    if (e == cudaErrorMemoryAllocation && spare() && spare()->give_back()) {
+        cudaGetLastError();
+        e = cudaMalloc(&p, n);
+    }
+    cuda_check(e, "cudaMalloc");
+    return p;
+}
+
 // Owning device buffer that only grows.
 struct DeviceBuffer {
     void* ptr = nullptr;
@@ -83,7 +116,7 @@ struct DeviceBuffer {
         if (n <= bytes && ptr) return ptr;
         release();
         if (n == 0) n = 16;
-        cuda_check(cudaMalloc(&ptr, n), "cudaMalloc");
+        ptr = device_alloc(n);
         bytes = n;
         return ptr;
     }
@@ -110,7 +143,7 @@ struct RasterFrame {
 
 // Scratch used by the device sort and scan, and the blocks that builds borrow
 // (ScratchBuffer): kept for the next build up to kKeep bytes in all, given
-// back by release().  A context's work is on one stream, so a block may be
+// back by release(), and when an allocation of the context fails (Spare).  A context's work is on one stream, so a block may be
 // lent again as soon as it is handed back.
 struct Workspace {
     DeviceBuffer a, b, c, d, e;
@@ -142,14 +175,7 @@ struct Workspace {
             return b;
         }
         Block b{nullptr, n ? n : 16};
-        if (cudaMalloc(&b.ptr, b.bytes) == cudaErrorMemoryAllocation && kept) {
-            cudaGetLastError();
-            drop_blocks();  // make room
-            cuda_check(cudaMalloc(&b.ptr, b.bytes), "cudaMalloc");
-        } else if (!b.ptr) {
-            cudaGetLastError();
-            cuda_check(cudaMalloc(&b.ptr, b.bytes), "cudaMalloc");
-        }
+        b.ptr = device_alloc(b.bytes);
         return b;
     }
     void hand_back(const Block& b) noexcept
@@ -217,6 +243,25 @@ struct RasterBuffers {
     DeviceBuffer jobs;    // triangles for warps (from the front) and blocks (from the back)
     DeviceBuffer list;    // pixels with more than the register path's chain
     DeviceBuffer stats;   // RasterStats
+    bool busy = false;    // a build or sun pass is using them
+    // The lists are rebuilt by every pass.
+    bool give_back()
+    {
+        bool any = false;
+        if (!busy)
+            for (DeviceBuffer* b : {&heads, &nodes, &planes, &jobs, &list}) {
+                any |= b->ptr != nullptr;
+                b->release();
+            }
+        return any;
+    }
+};
+struct RasterUse {
+    RasterBuffers& rb;
+    explicit RasterUse(RasterBuffers& r) : rb(r) { rb.busy = true; }
+    RasterUse(const RasterUse&) = delete;
+    RasterUse& operator=(const RasterUse&) = delete;
+    ~RasterUse() { rb.busy = false; }
 };
 
 struct RasterStats {
@@ -263,6 +308,14 @@ struct ColumnPlan {
     uint32_t ctas = 0, tiles = 0;
     DeviceBuffer shares, groups, meta, words, partial;
     void release();
+    // (Only a finished plan, and not between column_plan() and the sweeps that
+    // rely on it: no call allocates there.)
+    bool give_back()
+    {
+        if (state != kMade) return false;
+        release();
+        return true;
+    }
 };
 
 // ---- graph assembly (graph.cu) ------------------------------------------
