@@ -451,12 +451,21 @@ int facetcu_set_geometry(facetcu_context* ctx, const facetcu_vertex* vertices,
             throw Error(FACETCU_OVERFLOW_ERROR, "Geometry exceeds 2^30 facets");
         // checked on the device before anything of the old geometry changes
         // (in a buffer of this call, so that nothing gives it back meanwhile)
+        const size_t bytes = vertex_count * sizeof(facetcu_vertex);
         DeviceBuffer next;
         std::swap(next.ptr, ctx->vertices_next.ptr);
         std::swap(next.bytes, ctx->vertices_next.bytes);
-        upload(next, vertices, vertex_count * sizeof(facetcu_vertex), ctx->stream);
-        const GeometryCheck check =
-            check_geometry(next.as<facetcu_vertex>(), vertex_count, ctx->ws, ctx->stream);
+        GeometryCheck check;
+        try {
+            upload(next, vertices, bytes, ctx->stream);
+            check = check_geometry(next.as<facetcu_vertex>(), vertex_count, ctx->ws, ctx->stream);
+        } catch (const Error& e) {
+            // No room for both geometries: the new one is checked in pieces and
+            // takes the old one's place below.
+            if (e.code != FACETCU_OUT_OF_MEMORY) throw;
+            next.release();
+            check = check_geometry_in_pieces(vertices, vertex_count, ctx->ws, ctx->stream);
+        }
         if (check.bad_position != 0xffffffffu && check.bad_position <= check.bad_normal)
             throw Error(FACETCU_INVALID_ARGUMENT, "Geometry contains a non-finite position");
         if (check.bad_normal != 0xffffffffu)
@@ -465,11 +474,20 @@ int facetcu_set_geometry(facetcu_context* ctx, const facetcu_vertex* vertices,
         ctx->graph.changed();
         ctx->graph.scene_facets.clear();
         ctx->bvh_ready = false;
+        if (next.ptr) {
+            std::swap(ctx->vertices.ptr, next.ptr);
+            std::swap(ctx->vertices.bytes, next.bytes);
+        } else {
+            ctx->facets = 0;  // until the new geometry is there
+            ctx->vertices.release();
+            upload(ctx->vertices, vertices, bytes, ctx->stream);
+            FCU_CHECK(cudaStreamSynchronize(ctx->stream));
+        }
         ctx->facets = uint32_t(vertex_count / 3);
-        std::swap(ctx->vertices.ptr, next.ptr);
-        std::swap(ctx->vertices.bytes, next.bytes);
-        std::swap(next.ptr, ctx->vertices_next.ptr);  // the old one, for the next call
-        std::swap(next.bytes, ctx->vertices_next.bytes);
+        if (next.bytes <= Workspace::kKeep / 4) {  // the old buffer, for the next call
+            std::swap(next.ptr, ctx->vertices_next.ptr);
+            std::swap(next.bytes, ctx->vertices_next.bytes);
+        }
         for (int a = 0; a < 3; ++a) {
             ctx->bmin[a] = check.lo[a];
             ctx->bmax[a] = check.hi[a];

@@ -6,6 +6,7 @@
 // pass over the vertices took 3 ms for 200,000 facets, more than the raster
 // build that follows; here it is one read of the uploaded vertices (compiled
 // with -fmad=false: the normal's length rounds as the host's did).
+#include <algorithm>
 #include <cfloat>
 
 #include "internal.h"
@@ -110,6 +111,31 @@ GeometryCheck check_geometry(const facetcu_vertex* d_vertices, uint64_t count, W
         c.hi[k] = value_of(r.hi[k]);
     }
     return c;
+}
+
+GeometryCheck check_geometry_in_pieces(const facetcu_vertex* vertices, uint64_t count,
+                                       Workspace& ws, cudaStream_t s)
+{
+    constexpr uint64_t kPiece = 1u << 17;  // 3 MB
+    ScratchBuffer buf(ws);
+    facetcu_vertex* d = static_cast<facetcu_vertex*>(
+        buf.reserve(std::min(count, kPiece) * sizeof(facetcu_vertex)));
+    GeometryCheck all{0xffffffffu, 0xffffffffu, {FLT_MAX, FLT_MAX, FLT_MAX}, {-FLT_MAX, -FLT_MAX, -FLT_MAX}};
+    for (uint64_t first = 0; first < count; first += kPiece) {
+        const uint64_t n = std::min(kPiece, count - first);
+        FCU_CHECK(cudaMemcpyAsync(d, vertices + first, n * sizeof(facetcu_vertex),
+                                  cudaMemcpyHostToDevice, s));
+        const GeometryCheck c = check_geometry(d, n, ws, s);
+        if (c.bad_position != 0xffffffffu)
+            all.bad_position = std::min(all.bad_position, uint32_t(first) + c.bad_position);
+        if (c.bad_normal != 0xffffffffu)
+            all.bad_normal = std::min(all.bad_normal, uint32_t(first) + c.bad_normal);
+        for (int a = 0; a < 3; ++a) {
+            all.lo[a] = std::min(all.lo[a], c.lo[a]);
+            all.hi[a] = std::max(all.hi[a], c.hi[a]);
+        }
+    }
+    return all;
 }
 
 }  // namespace facetcu

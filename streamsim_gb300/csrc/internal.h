@@ -482,6 +482,9 @@ struct GeometryCheck {
 };
 GeometryCheck check_geometry(const facetcu_vertex* d_vertices, uint64_t count, Workspace& ws,
                              cudaStream_t s);
+// The same for vertices in host memory, a few MB on the device at a time.
+GeometryCheck check_geometry_in_pieces(const facetcu_vertex* vertices, uint64_t count,
+                                       Workspace& ws, cudaStream_t s);
 
 // ---- warm-start MLP (mlp.cu) -----------------------------------------------
 namespace mlp {

@@ -65,3 +65,54 @@ def test_solve_with_the_plan_in_the_way():
         torch.cuda.empty_cache()
     m.close()
     assert np.array_equal(got, want)
+
+
+def test_geometry_without_room_for_two():
+    """Both geometries don't fit: the new one is checked in pieces (more than five
+    here) and takes the old one's place; a refused one leaves the old one."""
+    require_gpu()
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(2)
+    F = 300_001
+
+    def geometry(seed):
+        g = np.random.default_rng(seed)
+        v = np.zeros((F, 3, 6), np.float32)
+        v[:, :, :3] = g.uniform(-8, 8, (F, 1, 3)) + g.uniform(-0.1, 0.1, (F, 3, 3))
+        v[:, :, 4] = 1.0
+        return v.reshape(-1, 6)
+
+    a, b = geometry(1), geometry(2)
+    b[rng.integers(0, len(b)), 0] = 9.5  # the bounds come from one vertex
+    b[len(b) - 1, 2] = -9.75
+    sun = np.float32([0.3, 0.9, 0.1])
+
+    def model(v):
+        m = facetcu.FacetrtCuda()
+        m.initialize(64, 64, 1024)
+        m.setGeometry(v)
+        return m
+
+    m = model(b)
+    want = m.computeSunlitFraction(sun)
+    m.close()
+    m = model(a)
+    torch.cuda.synchronize()
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - (12 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        for at, value, match in ((len(b) - 1, np.nan, "non-finite"), (200_000, np.inf, "non-finite")):
+            bad = b.copy()
+            bad[at, 1] = value
+            with pytest.raises(ValueError, match=match):
+                m.setGeometry(bad)
+        bad = b.copy()
+        bad[300_000, 4], bad[800_000, 0] = 2.0, np.nan
+        with pytest.raises(ValueError, match="normalized"):  # the earlier vertex
+            m.setGeometry(bad)
+        m.setGeometry(b)
+    finally:
+        del rest
+        torch.cuda.empty_cache()
+    got = m.computeSunlitFraction(sun)
+    m.close()
+    assert np.array_equal(got, want)
