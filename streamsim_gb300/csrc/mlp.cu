@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256, 2) k_layer(int rows, const float* __restr
     } else {
         for (int i = threadIdx.x; i < K * N; i += 256) Bs[i / N][i % N] = __bfloat162float(W[i]);
     }
-    float loss = 0.0f, loss_low = 0.0f;  // compensated: about twice the float precision
+    double loss = 0.0;
     for (int r0 = blockIdx.x * kRows; r0 < rows; r0 += gridDim.x * kRows) {
     float4 next[kFetch];
     auto fetch = [&](int k0) {
@@ -175,11 +175,7 @@ __global__ void __launch_bounds__(256, 2) k_layer(int rows, const float* __restr
                 if (E == kGeluBack) v[j] *= gelu_grad(w[j]);
                 if (E == kLoss) {
                     const float d = v[j] - w[j];
-                    const float q = __fmul_rn(d, d), t = __fadd_rn(loss, q);
-                    const float e = fabsf(loss) >= q ? __fadd_rn(__fadd_rn(loss, -t), q)
-                                                     : __fadd_rn(__fadd_rn(q, -t), loss);
-                    loss = t;
-                    loss_low = __fadd_rn(loss_low, __fadd_rn(e, __fmaf_rn(d, d, -q)));
+                    loss += double(d) * double(d);
                     v[j] = 2.0f * d * args.scale;
                 }
             }
@@ -192,7 +188,7 @@ __global__ void __launch_bounds__(256, 2) k_layer(int rows, const float* __restr
     }
     if (E == kLoss) {
         double* red = reinterpret_cast<double*>(smem);  // (the operands are done with)
-        red[threadIdx.x] = double(loss) + double(loss_low);
+        red[threadIdx.x] = loss;
         __syncthreads();
         for (int o = 128; o > 0; o >>= 1) {
             if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
