@@ -43,9 +43,13 @@ namespace {
 
 constexpr int kWarps = 8;
 constexpr uint32_t kSky = 0xFFFFFFFFu;
-// A node leaves up to 3 children waiting; the tree is at most 47 deep (30
-// Morton bits, then up to 17 of the facet's number among equal codes).
-constexpr int kStack = 144;
+// A visited node leaves up to 3 children waiting, and the next one lies below it.
+// Inner nodes below one another differ in the first bit that their leaves' keys
+// don't share: 30 Morton bits, then those of the facet's place among equal codes,
+// 30 for the 2^30 facets that setGeometry takes.
+constexpr int kMortonBits = 30, kPlaceBits = 30;
+constexpr int kStack = 180;
+static_assert(kStack >= 3 * (kMortonBits + kPlaceBits), "no accepted scene overflows the stack");
 constexpr int kKeptLeaves = 8;  // lanes with a leaf that make the warp test them (4, 12: equal; 16: +6 %)
 constexpr int kRefill = 8;      // idle lanes that make the warp fetch rays (4, 12: equal)
 constexpr int kSteps = 4;       // node steps between looks for idle lanes
@@ -750,7 +754,7 @@ void hemisphere_graph(const facetcu_vertex* d_vertices, uint32_t facets, const L
     unsigned long long host[3] = {0, 0, 0};
     FCU_CHECK(cudaMemcpyAsync(host, cnt, 24, cudaMemcpyDeviceToHost, s));
     FCU_CHECK(cudaStreamSynchronize(s));
-    if (uint32_t(host[2])) throw Error(FACETCU_DEVICE_CAPACITY, "BVH traversal stack exceeded 144 entries");
+    if (uint32_t(host[2])) throw Error(FACETCU_DEVICE_CAPACITY, "BVH traversal stack exceeded 180 entries");
     g.nnz = host[1];
     facetcu_csr_edge* edges = static_cast<facetcu_csr_edge*>(g.edges.reserve((g.nnz + 1) * 8));
     k_hemi_compact<<<(S * 32 + 255) / 256, 256, 0, s>>>(tmp_edges, rows, S, top_k, reinterpret_cast<uint2*>(edges));
@@ -785,7 +789,7 @@ void hemisphere_sunlit(const facetcu_vertex* d_vertices, uint32_t facets, const 
     uint32_t e = 0;
     FCU_CHECK(cudaMemcpyAsync(&e, d_error, 4, cudaMemcpyDeviceToHost, s));
     FCU_CHECK(cudaStreamSynchronize(s));
-    if (e) throw Error(FACETCU_DEVICE_CAPACITY, "BVH traversal stack exceeded 144 entries");
+    if (e) throw Error(FACETCU_DEVICE_CAPACITY, "BVH traversal stack exceeded 180 entries");
 }
 
 }  // namespace facetcu
