@@ -193,19 +193,23 @@ __global__ void __launch_bounds__(256) k_jacobi_any(
 // their edges in shared memory, and writes its new values into the others'.
 // Bound by that exchange and the cluster's barrier: 1 us a sweep for 1,152
 // sides, 2.5 for 8,192 (with blocks that wait on a count of received bytes
-// instead, 2.2 by bulk copies and 3.2 by asynchronous stores).  64 sweeps in
-// early launches and here, us:
-//     sides      1,152   2,048   3,200   4,608   6,272   8,192
-//     edges      6,708  18,923  33,350  50,392  72,020  98,058
-//     launches     160     173     187     202     211     243
-//     cluster      126     142     160     195     225     249
-// (two lanes a side; four: 125 and 279 for the first and the last; eight blocks:
-// 304 for the last.)  Setting up costs some launches: 8 sweeps of 6,708 edges
-// take 58 and 59, 12 take 64 and 60.
+// instead, 2.2 by bulk copies and 3.2 by asynchronous stores).  A call of 64 sweeps
+// in us, in early launches / here:
+//     edges     7,000      16,000     33,000     50,000     70,000     100,000
+//       256   157 / 131  158 / 159  196 / 281  248 / 283  255 / 359  337 / 465
+//       768   161 / 122  159 / 127  176 / 148  195 / 172  189 / 196  229 / 233
+//     1,152   169 / 125  170 / 138  171 / 147  191 / 162  182 / 176  205 / 200
+//     2,048   180 / 129  175 / 133  181 / 153  181 / 153  223 / 165  200 / 203
+//     3,200   190 / 145  180 / 148  187 / 158  199 / 159  199 / 170  216 / 182
+//     4,096              195 / 150  188 / 162  202 / 162  213 / 173  218 / 191
+// so rows of more than 64 edges, which two lanes read alone, go to the launches.
+// (8,192 sides of 98,058 edges: 243 / 249.  Four lanes a side: 125 for the first and
+// 279 for the last; eight blocks: 304 for the last.)  Setting up costs some
+// launches: 12 sweeps take 59 us and 57 on 256 sides, 65 and 67 on 1,152.
 constexpr uint32_t kCtas = 16, kClusterThreads = 1024, kGroup = 16, kDeltas = 64;
 constexpr int kClusterLanes = 2;
 constexpr uint32_t kClusterSides = 4096, kClusterSweeps = 12;
-constexpr uint64_t kClusterEdges = 100000;
+constexpr uint64_t kClusterEdges = 100000, kClusterMean = 64;
 constexpr size_t kClusterShared = 227 * 1024 - 1024;  // (static arrays besides)
 
 struct ClusterShape {
@@ -448,7 +452,7 @@ bool jacobi_sweeps_cluster(const DeviceGraph& g, const facetcu_surface_optics* d
 {
     const uint32_t S = g.surfaces;
     if (sweeps < kClusterSweeps || S < 2 || S > kClusterSides || g.nnz > kClusterEdges ||
-        g.max_count > 0xffffu)
+        g.nnz > kClusterMean * S || g.max_count > 0xffffu)
         return false;
     ClusterShape shape;
     const uint32_t groups = (S + kGroup - 1) / kGroup;

@@ -45,3 +45,18 @@ def test_lanes(S, mean):
         assert np.max(np.abs(b - want) / want) < _tolerance(graph)
     if S > 4096:  # one sweep kernel for both: the same order of additions
         assert np.array_equal(got, out.cpu().numpy())
+
+
+@pytest.mark.parametrize("mean", [63, 64, 65])
+def test_rows_around_the_cluster_limit(mean):
+    """Small graphs whose rows are too long for the cluster go to the sweeps."""
+    require_gpu()
+    S = 250
+    rng = np.random.default_rng(mean)
+    graph = _graph(S, np.full(S, mean), rng, counts=[255, 256, 65535])
+    o = _optics(S, rng)
+    m = _model(S, graph)
+    got = m.solve(o, SKY, 16, 0.75)["radiosity"]
+    m.close()
+    want = _jacobi(graph, o[:, 3].astype(np.float64), o[:, 2].astype(np.float64), 16, 0.75)
+    assert np.max(np.abs(got - want) / want) < _tolerance(graph)
