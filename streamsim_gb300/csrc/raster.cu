@@ -984,6 +984,16 @@ __global__ void k_fraction(uint32_t S, const uint32_t* total, const uint32_t* vi
 
 }  // namespace
 
+namespace {
+unsigned sm_count()
+{
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return unsigned(std::max(sms, 1));
+}
+}  // namespace
+
 void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame,
                       const RasterView* views, uint32_t dir_count, RasterBuffers& rb,
                       uint32_t* d_frags, RasterStats& stats, cudaStream_t s)
@@ -1008,6 +1018,7 @@ void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame
     // 200,000 facets has 0.29 a pixel over the 40 directions, 4,096 facets of
     // terrain 0.25.
     RasterStats host{};
+    const unsigned sms = sm_count();
     uint64_t capacity = std::max<uint64_t>(rb.nodes.bytes / 16, npix / 2 + 1);
     for (uint32_t* counted = d_frags;; counted = nullptr) {
         capacity = std::min<uint64_t>(capacity, 0xffffffffull);
@@ -1018,9 +1029,9 @@ void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame
         k_raster<<<dim3(unsigned((per_dir + 255) / 256), dir_count), 256, 0, s>>>(
             scene, planes, uint32_t(per_dir), pool, jobs, uint32_t(items), dstats, counted);
         FCU_LAUNCH("k_raster");
-        launch_early(k_raster_mid<kMidLanes>, unsigned(std::min<uint64_t>((items + 31) / 32, 8 * 152)),
+        launch_early(k_raster_mid<kMidLanes>, unsigned(std::min<uint64_t>((items + 31) / 32, 8u * sms)),
                      256, 0, s, scene, planes, uint32_t(per_dir), pool, jobs, &dstats->mid, counted);
-        launch_early(k_raster_big, dim3(unsigned(std::min<uint64_t>(items, 152)), 16), 256, 0, s, scene,
+        launch_early(k_raster_big, dim3(unsigned(std::min<uint64_t>(items, sms)), 16), 256, 0, s, scene,
                      planes, uint32_t(per_dir), pool, jobs + items, &dstats->big, counted);
         FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
         FCU_CHECK(cudaStreamSynchronize(s));
@@ -1054,7 +1065,7 @@ void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t
         frame.facets, frame.tiles, rb.heads.as<uint32_t>(), nodes, chain_cap, d_sky, d_pairs, d_pair_count, side_bits, list,
         dstats);
     FCU_LAUNCH("k_resolve_graph");
-    const unsigned list_blocks = 16 * 152;
+    const unsigned list_blocks = 16 * sm_count();
     k_resolve_list<kMidChain><<<list_blocks, 64, 0, s>>>(frame.facets, nodes, list, 0u, d_sky,
                                                          d_pairs, d_pair_count, side_bits, dstats);
     FCU_LAUNCH("k_resolve_list");
