@@ -831,14 +831,16 @@ int facetcu_set_graph(facetcu_context* ctx, uint32_t surface_count, const uint32
                 throw Error(FACETCU_INVALID_ARGUMENT, "graph contains an invalid surface index");
         DeviceGraph& g = ctx->graph;
         cudaStream_t s = ctx->stream;
+        // from here on the old graph is gone, also where a buffer cannot be had
+        ctx->graph_ready = false;
+        g.changed();
+        g.scene_facets.clear();
         g.surfaces = surface_count;
         g.nnz = nnz;
         upload(g.row_offsets, row_offsets, (size_t(surface_count) + 1) * 4, s);
         upload(g.edges, edges, nnz * 8 + 8, s);
         upload(g.denominators, denominators, size_t(surface_count) * 4, s);
         upload(g.sky, sky_counts, size_t(surface_count) * 4, s);
-        g.changed();
-        g.scene_facets.clear();
         float closure;
         uint32_t sampled;
         graph_closure(g, &closure, &sampled, ctx->ws, s);

@@ -116,3 +116,43 @@ def test_geometry_without_room_for_two():
     got = m.computeSunlitFraction(sun)
     m.close()
     assert np.array_equal(got, want)
+
+
+def test_graph_that_does_not_fit_leaves_none():
+    """setGraph gives the old graph up before it allocates: where there is no room
+    for the new one, solves are refused until a graph is set."""
+    require_gpu()
+    torch = pytest.importorskip("torch")
+    S = 4096
+    rng = np.random.default_rng(1)
+    v = np.zeros((3 * S // 2, 6), np.float32)
+    v[:, :3] = rng.uniform(-5, 5, (3 * S // 2, 3))
+    v[:, 4] = 1.0
+
+    def graph(degree):
+        cnt = np.ones(S * degree, np.uint32)
+        return ((np.arange(S + 1) * degree).astype(np.uint32),
+                rng.integers(0, S, S * degree).astype(np.uint32), cnt,
+                np.full(S, degree, np.uint32), np.zeros(S, np.uint32))
+
+    small, large = graph(4), graph(2000)  # 64 MB of edges
+    o = np.zeros((S, 4), np.float32)
+    o[:, 0], o[:, 3] = 0.4, 1.0
+    m = facetcu.FacetrtCuda()
+    m.initialize(64, 64, 64)
+    m.setGeometry(v)
+    m.setGraph(*small)
+    want = m.solve(o, 0.0, 20)["radiosity"]
+    torch.cuda.synchronize()
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - (16 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(facetcu.FacetcuError):
+            m.setGraph(*large)
+    finally:
+        del rest
+        torch.cuda.empty_cache()
+    with pytest.raises(RuntimeError, match="buildVisibilityGraph"):
+        m.solve(o, 0.0, 20)
+    m.setGraph(*small)
+    assert np.array_equal(m.solve(o, 0.0, 20)["radiosity"], want)
+    m.close()
