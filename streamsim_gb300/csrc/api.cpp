@@ -838,7 +838,8 @@ int facetcu_set_graph(facetcu_context* ctx, uint32_t surface_count, const uint32
         g.surfaces = surface_count;
         g.nnz = nnz;
         upload(g.row_offsets, row_offsets, (size_t(surface_count) + 1) * 4, s);
-        upload(g.edges, edges, nnz * 8 + 8, s);
+        g.edges.reserve(nnz * 8 + 8);
+        upload(g.edges, edges, nnz * 8, s);
         upload(g.denominators, denominators, size_t(surface_count) * 4, s);
         upload(g.sky, sky_counts, size_t(surface_count) * 4, s);
         float closure;
