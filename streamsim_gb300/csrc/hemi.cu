@@ -369,7 +369,17 @@ __device__ __forceinline__ uint32_t warp_exclusive(uint32_t v, int lane, uint32_
 // on 4,096 facets).
 constexpr uint32_t kBlockRays = 16384;
 constexpr uint32_t kMaxBlockFacets = 64;
-constexpr uint32_t kBlocksPerSm = 8;  // fewer facets per CTA where there would be fewer CTAs
+// Fewer facets per CTA where there would be fewer than 8 CTAs an SM, down to 768
+// rays (setting up and sorting a CTA costs as much as tracing some hundred), or one
+// CTA an SM.  The whole graph in us with a warp per side / 8 CTAs an SM and no
+// least number / so / 1,024 rays at least:
+//     1,936 facets  32 rays   172   238   173   176
+//                  100 rays   453   352   279   271
+//     2,916 facets  32 rays   186         188   194
+//     4,096 facets  32 rays   334   276   227   204
+//                   64 rays   415   356   302   286
+//    10,800 facets  48 rays   946   601   593   595
+constexpr uint32_t kBlocksPerSm = 8, kLeastRays = 768;
 constexpr uint32_t kBins = 4096;      // directions: 64 x 64 cells of the octahedral map
 constexpr int kTraceThreads = 512;
 
@@ -716,8 +726,11 @@ void hemisphere_graph(const facetcu_vertex* d_vertices, uint32_t facets, const L
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint32_t per_block = std::max(1u, std::min({kMaxBlockFacets, kBlockRays >> (shift + 1),
-                                                      facets / (kBlocksPerSm * uint32_t(std::max(sms, 1)))}));
+    sms = std::max(sms, 1);
+    const uint32_t even = std::max(facets / (kBlocksPerSm * uint32_t(sms)),
+                                   std::min(kLeastRays >> (shift + 1), facets / uint32_t(sms)));
+    const uint32_t per_block =
+        std::max(1u, std::min({kMaxBlockFacets, kBlockRays >> (shift + 1), even}));
     // hit ids of a run of facets at a time
     const uint32_t run = std::min(facets, std::max(per_block, uint32_t((size_t(1) << 30) / (size_t(8) * rays)) / per_block * per_block));
     ScratchBuffer traced_buf(ws);
