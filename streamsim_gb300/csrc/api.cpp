@@ -457,8 +457,12 @@ int facetcu_set_geometry(facetcu_context* ctx, const facetcu_vertex* vertices,
         std::swap(next.bytes, ctx->vertices_next.bytes);
         GeometryCheck check;
         try {
+            const bool checked = check_small_geometry(vertices, vertex_count, check);
             upload(next, vertices, bytes, ctx->stream);
-            check = check_geometry(next.as<facetcu_vertex>(), vertex_count, ctx->ws, ctx->stream);
+            if (checked)
+                FCU_CHECK(cudaStreamSynchronize(ctx->stream));
+            else
+                check = check_geometry(next.as<facetcu_vertex>(), vertex_count, ctx->ws, ctx->stream);
         } catch (const Error& e) {
             // No room for both geometries: the new one is checked in pieces and
             // takes the old one's place below.

@@ -482,6 +482,8 @@ struct GeometryCheck {
 };
 GeometryCheck check_geometry(const facetcu_vertex* d_vertices, uint64_t count, Workspace& ws,
                              cudaStream_t s);
+// The same on the host, where so few vertices are checked faster there (true).
+bool check_small_geometry(const facetcu_vertex* vertices, uint64_t count, GeometryCheck& check);
 // The same for vertices in host memory, a few MB on the device at a time.
 GeometryCheck check_geometry_in_pieces(const facetcu_vertex* vertices, uint64_t count,
                                        Workspace& ws, cudaStream_t s);
