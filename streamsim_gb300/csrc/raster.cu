@@ -439,6 +439,11 @@ __global__ void __launch_bounds__(256) k_raster_mid(const __grid_constant__ Scen
     }
 }
 
+// Triangles with boxes above kBigPixels.  A few share the grid, several blocks to
+// each; with more than the grid has warps, a warp takes one.  40 directions of 20,000
+// facets with boxes of some 3,000 pixels: 3.4 ms, 24.4 where every 16th block took
+// whole triangles and the others looked for parts beyond 8,192 pixels; a sheet over
+// the whole frame takes 16 blocks or more as before.
 __global__ void __launch_bounds__(256) k_raster_big(const __grid_constant__ Scene scene,
                                                     const float4* __restrict__ planes,
                                                     uint32_t per_dir, Pool pool,
@@ -450,16 +455,25 @@ __global__ void __launch_bounds__(256) k_raster_big(const __grid_constant__ Scen
     wait_for_previous();
     __shared__ Room room;
     const uint32_t count = *job_count, warp = threadIdx.x >> 5;
-    for (uint32_t k = blockIdx.x; k < count; k += gridDim.x) {
+    if (!count) return;
+    // spans of a job for each `stride` pixels from `first`, in step with the block
+    auto draw = [&](uint32_t item, bool on, uint32_t first, uint32_t stride) {
         Job j;
-        load_job<32>(scene, planes, per_dir, *(jobs_end - 1 - k), j);
-        const uint32_t box = uint32_t(j.b.x1 - j.b.x0 + 1) * uint32_t(j.b.y1 - j.b.y0 + 1);
-        for (uint32_t f = blockIdx.y * 8 * kBigPixels; f < box; f += gridDim.y * 8 * kBigPixels) {
-            const uint32_t first = f + warp * kBigPixels;
+        load_job<32>(scene, planes, per_dir, item, j);
+        const uint32_t box =
+            on ? uint32_t(j.b.x1 - j.b.x0 + 1) * uint32_t(j.b.y1 - j.b.y0 + 1) : 0u;
+        for (; __syncthreads_or(int(first < box)); first += stride)
             raster_span<32>(j.p, j.b, j.plane, scene.frame.width, j.key, first < box ? first : 0u,
-                        first < box ? min(box - first, kBigPixels) : 0u, pool, room,
-                        frags ? frags + j.side : nullptr);
-        }
+                            first < box ? min(box - first, kBigPixels) : 0u, pool, room,
+                            frags ? frags + j.side : nullptr);
+    };
+    if (count >= 8u * gridDim.x) {  // a warp each
+        for (uint32_t k = blockIdx.x * 8u; k < count; k += gridDim.x * 8u)
+            draw(*(jobs_end - 1 - min(k + warp, count - 1u)), k + warp < count, 0u, kBigPixels);
+    } else {  // several blocks, or one, to each
+        const uint32_t share = max(1u, gridDim.x / count), part = blockIdx.x % share;
+        for (uint32_t k = blockIdx.x / share; k < count; k += (gridDim.x + share - 1u) / share)
+            draw(*(jobs_end - 1 - k), true, (part * 8u + warp) * kBigPixels, share * 8u * kBigPixels);
     }
 }
 
@@ -1031,7 +1045,7 @@ void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame
         FCU_LAUNCH("k_raster");
         launch_early(k_raster_mid<kMidLanes>, unsigned(std::min<uint64_t>((items + 31) / 32, 8u * sms)),
                      256, 0, s, scene, planes, uint32_t(per_dir), pool, jobs, &dstats->mid, counted);
-        launch_early(k_raster_big, dim3(unsigned(std::min<uint64_t>(items, sms)), 16), 256, 0, s, scene,
+        launch_early(k_raster_big, unsigned(std::min<uint64_t>(items * 16, 8u * sms)), 256, 0, s, scene,
                      planes, uint32_t(per_dir), pool, jobs + items, &dstats->big, counted);
         FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
         FCU_CHECK(cudaStreamSynchronize(s));
