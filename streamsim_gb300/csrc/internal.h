@@ -241,7 +241,7 @@ struct RasterBuffers {
     DeviceBuffer nodes;   // fragments (depth bits, key, the older node)
     DeviceBuffer planes;  // facets as three planes of float4
     DeviceBuffer jobs;    // triangles for warps (from the front) and blocks (from the back)
-    DeviceBuffer list;    // pixels with more than the register path's chain
+    DeviceBuffer list;    // pixels with more than the register path's chain, by length
     DeviceBuffer stats;   // RasterStats
     bool busy = false;    // a build or sun pass is using them
     // The lists are rebuilt by every pass.
@@ -268,7 +268,7 @@ struct RasterStats {
     unsigned long long fragments;
     unsigned long long overflow;   // sum over pixels of max(0, count - cap)
     unsigned int mid, big;         // triangles listed for warps and for blocks
-    unsigned int listed;           // pixels in RasterBuffers::list
+    unsigned int listed[3];        // pixels in each part of RasterBuffers::list
     unsigned int capacity_error;
     unsigned int max_chain;
     unsigned long long pairs;      // (host copy only) pairs so far

@@ -691,8 +691,20 @@ __device__ __forceinline__ uint32_t frag_side(uint32_t key, uint32_t facets)
     return 2u * (order % facets) + (key >> 31);
 }
 
+// Room for `mine` pairs of each lane, one atomic a warp (one counter takes about
+// one atomic a clock).
+__device__ __forceinline__ unsigned long long take_pairs(uint32_t mine,
+                                                         unsigned long long* pair_count)
+{
+    const uint32_t incl = scan_inclusive(mine);
+    unsigned long long base = 0;
+    if ((threadIdx.x & 31u) == 31u && incl) base = atomicAdd(pair_count, (unsigned long long)incl);
+    return __shfl_sync(0xffffffffu, base, 31) + (incl - mine);
+}
+
 // Emit sky counts and adjacent pairs of an ordered chain
-// (facetrtcore.cpp:1374-1392; visibility_resolve.comp:102-116).
+// (facetrtcore.cpp:1374-1392; visibility_resolve.comp:102-116).  Called by whole
+// warps (n = 0: no chain), which take their room in `pairs` with one atomic.
 __device__ void emit_chain(const Frag* f, int n, uint32_t facets, uint32_t* sky, uint64_t* pairs,
                            unsigned long long* pair_count, int side_bits)
 {
@@ -706,8 +718,8 @@ __device__ void emit_chain(const Frag* f, int n, uint32_t facets, uint32_t* sky,
         const uint32_t b = frag_side(f[i + 1].key, facets);
         if ((a >> 1) != (b >> 1)) ++np;
     }
-    unsigned long long base = 0;
-    if (np) base = atomicAdd(pair_count, (unsigned long long)np);
+    __syncwarp();
+    unsigned long long base = take_pairs(np, pair_count);
     uint32_t k = 0;
     for (int i = 0; i + 1 < n; ++i) {
         const uint32_t a = frag_side(f[i].key, facets) ^ 1u;
@@ -797,8 +809,14 @@ __device__ __forceinline__ uint32_t gather_covered(const uint32_t* heads, Covere
     return (all & 0xffffu) + (all >> 16);
 }
 
+// Pixels with longer chains than kFast, by length: for networks of 16 and of 32
+// keys, and the rest.
+struct Lists {
+    uint2 *at16, *at32, *rest;  // {1 + the newest node, fragments}
+};
+
 // A thread per covered pixel, chains of at most kFast fragments ordered in
-// registers (most have one); longer ones are listed for k_resolve_list.  The
+// registers (most have one); longer ones are listed.  The
 // block's pairs wait in shared memory and leave together: with one atomic and a
 // barrier per 256 pixels this took 208 us for the terrain's 42 M pixels and 252
 // for the forest's, now 171 and 181; 64 fragments of local memory for every
@@ -807,9 +825,10 @@ __device__ __forceinline__ uint32_t gather_covered(const uint32_t* heads, Covere
 constexpr uint32_t kHeldPairs = 1024;
 __global__ void __launch_bounds__(256) k_resolve_graph(
     uint32_t facets, uint32_t tiles, const uint32_t* __restrict__ heads, const uint4* __restrict__ nodes, uint32_t cap,
-    uint32_t* sky, uint64_t* pairs, unsigned long long* pair_count, int side_bits, uint2* list,
+    uint32_t* sky, uint64_t* pairs, unsigned long long* pair_count, int side_bits, Lists lists,
     RasterStats* stats)
 {
+    start_next();
     __shared__ Covered c;
     __shared__ uint64_t held[kHeldPairs];
     __shared__ uint32_t held_count, held_end;
@@ -850,12 +869,23 @@ __global__ void __launch_bounds__(256) k_resolve_graph(
                 ++n;
             }
         }
-        if (next) {
-            while (next) {
-                next = nodes[next - 1u].z;
-                ++n;
+        const bool is_long = next != 0u;
+        while (next) {
+            next = nodes[next - 1u].z;
+            ++n;
+        }
+        if (__any_sync(0xffffffffu, is_long)) {
+            const uint32_t which = n <= 16u ? 0u : n <= 32u ? 1u : 2u;
+#pragma unroll
+            for (uint32_t l = 0; l < 3; ++l) {  // one atomic a warp and list
+                const uint32_t lanes = __ballot_sync(0xffffffffu, is_long && which == l);
+                if (!lanes) continue;
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(&stats->listed[l], uint32_t(__popc(lanes)));
+                at = __shfl_sync(0xffffffffu, at, 0) + uint32_t(__popc(lanes & ((1u << lane) - 1u)));
+                if (lanes >> lane & 1u)
+                    (l == 0 ? lists.at16 : l == 1 ? lists.at32 : lists.rest)[at] = make_uint2(head, n);
             }
-            list[atomicAdd(&stats->listed, 1u)] = make_uint2(head, n);
         }
         if (n > cap) atomicAdd(&stats->overflow, (unsigned long long)(n - cap));
         longest = max(longest, n);
@@ -931,25 +961,112 @@ __global__ void __launch_bounds__(256) k_resolve_graph(
     for (uint32_t i = threadIdx.x; i < keep; i += 256) pairs[out + i] = held[i];
 }
 
-// The listed pixels with more than `above` and at most kCap fragments, a thread
-// each, in local memory; chains above kDeepChain are an error.
+// Batcher's odd-even merge sort of N keys, from merges of P with strides of Q on.
+template <int N, int P, int Q>
+__device__ __forceinline__ void network(uint64_t (&k)[N])
+{
+    constexpr int first = Q % P;
+#pragma unroll
+    for (int i = first; i < N - Q; ++i)
+        if ((i - first) / Q % 2 == 0 && i / (2 * P) == (i + Q) / (2 * P)) order2(k[i], k[i + Q]);
+    if constexpr (Q > 1) network<N, P, Q / 2>(k);
+    else if constexpr (2 * P < N) network<N, 2 * P, 2 * P>(k);
+}
+
+// Listed pixels with at most N fragments, a thread each, ordered by Batcher's
+// network in registers, without local memory and in step (insertion sorts in local
+// memory kept 10 of 32 lanes busy).  40 directions of 60,000 facets of some 0.4 m:
+// chains of 9 to 16 take 1.15 ms and of 17 to 32 0.39, 9.5 by sorts in local memory
+// and an atomic for each pixel's pairs.  Bound by the loads along the chain.  Where two of more than 16 fragments
+// share a depth, std::sort's order is not the append order, and the pixel goes to the
+// rest's list.
+template <int N>
+__global__ void __launch_bounds__(128) k_resolve_network(
+    uint32_t facets, uint32_t tiles, const uint4* __restrict__ nodes, const uint2* list,
+    const uint32_t* count, uint32_t* sky, uint64_t* pairs, unsigned long long* pair_count,
+    int side_bits, uint2* rest, uint32_t* rest_count)
+{
+    start_next();
+    wait_for_previous();
+    const uint32_t listed = *count;
+    for (uint32_t j0 = blockIdx.x * 128 + (threadIdx.x & ~31u); j0 < listed; j0 += gridDim.x * 128) {
+        const uint32_t j = j0 + (threadIdx.x & 31u);
+        const uint2 mine = j < listed ? list[j] : make_uint2(0u, 0u);
+        uint32_t next = mine.x, n = mine.y;
+        uint64_t k[N];
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            k[q] = ~0ull;
+            if (next) {
+                const uint4 node = __ldcs(nodes + (next - 1u));
+                k[q] = chain_key(node);
+                next = node.z;
+            }
+        }
+        __syncwarp();
+        network<N, 1, 1>(k);
+        if (N > 16) {
+            bool tie = false;
+#pragma unroll
+            for (int q = 1; q < N; ++q) tie |= uint32_t(q) < n && k[q] >> 32 == k[q - 1] >> 32;
+            if (tie) {
+                rest[atomicAdd(rest_count, 1u)] = mine;
+                n = 0;
+            }
+            __syncwarp();
+        }
+        uint32_t before = key_side(k[0], facets, tiles), np = 0;
+        const uint32_t nearest = before;
+#pragma unroll
+        for (int q = 1; q < N; ++q)
+            if (uint32_t(q) < n) {
+                const uint32_t side = key_side(k[q], facets, tiles);
+                np += (before >> 1) != (side >> 1) ? 1u : 0u;
+                before = side;
+            }
+        if (n) {
+            atomicAdd(&sky[nearest], 1u);
+            atomicAdd(&sky[before ^ 1u], 1u);
+        }
+        __syncwarp();
+        uint64_t* to = pairs + take_pairs(np, pair_count);
+        before = nearest;
+#pragma unroll
+        for (int q = 1; q < N; ++q)
+            if (uint32_t(q) < n) {
+                const uint32_t side = key_side(k[q], facets, tiles), a = before ^ 1u;
+                if ((before >> 1) != (side >> 1))
+                    *to++ = (uint64_t(min(a, side)) << side_bits) | max(a, side);
+                before = side;
+            }
+    }
+}
+
+// The rest, pixels with more than `above` and at most kCap fragments, a thread
+// each, in local memory; chains above kDeepChain are an error.  A list begins with
+// its newest fragment, so it is laid out from the back: near the append order that
+// long chains are brought into first.
 template <uint32_t kCap>
 __global__ void __launch_bounds__(64) k_resolve_list(
-    uint32_t facets, const uint4* __restrict__ nodes, const uint2* __restrict__ list, uint32_t above, uint32_t* sky,
+    uint32_t facets, const uint4* __restrict__ nodes, const uint2* list, uint32_t above, uint32_t* sky,
     uint64_t* pairs, unsigned long long* pair_count, int side_bits, RasterStats* stats)
 {
-    const uint32_t listed = stats->listed;
-    for (uint32_t j = blockIdx.x * 64 + threadIdx.x; j < listed; j += gridDim.x * 64) {
-        const uint32_t n = list[j].y;
+    start_next();
+    wait_for_previous();
+    const uint32_t listed = stats->listed[2];
+    for (uint32_t j0 = blockIdx.x * 64 + (threadIdx.x & ~31u); j0 < listed; j0 += gridDim.x * 64) {
+        const uint32_t j = j0 + (threadIdx.x & 31u);
+        uint32_t n = j < listed ? list[j].y : 0u;
         if (n > kCap) {
             // (kMidChain: the next launch's)
             if (kCap == kDeepChain) atomicAdd(&stats->capacity_error, 1u);
-            continue;
+            n = 0;
         }
-        if (n <= above) continue;
+        if (n <= above) n = 0;
+        if (!__any_sync(0xffffffffu, n != 0u)) continue;
         Frag f[kCap];
-        uint32_t next = list[j].x;
-        for (uint32_t k = 0; k < n; ++k) {
+        uint32_t next = n ? list[j].x : 0u;
+        for (uint32_t k = n; k-- > 0;) {
             const uint4 node = nodes[next - 1u];
             f[k].depth = __uint_as_float(node.x);
             f[k].key = node.y;
@@ -1073,16 +1190,24 @@ void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t
 {
     const uint64_t npix = uint64_t(dir_count) * frame.width * frame.height;
     RasterStats* dstats = rb.stats.as<RasterStats>();
-    uint2* list = static_cast<uint2*>(rb.list.reserve((stats.fragments / (kFast + 1) + 1) * 8));
+    // (pixels of 9, 17 and 17 fragments at least: the last list takes the ties too)
+    const size_t room16 = stats.fragments / (kFast + 1) + 1, room32 = stats.fragments / 17 + 1;
+    uint2* list = static_cast<uint2*>(rb.list.reserve((room16 + 2 * room32) * 8));
+    const Lists lists{list, list + room16, list + room16 + room32};
     const uint4* nodes = rb.nodes.as<uint4>();
     k_resolve_graph<<<unsigned((npix + kResolvePixels - 1) / kResolvePixels), 256, 0, s>>>(
-        frame.facets, frame.tiles, rb.heads.as<uint32_t>(), nodes, chain_cap, d_sky, d_pairs, d_pair_count, side_bits, list,
-        dstats);
+        frame.facets, frame.tiles, rb.heads.as<uint32_t>(), nodes, chain_cap, d_sky, d_pairs,
+        d_pair_count, side_bits, lists, dstats);
     FCU_LAUNCH("k_resolve_graph");
     const unsigned list_blocks = 16 * sm_count();
-    k_resolve_list<kMidChain><<<list_blocks, 64, 0, s>>>(frame.facets, nodes, list, 0u, d_sky,
-                                                         d_pairs, d_pair_count, side_bits, dstats);
-    FCU_LAUNCH("k_resolve_list");
+    launch_early(k_resolve_network<16>, list_blocks, 128, 0, s, frame.facets, frame.tiles, nodes,
+                 lists.at16, &dstats->listed[0], d_sky, d_pairs, d_pair_count, side_bits, lists.rest,
+                 &dstats->listed[2]);
+    launch_early(k_resolve_network<32>, list_blocks, 128, 0, s, frame.facets, frame.tiles, nodes,
+                 lists.at32, &dstats->listed[1], d_sky, d_pairs, d_pair_count, side_bits, lists.rest,
+                 &dstats->listed[2]);
+    launch_early(k_resolve_list<kMidChain>, list_blocks, 64, 0, s, frame.facets, nodes, lists.rest, 0u,
+                 d_sky, d_pairs, d_pair_count, side_bits, dstats);
     RasterStats host{};
     auto read = [&] {
         FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
@@ -1092,8 +1217,9 @@ void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t
     read();
     if (host.max_chain > kMidChain) {
         // (launched only then: its local memory is a few GB)
-        k_resolve_list<kDeepChain><<<list_blocks, 64, 0, s>>>(
-            frame.facets, nodes, list, kMidChain, d_sky, d_pairs, d_pair_count, side_bits, dstats);
+        k_resolve_list<kDeepChain><<<list_blocks, 64, 0, s>>>(frame.facets, nodes, lists.rest, kMidChain,
+                                                              d_sky, d_pairs, d_pair_count,
+                                                              side_bits, dstats);
         FCU_LAUNCH("k_resolve_list");
         read();
     }
