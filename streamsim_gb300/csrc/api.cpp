@@ -665,9 +665,10 @@ namespace {
 
 // The rays of each sample set in the order of their directions: a Morton
 // curve over the direction's tangent-plane components (dx, dy), 8 bits each.
-// A warp traces 32 consecutive rays at a time, so neighbouring directions
-// keep its BVH traversal coherent.  A side's row depends only on the set of
-// its rays (hits are sorted and counted), so the graph is unchanged.
+// A side's row depends only on the set of its rays (hits are sorted and
+// counted), so the graph is unchanged.  (The caster sorts a block's rays by
+// direction itself, so its traversal no longer depends on this order; it costs
+// some 0.5 ms of a call of 256 rays and 32 sets on the host.)
 void order_samples(const float* uv, const float* dir, uint32_t sets, uint32_t rays,
                    std::vector<float>& uv_out, std::vector<float>& dir_out)
 {
