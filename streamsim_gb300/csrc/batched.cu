@@ -623,6 +623,7 @@ __global__ void __launch_bounds__(kWarps * 32, SweepBlocks<P>::value) k_sweep_wi
                                                             const uint32_t* done)
 {
     start_next();
+    wait_for_previous();
     if (*done) return;
     constexpr int CPL = 4;
     constexpr int L = P / CPL;
@@ -2128,10 +2129,11 @@ __device__ __forceinline__ float cheb_advance(float* cheb, int c, int mode, floa
 __global__ void k_check(uint32_t* stats, uint32_t* flag, int P, float tol, uint32_t it,
                         uint32_t* counter, float* scale_a, float* scale_b, uint32_t* it_dev,
                         bool per_side, float* colmax, float* cheb = nullptr, int cheb_mode = 0,
-                        const float* scale_prev = nullptr)
+                        const float* scale_prev = nullptr, bool late = false)
 {
-    start_next();
+    if (!late) start_next();
     wait_for_previous();
+    if (late) start_next();  // the sweep before has ended and its panel is written
     __shared__ int all_ok, abs_ok;
     __shared__ float worst;
     if (it_dev) it = *it_dev;  // the sweep index kept on the device (graph replays)
@@ -2446,16 +2448,24 @@ int grid_for(K kernel)
     return std::max(1, sms) * std::max(1, per_sm);
 }
 
-// (The 8- and 16-column sweeps and k_check are launched while the kernel in front
-// of them ends and wait inside.  k_sweep_wide is not: it gathers its panel through
-// the read-only path, which an early kernel may not do, and with plain loads the
-// 32-column sweeps cost more than the 2 us of a launch: the energy node 28.7 ms
-// instead of 27.8.)
+// (The FP32 sweeps and k_check are launched while the kernel in front of them ends
+// and wait inside.  k_sweep_wide gathers its panel through the read-only path, so it
+// may not be there while the sweep before it writes that panel: `follows` says that
+// a k_check with `late` stands between them, which starts it when that sweep has
+// ended.  With plain loads instead the 32-column sweeps cost more than a launch: the
+// energy node 28.7 ms instead of 27.8.)
 template <typename T>
 void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in, T* out,
-                  uint32_t* stats, uint32_t* counter, const uint32_t* done, cudaStream_t s)
+                  uint32_t* stats, uint32_t* counter, const uint32_t* done, bool follows,
+                  cudaStream_t s)
 {
     if constexpr (sizeof(T) == 4) {
+        auto wide = [&](auto kernel, int grid) {
+            if (follows)
+                launch_early(kernel, grid, kWarps * 32, 0, s, g, pp, in, out, stats, counter, done);
+            else
+                kernel<<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+        };
         if (in == nullptr && P >= 8) {
             // a solve from zero: its first sweep has nothing to gather
             static const int grid = [] {
@@ -2489,10 +2499,10 @@ void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in,
             // 16-byte row vectors in rounds of 8 loads per lane
             if (P == 8) {
                 static const int grid = grid_for(k_sweep_wide<8>);
-                k_sweep_wide<8><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                wide(k_sweep_wide<8>, grid);
             } else {
                 static const int grid = grid_for(k_sweep_wide<16>);
-                k_sweep_wide<16><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                wide(k_sweep_wide<16>, grid);
             }
             FCU_LAUNCH("k_sweep_wide");
             return;
@@ -2501,17 +2511,17 @@ void launch_sweep(int P, const GraphView& g, const PanelParams& pp, const T* in,
             switch (P) {
             case 32: {
                 static const int grid = grid_for(k_sweep_wide<32>);
-                k_sweep_wide<32><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                wide(k_sweep_wide<32>, grid);
                 break;
             }
             case 64: {
                 static const int grid = grid_for(k_sweep_wide<64>);
-                k_sweep_wide<64><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                wide(k_sweep_wide<64>, grid);
                 break;
             }
             default: {
                 static const int grid = grid_for(k_sweep_wide<128>);
-                k_sweep_wide<128><<<grid, kWarps * 32, 0, s>>>(g, pp, in, out, stats, counter, done);
+                wide(k_sweep_wide<128>, grid);
                 break;
             }
             }
@@ -3100,6 +3110,8 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
         const char* final_buf = x0;
         uint32_t host_flag[3] = {0, 0, 0};
         if (!low) {
+            // (k_sweep_wide's panels: see launch_sweep)
+            const bool wide = !column && !fp64 && (P >= 32 || !g.packed);
             while (it < max_it) {
                 const uint32_t batch = std::min(timed ? 1u : check_every, max_it - it);
                 for (uint32_t k = 0; k < batch; ++k) {
@@ -3114,14 +3126,14 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
                         else if (fp64)
                             launch_sweep<double>(P, g, pp, reinterpret_cast<const double*>(in),
                                                  reinterpret_cast<double*>(out), stats, counter,
-                                                 flag, s);
+                                                 flag, false, s);
                         else
                             launch_sweep<float>(P, g, pp, reinterpret_cast<const float*>(in),
                                                 reinterpret_cast<float*>(out), stats, counter,
-                                                flag, s);
+                                                flag, k > 0, s);
                     });
                     launch_early(k_check, 1, kMaxP, 0, s, stats, flag, P, tol, sweep, counter, nullptr,
-                                 nullptr, nullptr, true, colmax, nullptr, 0, nullptr);
+                                 nullptr, nullptr, true, colmax, nullptr, 0, nullptr, wide);
                     ++launches;
                 }
                 it += batch;
@@ -3153,7 +3165,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
             while (it < max_it) {
                 timed_sweep(false, [&] {
                     launch_sweep<float>(P, g, pp, it == 0 && zero_start ? nullptr : X, Y, stats,
-                                        counter, flag, s);
+                                        counter, flag, false, s);
                 });
                 k_check<<<1, kMaxP, 0, s>>>(stats, flag, P, tol, it, counter, slot[0], slot[1],
                                             nullptr, true, colmax, cheb, 1);
@@ -3285,7 +3297,7 @@ int batched_solve(const DeviceGraph& gr_in, const BatchProblem& p, const facetcu
             while (it < max_it) {
                 timed_sweep(false, [&] {
                     launch_sweep<float>(P, g, pp, it == 0 && zero_start ? nullptr : X, Y, stats,
-                                        counter, flag, s);
+                                        counter, flag, false, s);
                 });
                 k_check<<<1, kMaxP, 0, s>>>(stats, flag, P, tol, it, counter, nullptr, nullptr,
                                             nullptr, true, colmax);

@@ -43,6 +43,8 @@ def _early_kernels():
         found = set(re.findall(r"launch_early\(\s*(k_\w+)", text))
         if name == "solve.cu":  # launched through a generic lambda
             found.add("k_jacobi_rows")
+        if name == "batched.cu":
+            found.add("k_sweep_wide")
         for kernel in sorted(found):
             yield name, kernel
 
@@ -55,6 +57,8 @@ def test_early_kernel(source, kernel):
     written = WRITTEN
     if kernel == "k_jacobi_rows":  # see test_first_sweep
         written = tuple(w for w in WRITTEN if w != "optics")
+    if kernel == "k_sweep_wide":  # see test_wide_sweeps
+        written = tuple(w for w in WRITTEN if w != "Bin")
     for p in params.split(","):
         words = p.replace("*", " ").split()
         if words and words[-1].split("=")[0] in written and "*" in p:
@@ -76,3 +80,21 @@ def test_first_sweep():
     solve = dict(_sources())["solve.cu"]
     assert re.search(r"follows \? sweep_rows<true> : sweep_rows<false>", solve)
     assert len(re.findall(r"sweep_rows<true>", solve)) == 1
+
+
+def test_wide_sweeps():
+    """k_sweep_wide gathers its panel through the read-only path.  It starts early
+    only behind a k_check that lets it start after its own wait, when the sweep that
+    wrote the panel has ended."""
+    text = dict(_sources())["batched.cu"]
+    _, check = _kernel(text, "k_check")
+    early, wait, late = (check.index(x) for x in (
+        "if (!late) start_next();", "wait_for_previous();", "if (late) start_next();"))
+    assert early < wait < late
+    assert check.count("start_next") == 2
+    assert re.search(r"if \(follows\)\s*launch_early\(kernel,", text)
+    # the only call with follows other than false: behind a k_check of the same loop
+    calls = re.findall(r"launch_sweep<(?:float|double)>\([^;]*;", text)
+    assert [c.split(",")[-2].strip() for c in calls].count("false") == len(calls) - 1
+    loop = text[text.index("const bool wide = !column && !fp64 && (P >= 32 || !g.packed);"):]
+    assert re.search(r"flag, k > 0, s\);.*?launch_early\(k_check,[^;]*, wide\);", loop, re.S)
