@@ -710,7 +710,7 @@ def run_gpu(args, rank, world, local):
             perr = max(perr, rel_err_floor(pout.cpu().numpy()[None, :], truth[b][None, :]))
         plain = {"value": sc.facet_count * len(picks) / pt, "unit": UNIT,
                  "sample": f"{len(picks)} bands x 64 sweeps of the reference-semantics kernel "
-                           "(k_jacobi_rows), device-resident inputs, CUDA events",
+                           "(k_jacobi_any), device-resident inputs, CUDA events",
                  "max_rel_err_vs_fp64": perr}
         del dg, opt, pout
 
