@@ -563,12 +563,19 @@ void render(const Camera& c, uint32_t F, const facetcu_vertex* V, const float* v
     FCU_CHECK(cudaMemsetAsync(counts, 0, 3 * sizeof(uint32_t), s));
     FCU_CHECK(cudaMemsetAsync(w.zbuf, 0, n * sizeof(ulonglong2), s));
     if (F) {
-        // 16 warps an SM before a warp takes more than one facet: enough to hide
-        // the divisions; more would do the projection's doubles in idle lanes
+        // A warp takes as many facets as share some 512 of the image's pixels, fewer
+        // lanes than that do the projection's doubles (a warp of them costs the same)
+        // for nothing, more leave too long a queue of boxes; and no more than leave
+        // 16 warps an SM, unless the image is small.  Side images in us with 32 facets
+        // a warp / 2, 4 and 16 warps an SM: 2,000 facets on 64 x 64 57 / 57, 69, 81 (a
+        // warp per facet of old: 86), 4,000 on 1,024 x 1,024 2,751 / 917, 743, 659
+        // (1,547), 30,000 1,605 / 1,654, 1,655, 1,498 (2,522).
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const uint32_t per_warp = std::clamp(F / (16u * uint32_t(std::max(sms, 1))), 1u, 32u);
+        const uint32_t spread = F / (16u * uint32_t(std::max(sms, 1)));
+        const uint32_t of_image = uint32_t(std::min<size_t>(512 * size_t(F) / n, 32u));
+        const uint32_t per_warp = std::clamp(std::max(spread, of_image), 1u, 32u);
         k_raster<<<blocks(F, per_warp * kRasterThreads / 32), kRasterThreads, 0, s>>>(
             F, per_warp, V, c, w.zbuf, w.side, w.large, counts + 2);
         FCU_LAUNCH("k_raster");
