@@ -255,9 +255,9 @@ __global__ void __launch_bounds__(kRasterThreads, 6) k_raster(
     }
 }
 
-// Bound by FP64, as k_raster.  The listed facets: with few of them the blocks share a facet, taking parts of
+// The listed facets: with few of them the blocks share a facet, taking parts of
 // kPartPixels pixels of its box in turn; with more than blocks each takes whole
-// ones (the projection is done once a block and facet).
+// ones (the projection is done once a block and facet).  Bound by FP64, as k_raster.
 constexpr uint32_t kPartPixels = 2048;
 __global__ void __launch_bounds__(256) k_raster_large(const facetcu_vertex* __restrict__ V, Camera c,
                                                       ulonglong2* __restrict__ zbuf,
