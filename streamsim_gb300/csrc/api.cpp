@@ -630,10 +630,9 @@ int facetcu_compute_sunlit_fraction(facetcu_context* ctx, const facetcu_directio
         uint32_t* visible = static_cast<uint32_t*>(ctx->sun_visible.reserve(size_t(S) * 4));
         FCU_CHECK(cudaMemsetAsync(total, 0, size_t(S) * 4, s));
         FCU_CHECK(cudaMemsetAsync(visible, 0, size_t(S) * 4, s));
-        raster_fragments(ctx->vertices.as<facetcu_vertex>(), frame, &view, 1, ctx->raster, total, st,
-                         s);
         float* d_fraction = static_cast<float*>(ctx->fraction.reserve(size_t(S) * 4));
-        raster_resolve_sunlit(frame, chain_cap(ctx), ctx->raster, total, visible, d_fraction, st, s);
+        raster_sunlit(ctx->vertices.as<facetcu_vertex>(), frame, view, chain_cap(ctx), ctx->raster,
+                      total, visible, d_fraction, st, s);
         if (st.overflow)
             throw Error(FACETCU_RUNTIME_ERROR,
                         "Direct-light A-buffer overflow; increase Config::maxFragmentsPerPixel");

@@ -238,7 +238,9 @@ void radix_sort_u64(uint64_t*& keys, uint64_t*& keys_alt, uint32_t*& values,
 // ---- raster visibility (raster.cu) --------------------------------------
 struct RasterBuffers {
     DeviceBuffer heads;   // dirs * pixels: 1 + the newest node of the pixel's list, or 0
-    DeviceBuffer nodes;   // fragments (depth bits, key, the older node)
+                          // (sun pass: the pixel's fragments)
+    DeviceBuffer nodes;   // fragments (depth bits, key, the older node; sun pass: the
+                          // pixels' nearest)
     DeviceBuffer planes;  // facets as three planes of float4
     DeviceBuffer jobs;    // triangles for warps (from the front) and blocks (from the back)
     DeviceBuffer list;    // pixels with more than the register path's chain, by length
@@ -292,11 +294,11 @@ void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t
                           RasterBuffers& rb, uint32_t* d_sky, uint64_t* d_pairs,
                           unsigned long long* d_pair_count, int side_bits, RasterStats& stats,
                           cudaStream_t s);
-// Resolve one direction's lists into visible counts per side, and their ratio
-// to the totals (the raster's d_frags; 0 where there are none).
-void raster_resolve_sunlit(const RasterFrame& frame, uint32_t chain_cap, RasterBuffers& rb,
-                           const uint32_t* d_total, uint32_t* d_visible, float* d_fraction,
-                           RasterStats& stats, cudaStream_t s);
+// One direction's fragments per side (added to d_total), visible counts per side
+// (added to d_visible), and their ratio (0 where there are none).
+void raster_sunlit(const facetcu_vertex* d_vertices, const RasterFrame& frame, const RasterView& view,
+                   uint32_t chain_cap, RasterBuffers& rb, uint32_t* d_total, uint32_t* d_visible,
+                   float* d_fraction, RasterStats& stats, cudaStream_t s);
 
 // ---- one-column sweeps from shared memory (column.cu) --------------------
 // The edge words of a graph laid out by tiles of the column, and the sums of

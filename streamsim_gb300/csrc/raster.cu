@@ -20,7 +20,8 @@
 // takes its room in the pool with one atomic.  A pool that turns out too small
 // is grown to the exact number and the chunk rasterised again.  A facet's
 // fragments are counted by the threads that rasterise it, not fragment by
-// fragment when the lists are resolved.
+// fragment when the lists are resolved.  The sun pass needs a pixel's nearest
+// fragment and their number only: no lists, two atomics a fragment.
 #include <algorithm>
 
 #include "internal.h"
@@ -34,8 +35,8 @@ namespace {
 //   a thread up to 8, 16, 32 pixels:  925 / 5288,  929 / 2095,  876 / 2005
 //   above, 4, 8, 16, 32 lanes:        839 / 1709,  848 / 1777,  870 / 1904,
 //                                     894 / 2194
-// and the one direction of the sun pass with 4, 8, 32 lanes: 144 / 157,
-// 121 / 155, 110 / 169.
+// and the one direction of the sun pass, when it had lists too, with 4, 8, 32
+// lanes: 144 / 157, 121 / 155, 110 / 169.
 constexpr uint32_t kSmallPixels = 32;  // (a thread's covered pixels are bits of a word)
 constexpr uint32_t kMidLanes = 8;
 constexpr uint32_t kBigPixels = 1024;  // above: blocks
@@ -199,11 +200,32 @@ struct Pool {
     uint4* nodes;                    // depth bits, key, the older node (1 + index, or 0)
     uint64_t capacity;
     unsigned long long* used;        // also counts what found no room
+    // kNearest, the sun pass: heads count a pixel's fragments, and this keeps the
+    // chain key of its first one.  (From lists, a thread walked its pixel's nodes
+    // for it.  With / without them: 900 sheets over 128 x 128 pixels 1,474 / 93 us,
+    // 20,000 leaves with 0.9 m edges over 1,024 x 1,024 432 / 262, 4,050 facets of
+    // terrain 96 / 88, one facet over 64 x 64 88 / 72.)
+    unsigned long long* nearest;
 };
 
+// A fragment as a number whose order is the chain's: depth, then append order
+// (frag_less_stable); the flip bit lies below both.
+__device__ __forceinline__ uint64_t chain_key(float depth, uint32_t key)
+{
+    const uint32_t bits = __float_as_uint(depth + 0.0f);  // -0 is 0
+    const uint32_t ordered = bits & 0x80000000u ? ~bits : bits | 0x80000000u;
+    return (uint64_t(ordered) << 32) | uint64_t((key << 1) | (key >> 31));
+}
+
+template <bool kNearest>
 __device__ __forceinline__ void put(const Pool& pool, size_t pix, uint64_t slot, float depth,
                                     uint32_t key)
 {
+    if (kNearest) {
+        atomicMin(&pool.nearest[pix], (unsigned long long)chain_key(depth, key));
+        atomicAdd(&pool.heads[pix], 1u);
+        return;
+    }
     if (slot >= pool.capacity) return;
     const uint32_t older = atomicExch(&pool.heads[pix], uint32_t(slot) + 1u);
     pool.nodes[slot] = make_uint4(__float_as_uint(depth), key, older, 0u);
@@ -249,6 +271,7 @@ __device__ __forceinline__ uint32_t scan_inclusive(uint32_t v)
 // Bound by instructions (69 % of the issue slots; nine IEEE divides to project
 // a triangle): 351 us for the 8 M triangles of the forest, where counting and
 // filling in two passes took 268 + 448.
+template <bool kNearest>
 __global__ void __launch_bounds__(256) k_raster(const __grid_constant__ Scene scene,
                                                 const float4* __restrict__ planes, uint32_t per_dir,
                                                 Pool pool, uint32_t* jobs, uint32_t items,
@@ -307,7 +330,7 @@ __global__ void __launch_bounds__(256) k_raster(const __grid_constant__ Scene sc
                 if (!(mask & 1u)) continue;
                 float depth;
                 cover(p, b.area, x, y, depth);
-                put(pool, plane + size_t(y) * width + size_t(x), slot++, depth, key);
+                put<kNearest>(pool, plane + size_t(y) * width + size_t(x), slot++, depth, key);
             }
         }
     }
@@ -324,7 +347,7 @@ __global__ void __launch_bounds__(256) k_raster(const __grid_constant__ Scene sc
 // its box, at most 32 kLanes, so that a lane's covered ones are the bits of a
 // word.  Called by all threads of the block (count 0 where there is none).
 // The atomics of four steps are in flight together.
-template <uint32_t kLanes>
+template <uint32_t kLanes, bool kNearest>
 __device__ __forceinline__ void raster_span(const Projected& p, const Bbox& b, size_t plane,
                                             uint32_t width, uint32_t key, uint32_t first, uint32_t count,
                                             const Pool& pool, Room& room, uint32_t* count_at)
@@ -367,7 +390,13 @@ __device__ __forceinline__ void raster_span(const Projected& p, const Bbox& b, s
             const uint32_t lanes = __ballot_sync(0xffffffffu, on);
             at[k] = on ? slot + uint32_t(__popc(lanes & ((1u << lane) - 1u))) : ~0ull;
             slot += uint32_t(__popc(lanes));
-            if (at[k] < pool.capacity) {
+            if (kNearest) {
+                if (on) {
+                    const int x = b.x0 + int(cx), y = b.y0 + int(cy);
+                    cover(p, b.area, x, y, depth[k]);
+                    put<true>(pool, plane + size_t(y) * width + size_t(x), 0, depth[k], key);
+                }
+            } else if (at[k] < pool.capacity) {
                 const int x = b.x0 + int(cx), y = b.y0 + int(cy);
                 cover(p, b.area, x, y, depth[k]);
                 older[k] = atomicExch(&pool.heads[plane + size_t(y) * width + size_t(x)],
@@ -382,7 +411,7 @@ __device__ __forceinline__ void raster_span(const Projected& p, const Bbox& b, s
         }
 #pragma unroll
         for (uint32_t k = 0; k < 4; ++k)
-            if (at[k] < pool.capacity)
+            if (!kNearest && at[k] < pool.capacity)
                 pool.nodes[at[k]] = make_uint4(__float_as_uint(depth[k]), key, older[k], 0u);
     }
     __syncthreads();  // room is free again
@@ -413,7 +442,7 @@ __device__ __forceinline__ void load_job(const Scene& scene, const float4* plane
 // Bound by instructions and the latency of its rounds (issue 57 %): 323 us for
 // the forest's 0.8 M ground triangles, 190 us for the terrain's 164,000, which
 // took 160 + 495 in two passes of a thread each.
-template <uint32_t kLanes>
+template <uint32_t kLanes, bool kNearest>
 __global__ void __launch_bounds__(256) k_raster_mid(const __grid_constant__ Scene scene,
                                                     const float4* __restrict__ planes,
                                                     uint32_t per_dir, Pool pool,
@@ -433,7 +462,7 @@ __global__ void __launch_bounds__(256) k_raster_mid(const __grid_constant__ Scen
         const uint32_t box = mine < count ? uint32_t(j.b.x1 - j.b.x0 + 1) *
                                                 uint32_t(j.b.y1 - j.b.y0 + 1) : 0u;
         for (uint32_t first = 0; __syncthreads_or(int(first < box)); first += kSpan)
-            raster_span<kLanes>(j.p, j.b, j.plane, scene.frame.width, j.key, first,
+            raster_span<kLanes, kNearest>(j.p, j.b, j.plane, scene.frame.width, j.key, first,
                                 first < box ? min(box - first, kSpan) : 0u, pool, room,
                                 frags ? frags + j.side : nullptr);
     }
@@ -444,6 +473,7 @@ __global__ void __launch_bounds__(256) k_raster_mid(const __grid_constant__ Scen
 // facets with boxes of some 3,000 pixels: 3.4 ms, 24.4 where every 16th block took
 // whole triangles and the others looked for parts beyond 8,192 pixels; a sheet over
 // the whole frame takes 16 blocks or more as before.
+template <bool kNearest>
 __global__ void __launch_bounds__(256) k_raster_big(const __grid_constant__ Scene scene,
                                                     const float4* __restrict__ planes,
                                                     uint32_t per_dir, Pool pool,
@@ -463,7 +493,7 @@ __global__ void __launch_bounds__(256) k_raster_big(const __grid_constant__ Scen
         const uint32_t box =
             on ? uint32_t(j.b.x1 - j.b.x0 + 1) * uint32_t(j.b.y1 - j.b.y0 + 1) : 0u;
         for (; __syncthreads_or(int(first < box)); first += stride)
-            raster_span<32>(j.p, j.b, j.plane, scene.frame.width, j.key, first < box ? first : 0u,
+            raster_span<32, kNearest>(j.p, j.b, j.plane, scene.frame.width, j.key, first < box ? first : 0u,
                             first < box ? min(box - first, kBigPixels) : 0u, pool, room,
                             frags ? frags + j.side : nullptr);
     };
@@ -731,13 +761,9 @@ __device__ void emit_chain(const Frag* f, int n, uint32_t facets, uint32_t* sky,
     }
 }
 
-// A fragment as a number whose order is the chain's: depth, then append order
-// (frag_less_stable); the flip bit lies below both.
 __device__ __forceinline__ uint64_t chain_key(const uint4& node)
 {
-    const uint32_t bits = __float_as_uint(__uint_as_float(node.x) + 0.0f);  // -0 is 0
-    const uint32_t depth = bits & 0x80000000u ? ~bits : bits | 0x80000000u;
-    return (uint64_t(depth) << 32) | uint64_t((node.y << 1) | (node.y >> 31));
+    return chain_key(__uint_as_float(node.x), node.y);
 }
 __device__ __forceinline__ uint32_t key_side(uint64_t k, uint32_t facets, uint32_t tiles)
 {
@@ -1079,29 +1105,25 @@ __global__ void __launch_bounds__(64) k_resolve_list(
 
 // computeCpuSunlit per pixel (facetrtcore.cpp:1448-1466): the nearest fragment
 // (first in append order among equal depths) is visible.  (Every fragment
-// counts towards its side's total: counted by the raster.)
+// counts towards its side's total: counted by the raster.)  Bound by reading the
+// counts; a warp without fragments reads nothing else.
 __global__ void __launch_bounds__(256) k_resolve_sunlit(uint32_t facets, uint32_t tiles,
-                                                        const uint32_t* __restrict__ heads,
-                                                        const uint4* __restrict__ nodes,
-                                                        uint32_t cap, uint32_t* visible,
-                                                        RasterStats* stats)
+                                                        const uint32_t* __restrict__ counts,
+                                                        const uint64_t* __restrict__ nearest,
+                                                        uint64_t npix, uint32_t cap,
+                                                        uint32_t* visible, RasterStats* stats)
 {
-    __shared__ Covered c;
-    const uint32_t covered = gather_covered(heads, c), lane = threadIdx.x & 31u;
     uint32_t longest = 0;
-    for (uint32_t first = threadIdx.x & ~31u; first < covered; first += 256) {
-        uint32_t next = first + lane < covered ? c.queue[first + lane] : 0u, n = 0;
-        uint64_t best = ~0ull;
-        while (next) {
-            const uint4 node = __ldcs(nodes + (next - 1u));
-            const uint64_t key = chain_key(node);
-            best = key < best ? key : best;
-            next = node.z;
-            ++n;
-        }
-        __syncwarp();
+    const uint64_t stride = uint64_t(gridDim.x) * 256;
+    for (uint64_t first = uint64_t(blockIdx.x) * 256 + (threadIdx.x & ~31u); first < npix;
+         first += stride) {
+        const uint64_t i = first + (threadIdx.x & 31u);
+        const uint32_t n = i < npix ? __ldcs(counts + i) : 0u;
+        if (!__any_sync(0xffffffffu, n != 0u)) continue;
+        const uint64_t best = n ? __ldcs(nearest + i) : ~0ull;
         if (n > cap) atomicAdd(&stats->overflow, (unsigned long long)(n - cap));
         longest = max(longest, n);
+        __syncwarp();
         add_sides(visible, key_side(best, facets, tiles), n != 0u);
     }
     note_longest(stats, longest);
@@ -1125,49 +1147,80 @@ unsigned sm_count()
 }
 }  // namespace
 
+namespace {
+
+// The rasters of all directions, into the pool's lists or nearest fragments.
+struct RasterPass {
+    Scene scene{};
+    uint64_t npix = 0, per_dir = 0, items = 0;
+    unsigned sms = 0;
+    uint32_t* jobs = nullptr;
+    float4* planes = nullptr;
+    RasterStats* stats = nullptr;
+    RasterPass(const facetcu_vertex* d_vertices, const RasterFrame& frame, const RasterView* views,
+               uint32_t dir_count, RasterBuffers& rb, cudaStream_t s)
+    {
+        if (dir_count > kMaxViews)
+            throw Error(FACETCU_INVALID_ARGUMENT, "raster chunk exceeds 64 directions");
+        scene.frame = frame;
+        std::copy(views, views + dir_count, scene.views);
+        npix = uint64_t(dir_count) * frame.width * frame.height;
+        per_dir = uint64_t(frame.tiles) * frame.facets;
+        items = dir_count * per_dir;
+        if (items >= (1ull << 32))
+            throw Error(FACETCU_OVERFLOW_ERROR, "raster work exceeds 2^32 triangles");
+        sms = sm_count();
+        jobs = static_cast<uint32_t*>(rb.jobs.reserve(items * 4));
+        planes = static_cast<float4*>(rb.planes.reserve(size_t(frame.facets) * 48));
+        stats = static_cast<RasterStats*>(rb.stats.reserve(sizeof(RasterStats)));
+        k_planes<<<(frame.facets + 255) / 256, 256, 0, s>>>(d_vertices, frame.facets, planes);
+        FCU_LAUNCH("k_planes");
+    }
+    template <bool kNearest>
+    void run(const Pool& pool, uint32_t* d_frags, uint32_t dir_count, cudaStream_t s) const
+    {
+        FCU_CHECK(cudaMemsetAsync(stats, 0, sizeof(RasterStats), s));
+        k_raster<kNearest><<<dim3(unsigned((per_dir + 255) / 256), dir_count), 256, 0, s>>>(
+            scene, planes, uint32_t(per_dir), pool, jobs, uint32_t(items), stats, d_frags);
+        FCU_LAUNCH("k_raster");
+        launch_early(k_raster_mid<kMidLanes, kNearest>,
+                     unsigned(std::min<uint64_t>((items + 31) / 32, 8u * sms)), 256, 0, s, scene, planes,
+                     uint32_t(per_dir), pool, jobs, &stats->mid, d_frags);
+        launch_early(k_raster_big<kNearest>, unsigned(std::min<uint64_t>(items * 16, 8u * sms)), 256, 0,
+                     s, scene, planes, uint32_t(per_dir), pool, jobs + items, &stats->big, d_frags);
+    }
+};
+
+void refuse_fragments(const RasterStats& host)
+{
+    if (host.fragments >= (1ull << 32))
+        throw Error(FACETCU_OVERFLOW_ERROR, "more than 2^32 fragments in one raster chunk");
+}
+
+}  // namespace
+
 void raster_fragments(const facetcu_vertex* d_vertices, const RasterFrame& frame,
                       const RasterView* views, uint32_t dir_count, RasterBuffers& rb,
                       uint32_t* d_frags, RasterStats& stats, cudaStream_t s)
 {
-    if (dir_count > kMaxViews)
-        throw Error(FACETCU_INVALID_ARGUMENT, "raster chunk exceeds 64 directions");
-    Scene scene{};
-    scene.frame = frame;
-    std::copy(views, views + dir_count, scene.views);
-    const uint64_t npix = uint64_t(dir_count) * frame.width * frame.height;
-    const uint64_t per_dir = uint64_t(frame.tiles) * frame.facets, items = dir_count * per_dir;
-    if (items >= (1ull << 32)) throw Error(FACETCU_OVERFLOW_ERROR, "raster work exceeds 2^32 triangles");
+    const RasterPass pass(d_vertices, frame, views, dir_count, rb, s);
     // whole blocks of the resolve
-    const uint64_t padded = (npix + kResolvePixels - 1) / kResolvePixels * kResolvePixels;
+    const uint64_t padded = (pass.npix + kResolvePixels - 1) / kResolvePixels * kResolvePixels;
     uint32_t* heads = static_cast<uint32_t*>(rb.heads.reserve(padded * 4));
-    uint32_t* jobs = static_cast<uint32_t*>(rb.jobs.reserve(items * 4));
-    float4* planes = static_cast<float4*>(rb.planes.reserve(size_t(frame.facets) * 48));
-    RasterStats* dstats = static_cast<RasterStats*>(rb.stats.reserve(sizeof(RasterStats)));
-    k_planes<<<(frame.facets + 255) / 256, 256, 0, s>>>(d_vertices, frame.facets, planes);
-    FCU_LAUNCH("k_planes");
     // A pool of one fragment for two pixels to begin with: the forest of
     // 200,000 facets has 0.29 a pixel over the 40 directions, 4,096 facets of
     // terrain 0.25.
     RasterStats host{};
-    const unsigned sms = sm_count();
-    uint64_t capacity = std::max<uint64_t>(rb.nodes.bytes / 16, npix / 2 + 1);
+    uint64_t capacity = std::max<uint64_t>(rb.nodes.bytes / 16, pass.npix / 2 + 1);
     for (uint32_t* counted = d_frags;; counted = nullptr) {
         capacity = std::min<uint64_t>(capacity, 0xffffffffull);
         const Pool pool{heads, static_cast<uint4*>(rb.nodes.reserve(capacity * 16)), capacity,
-                        &dstats->fragments};
+                        &pass.stats->fragments, nullptr};
         FCU_CHECK(cudaMemsetAsync(heads, 0, padded * 4, s));
-        FCU_CHECK(cudaMemsetAsync(dstats, 0, sizeof(RasterStats), s));
-        k_raster<<<dim3(unsigned((per_dir + 255) / 256), dir_count), 256, 0, s>>>(
-            scene, planes, uint32_t(per_dir), pool, jobs, uint32_t(items), dstats, counted);
-        FCU_LAUNCH("k_raster");
-        launch_early(k_raster_mid<kMidLanes>, unsigned(std::min<uint64_t>((items + 31) / 32, 8u * sms)),
-                     256, 0, s, scene, planes, uint32_t(per_dir), pool, jobs, &dstats->mid, counted);
-        launch_early(k_raster_big, unsigned(std::min<uint64_t>(items * 16, 8u * sms)), 256, 0, s, scene,
-                     planes, uint32_t(per_dir), pool, jobs + items, &dstats->big, counted);
-        FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
+        pass.run<false>(pool, counted, dir_count, s);
+        FCU_CHECK(cudaMemcpyAsync(&host, pass.stats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
         FCU_CHECK(cudaStreamSynchronize(s));
-        if (host.fragments >= (1ull << 32))
-            throw Error(FACETCU_OVERFLOW_ERROR, "more than 2^32 fragments in one raster chunk");
+        refuse_fragments(host);
         if (host.fragments <= capacity) break;
         capacity = host.fragments;
     }
@@ -1228,24 +1281,26 @@ void raster_resolve_graph(const RasterFrame& frame, uint32_t dir_count, uint32_t
     stats.capacity_error = host.capacity_error;
 }
 
-void raster_resolve_sunlit(const RasterFrame& frame, uint32_t chain_cap, RasterBuffers& rb,
-                           const uint32_t* d_total, uint32_t* d_visible, float* d_fraction,
-                           RasterStats& stats, cudaStream_t s)
+void raster_sunlit(const facetcu_vertex* d_vertices, const RasterFrame& frame, const RasterView& view,
+                   uint32_t chain_cap, RasterBuffers& rb, uint32_t* d_total, uint32_t* d_visible,
+                   float* d_fraction, RasterStats& stats, cudaStream_t s)
 {
-    const uint64_t npix = uint64_t(frame.width) * frame.height;
-    RasterStats* dstats = rb.stats.as<RasterStats>();
-    k_resolve_sunlit<<<unsigned((npix + kResolvePixels - 1) / kResolvePixels), 256, 0, s>>>(
-        frame.facets, frame.tiles, rb.heads.as<uint32_t>(), rb.nodes.as<uint4>(), chain_cap,
-        d_visible, dstats);
+    const RasterPass pass(d_vertices, frame, &view, 1, rb, s);
+    uint32_t* counts = static_cast<uint32_t*>(rb.heads.reserve(pass.npix * 4));
+    unsigned long long* nearest = static_cast<unsigned long long*>(rb.nodes.reserve(pass.npix * 8));
+    FCU_CHECK(cudaMemsetAsync(counts, 0, pass.npix * 4, s));
+    FCU_CHECK(cudaMemsetAsync(nearest, 0xff, pass.npix * 8, s));
+    pass.run<true>({counts, nullptr, 0, &pass.stats->fragments, nearest}, d_total, 1, s);
+    k_resolve_sunlit<<<unsigned(std::min<uint64_t>((pass.npix + 255) / 256, 16u * pass.sms)), 256, 0, s>>>(
+        frame.facets, frame.tiles, counts, reinterpret_cast<const uint64_t*>(nearest), pass.npix,
+        chain_cap, d_visible, pass.stats);
     FCU_LAUNCH("k_resolve_sunlit");
     k_fraction<<<(2 * frame.facets + 255) / 256, 256, 0, s>>>(2 * frame.facets, d_total, d_visible,
                                                               d_fraction);
     FCU_LAUNCH("k_fraction");
-    RasterStats host{};
-    FCU_CHECK(cudaMemcpyAsync(&host, dstats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
+    FCU_CHECK(cudaMemcpyAsync(&stats, pass.stats, sizeof(RasterStats), cudaMemcpyDeviceToHost, s));
     FCU_CHECK(cudaStreamSynchronize(s));
-    stats.overflow = host.overflow;
-    stats.max_chain = host.max_chain;
+    refuse_fragments(stats);
 }
 
 }  // namespace facetcu
